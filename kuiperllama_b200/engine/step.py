@@ -76,6 +76,24 @@ class _Staging:
         return self.dev
 
 
+def _places(want: Sequence[int], n: int, slot: int) -> np.ndarray:
+    """The wanted places as int32, all of them within a sequence's ``n`` tokens.  Checked as one array: a prompt whose every token's
+    logits are wanted names thousands of places (6,000: 0.55 ms one by one, 0.24 ms as a list, a few microseconds as a range)."""
+    if isinstance(want, range):
+        ends = (want[0], want[-1]) if len(want) else ()
+        bad = [w for w in ends if not 0 <= w < n]
+        if not bad:
+            return np.arange(want.start, want.stop, want.step, dtype=np.int32)
+        want = bad
+    a = np.asarray(want)
+    if a.ndim != 1:
+        a = np.asarray([w for w in want])
+    bad = np.flatnonzero(~((a >= 0) & (a < n)))
+    if bad.size:
+        raise StepError(f"slot {slot}: wanted place {a[bad[0]]} is outside its {n} tokens")
+    return a.astype(np.int32)
+
+
 def context_class(max_context: int) -> int:
     """The class of a step by its longest sequence: 0 up to 16 cache pages, then one class per
     doubling.  A captured decode step is replayed only for steps of its own class, so a part may
@@ -128,7 +146,7 @@ class Engine:
         if not inputs:
             raise StepError("an empty batch")
         vocab = self.model.spec.vocab_size
-        slots, starts, news, token_arrays = [], [], [], []
+        slots, starts, news, token_arrays, places = [], [], [], [], []
         seen = set()
         for s in inputs:
             if not self.cache.slots.is_held(s.slot):
@@ -139,9 +157,7 @@ class Engine:
             n = len(s.tokens)
             if n < 1:
                 raise StepError(f"the sequence in slot {s.slot} brings no token")
-            for w in s.want:
-                if not 0 <= w < n:
-                    raise StepError(f"slot {s.slot}: wanted place {w} is outside its {n} tokens")
+            places.append(_places(s.want, n, s.slot) if len(s.want) else None)
             toks = np.asarray(s.tokens, dtype=np.int64)
             lo, hi = int(toks.min()), int(toks.max())
             if lo < 0 or hi >= vocab:
@@ -169,7 +185,7 @@ class Engine:
         pad = np.zeros(pad_rows, dtype=i32)
         cu = np.zeros(n_seqs + 1, dtype=i32)
         np.cumsum(news, out=cu[1:])
-        want = [cu[j] + np.asarray(s.want, dtype=i32) for j, s in enumerate(inputs) if len(s.want)]
+        want = [cu[j] + p for j, p in enumerate(places) if p is not None]
         flat = (token_arrays + [pad]
                 + [np.arange(st, st + n, dtype=i32) for st, n in zip(starts, news)] + [pad]
                 + [np.full(n, sl, dtype=i32) for sl, n in zip(slots, news)] + [np.full(pad_rows, -1, dtype=i32)]
