@@ -16,7 +16,7 @@
 //       through shared memory; per token every thread decays and updates its rows, multiplies them by q and the
 //       lanes' sums are added by shuffles.  Tokens are walked in order from the slot's state, so a result does not
 //       depend on how a prompt was cut.
-//   outer_recurrence_slab_kernel<TI, R, C>   the form that runs where the sizes allow: R x C of S per thread (see there).
+//   outer_recurrence_slab_kernel<TI, R, L, MODE>   the form that runs where the sizes allow: R x 2 of S per thread (see there).
 //   outer_recurrence_single_kernel<TI, CL>   a step of single tokens, bound by reading and writing S once: neighbouring lanes hold
 //       neighbouring columns of a row, eight rows a thread on their way at a time.
 //   decay_softplus_kernel     dt = softplus(raw + bias), a = exp(-exp(A_log) dt) per (token, head), 32-bit.
@@ -29,7 +29,8 @@
 namespace kl {
 
 constexpr int OR_THREADS = 512;          // the most threads of a CTA; a launch takes 128, 256 or 512
-constexpr int OR_TILE = 32;           // tokens per shared-memory tile
+constexpr int OR_TILE = 32;           // tokens per shared-memory tile (the lane form)
+constexpr int SLAB_WARPS = 10;         // warps an SM below which the slab form cuts S into smaller pieces
 
 struct OuterArgs {
     const void* q; long long ld_q; int q_col;        // [rows, >= q_col + groups * N]
@@ -191,165 +192,249 @@ __device__ __forceinline__ void or_ld4(const bf16* p, float (&x)[4]) {
     x[2] = __uint_as_float(v.y << 16); x[3] = __uint_as_float(v.y & 0xffff0000u);
 }
 
-// The same recurrence with R rows x C columns of S in a thread's registers: per token a thread reads R values each of
-// k, q (and a) and C of v for 3 R C multiply-adds, and only the column sums cross lanes.  A warp holds LR = 32 / CGW lanes
-// along the rows (lane = column group + CGW * row group; row n = row group + LR * i), so neighbouring lanes hold
-// neighbouring columns of a row.  Rows from N to LR * R are zero in shared memory and change nothing.
-// NORM: with the normaliser, which the warp of the CTA's first columns of S carries (every column group of it alike).
-template <typename TI, int R, int C, bool NORM>
-__global__ void __launch_bounds__(256)
+typedef unsigned long long f32x2;                              // two float32 numbers, one instruction for both
+__device__ __forceinline__ f32x2 or_pair(float x, float y) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 or_unpair(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 or_fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 or_mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+template <int BYTES>
+__device__ __forceinline__ void or_copy(void* dst, const void* src, bool live) {         // not live: the piece becomes zero, nothing is read
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if constexpr (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(live ? 16 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(BYTES), "r"(live ? BYTES : 0) : "memory");
+}
+
+// The same recurrence with R rows x 2 columns of S in a thread's registers, for prompts.  What bounds it is the chain of tokens: the
+// arithmetic of a token is three multiply-adds an element, and a kernel that waits for shared memory, for shuffles and for the next
+// tile of tokens between tokens spends most of its time there.  So: rows of S are packed in pairs (one instruction for two rows,
+// and k, q and a of a pair come as they lie in shared memory), a thread reads four rows of k and q at once (L lanes read 16 L
+// neighbouring bytes), four tokens are worked between reductions, whose eight sums the L lanes share out among themselves (seven
+// shuffles for four tokens and two columns), and the next tile of tokens is copied while this one is worked.  One prompt of 2,048
+// tokens, us with R x C of S per thread and a reduction per token and column / now: 64 heads of 128 x 64 (state-space) 1,043 / 405, 16
+// heads of 64 x 128 with a decay per row (gated linear attention) 725 / 393; three prompts of 446, 1,333 and 2,222 tokens 1,668 / 585.
+// Rows: lane rg holds rows 4 rg + 4 L i + (0..3), i < R / 4; rows from N to R L are zero and change nothing.
+// MODE 0: one decay per head; 1: one per row of S; 2: one per head and the normaliser, which the first warp of the first columns carries.
+constexpr int OSL_TOKENS = 4;             // tokens between reductions
+constexpr int OSL_THREADS = 128;
+// four neighbouring numbers as two pairs
+__device__ __forceinline__ ulonglong2 or_quad(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+__device__ __forceinline__ ulonglong2 or_quad(const bf16* p) {
+    float x[4];
+    or_ld4(p, x);
+    return make_ulonglong2(or_pair(x[0], x[1]), or_pair(x[2], x[3]));
+}
+__device__ __forceinline__ float2 or_two(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 or_two(const bf16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
+
+template <typename TI, int R, int L, int MODE>
+__global__ void __launch_bounds__(OSL_THREADS, 2)
 outer_recurrence_slab_kernel(const OuterArgs A) {
     pdl_launch_dependents();
     pdl_wait();
-    extern __shared__ __align__(16) float sm[];
+    constexpr int Np = R * L, H2 = R / 2, ES = sizeof(TI);
+    constexpr int A_BYTES = MODE == 1 ? Np * 4 : 0;
+    extern __shared__ __align__(16) unsigned char osl_smem[];
     const int s = blockIdx.z, h = blockIdx.y;
     const int row0 = A.cu_tokens[s], n_new = A.cu_tokens[s + 1] - row0;
     if (n_new <= 0) return;
-    const int N = A.N, P = A.P, LR = A.L, Np = LR * R;
-    const int threads = blockDim.x;
-    const int cgw = 32 / LR;                                   // column groups per warp
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int rg = lane / cgw, cg = warp * cgw + lane % cgw;   // the thread's row group, and its column group in the CTA
-    const int cols_per_cta = (threads / LR) * C;
-    const int col0 = blockIdx.x * cols_per_cta + cg * C;
-    const bool live = col0 < P;                                // P is a multiple of C
+    const int N = A.N, P = A.P, T = A.tile;
+    const int threads = blockDim.x, lane = threadIdx.x & 31;
+    const int rg = threadIdx.x % L, cg = threadIdx.x / L;      // the thread's lane along the rows, and its column pair in the CTA
+    const int cols = threads / L * 2;                          // a multiple of four
+    const int col0 = blockIdx.x * cols + cg * 2;
+    const bool live = col0 < P;                                // P is even
     const int g = h / (A.heads / A.groups);
-    const int a_len = A.a_per_row ? Np : 4;                    // one decay per head: a piece of four, so that rows stay aligned
-    const int per_tok = 2 * Np + a_len + cols_per_cta;         // k (times c), q (times q_scale), a, v
+    const int tok = (2 * Np * ES + A_BYTES + cols * ES + 15) / 16 * 16;       // bytes of a token: k, q, a, v
+    const int scal = T * tok;                                  // behind them the tile's decays and factors c
+    const int stage = (scal + 2 * T * 4 + 15) / 16 * 16;
     float* S_slot = A.state + (size_t)A.seq_slots[s] * A.ld_state + (size_t)h * N * P;
-    float S[R][C];
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const int n = rg + LR * i;
-        if (C == 4 && A.vec_state && live && n < N) {                         // P and col0 are multiples of 4
-            const float4 v4 = *reinterpret_cast<const float4*>(S_slot + (size_t)n * P + col0);
-            S[i][0] = v4.x; S[i][1] = v4.y; S[i][2] = v4.z; S[i][C - 1] = v4.w;
-        } else {
-#pragma unroll
-            for (int j = 0; j < C; ++j) S[i][j] = (live && n < N) ? S_slot[(size_t)n * P + col0 + j] : 0.f;
-        }
-    }
-    const bool norm = NORM && blockIdx.x == 0 && warp == 0;
-    float* n_slot = NORM ? A.norm_state + (size_t)A.seq_slots[s] * A.ld_state + (size_t)h * N : nullptr;
-    float nS[NORM ? R : 1];
-    if constexpr (NORM) {
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-            const int n = rg + LR * i;
-            nS[i] = (norm && n < N) ? n_slot[n] : 0.f;
-        }
-    }
-    const TI* qp = (const TI*)A.q; const TI* kp = (const TI*)A.k; const TI* vp = (const TI*)A.v;
-    const float skip = A.skip != nullptr ? A.skip[h] : 0.f;
-    // one tile's tokens: decay, update, multiply by q, add the lanes' column sums
-    auto compute = [&](int t0, int nt) {
-        for (int tt = 0; tt < nt; ++tt) {
-            const float* kk = sm + tt * per_tok;
-            const float* qq = kk + Np;
-            const float* aa = qq + Np;
-            float v[C], acc[C];
-#pragma unroll
-            for (int j = 0; j < C; ++j) { v[j] = aa[a_len + cg * C + j]; acc[j] = 0.f; }
-            const float a0 = aa[0];
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-                const int n = rg + LR * i;
-                const float kn = kk[n], qn = qq[n], an = A.a_per_row ? aa[n] : a0;
-#pragma unroll
-                for (int j = 0; j < C; ++j) {
-                    S[i][j] = fmaf(an, S[i][j], kn * v[j]);
-                    acc[j] = fmaf(S[i][j], qn, acc[j]);
+
+    // a thread copies the same four columns of every token of a tile
+    auto copy_tile = [&](int t0, unsigned char* dst) {
+        const int nt = min(T, n_new - t0);
+        const size_t row = (size_t)(row0 + t0);
+        const int kq = Np / 4, pieces = 2 * kq + (MODE == 1 ? kq : 0) + cols / 4;
+        for (int j = threadIdx.x; j < pieces; j += threads) {
+            const int which = j < kq ? 0 : j < 2 * kq ? 1 : (MODE == 1 && j < 3 * kq) ? 2 : 3;
+            const int e = (j - (which == 3 && MODE != 1 ? 2 : which) * kq) * 4;
+            const int c = which == 3 ? blockIdx.x * cols + e : e;                  // the element in its head's row
+            const int n = min(4, (which == 3 ? P : N) - c);                        // elements that exist
+            unsigned char* to = dst + (which == 0 ? e * ES : which == 1 ? (Np + e) * ES : which == 2 ? 2 * Np * ES + e * 4 : 2 * Np * ES + A_BYTES + e * ES);
+            if (MODE == 1 && which == 2) {
+                const float* src = A.a + row * A.ld_a + (size_t)h * N + c;
+                for (int tt = 0; tt < T; ++tt, to += tok, src += A.ld_a) {
+                    if (tt >= nt) *reinterpret_cast<float4*>(to) = make_float4(1.f, 1.f, 1.f, 1.f);      // a token past the end leaves S as it is
+                    else if (A.vec_in) or_copy<16>(to, n > 0 ? src : A.a, n > 0);
+                    else
+                        for (int u = 0; u < 4; ++u) reinterpret_cast<float*>(to)[u] = u < n ? src[u] : 0.f;
                 }
+                continue;
             }
-            for (int o = cgw; o < 32; o <<= 1) {
-#pragma unroll
-                for (int j = 0; j < C; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-            }
-            if (rg == 0 && live) {
-                float* y = A.y + (size_t)(row0 + t0 + tt) * A.ld_y + (size_t)h * P + col0;
-#pragma unroll
-                for (int j = 0; j < C; ++j) y[j] = fmaf(skip, v[j], acc[j]);
-            }
-            if constexpr (NORM) {
-                if (norm) {
-                    float dot = 0.f;
-#pragma unroll
-                    for (int i = 0; i < R; ++i) {
-                        const int n = rg + LR * i;
-                        nS[i] = fmaf(A.a_per_row ? aa[n] : a0, nS[i], kk[n]);
-                        dot = fmaf(nS[i], qq[n], dot);
-                    }
-                    for (int o = cgw; o < 32; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-                    if (lane == 0) A.den[(size_t)(row0 + t0 + tt) * A.heads + h] = or_den(A, (size_t)(row0 + t0 + tt), h, dot);
+            const TI* base = (const TI*)(which == 0 ? A.k : which == 1 ? A.q : A.v);
+            const long long ld = which == 0 ? A.ld_k : which == 1 ? A.ld_q : A.ld_v;
+            const TI* src = base + row * ld + (which == 0 ? A.k_col + (size_t)g * N : which == 1 ? A.q_col + (size_t)g * N : A.v_col + (size_t)h * P) + c;
+            if (A.vec_in) {                                                        // N and P are multiples of four
+                for (int tt = 0; tt < T; ++tt, to += tok, src += ld) {
+                    const bool in = n > 0 && tt < nt;
+                    or_copy<4 * ES>(to, in ? src : base, in);
                 }
+            } else {
+                for (int tt = 0; tt < T; ++tt, to += tok, src += ld)
+                    for (int u = 0; u < 4; ++u) reinterpret_cast<TI*>(to)[u] = tt < nt && u < n ? src[u] : from_f32<TI>(0.f);
             }
         }
+        for (int t = threadIdx.x; t < 2 * T; t += threads) {
+            const int tt = t < T ? t : t - T;
+            float* to = reinterpret_cast<float*>(dst + scal) + t;
+            const float* src = t < T ? (MODE != 1 ? A.a + (row + min(tt, nt - 1)) * A.ld_a + h : nullptr)
+                                     : A.c != nullptr ? A.c + (row + min(tt, nt - 1)) * A.ld_c + h : nullptr;
+            if (src != nullptr && tt < nt) or_copy<4>(to, src, true);
+            else *to = 1.f;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    for (int t0 = 0; t0 < n_new; t0 += OR_TILE) {
-        const int nt = min(OR_TILE, n_new - t0);
-        __syncthreads();
-        if (A.vec_in) {                                        // four elements a turn; N, Np and per_tok are multiples of 4
-            const int quads = Np / 4;
-#pragma unroll 4
-            for (int idx = threadIdx.x; idx < nt * quads; idx += threads) {
-                const int tt = idx / quads, j = (idx - tt * quads) * 4;
-                const size_t row = (size_t)(row0 + t0 + tt);
-                float kv[4] = {0.f, 0.f, 0.f, 0.f}, qv[4] = {0.f, 0.f, 0.f, 0.f}, av[4] = {0.f, 0.f, 0.f, 0.f};
-                if (j < N) {
-                    or_ld4(kp + row * A.ld_k + A.k_col + (size_t)g * N + j, kv);
-                    or_ld4(qp + row * A.ld_q + A.q_col + (size_t)g * N + j, qv);
-                    const float cc = A.c != nullptr ? A.c[row * A.ld_c + h] : 1.0f;
+    copy_tile(0, osl_smem);
+
+    f32x2 S[H2][2];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) { kv[e] *= cc; qv[e] *= A.q_scale; }
-                    if (A.a_per_row) or_ld4(A.a + row * A.ld_a + (size_t)h * N + j, av);
+    for (int i = 0; i < H2; ++i) {
+        const int n = 4 * rg + 4 * L * (i / 2) + 2 * (i % 2);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            S[i][j] = or_pair(live && n < N ? S_slot[(size_t)n * P + col0 + j] : 0.f, live && n + 1 < N ? S_slot[(size_t)(n + 1) * P + col0 + j] : 0.f);
+    }
+    const bool norm = MODE == 2 && blockIdx.x == 0 && threadIdx.x < 32;
+    float* n_slot = MODE == 2 ? A.norm_state + (size_t)A.seq_slots[s] * A.ld_state + (size_t)h * N : nullptr;
+    f32x2 nS[MODE == 2 ? H2 : 1];
+    if constexpr (MODE == 2) {
+#pragma unroll
+        for (int i = 0; i < H2; ++i) {
+            const int n = 4 * rg + 4 * L * (i / 2) + 2 * (i % 2);
+            nS[i] = or_pair(norm && n < N ? n_slot[n] : 0.f, norm && n + 1 < N ? n_slot[n + 1] : 0.f);
+        }
+    }
+    const float skip = A.skip != nullptr ? A.skip[h] : 0.f;
+
+    int buf = 0;
+    for (int t0 = 0; t0 < n_new; t0 += T, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                       // this tile is here, and everyone is done with the one before
+        const unsigned char* tile = osl_smem + buf * stage;
+        if (t0 + T < n_new) copy_tile(t0 + T, osl_smem + (buf ^ 1) * stage);
+        const int nt = min(T, n_new - t0);
+        const float* decay = reinterpret_cast<const float*>(tile + scal);
+        const float* factor = decay + T;
+        for (int tb = 0; tb < nt; tb += OSL_TOKENS) {
+            float sums[OSL_TOKENS * 2];
+            float dots[MODE == 2 ? OSL_TOKENS : 1];
+#pragma unroll
+            for (int u = 0; u < OSL_TOKENS; ++u) {             // T is a multiple of OSL_TOKENS; tokens past the end are zeros
+                const unsigned char* at = tile + (tb + u) * tok;
+                const TI* kk = reinterpret_cast<const TI*>(at) + 4 * rg;
+                const float2 v = or_two(reinterpret_cast<const TI*>(at + 2 * Np * ES + A_BYTES) + 2 * cg);
+                const float c = factor[tb + u], a0 = MODE == 1 ? 0.f : decay[tb + u];
+                const f32x2 v0 = or_pair(c * v.x, c * v.x), v1 = or_pair(c * v.y, c * v.y), ad = or_pair(a0, a0), cd = or_pair(c, c);
+                f32x2 y0[2] = {0, 0}, y1[2] = {0, 0}, dot = 0;
+#pragma unroll
+                for (int i = 0; i < R / 4; ++i) {
+                    const ulonglong2 k4 = or_quad(kk + 4 * L * i), q4 = or_quad(kk + Np + 4 * L * i);
+                    ulonglong2 a4 = make_ulonglong2(ad, ad);
+                    if constexpr (MODE == 1) a4 = or_quad(reinterpret_cast<const float*>(at + 2 * Np * ES) + 4 * rg + 4 * L * i);
+                    S[2 * i][0] = or_fma2(a4.x, S[2 * i][0], or_mul2(k4.x, v0));
+                    S[2 * i][1] = or_fma2(a4.x, S[2 * i][1], or_mul2(k4.x, v1));
+                    S[2 * i + 1][0] = or_fma2(a4.y, S[2 * i + 1][0], or_mul2(k4.y, v0));
+                    S[2 * i + 1][1] = or_fma2(a4.y, S[2 * i + 1][1], or_mul2(k4.y, v1));
+                    y0[0] = or_fma2(S[2 * i][0], q4.x, y0[0]);
+                    y1[0] = or_fma2(S[2 * i][1], q4.x, y1[0]);
+                    y0[1] = or_fma2(S[2 * i + 1][0], q4.y, y0[1]);
+                    y1[1] = or_fma2(S[2 * i + 1][1], q4.y, y1[1]);
+                    if constexpr (MODE == 2) {
+                        if (norm) {
+                            nS[2 * i] = or_fma2(ad, nS[2 * i], or_mul2(k4.x, cd));
+                            nS[2 * i + 1] = or_fma2(ad, nS[2 * i + 1], or_mul2(k4.y, cd));
+                            dot = or_fma2(nS[2 * i], q4.x, dot);
+                            dot = or_fma2(nS[2 * i + 1], q4.y, dot);
+                        }
+                    }
                 }
-                float* dst = sm + tt * per_tok + j;
-                *reinterpret_cast<float4*>(dst) = make_float4(kv[0], kv[1], kv[2], kv[3]);
-                *reinterpret_cast<float4*>(dst + Np) = make_float4(qv[0], qv[1], qv[2], qv[3]);
-                if (A.a_per_row) *reinterpret_cast<float4*>(dst + 2 * Np) = make_float4(av[0], av[1], av[2], av[3]);
+                const float2 s0 = or_unpair(y0[0]), s1 = or_unpair(y1[0]), s2 = or_unpair(y0[1]), s3 = or_unpair(y1[1]);
+                sums[2 * u] = (s0.x + s0.y) + (s2.x + s2.y);
+                sums[2 * u + 1] = (s1.x + s1.y) + (s3.x + s3.y);
+                if constexpr (MODE == 2) { const float2 d = or_unpair(dot); dots[u] = d.x + d.y; }
             }
-        } else
-#pragma unroll 8
-        for (int idx = threadIdx.x; idx < nt * Np; idx += threads) {
-            const int tt = idx / Np, j = idx - tt * Np;
-            const size_t row = (size_t)(row0 + t0 + tt);
-            float kv = 0.f, qv = 0.f;
-            if (j < N) {
-                kv = to_f32(kp[row * A.ld_k + A.k_col + (size_t)g * N + j]);
-                if (A.c != nullptr) kv *= A.c[row * A.ld_c + h];
-                qv = to_f32(qp[row * A.ld_q + A.q_col + (size_t)g * N + j]) * A.q_scale;
+            // the lanes add each other's sums and keep a share: bit 0 of the lane the column, bits 1 and 2 the token (four lanes: two tokens each)
+            int left = OSL_TOKENS * 2;
+#pragma unroll
+            for (int o = 1; o < L; o <<= 1) {
+                if (left > 1) {
+                    left >>= 1;
+#pragma unroll
+                    for (int j = 0; j < left; ++j) {
+                        const float give = (lane & o) ? sums[2 * j] : sums[2 * j + 1], keep = (lane & o) ? sums[2 * j + 1] : sums[2 * j];
+                        sums[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                    }
+                } else {
+                    sums[0] += __shfl_xor_sync(0xffffffffu, sums[0], o);
+                }
             }
-            sm[tt * per_tok + j] = kv;
-            sm[tt * per_tok + Np + j] = qv;
-            if (A.a_per_row) sm[tt * per_tok + 2 * Np + j] = j < N ? A.a[row * A.ld_a + (size_t)h * N + j] : 0.f;
+            constexpr int KEPT = L >= 8 ? 1 : 8 / L;
+            if (live && rg < 8) {
+#pragma unroll
+                for (int j = 0; j < KEPT; ++j) {
+                    const int idx = rg % 8 + j * (8 / KEPT), u = tb + idx / 2, cc = idx % 2;
+                    if (u < nt) {
+                        const float v = to_f32(reinterpret_cast<const TI*>(tile + u * tok + 2 * Np * ES + A_BYTES)[2 * cg + cc]);
+                        A.y[(size_t)(row0 + t0 + u) * A.ld_y + (size_t)h * P + col0 + cc] = fmaf(skip, v, A.q_scale * sums[j]);
+                    }
+                }
+            }
+            if constexpr (MODE == 2) {
+                if (norm) {
+#pragma unroll
+                    for (int u = 0; u < OSL_TOKENS; ++u) {
+                        float d = dots[u];
+#pragma unroll
+                        for (int o = 1; o < L; o <<= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+                        if (threadIdx.x == 0 && tb + u < nt) {
+                            const size_t row = (size_t)(row0 + t0 + tb + u);
+                            A.den[row * A.heads + h] = or_den(A, row, h, A.q_scale * d);
+                        }
+                    }
+                }
+            }
         }
-        for (int idx = threadIdx.x; idx < nt * cols_per_cta; idx += threads) {
-            const int tt = idx / cols_per_cta, j = idx - tt * cols_per_cta;
-            const size_t row = (size_t)(row0 + t0 + tt);
-            const int cc = blockIdx.x * cols_per_cta + j;
-            sm[tt * per_tok + 2 * Np + a_len + j] = cc < P ? to_f32(vp[row * A.ld_v + A.v_col + (size_t)h * P + cc]) : 0.f;
-        }
-        if (!A.a_per_row)
-            for (int tt = threadIdx.x; tt < nt; tt += threads) sm[tt * per_tok + 2 * Np] = A.a[(size_t)(row0 + t0 + tt) * A.ld_a + h];
-        __syncthreads();
-        compute(t0, nt);
     }
-    if constexpr (NORM) {
 #pragma unroll
-        for (int i = 0; i < R; ++i) {
-            const int n = rg + LR * i;
-            if (norm && lane % cgw == 0 && n < N) n_slot[n] = nS[i];
+    for (int i = 0; i < H2; ++i) {
+        const int n = 4 * rg + 4 * L * (i / 2) + 2 * (i % 2);
+        if constexpr (MODE == 2) {
+            const float2 z = or_unpair(nS[i]);
+            if (norm && cg == 0 && n < N) n_slot[n] = z.x;
+            if (norm && cg == 0 && n + 1 < N) n_slot[n + 1] = z.y;
         }
-    }
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const int n = rg + LR * i;
-        if (!(live && n < N)) continue;
-        if (C == 4 && A.vec_state) {
-            *reinterpret_cast<float4*>(S_slot + (size_t)n * P + col0) = make_float4(S[i][0], S[i][1], S[i][2], S[i][C - 1]);
-        } else {
-#pragma unroll
-            for (int j = 0; j < C; ++j) S_slot[(size_t)n * P + col0 + j] = S[i][j];
+        for (int j = 0; j < 2; ++j) {
+            const float2 x = or_unpair(S[i][j]);
+            if (live && n < N) S_slot[(size_t)n * P + col0 + j] = x.x;
+            if (live && n + 1 < N) S_slot[(size_t)(n + 1) * P + col0 + j] = x.y;
         }
     }
 }
@@ -509,58 +594,58 @@ KL_API int kl_outer_recurrence(const void* q, long long ld_q, int q_col, const v
         KL_LAUNCH_CHECK();
         return KL_OK;
     }
-    {   // slabs of R x C in registers: the largest slab that still gives every SM eight warps, else the smallest that fits
-        const int slabs[3][2] = {{8, 4}, {4, 4}, {2, 2}};
-        int pick = -1, pick_lr = 0;
-        for (int z = 0; z < 3; ++z) {
-            const int R = slabs[z][0], C = slabs[z][1];
-            if (P % C) continue;
-            int LR = 1;
-            while (LR * R < N) LR <<= 1;
-            if (LR > 32) continue;
-            pick = z; pick_lr = LR;
-            if ((long long)n_seqs * heads * LR * (P / C) / 32 >= 8LL * sms) break;
+    // slabs of R x 2 in registers: the most rows a thread that still give the device SLAB_WARPS warps an SM, else the fewest.  us at R = 16 / 8
+    // / 4: one prompt of 2,048 tokens, 64 heads of 128 x 64 (3.5 / 7 / 14 warps an SM) 478 / 427 / 405, 16 heads of 64 x 128 (1.7 / 3.5 / 6.9)
+    // 620 / 528 / 398, eight prompts of 256 of the latter (14 / 28 / 55) 93 / 131 / 133.
+    const int mode = norm_state != nullptr ? 2 : a_per_row ? 1 : 0;
+    if (P % 2 == 0 && N <= 512 && !(mode == 2 && a_per_row)) {
+        int R = 0, L = 0;
+        for (int r = 16; r >= 4; r >>= 1) {
+            int l = 4;
+            while (l * r < N) l <<= 1;
+            if (l > 32) continue;
+            R = r; L = l;
+            if (1LL * n_seqs * heads * l * (P / 2) / 32 >= (long long)SLAB_WARPS * sms) break;
         }
-        if (pick >= 0) {
-            const int R = slabs[pick][0], C = slabs[pick][1], LR = pick_lr;
-            int threads = LR * (P / C);
-            threads = threads > 256 ? 256 : ((threads + 31) & ~31);
-            auto ctas = [&](int th) { return (long long)((P / C + th / LR - 1) / (th / LR)) * heads * n_seqs; };
-            // short runs (decode): smaller CTAs until every SM has two.  Long runs: a CTA's threads share the loading of
-            // each tile of tokens, which is the same for every column of a head, so the CTA stays wide
-            while (max_new <= 16 && threads > 32 && (threads / 2) % 32 == 0 && ctas(threads) < 2LL * sms) threads >>= 1;
-            A.L = LR;
-            const int cols = (threads / LR) * C;
-            dim3 grid((P + cols - 1) / cols, heads, n_seqs);
-            const int per_tok = 2 * LR * R + (a_per_row ? LR * R : 4) + cols;
-            const size_t smem = (size_t)OR_TILE * per_tok * sizeof(float);
-            const int es = in_dtype == KL_F32 ? 4 : 2;
-            auto quad = [&](const void* p, long long ld, int col) { return (uintptr_t)p % (4 * es) == 0 && ld % 4 == 0 && col % 4 == 0; };
-            A.vec_in = (N % 4 == 0 && (LR * R) % 4 == 0 && per_tok % 4 == 0 && quad(q, ld_q, q_col) && quad(k, ld_k, k_col) &&
-                        (!a_per_row || ((uintptr_t)a % 16 == 0 && ld_a % 4 == 0))) ? 1 : 0;
-            if (smem <= 200 * 1024) {
-#define KL_SLAB(TI, R_, C_, NM)                                                                                      \
+        const int pairs = P / 2, es = in_dtype == KL_F32 ? 4 : 2;
+        // CTAs of 128 threads: a CTA's threads share the copies of a tile, two CTAs on an SM fill each other's waits
+        const int fewest = 2 * L > 32 ? 2 * L : 32;            // four columns of S at least: pieces of four stay aligned
+        int threads = (L * pairs + 31) / 32 * 32;
+        threads = threads < fewest ? fewest : threads > OSL_THREADS ? OSL_THREADS : threads;
+        while (threads > fewest && threads % 64 == 0 && (long long)((pairs * L + threads - 1) / threads) * heads * n_seqs < sms) threads >>= 1;
+        const int cols = threads / L * 2, Np = R * L, tok = (2 * Np * es + (mode == 1 ? Np * 4 : 0) + cols * es + 15) / 16 * 16;
+        auto quad = [&](const void* p, long long ld, int col) { return (uintptr_t)p % (4 * es) == 0 && ld % 4 == 0 && col % 4 == 0; };
+        A.vec_in = (N % 4 == 0 && P % 4 == 0 && quad(q, ld_q, q_col) && quad(k, ld_k, k_col) && quad(v, ld_v, v_col) &&
+                    (!a_per_row || ((uintptr_t)a % 16 == 0 && ld_a % 4 == 0))) ? 1 : 0;
+        A.tile = max_new <= 4 ? 4 : max_new <= 8 || Np > 256 ? 8 : 16;
+        A.L = L;
+        const size_t smem = (size_t)2 * ((A.tile * tok + 2 * A.tile * 4 + 15) / 16 * 16);
+        const dim3 grid((P + cols - 1) / cols, heads, n_seqs);
+#define KL_SLAB(TI, R_, L_, M_)                                                                                      \
     do {                                                                                                            \
         if (smem > 48 * 1024)                                                                                       \
-            KL_CUDA(cudaFuncSetAttribute(outer_recurrence_slab_kernel<TI, R_, C_, NM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        launch_kernel(outer_recurrence_slab_kernel<TI, R_, C_, NM>, grid, threads, smem, stream, A);                \
+            KL_CUDA(cudaFuncSetAttribute(outer_recurrence_slab_kernel<TI, R_, L_, M_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        launch_kernel(outer_recurrence_slab_kernel<TI, R_, L_, M_>, grid, threads, smem, stream, A);                \
     } while (0)
-#define KL_SLAB_N(TI, R_, C_)                                                                                       \
+#define KL_SLAB_M(TI, R_, L_)                                                                                        \
     do {                                                                                                            \
-        if (norm_state != nullptr) KL_SLAB(TI, R_, C_, true); else KL_SLAB(TI, R_, C_, false);                      \
+        if (mode == 0) KL_SLAB(TI, R_, L_, 0); else if (mode == 1) KL_SLAB(TI, R_, L_, 1); else KL_SLAB(TI, R_, L_, 2); \
     } while (0)
-#define KL_SLAB_BY(TI)                                                                                              \
+#define KL_SLAB_L(TI, R_)                                                                                            \
     do {                                                                                                            \
-        if (R == 8) KL_SLAB_N(TI, 8, 4); else if (R == 4) KL_SLAB_N(TI, 4, 4); else KL_SLAB_N(TI, 2, 2);            \
+        if (L == 4) KL_SLAB_M(TI, R_, 4); else if (L == 8) KL_SLAB_M(TI, R_, 8); else if (L == 16) KL_SLAB_M(TI, R_, 16); else KL_SLAB_M(TI, R_, 32); \
     } while (0)
-                if (in_dtype == KL_F32) KL_SLAB_BY(float); else KL_SLAB_BY(bf16);
-#undef KL_SLAB_BY
-#undef KL_SLAB_N
+#define KL_SLAB_R(TI)                                                                                                \
+    do {                                                                                                            \
+        if (R == 16) KL_SLAB_L(TI, 16); else if (R == 8) KL_SLAB_L(TI, 8); else KL_SLAB_L(TI, 4);                   \
+    } while (0)
+        if (in_dtype == KL_F32) KL_SLAB_R(float); else KL_SLAB_R(bf16);
+#undef KL_SLAB_R
+#undef KL_SLAB_L
+#undef KL_SLAB_M
 #undef KL_SLAB
-                KL_LAUNCH_CHECK();
-                return KL_OK;
-            }
-        }
+        KL_LAUNCH_CHECK();
+        return KL_OK;
     }
     // any other size: a column of S over L lanes, rows of S in registers per thread at most 16 where 32 lanes allow it
     int L = 1;
