@@ -494,6 +494,61 @@ head_rmsnorm_gate_vec_kernel(const float* __restrict__ x, const T* __restrict__ 
     }
 }
 
+// The same for longer heads (a state-space layer's inner channels as one): a CTA of THREADS threads holds a head in registers, four
+// elements an access, so that x and the gate are read once.  Bound by bytes: 4,001 rows of 4,096 (131 MB) 34 us, 113 in two passes of
+// single elements.
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+head_rmsnorm_gate_row_kernel(const float* __restrict__ x, const T* __restrict__ gate, long long gate_ld, const float* __restrict__ w,
+                             T* __restrict__ out, long long out_ld, float out_scale, int heads, int dim, float eps, int gate_first,
+                             int wide_weight, const float* __restrict__ divisor, int sigmoid) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int VPT = 4;
+    __shared__ float scratch[33];
+    const int n4 = dim >> 2, t = blockIdx.x / heads, h = blockIdx.x - t * heads;
+    const float* xr = x + ((size_t)t * heads + h) * dim;
+    const T* g = gate ? gate + (size_t)t * gate_ld + (size_t)h * dim : nullptr;
+    const float* wr = w != nullptr ? w + (wide_weight ? (size_t)h * dim : 0) : nullptr;
+    T* o = out + (size_t)t * out_ld + (size_t)h * dim;
+    const float pre = divisor != nullptr ? 1.0f / divisor[(size_t)t * heads + h] : 1.0f;
+    float4 v[VPT], f[VPT];
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+        const int i4 = threadIdx.x + THREADS * j;
+        v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        f[j] = make_float4(1.f, 1.f, 1.f, 1.f);
+        if (i4 >= n4) continue;
+        v[j] = *reinterpret_cast<const float4*>(xr + 4 * i4);
+        if (g != nullptr) f[j] = Vec4<T>::load(g + 4 * i4);
+    }
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+        if (g != nullptr) {
+            f[j].x = gate_factor(f[j].x, sigmoid); f[j].y = gate_factor(f[j].y, sigmoid);
+            f[j].z = gate_factor(f[j].z, sigmoid); f[j].w = gate_factor(f[j].w, sigmoid);
+        }
+        v[j].x *= pre; v[j].y *= pre; v[j].z *= pre; v[j].w *= pre;
+        if (gate_first) { v[j].x *= f[j].x; v[j].y *= f[j].y; v[j].z *= f[j].z; v[j].w *= f[j].w; }
+        ss += (v[j].x * v[j].x + v[j].y * v[j].y) + (v[j].z * v[j].z + v[j].w * v[j].w);
+    }
+    ss = block_sum(ss, scratch);
+    const float inv = 1.0f / sqrtf(ss / (float)dim + eps);
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+        const int i4 = threadIdx.x + THREADS * j;
+        if (i4 >= n4) continue;
+        float4 y = make_float4(v[j].x * inv, v[j].y * inv, v[j].z * inv, v[j].w * inv);
+        if (wr != nullptr) {
+            const float4 ww = *reinterpret_cast<const float4*>(wr + 4 * i4);
+            y.x *= ww.x; y.y *= ww.y; y.z *= ww.z; y.w *= ww.w;
+        }
+        if (!gate_first) { y.x *= f[j].x; y.y *= f[j].y; y.z *= f[j].z; y.w *= f[j].w; }
+        Vec4<T>::store(o + 4 * i4, make_float4(y.x * out_scale, y.y * out_scale, y.z * out_scale, y.w * out_scale));
+    }
+}
+
 }  // namespace kl
 
 using namespace kl;
@@ -564,8 +619,19 @@ KL_API int kl_head_rmsnorm_gate(const float* x, const void* gate, long long gate
     const long long items = (long long)tokens * heads;
     {   // heads that fit a warp's registers, on boundaries of four elements
         const uintptr_t m = dtype == KL_BF16 ? 7 : 15;
-        if ((dtype == KL_F32 || dtype == KL_BF16) && dim % 4 == 0 && dim <= 1024 && gate_ld % 4 == 0 && out_ld % 4 == 0 &&
-            (((uintptr_t)gate | (uintptr_t)out) & m) == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
+        const bool fours = (dtype == KL_F32 || dtype == KL_BF16) && dim % 4 == 0 && gate_ld % 4 == 0 && out_ld % 4 == 0 &&
+                           (((uintptr_t)gate | (uintptr_t)out) & m) == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
+        if (fours && dim > 1024 && dim <= 8192) {              // a CTA per head, 16 elements a thread
+#define KL_HR(T, TH)                                                                                                                     \
+    launch_kernel(head_rmsnorm_gate_row_kernel<T, TH>, (int)items, TH, 0, stream, x, (const T*)gate, gate_ld, w, (T*)out, out_ld, out_scale, \
+                  heads, dim, eps, gate_first, wide_weight, divisor, sigmoid)
+            if (dtype == KL_F32) { if (dim <= 4096) KL_HR(float, 256); else KL_HR(float, 512); }
+            else { if (dim <= 4096) KL_HR(bf16, 256); else KL_HR(bf16, 512); }
+#undef KL_HR
+            KL_LAUNCH_CHECK();
+            return KL_OK;
+        }
+        if (fours && dim <= 1024) {
             const int blocks = (int)((items + 3) / 4);
 #define KL_HV(T, VPL)                                                                                                                    \
     launch_kernel(head_rmsnorm_gate_vec_kernel<T, VPL>, blocks, 128, 0, stream, x, (const T*)gate, gate_ld, w, (T*)out, out_ld, out_scale, \

@@ -241,6 +241,7 @@ class Engine:
         rows = -(-n_real // PAGE) * PAGE
         ctx, want_rows, n_want = self._pack(inputs, rows - n_real)
         ctx.max_new = rows                                # every length a replay may bring
+        ctx.captured = True
         key = (ctx.n_seqs, rows, n_want)
         g = self._step_graphs.get(key)
         if g is not None and g.staging_ptr != self._staging.dev.data_ptr():

@@ -93,7 +93,7 @@ class AttentionMixer(Mixer):
                           cache.k if cache.writable else None, cache.v if cache.writable else None,
                           self.H, self.KV, self.hd, values_are_keys=self.values_are_keys)
         # rows that belong to no sequence (a small step's padding) are not written by the kernels: keep them defined
-        make = torch.empty if n == step.n_seqs else torch.zeros
+        make = torch.zeros if step.padded else torch.empty
         attn = make((n, self.H * self.hd), dtype=self.runtime.dtype, device=x.device)
         ops.attention(proj, proj.stride(0), attn, cache.k, cache.v, cache.block_table, step, self.H, self.KV, self.hd,
                       self.scale, int(self.window or 0))

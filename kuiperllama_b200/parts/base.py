@@ -66,14 +66,16 @@ class StepContext:
     # the residual stream into the products at all.
     next_norm: Optional["Norm"] = None
     allow_stream_fusion: bool = False
+    # Whether the step is captured and replayed for steps that bring fewer tokens: rows that are real now are padding then.
+    captured: bool = False
     # What a layer leaves for later layers of the same step, by a name the parts agree on (the values that later layers mix
     # into theirs, for instance).  It starts empty with every step.
     shared: Dict[str, torch.Tensor] = field(default_factory=dict)
 
     @property
     def padded(self) -> bool:
-        """Whether the step has rows that belong to no sequence (kernels write nothing there)."""
-        return self.n_tokens > sum(self.host_new)
+        """Whether the step has, or in a replay may have, rows that belong to no sequence (kernels write nothing there)."""
+        return self.captured or self.n_tokens > sum(self.host_new)
 
 
 @dataclass

@@ -105,7 +105,7 @@ class InputConvMixer(Mixer):
     def forward(self, x, step: StepContext, cache: CacheView) -> torch.Tensor:
         if isinstance(x, NormedLazy):
             x = x.dense()
-        make = torch.empty if step.n_tokens == step.n_seqs else torch.zeros
+        make = torch.zeros if step.padded else torch.empty
         h = make((step.n_tokens, self.hidden), dtype=self.runtime.dtype, device=x.device)
         if self.own_state:
             own = cache.state[:, self.inner_state:]

@@ -75,7 +75,7 @@ class Mamba2Mixer(Mixer):
         inner, C, GN = self.inner, self.channels, self.G * self.N
         proj = self.input.forward(x)
         # rows that belong to no sequence (a small step's padding) are not written by the kernels: keep them defined
-        make = torch.empty if n == step.n_seqs else torch.zeros
+        make = torch.zeros if step.padded else torch.empty
         xbc = make((n, C), dtype=torch.float32, device=dev)
         conv_state = cache.state[:, self.conv_off:] if self.taps > 1 else cache.state
         ops.short_conv(proj[:, inner:inner + C], self.conv_weight, self.conv_bias, conv_state, step, xbc, silu=True,
@@ -143,7 +143,7 @@ class GatedLinearAttentionMixer(BranchMixer):
         n, dev = step.n_tokens, out.device
         alpha = torch.empty((n, self.H * self.d), dtype=torch.float32, device=dev)
         ops.decay_lowrank(stacked.view(tag + "a1"), self.a2, self.a2_bias, self.tau, n, alpha)
-        make = torch.empty if n == step.n_seqs else torch.zeros
+        make = torch.zeros if step.padded else torch.empty
         o = make((n, self.H * self.dv), dtype=torch.float32, device=dev)
         ops.outer_recurrence(stacked.view(tag + "q"), stacked.view(tag + "k"), stacked.view(tag + "v"), alpha, cache.state, o, step,
                              self.H, self.H, self.d, self.dv, q_scale=self.q_scale)

@@ -55,7 +55,7 @@ class MinGRUMixer(Mixer):
         proj = self.inputs.forward(x)
         col = self.inputs.column
         # rows that belong to no sequence (a small step's padding) are not written by the scan: keep them defined
-        make = torch.empty if step.n_tokens == step.n_seqs else torch.zeros
+        make = torch.zeros if step.padded else torch.empty
         mixed = make((step.n_tokens, self.width), dtype=self.runtime.dtype, device=x.device)
         ops.mingru_scan(proj, col("z"), col("x"), col("g"), self.bias_z, self.bias_x, cache.state, mixed, step, self.width)
         return self.o.forward(mixed, allow_partials=True)
@@ -128,7 +128,7 @@ class GatedDeltaMixer(Mixer):
         col = self.inputs.column
         n = step.n_tokens
         # rows that belong to no sequence (a small step's padding) are not written by the scan: keep them defined
-        make = torch.empty if n == step.n_seqs else torch.zeros
+        make = torch.zeros if step.padded else torch.empty
         o = make((n, self.H * self.dv), dtype=torch.float32, device=x.device)
         ops.gated_delta_rule(proj, col("qkv"), col("beta"), col("a"), self.conv_weight, self.A_log, self.dt_bias, cache.state,
                              self.conv_off, o, step, self.H, self.G, self.d, self.dv, self.q_scale, self.unit_eps)
@@ -193,7 +193,7 @@ class RGLRUMixer(Mixer):
         proj = self.inputs.forward(x)
         y_col, x_col = self.inputs.column("y"), self.inputs.column("x")
         # rows that belong to no sequence (a small step's padding) are not written by the kernels: keep them defined
-        make = torch.empty if n == step.n_seqs else torch.zeros
+        make = torch.zeros if step.padded else torch.empty
         u = make((n, w), dtype=torch.float32, device=dev)
         ops.causal_conv(proj, x_col, self.x_bias, self.conv_weight, self.conv_bias, cache.state, step, w, u)
         gates = torch.empty((n, 2 * w), dtype=torch.float32, device=dev)
