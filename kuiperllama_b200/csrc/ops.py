@@ -1258,7 +1258,8 @@ def attention_mixed(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Te
     r1_h ln(1 + r2_h (i - j)) taken off, a sliding window that also keeps the first ``keep_first`` keys, the heads' softmax
     weights mixed by ``talk`` [heads, heads], and head h's result times out_scale * sigmoid(gate[t, h]) (see
     attention_mixed.cu).  ``q`` [rows, heads * dim], ``gate`` [rows, heads], ``out`` [rows, heads * vdim]: the compute dtype,
-    any row stride.  The tiled kernel (attention_mixed_tiled.cu) runs where its shared memory holds the sizes, else the
+    any row stride.  Prompts of bfloat16 rows run on the tensor cores where the sizes allow (attention_mixed_mma.cu); else the
+    tiled kernel (attention_mixed_tiled.cu) runs where its shared memory holds the sizes (``tiled=True`` asks for it), else the
     plain one; ``tiled=False`` asks for the plain one, and ``splits`` (1 to 32) sets into how many pieces a step of single
     tokens cuts each sequence's keys instead of ``mixed_attention_splits``."""
     _cuda(q, gate, out, k_cache, v_cache, block_table, r1, r2, talk)
@@ -1273,8 +1274,20 @@ def attention_mixed(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Te
         _need(t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.numel() == count), "attention_mixed: float32 per-head tensors")
     _need((r1 is None) == (r2 is None), "attention_mixed: the distance bias needs both of its numbers")
     _need(heads % kv_heads == 0, "attention_mixed: heads must be a multiple of kv heads")
-    L = lib("attention_mixed_tiled")
     max_new = int(step.max_new)
+    if tiled is None and splits is None and q.dtype == torch.bfloat16 and max_new > 1:
+        M = lib("attention_mixed_mma")
+        if (M.kl_attention_mixed_mma_fits(heads, kv_heads, dim, vdim, BF16, max_new) and q.stride(0) % 2 == 0 and out.stride(0) % 2 == 0
+                and (q.data_ptr() | out.data_ptr()) % 4 == 0 and (talk is None or talk.data_ptr() % 8 == 0)):
+            ml = torch.empty((n, heads, 2), dtype=torch.float32, device=q.device)
+            _check(M.kl_attention_mixed_mma(
+                _ptr(q), ctypes.c_longlong(q.stride(0)), _ptr(gate), ctypes.c_longlong(gate.stride(0) if gate is not None else 0), _ptr(out),
+                ctypes.c_longlong(out.stride(0)), _ptr(k_cache), _ptr(v_cache), _ptr(block_table), block_table.shape[1], _ptr(step.cu_tokens),
+                _ptr(step.seq_slots), _ptr(step.seq_starts), n, step.n_seqs, max_new, heads, kv_heads, dim, ctypes.c_float(scale),
+                ctypes.c_float(softcap or 0.0), _ptr(r1), _ptr(r2), _ptr(talk), int(window or 0), int(keep_first or 0),
+                ctypes.c_float(out_scale), _ptr(ml), _stream()), "attention_mixed_mma", 2)
+            return
+    L = lib("attention_mixed_tiled")
     fits = L.kl_attention_mixed_tiled_fits(heads, kv_heads, dim, vdim, dtype_code(q.dtype), int(talk is not None), max_new)
     _need(not (tiled and not fits), "attention_mixed: the tiled kernel cannot hold these sizes")
     if fits and tiled is not False:
