@@ -70,8 +70,7 @@ template <int D> __device__ __forceinline__ int mx_at(int r, int c) {
     else return r * D + ((c ^ ((r / (8 / P)) & (P - 1))) << 3);
 }
 
-template <int H, int D>
-constexpr size_t mx_smem_bytes(int G, int phase) {
+inline size_t mx_smem_bytes(int H, int D, int G, int phase) {
     return (size_t)(phase == 1 ? 3 : 2) * G * MX_CH * D * 2 + (size_t)(H / 2) * 2 * MX_BIAS * 4 +
            (phase == 1 ? (size_t)H * MX_PH * 4 + (size_t)3 * H * (H + 8) * 2 : 0);
 }
@@ -328,7 +327,7 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
 
 template <int H, int D, int PHASE>
 static int launch_mixed_mma(const MixedMmaArgs& A, dim3 grid, cudaStream_t stream) {
-    const size_t smem = mx_smem_bytes<H, D>(A.kv_heads, PHASE);
+    const size_t smem = mx_smem_bytes(H, D, A.kv_heads, PHASE);
     KL_CUDA(cudaFuncSetAttribute(attention_mixed_mma_kernel<H, D, PHASE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     launch_kernel(attention_mixed_mma_kernel<H, D, PHASE>, grid, H * 16, smem, stream, A);
     KL_LAUNCH_CHECK();
@@ -340,11 +339,11 @@ static int launch_mixed_mma(const MixedMmaArgs& A, dim3 grid, cudaStream_t strea
 using namespace kl;
 
 // Whether kl_attention_mixed_mma runs these sizes: 16 or 32 heads, an even number of them to a key/value head, keys and values of 32 or
-// 64 (larger heads leave no room for the chunks beside P), and steps of more than four tokens a sequence (a tile of eight mostly
+// 64 (larger heads, and 16 key/value heads of 64, leave no room for the chunks beside P), and steps of more than four tokens a sequence (a tile of eight mostly
 // empty is no gain).
 KL_API int kl_attention_mixed_mma_fits(int heads, int kv_heads, int dim, int vdim, int dtype, int max_new) {
     return dtype == KL_BF16 && (heads == 16 || heads == 32) && kv_heads > 0 && heads % kv_heads == 0 && heads / kv_heads % 2 == 0 && dim == vdim &&
-           (dim == 32 || dim == 64) && max_new > 4;
+           (dim == 32 || dim == 64) && max_new > 4 && mx_smem_bytes(heads, dim, kv_heads, 1) <= 227 * 1024;
 }
 
 // ml: float32 [rows, heads, 2].  q and out: rows and heads on 4-byte boundaries; the caches on 16-byte ones.
