@@ -1,0 +1,230 @@
+"""Kernels that prompts take, alone against float64 at the sizes where they can go wrong: remainders of tiles, every split of a state over
+lanes, rows on no 16-byte boundary, windows and kept keys, portions that start inside a page."""
+from __future__ import annotations
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+F64 = torch.float64
+U = 2.0 ** -24                                              # half a unit in the last place of 1.0 in float32
+
+
+def _step(starts, news):
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    cu = [0]
+    for n in news:
+        cu.append(cu[-1] + n)
+    return SimpleNamespace(n_tokens=cu[-1], n_seqs=len(news), cu_tokens=i32(cu), seq_slots=i32(list(range(len(news)))), seq_starts=i32(starts),
+                           seq_new=i32(news), max_new=max(news), token_slot=i32([s for s, n in enumerate(news) for _ in range(n)]),
+                           positions=i32([a + t for a, n in zip(starts, news) for t in range(n)]), host_new=news, cu=cu)
+
+
+def _recurrence(q, k, v, a, c, skip, state, cu, scale):
+    """y and S in float64; with every operand replaced by its magnitude it is the sum that bounds the rounding."""
+    y, out = torch.zeros(v.shape, dtype=F64, device=DEV), []
+    for s in range(len(cu) - 1):
+        S = state[s].clone()
+        for t in range(cu[s], cu[s + 1]):
+            S = S * a[t][:, :, None] + (c[t][:, None] * k[t])[:, :, None] * v[t][:, None, :]
+            y[t] = (q[t][:, None] @ S)[:, 0] * scale + skip[:, None] * v[t]
+        out.append(S)
+    return y, torch.stack(out)
+
+
+# heads, groups, N, P: N fills 4, 8, 16 and 32 lanes or leaves some empty; P of one column pair, of a remainder of a CTA's columns; odd
+# sizes that no 16-byte copy takes; many heads, so that the larger pieces of S are chosen
+@pytest.mark.parametrize("heads,groups,n,p", [(1, 1, 4, 4), (4, 2, 16, 8), (3, 3, 9, 6), (5, 1, 33, 14), (2, 1, 128, 64), (2, 2, 500, 4), (1, 1, 512, 2),
+                                              (64, 1, 128, 64), (16, 16, 64, 128), (96, 32, 20, 50)])
+@pytest.mark.parametrize("form", ["head", "row", "normaliser"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_recurrence_of_prompts(heads, groups, n, p, form, dtype):
+    from kuiperllama_b200.csrc import ops
+    step = _step([0, 0, 0, 0], [39, 1, 16, 5])
+    rows = step.n_tokens
+    g = torch.Generator(device=DEV).manual_seed(heads * n + p)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    q, k, v = rand(rows, groups * n).to(dtype), (0.3 * rand(rows, groups * n)).to(dtype), rand(rows, heads * p).to(dtype)
+    a = 0.75 + 0.25 * torch.rand(rows, heads * n if form == "row" else heads, device=DEV, generator=g)
+    a[3] = 0.0                                             # a decay that underflowed: what was before is gone
+    c, skip = torch.rand(rows, heads, device=DEV, generator=g), rand(heads)
+    size = heads * n * p
+    state0 = torch.cat([0.1 * rand(4, size), 0.1 * rand(4, heads * n)], dim=1)
+    state = state0.clone()
+    y = torch.full((rows, heads * p), 7.0, device=DEV)
+    norm, floor, den = None, torch.full((rows, heads), 0.05, device=DEV), torch.empty(rows, heads, device=DEV)
+    if form == "normaliser":
+        norm = (state[:, size:], floor, den, 1e-3)
+    ops.outer_recurrence(q, k, v, a, state, y, step, heads, groups, n, p, c=c, skip=skip, q_scale=0.7, normaliser=norm)
+    wide = lambda x: x.double().view(rows, groups, n).repeat_interleave(heads // groups, dim=1)
+    args = [wide(q), wide(k), v.double().view(rows, heads, p), a.double().view(rows, heads, -1), c.double(), skip.double(),
+            state0[:, :size].double().view(4, heads, n, p)]
+    want, S = _recurrence(*args, step.cu, 0.7)
+    most, S_most = _recurrence(*[x.abs() for x in args], step.cu, 0.7)
+    # an element of S takes three roundings a token, y one more for each of n terms and a few for scale and skip
+    tokens = max(step.host_new)
+    assert bool(((y.double().view(want.shape) - want).abs() <= (3 * tokens + n + 8) * U * most).all())
+    assert bool(((state[:, :size].double().view(S.shape) - S).abs() <= (3 * tokens + 2) * U * S_most).all())
+    if form == "normaliser":
+        args[2], args[5], args[6] = torch.ones(rows, heads, 1, dtype=F64, device=DEV), torch.zeros(heads, dtype=F64, device=DEV), state0[:, size:].double().view(4, heads, n, 1)
+        dot, z = _recurrence(*args, step.cu, 0.7)
+        dot_most, z_most = _recurrence(*[x.abs() for x in args], step.cu, 0.7)
+        near = (3 * tokens + n + 8) * U * dot_most[:, :, 0] + 4 * U
+        assert bool(((den.double() - (torch.clamp(dot[:, :, 0].abs(), min=0.05) + 1e-3)).abs() <= near).all())
+        assert bool(((state[:, size:].double().view(z.shape) - z).abs() <= (3 * tokens + 2) * U * z_most).all())
+    else:
+        assert torch.equal(state[:, size:], state0[:, size:])
+
+
+@pytest.mark.parametrize("channels", [4, 36, 512, 1028])
+@pytest.mark.parametrize("dtype,out_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
+def test_four_taps_in_tiles(channels, dtype, out_dtype):
+    """The vector form against the plain one (the same rows at a stride that it does not take): the same bits, outputs and state."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(channels)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    w, b = rand(channels, 4), rand(channels)
+    for news in ([1, 1, 1], [2, 4, 3], [3, 17, 1], [70, 5, 33], [500]):
+        step = _step([0] * len(news), news)
+        x = rand(step.n_tokens, channels).to(dtype)
+        loose = torch.zeros(step.n_tokens, channels + 1, dtype=dtype, device=DEV)
+        loose[:, :channels] = x
+        state0 = rand(len(news), 3 * channels)
+        for add, silu in ((True, False), (False, True)):
+            got = []
+            for rows in (x, loose[:, :channels]):
+                state, out = state0.clone(), torch.empty(step.n_tokens, channels, dtype=out_dtype, device=DEV)
+                ops.short_conv(rows, w, b, state, step, out, add_input=add, silu=silu)
+                got.append((out, state))
+            assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1]), (news, add)
+
+
+@pytest.mark.parametrize("rows,channels", [(1, 5), (3, 256), (65, 300), (700, 1024)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_low_rank_decays_of_rank_16(rows, channels, dtype):
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(rows)
+    r1 = torch.randn(rows, 40, device=DEV, generator=g).to(dtype)[:, 3:19]
+    W2, b = torch.randn(channels, 16, device=DEV, generator=g), 8.0 * torch.randn(channels, device=DEV, generator=g)
+    a = torch.empty(rows, channels, device=DEV)
+    ops.decay_lowrank(r1, W2, b, 16.0, rows, a)
+    z = r1.double() @ W2.double().T + b.double()
+    want = torch.exp(-torch.nn.functional.softplus(-z, threshold=200.0) / 16.0)
+    most = r1.double().abs() @ W2.double().abs().T + b.double().abs()
+    # 17 roundings of z, whose error enters the exponent by at most a sixteenth, and a few units for exp and log1p
+    assert bool(((a.double() - want).abs() <= want * (17 * U * most / 16 + 32 * U)).all())
+
+
+@pytest.mark.parametrize("heads,dim", [(1, 1028), (2, 2048), (1, 4096), (1, 4100), (1, 8192)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gated_norm_of_long_heads(heads, dim, dtype):
+    """One pass in registers: the gate before and after the norm, a divisor; off by a sum of dim squares and the output's rounding."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(dim)
+    x, gate = 3 * torch.randn(37, heads * dim, device=DEV, generator=g), torch.randn(37, heads * dim, device=DEV, generator=g).to(dtype)
+    w, div = 1 + 0.2 * torch.randn(heads * dim, device=DEV, generator=g), 0.5 + torch.rand(37, heads, device=DEV, generator=g)
+    for first in (True, False):
+        out = torch.empty(37, heads * dim, dtype=dtype, device=DEV)
+        ops.head_rmsnorm_gate(x, gate, w, out, heads, dim, 1e-5, gate_first=first, out_scale=0.7, divisor=div)
+        xs, gs = x.double().view(37, heads, dim) / div.double()[..., None], torch.nn.functional.silu(gate.double()).view(37, heads, dim)
+        y = xs * gs if first else xs
+        y = y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5) * w.double().view(heads, dim)
+        want = (y if first else y * gs) * 0.7
+        tol = (dim ** 0.5 + 32) * U + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
+        assert bool(((out.double().view(want.shape) - want).abs() <= tol * want.abs() + 1e-9).all())
+
+
+# heads on key/value heads with keys and values of one size, window, kept first keys
+@pytest.mark.parametrize("H,G,d,window,keep", [(32, 8, 64, 96, 16), (16, 4, 64, 0, 0), (32, 16, 32, 130, 64), (16, 2, 32, 40, 5), (32, 2, 64, 1, 3),
+                                               (32, 16, 64, 70, 0)])
+def test_mixed_heads_on_the_tensor_cores(H, G, d, window, keep):
+    """Outputs are off by their own rounding (2^-9) and by what 32-bit scores, exponentials and sums leave: scores up to 30 in magnitude
+    after the soft cap have errors of a few 2^-24 * 30, which the exponential passes on as a relative error of about 1e-5."""
+    from kuiperllama_b200.csrc import ops
+    T, dev, dt = 256, DEV, torch.bfloat16
+    g = torch.Generator().manual_seed(H + G + d)
+    table = torch.tensor([[5, 2, 9, 0], [1, 7, 3, 11], [4, 6, 8, 10]], dtype=torch.int32, device=dev)
+    ks, vs = (torch.randn(3, T, G, d, generator=g).to(dt).to(dev) for _ in range(2))
+    qs, gates = (1.5 * torch.randn(3, T, H, d, generator=g)).to(dt).to(dev), torch.randn(3, T, H, generator=g).to(dt).to(dev)
+    kc, vc = torch.zeros(12, G, 64, d, dtype=dt, device=dev), torch.zeros(12, G, 64, d, dtype=dt, device=dev)
+    for s in range(3):
+        for p in range(T):
+            kc[int(table[s, p // 64]), :, p % 64], vc[int(table[s, p // 64]), :, p % 64] = ks[s, p], vs[s, p]
+    r1, r2 = (torch.rand(H, generator=g) * 0.5 + 0.1).to(dev), (torch.rand(H, generator=g) + 0.05).to(dev)
+    talk = (torch.eye(H) + 0.4 * torch.randn(H, H, generator=g)).to(dev)
+    i, j = torch.arange(T, device=dev)[:, None], torch.arange(T, device=dev)[None]
+    hidden = (j > i) | ((i - j >= window) & (j >= keep) if window else torch.zeros(T, T, dtype=torch.bool, device=dev))
+    for full in (True, False):
+        want, most = [], []
+        for s in range(3):
+            sc = torch.einsum("ihd,jhd->hij", qs[s].double(), ks[s].double().repeat_interleave(H // G, 1)) * 0.3
+            if full:
+                sc = 30.0 * torch.tanh(sc / 30.0) - r1.double()[:, None, None] * torch.log1p(r2.double()[:, None, None] * (i - j).clamp(min=0).double())
+            w = torch.softmax(sc.masked_fill(hidden, float("-inf")), -1)
+            u = torch.einsum("hg,gij->hij", talk.double().abs(), w) if full else w
+            w = torch.einsum("hg,gij->hij", talk.double(), w) if full else w
+            gate = 1.25 * (torch.sigmoid(gates[s].double()) if full else torch.ones(T, H, dtype=F64, device=dev))[..., None]
+            v = vs[s].double().repeat_interleave(H // G, 1)
+            want.append(torch.einsum("hij,jhd->ihd", w, v) * gate)
+            most.append(torch.einsum("hij,jhd->ihd", u, v.abs()) * gate)
+        for starts, news in (([0, 0, 0], [256, 1, 67]), ([100, 63, 200], [30, 2, 56]), ([0, 39, 129], [5, 110, 127])):
+            step = _step(starts, news)
+            cut = lambda x: torch.cat([x[s][a:a + n].reshape(n, -1) for s, (a, n) in enumerate(zip(starts, news))]).contiguous()
+            ref, bound = cut(want), cut(most)
+            for tiled in (None, False):                     # the kernel that the sizes choose and the plain one, within the same bound
+                out = torch.full((step.n_tokens, H * d), 9.0, dtype=dt, device=dev)
+                ops.attention_mixed(cut(qs), cut(gates) if full else None, out, kc, vc, table, step, H, G, d, d, 0.3, 30.0 if full else 0.0,
+                                    r1 if full else None, r2 if full else None, talk if full else None, window, keep, 1.25, tiled=tiled)
+                off = (out.double() - ref).abs()
+                assert bool((off <= 2.0 ** -8 * ref.abs() + 2e-5 * bound + 1e-30).all()), (full, starts, tiled, float((off / (bound + 1e-30)).max()))
+
+
+@pytest.mark.parametrize("H,KV,hd,vd", [(4, 2, 64, 64), (2, 1, 128, 128), (3, 3, 20, 20), (4, 1, 48, 32)])
+def test_float32_attention_of_runs_has_the_same_bits(H, KV, hd, vd):
+    """Tiles of eight rows, a CTA per row, and the plain kernel (which a distance bias of zeros asks for): prompts, portions, single tokens
+    and padding rows in one step, with and without a sink, and a cache that holds infinities past every row's keys."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator().manual_seed(hd)
+    table = torch.tensor([[5, 2, 9, 0], [1, 7, 3, 11], [4, 6, 8, 10]], dtype=torch.int32, device=DEV)
+    kc, vc = torch.randn(12, KV, 64, hd, generator=g).to(DEV), torch.randn(12, KV, 64, hd, generator=g).to(DEV)
+    for starts, news in (([0, 0, 0], [200, 1, 67]), ([100, 63, 200], [30, 2, 56]), ([150, 64, 255], [1, 1, 1]), ([0, 39, 129], [8, 16, 9])):
+        pos = [a + t for a, n in zip(starts, news) for t in range(n)] + [0, 0, 0]
+        slot = [s for s, n in enumerate(news) for _ in range(n)] + [-1, -1, -1]
+        pos, slot = (torch.tensor(x, dtype=torch.int32, device=DEV) for x in (pos, slot))
+        ks, vs = kc.clone(), vc.clone()
+        for s, (a, n) in enumerate(zip(starts, news)):
+            for p in range(a + n, 256):
+                ks[int(table[s, p // 64]), :, p % 64], vs[int(table[s, p // 64]), :, p % 64] = float("inf"), float("nan")
+        q = torch.randn(len(pos), H * hd, generator=g).to(DEV)
+        for sink in (None, torch.randn(H, generator=g).to(DEV)):
+            got = []
+            for runs, zeros in ((False, None), (True, None), (False, torch.zeros(H, 1, device=DEV))):
+                out = torch.full((len(pos), H * vd), 3.0, device=DEV)
+                ops.attention_simt(q, H * hd, out, ks, vs, table, pos, slot, len(pos), H, KV, hd, 0.2, value_dim=vd, sink=sink, distance_bias=zeros, runs=runs)
+                got.append(out)
+            assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2]) and bool(torch.isfinite(got[0]).all()) and bool((got[0][-3:] == 3.0).all())
+
+
+@pytest.mark.parametrize("H,G,d,dv", [(4, 2, 16, 24), (2, 1, 32, 8), (4, 4, 64, 48), (2, 1, 100, 36), (3, 1, 256, 20)])
+def test_delta_rule_has_the_same_bits_however_a_prompt_is_cut(H, G, d, dv):
+    """Whole tiles of eight tokens and tokens one by one, over every number of lanes a column is cut into."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(d)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    C, T = 2 * G * d + H * dv, 37
+    proj, taps = rand(T, C + 2 * H), rand(C, 4)
+    A_log, dt_bias = 0.1 * rand(H), rand(H) - 3.0
+    got = []
+    for cuts in ([T], [8, 8, 21], [1] * T, [5, 16, 3, 13]):
+        state, outs, at = torch.zeros(1, H * d * dv + 3 * C, device=DEV), [], 0
+        for n in cuts:
+            out = torch.empty(n, H * dv, device=DEV)
+            ops.gated_delta_rule(proj[at:at + n], 0, C, C + H, taps, A_log, dt_bias, state, H * d * dv, out, _step([at], [n]), H, G, d, dv, d ** -0.5, 1e-6)
+            outs.append(out)
+            at += n
+        got.append((torch.cat(outs), state))
+    for out, state in got[1:]:
+        assert torch.equal(out, got[0][0]) and torch.equal(state, got[0][1])
