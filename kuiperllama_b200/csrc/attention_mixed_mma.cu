@@ -79,7 +79,6 @@ template <int H, int D, int PHASE>
 __global__ void __launch_bounds__(H * 16, PHASE == 1 ? 1 : 512 / (H * 16) + 1)
 attention_mixed_mma_kernel(const MixedMmaArgs A) {
     constexpr int THREADS = H * 16, WARPS = H / 2, KS = D / 16, NT = MX_CH / 8;
-    pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(128) unsigned char mx_raw[];
     const int s = blockIdx.y, tile = gridDim.x - 1 - blockIdx.x;           // late tiles see the most keys: they start first
@@ -304,6 +303,7 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
         c = cn;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    pdl_launch_dependents();
     if (r >= nrows) return;
     const size_t row = (size_t)(row0 + r);
     if constexpr (PHASE == 0) {

@@ -61,10 +61,10 @@ inline bool pdl_enabled() {
 }
 
 // Launch on `stream`; a failure is left for cudaGetLastError (KL_LAUNCH_CHECK).  `cluster_x` > 1
-// launches thread-block clusters of that many CTAs along x (the grid's x must be a multiple of it).
+// launches thread-block clusters of that many CTAs along x (the grid's x must be a multiple of it).  `early`: with the attribute.
 template <typename... KArgs, typename... Args>
-inline void launch_kernel_clustered(void (*kernel)(KArgs...), int cluster_x, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                    Args&&... args) {
+inline void launch_kernel_with(bool early, void (*kernel)(KArgs...), int cluster_x, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                               Args&&... args) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = grid;
@@ -73,7 +73,7 @@ inline void launch_kernel_clustered(void (*kernel)(KArgs...), int cluster_x, dim
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int n = 0;
-    if (pdl_enabled()) {
+    if (early && pdl_enabled()) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n].val.programmaticStreamSerializationAllowed = 1;
         ++n;
@@ -90,8 +90,20 @@ inline void launch_kernel_clustered(void (*kernel)(KArgs...), int cluster_x, dim
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 template <typename... KArgs, typename... Args>
+inline void launch_kernel_clustered(void (*kernel)(KArgs...), int cluster_x, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                    Args&&... args) {
+    launch_kernel_with(true, kernel, cluster_x, grid, block, smem, stream, static_cast<Args&&>(args)...);
+}
+template <typename... KArgs, typename... Args>
 inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
     launch_kernel_clustered(kernel, 1, grid, block, smem, stream, static_cast<Args&&>(args)...);
+}
+// For a kernel of about one long CTA a multiprocessor (a walk over a prompt's tokens): it starts when the kernel ahead has finished.
+// Started early its CTAs crowd onto the multiprocessors that are free first and stay there: a recurrence of 128 CTAs over 2,048 tokens took 731
+// us beside the kernels ahead of it, 386 after them.  Such a kernel calls pdl_launch_dependents() at its end, for the same reason.
+template <typename... KArgs, typename... Args>
+inline void launch_kernel_after(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    launch_kernel_with(false, kernel, 1, grid, block, smem, stream, static_cast<Args&&>(args)...);
 }
 
 // Streaming multiprocessors of the current device (asked of the driver once per device; 0 on error).

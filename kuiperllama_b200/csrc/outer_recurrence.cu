@@ -247,7 +247,6 @@ __device__ __forceinline__ float2 or_two(const bf16* p) { return __bfloat1622flo
 template <typename TI, int R, int L, int MODE>
 __global__ void __launch_bounds__(OSL_THREADS, 2)
 outer_recurrence_slab_kernel(const OuterArgs A) {
-    pdl_launch_dependents();
     pdl_wait();
     constexpr int Np = R * L, H2 = R / 2, ES = sizeof(TI);
     constexpr int A_BYTES = MODE == 1 ? Np * 4 : 0;
@@ -255,6 +254,7 @@ outer_recurrence_slab_kernel(const OuterArgs A) {
     const int s = blockIdx.z, h = blockIdx.y;
     const int row0 = A.cu_tokens[s], n_new = A.cu_tokens[s + 1] - row0;
     if (n_new <= 0) return;
+    if (A.tile <= 8) pdl_launch_dependents();                  // a step of a few tokens
     const int N = A.N, P = A.P, T = A.tile;
     const int threads = blockDim.x, lane = threadIdx.x & 31;
     const int rg = threadIdx.x % L, cg = threadIdx.x / L;      // the thread's lane along the rows, and its column pair in the CTA
@@ -422,6 +422,7 @@ outer_recurrence_slab_kernel(const OuterArgs A) {
             }
         }
     }
+    pdl_launch_dependents();
 #pragma unroll
     for (int i = 0; i < H2; ++i) {
         const int n = 4 * rg + 4 * L * (i / 2) + 2 * (i % 2);
@@ -653,7 +654,7 @@ KL_API int kl_outer_recurrence(const void* q, long long ld_q, int q_col, const v
         auto quad = [&](const void* p, long long ld, int col) { return (uintptr_t)p % (4 * es) == 0 && ld % 4 == 0 && col % 4 == 0; };
         A.vec_in = (N % 4 == 0 && P % 4 == 0 && quad(q, ld_q, q_col) && quad(k, ld_k, k_col) && quad(v, ld_v, v_col) &&
                     (!a_per_row || ((uintptr_t)a % 16 == 0 && ld_a % 4 == 0))) ? 1 : 0;
-        A.tile = max_new <= 4 ? 4 : max_new <= 8 || Np > 256 ? 8 : 16;
+        A.tile = max_new <= 4 ? 4 : max_new <= 8 || Np > 256 ? 8 : 16;       // (a prompt of long rows of S: 8)
         A.L = L;
         const size_t smem = (size_t)2 * ((A.tile * tok + 2 * A.tile * 4 + 15) / 16 * 16);
         const dim3 grid((P + cols - 1) / cols, heads, n_seqs);
@@ -661,7 +662,8 @@ KL_API int kl_outer_recurrence(const void* q, long long ld_q, int q_col, const v
     do {                                                                                                            \
         if (smem > 48 * 1024)                                                                                       \
             KL_CUDA(cudaFuncSetAttribute(outer_recurrence_slab_kernel<TI, R_, L_, M_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        launch_kernel(outer_recurrence_slab_kernel<TI, R_, L_, M_>, grid, threads, smem, stream, A);                \
+        if (max_new > 8) launch_kernel_after(outer_recurrence_slab_kernel<TI, R_, L_, M_>, grid, threads, smem, stream, A); \
+        else launch_kernel(outer_recurrence_slab_kernel<TI, R_, L_, M_>, grid, threads, smem, stream, A);           \
     } while (0)
 #define KL_SLAB_M(TI, R_, L_)                                                                                        \
     do {                                                                                                            \

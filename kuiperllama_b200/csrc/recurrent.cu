@@ -512,8 +512,9 @@ KL_API int kl_gated_delta_rule(const void* proj, long long ld, int conv_col, int
     const dim3 grid1((max_new + tpc - 1) / tpc, n_seqs, G + H);
     const dim3 grid2((dv + DR_THREADS / lpc - 1) / (DR_THREADS / lpc), H, n_seqs);
     if (grid2.y > 65535) return KL_ERR_BAD_SIZE;
-#define KL_DR(T, L, D) launch_kernel(delta_rule_kernel<T, L, D>, grid2, DR_THREADS, 0, stream, (const float*)prep, (const float*)bg, (const T*)proj, ld, \
-                                     conv_col, taps, state, state_ld, conv_off, out, cu_tokens, seq_slots, H, G, d, dv)
+#define KL_DR(T, L, D) launch_kernel_with(max_new <= DR_TILE, delta_rule_kernel<T, L, D>, 1, grid2, DR_THREADS, 0, stream, (const float*)prep,          \
+                                          (const float*)bg, (const T*)proj, ld, conv_col, taps, state, state_ld, conv_off, out, cu_tokens,      \
+                                          seq_slots, H, G, d, dv)
 #define KL_DELTA(T)                                                                                                          \
     do {                                                                                                                     \
         launch_kernel(delta_prepare_kernel<T>, grid1, DP_THREADS, smem, stream, (const T*)proj, ld, conv_col, b_col, a_col, taps_w, taps, A_log, \

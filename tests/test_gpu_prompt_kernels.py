@@ -174,7 +174,7 @@ def test_mixed_heads_on_the_tensor_cores(H, G, d, window, keep):
             step = _step(starts, news)
             cut = lambda x: torch.cat([x[s][a:a + n].reshape(n, -1) for s, (a, n) in enumerate(zip(starts, news))]).contiguous()
             ref, bound = cut(want), cut(most)
-            for tiled in (None, False):                     # the kernel that the sizes choose and the plain one, within the same bound
+            for tiled in (None, True):                      # the kernel that the sizes choose and the tiled one, within the same bound
                 out = torch.full((step.n_tokens, H * d), 9.0, dtype=dt, device=dev)
                 ops.attention_mixed(cut(qs), cut(gates) if full else None, out, kc, vc, table, step, H, G, d, d, 0.3, 30.0 if full else 0.0,
                                     r1 if full else None, r2 if full else None, talk if full else None, window, keep, 1.25, tiled=tiled)
