@@ -10,8 +10,9 @@
 //
 // Ways of laying a product on tiles:
 //   * tokens as rows (prefill): A = activations [M, K], B = weights [N, K]; out[m, n] in bfloat16
-//     or float32.  Tiles of 256 x 256 worked by pairs of CTAs as one (gemm_pair_kernel, cta_group::2)
-//     where the token count suits, else tiles of 128 x 256 by single CTAs.
+//     or float32.  Tiles of 128 x 128 by single CTAs where all of them run at once; tiles of 256 x 256
+//     worked by pairs of CTAs as one (gemm_pair_kernel, cta_group::2) where the token count suits, else
+//     tiles of 128 x 256 by single CTAs.
 //   * weights as rows (decode, few tokens): A = weights [N, K], B = activations [M <= 64, K],
 //     tile 128 x {16, 32, 64}; the K range may be cut over blockIdx.z, each cut writing
 //     float32 partial sums [z, M, N] that the caller's reduction adds in a fixed order.  Every
@@ -750,28 +751,36 @@ KL_API int kl_gemm_tcgen05(const void* a, long long lda, const void* w, long lon
     CUtensorMap ma, mb;
     int rc;
     if ((rc = make_map(&ma, a, M, K, lda, TC_BM)) != KL_OK) return rc;
+    const int sms = kl::sm_count();
+    if (sms <= 1) return KL_ERR_SETUP;
+    const int tiles_m = (M + TC_BM - 1) / TC_BM;
+    // Tiles of 128 tokens x 128 features where all of them run at once.  Such a product is bound by what each multiprocessor
+    // has on its way from memory and by the chain of its k blocks: twice the CTAs, each with 7 stages of 32 KB instead of 4 of
+    // 48 KB, and k blocks of half the products.  us with tiles of 256 features (pairs from 129 tokens on) / of 128:
+    //   64 tokens:    gate/up of 16,384 x 2,048 18.3 / 14.2, 4,096 x 2,048 14.1 / 8.7, 4,096 x 14,336 81.0 / 44.2
+    //   500 tokens:   2,048 x 2,048 14.4 / 9.7, 4,096 x 14,336 69.5 / 53.3
+    //   1,024 tokens: 2,048 x 2,048 14.8 / 10.9, 2,048 x 8,192 42.6 / 30.3
+    // With more tiles than multiprocessors the second wave costs what the first one gained, and the larger tiles fetch less.
+    // The sums run over the same k blocks in the same order either way.
+    const bool narrow = (long long)tiles_m * ((N + 127) / 128) <= sms;
     // Pairs of CTAs on tiles of 256 tokens where that wastes no rows to speak of: an even number of
     // 128-token tiles, or so many tokens that half a tile of padding is little.
-    if (pairs_enabled() && (((M + TC_BM - 1) / TC_BM) % 2 == 0 || M >= 1024)) {
-        const int sms2 = kl::sm_count();
-        if (sms2 <= 1) return KL_ERR_SETUP;
+    if (!narrow && pairs_enabled() && (tiles_m % 2 == 0 || M >= 1024)) {
         if ((rc = make_map(&mb, w, N, K, ldw, 128)) != KL_OK) return rc;
         const int tiles_m2 = (M + 2 * TC_BM - 1) / (2 * TC_BM), tiles_n2 = (N + 255) / 256;
         if ((long long)tiles_m2 * tiles_n2 > 0x3fffffffLL) return KL_ERR_BAD_SIZE;
         GemmArgs pargs{out, ldo, 0, M, N, (K + TC_BK - 1) / TC_BK, out_f32, status, tiles_m2, tiles_n2, swiglu};
         set_gated(pargs, swiglu, limit, alpha, shift);
-        return launch_pairs(ma, mb, pargs, 2 * min(tiles_m2 * tiles_n2, sms2 / 2), stream);
+        return launch_pairs(ma, mb, pargs, 2 * min(tiles_m2 * tiles_n2, sms / 2), stream);
     }
-    if ((rc = make_map(&mb, w, N, K, ldw, 256)) != KL_OK) return rc;
-    const int tiles_m = (M + TC_BM - 1) / TC_BM, tiles_n = (N + 255) / 256;
+    const int bn = narrow ? 128 : 256;
+    if ((rc = make_map(&mb, w, N, K, ldw, bn)) != KL_OK) return rc;
+    const int tiles_n = (N + bn - 1) / bn;
     GemmArgs args{out, ldo, 0, M, N, (K + TC_BK - 1) / TC_BK, out_f32, status, tiles_m, tiles_n, swiglu};
     set_gated(args, swiglu, limit, alpha, shift);
     if ((long long)tiles_m * tiles_n > 0x7fffffffLL) return KL_ERR_BAD_SIZE;
-    const int sms = kl::sm_count();
-    if (sms <= 0) return KL_ERR_SETUP;
-    const int tiles = tiles_m * tiles_n;
-    const int grid_x = min(tiles, sms);               // one CTA per SM walks the tiles
-    dim3 grid(grid_x, 1, 1);
+    dim3 grid(min(tiles_m * tiles_n, sms), 1, 1);     // one CTA per SM walks the tiles
+    if (bn == 128) return launch<128, 7, false>(ma, mb, args, grid, stream);
     return launch<256, 4, false>(ma, mb, args, grid, stream);
 }
 

@@ -1467,8 +1467,8 @@ def skinny_splits(N: int, K: int, M: int = 1) -> int:
 
 
 def gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, swiglu: bool = False, activation="silu") -> None:
-    """out[M, N] = a @ w^T on the tensor cores, tokens as tile rows (any M; pairs of CTAs on tiles of
-    256 tokens where the token count suits, single CTAs on tiles of 128 otherwise).  With ``swiglu``
+    """out[M, N] = a @ w^T on the tensor cores, tokens as tile rows (any M; tiles of 128 x 128 where they all run at
+    once, else pairs of CTAs on tiles of 256 tokens where the token count suits, single CTAs on tiles of 128 otherwise).  With ``swiglu``
     the rows of ``w`` alternate 64 gate rows and 64 up rows and out[M, N / 2] receives
     act(gate) * up (``activation`` one of ``GATED_ACTIVATIONS``, or a (limit, alpha, shift))."""
     _cuda(a, w, out)
@@ -1559,31 +1559,45 @@ def gemm_skinny_stream(w: torch.Tensor, a: torch.Tensor, row_scale=None, sink=No
 
 # Which way round a product of M tokens and N features runs.  Weights as tile rows (tiles of 128
 # features x 16 to 128 tokens, the K range cut so that all SMs stream): every weight crosses from HBM
-# once and 16 KB of it per CTA and k block.  Tokens as tile rows (128 x 256 or 256 x 256): both operands
-# are reused, but a product of 128 tokens and 4,096 features has 16 tiles for 148 SMs (8B shape, 96
-# sequences: 7.6 ms per decode step that way, 5.5 ms with weights as rows).  Measured per product on
-# the 8B shape, us with tokens / weights as rows:
-#   128 tokens: q/k/v (24 tiles) 29.2 / 18.2, output (16) 26.7 / 13.9, gate/up (112) 43.1 / 53.6, down (16) 82.9 / 28.9
-#   384 tokens: q/k/v (72) 29.6 / 23.2, output (48) 26.8 / 21.7, gate/up (336) 85.0 / -, down (48) 82.6 / 46.1
-#   512 tokens: q/k/v (96) 27.6 / 34.1, output (64) 24.2 / 21.9, down (64) 70.2 / 58.5
-# and on the 1B shape at 128 tokens: gate/up (64 tiles) 18.0 / 25.9.  So beyond 64 tokens: weights as rows
-# while the other way has fewer tiles than 0.6 of the SMs; the gate/up product, whose K range cannot be
-# cut (its epilogue needs whole sums), while it has fewer than a third of them, and already from 33 tokens on
-# (8B shape, ms per decode step with the gate/up product's weights / tokens as rows: 48 sequences 4.06 / 4.02,
-# 64 sequences 4.44 / 4.36; 24 and 32 sequences, were they included: 3.42 / 3.49 and 3.52 / 3.62).
+# once and 16 KB of it per CTA and k block.  Tokens as tile rows (128 x 128, 128 x 256 or 256 x 256):
+# both operands are reused, but a product of 128 tokens and 4,096 features has 32 tiles for 148 SMs,
+# each of which walks all of K.  Measured per product, us with tokens / weights as rows (plain products
+# with their K cuts added up; features x K):
+#   48 tokens:  3,072 x 2,048 8.6 / 9.7, 1,024 x 1,024 5.3 / 7.4, 8,192 x 2,048 9.6 / 13.9, 4,096 x 4,096 14.8 / 13.0, 2,048 x 8,192 25.7 / 12.9
+#   128 tokens: 2,048 x 2,048 9.1 / 14.4, 8,192 x 2,048 10.3 / 21.1, 4,096 x 4,096 15.6 / 18.1, 1,024 x 4,096 14.7 / 13.1, 4,096 x 14,336 45.3 / 35.2
+#   256 tokens: 4,096 x 4,096 15.8 / 23.0, 1,024 x 4,096 14.7 / 17.2, 2,048 x 8,192 27.0 / 19.8
+#   32 tokens:  3,072 x 2,048 8.3 / 7.0, 1,024 x 4,096 14.1 / 7.7
+# (``tokens_first``: the lines of K where tokens as rows win while their tiles run at once.)  The gate/up product cannot cut
+# its K range (its epilogue needs whole sums):
+#   16,384 x 2,048: 16 tokens 18.1 / 14.5, 32 tokens 14.0 / 16.5, 64 tokens 14.1 / 21.4
+#   8,192 x 1,024:  16 tokens 8.2 / 7.8, 32 tokens 8.0 / 9.8, 128 tokens 7.2 / 23.5
+#   28,672 x 4,096: 16 tokens 41.1 / 39.4, 32 tokens 41.5 / 41.0, 48 tokens 41.8 / 45.7 (more tiles than SMs)
+# The pieces of a cut product that its consumer adds itself (``gemm_skinny_partials``) stay 32-bit numbers: there weights as
+# rows run up to the number of tokens at which the tiles of 128 x 256 reach 0.6 of the SMs.
 SKINNY_MAX_ROWS = 512
 
 
-SWIGLU_WEIGHT_ROWS_MAX = 32     # tokens up to which the gate/up product takes the weights as tile rows
+SWIGLU_WEIGHT_ROWS_MAX = 32     # tokens up to which the gate/up product takes the weights as tile rows (16 where the other way's tiles run at once)
+
+
+def one_wave(M: int, N: int) -> bool:
+    """Whether the tiles of 128 tokens x 128 features of a product all run at once (gemm_tcgen05 then takes them)."""
+    return ((M + 127) // 128) * ((N + 127) // 128) <= sm_count()
 
 
 def weights_as_rows(M: int, N: int, swiglu: bool = False) -> bool:
-    if M <= (SWIGLU_WEIGHT_ROWS_MAX if swiglu else 64):
+    if swiglu:
+        return M <= 16 or (M <= SWIGLU_WEIGHT_ROWS_MAX and not one_wave(M, N))
+    if M <= 64:
         return True
     if M > SKINNY_MAX_ROWS:
         return False
-    tiles = ((M + 127) // 128) * ((N + 255) // 256)
-    return tiles * 3 < sm_count() if swiglu else tiles * 5 < sm_count() * 3
+    return ((M + 127) // 128) * ((N + 255) // 256) * 5 < sm_count() * 3
+
+
+def tokens_first(M: int, N: int, K: int) -> bool:
+    """Whether a product whose K cuts would be added by a kernel of their own runs with tokens as tile rows all the same."""
+    return M > 32 and one_wave(M, N) and (K <= 2048 or (M > 128 and K <= 4096) or skinny_splits(N, K, M) == 1)
 
 
 def gemm_skinny_partials(a: torch.Tensor, w: torch.Tensor, splits: Optional[int] = None) -> Optional[torch.Tensor]:
@@ -1639,7 +1653,7 @@ def matmul(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     always take the plain 32-bit kernel; bfloat16 operands take the tensor-core kernels when
     their rows are 16-byte aligned (few tokens: weights as tile rows), else the plain kernel."""
     if a.dtype == torch.bfloat16 and _tc_ok(a, w, out):
-        if weights_as_rows(a.shape[0], w.shape[0]):
+        if weights_as_rows(a.shape[0], w.shape[0]) and not tokens_first(a.shape[0], *w.shape):
             gemm_skinny(a, w, out)
         else:
             gemm_tcgen05(a, w, out)

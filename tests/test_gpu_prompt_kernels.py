@@ -228,3 +228,54 @@ def test_delta_rule_has_the_same_bits_however_a_prompt_is_cut(H, G, d, dv):
         got.append((torch.cat(outs), state))
     for out, state in got[1:]:
         assert torch.equal(out, got[0][0]) and torch.equal(state, got[0][1])
+
+
+# ------------------------------------------------------------------------------------------------ products with few tiles
+
+def _rand(rows, cols, seed):
+    return (torch.randn(rows, cols, generator=torch.Generator().manual_seed(seed)) / cols ** 0.25).to(torch.bfloat16).to(DEV)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 64), (64, 1024, 72), (127, 136, 8), (129, 128, 512), (200, 2056, 640), (1025, 2048, 1032), (640, 3712, 128)])
+@pytest.mark.parametrize("f32_out", [False, True])
+def test_tiles_of_128_features_give_the_sums_of_the_larger_tiles(M, N, K, f32_out):
+    from kuiperllama_b200.csrc import ops
+    # the first rows of a product with too many tokens for the small tiles have the same sums, added in the same order
+    many = 128 * (148 // -(-N // 128) + 2)
+    if M >= many:
+        many = M + 128
+    a, w = _rand(many, K, seed=M), _rand(N, K, seed=N)
+    dt = torch.float32 if f32_out else torch.bfloat16
+    few, all_rows = torch.full((M + 1, N), 7.0, dtype=dt, device=DEV), torch.empty(many, N, dtype=dt, device=DEV)
+    assert ops.one_wave(M, N) and not ops.one_wave(many, N)
+    ops.gemm_tcgen05(a[:M], w, few[:M])
+    ops.gemm_tcgen05(a, w, all_rows)
+    assert torch.equal(few[:M], all_rows[:M])
+    assert bool((few[M] == 7.0).all())
+    exact = a[:M].double() @ w.double().T
+    # K exact products added in 32 bits (and one rounding to 8 bits of the bfloat16 result)
+    bound = (a[:M].double().abs() @ w.double().abs().T) * K * 2.0 ** -24 + (0 if f32_out else exact.abs() * 2.0 ** -8) + 1e-30
+    assert bool(((few[:M].double() - exact).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M", [16, 17, 32, 33, 128, 129, 512, 513])
+@pytest.mark.parametrize("N,K", [(256, 2048), (256, 2056), (2048, 4096), (1280, 4104), (19072, 256)])
+def test_products_on_both_sides_of_the_lines_between_the_ways_round(M, N, K):
+    from kuiperllama_b200.csrc import ops
+    a, w = _rand(M, K, seed=M), _rand(N, K, seed=K)
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    ops.matmul(a, w, out)
+    exact = a.double() @ w.double().T
+    bound = (a.double().abs() @ w.double().abs().T) * K * 2.0 ** -24 + exact.abs() * 2.0 ** -8 + 1e-30
+    assert bool(((out.double() - exact).abs() <= bound).all())
+    # the gated form of the same product: rows alternate 64 gate rows and 64 up rows
+    gated = torch.empty(M, N // 2, dtype=torch.bfloat16, device=DEV)
+    ops.matmul_swiglu(a, w, gated)
+    blocks = exact.view(M, N // 128, 2, 64)
+    g, u = blocks[:, :, 0].reshape(M, -1), blocks[:, :, 1].reshape(M, -1)
+    want = g * torch.sigmoid(g) * u
+    slack = (a.double().abs() @ w.double().abs().T).view(M, N // 128, 2, 64) * K * 2.0 ** -24
+    dg, du = slack[:, :, 0].reshape(M, -1), slack[:, :, 1].reshape(M, -1)
+    # |d silu / dg| <= 1.1; the two units' exponential and quotient are good to about 2^-20; one rounding to 8 bits
+    bound = 1.1 * dg * u.abs() + (g * torch.sigmoid(g)).abs() * du + want.abs() * (2.0 ** -8 + 2.0 ** -18) + 1e-30
+    assert bool(((gated.double() - want).abs() <= bound + 1e-6).all())
