@@ -15,7 +15,7 @@
 //   lane one row and one block; the warp copies its weights by 16-byte cp.async into a ring of its own, two chunks (17 KB a warp, 139 KB
 //   an SM) ahead of the arithmetic, without a break between one set of rows and the next, the first ones before the kernel ahead has
 //   finished.  W of 16,384 x 2,048: 28.7 us for one row of A (4.7 TB/s), 68 for eight (the shared-memory reads of A bind); a decode step
-//   of one sequence through two layers of width 2,048: 266 us, 4,051 with 64 x 64 tiles of which one row was used.
+//   of one sequence through two layers of width 2,048: 183 us, 4,051 with 64 x 64 tiles of which one row was used.
 // * gemm_tile_kernel (everything else) is bound by the FMA pipe.  128 threads make a tile of 64 x 128 outputs, 8 x 8 each, as
 //   packed pairs of rows of A (fma.rn.f32x2: the same two results in one instruction, whose operands come from both register
 //   banks; scalar multiply-adds of this form stay at 39 TFLOP/s whatever the tile and the occupancy).  A lies in shared memory with the row
