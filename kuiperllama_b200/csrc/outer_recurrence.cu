@@ -258,7 +258,7 @@ outer_recurrence_slab_kernel(const OuterArgs A) {
     const int N = A.N, P = A.P, T = A.tile;
     const int threads = blockDim.x, lane = threadIdx.x & 31;
     const int rg = threadIdx.x % L, cg = threadIdx.x / L;      // the thread's lane along the rows, and its column pair in the CTA
-    const int cols = threads / L * 2;                          // a multiple of four
+    const int cols = threads / L * 2;                          // a multiple of four (the launch rounds its threads to that)
     const int col0 = blockIdx.x * cols + cg * 2;
     const bool live = col0 < P;                                // P is even
     const int g = h / (A.heads / A.groups);
@@ -646,10 +646,11 @@ KL_API int kl_outer_recurrence(const void* q, long long ld_q, int q_col, const v
         }
         const int pairs = P / 2, es = in_dtype == KL_F32 ? 4 : 2;
         // CTAs of 128 threads: a CTA's threads share the copies of a tile, two CTAs on an SM fill each other's waits
-        const int fewest = 2 * L > 32 ? 2 * L : 32;            // four columns of S at least: pieces of four stay aligned
-        int threads = (L * pairs + 31) / 32 * 32;
-        threads = threads < fewest ? fewest : threads > OSL_THREADS ? OSL_THREADS : threads;
-        while (threads > fewest && threads % 64 == 0 && (long long)((pairs * L + threads - 1) / threads) * heads * n_seqs < sms) threads >>= 1;
+        const int fewest = 2 * L > 32 ? 2 * L : 32;            // whole warps and four columns of S at least
+        // always a multiple of `fewest`, so that a CTA's columns are a multiple of four: v is copied in pieces of four columns
+        int threads = (L * pairs + fewest - 1) / fewest * fewest;
+        threads = threads > OSL_THREADS ? OSL_THREADS : threads;
+        while (threads % (2 * fewest) == 0 && (long long)((pairs * L + threads - 1) / threads) * heads * n_seqs < sms) threads >>= 1;
         const int cols = threads / L * 2, Np = R * L, tok = (2 * Np * es + (mode == 1 ? Np * 4 : 0) + cols * es + 15) / 16 * 16;
         auto quad = [&](const void* p, long long ld, int col) { return (uintptr_t)p % (4 * es) == 0 && ld % 4 == 0 && col % 4 == 0; };
         A.vec_in = (N % 4 == 0 && P % 4 == 0 && quad(q, ld_q, q_col) && quad(k, ld_k, k_col) && quad(v, ld_v, v_col) &&

@@ -42,8 +42,21 @@ def _recurrence(q, k, v, a, c, skip, state, cu, scale):
 @pytest.mark.parametrize("form", ["head", "row", "normaliser"])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_recurrence_of_prompts(heads, groups, n, p, form, dtype):
+    _check_recurrence(heads, groups, n, p, form, dtype, [39, 1, 16, 5])
+
+
+# 32 lanes a column and three pairs of columns: 96 threads would be whole warps but no multiple of four columns
+@pytest.mark.parametrize("heads,groups,n,p", [(2, 1, 65, 6), (2, 2, 128, 6), (1, 1, 256, 6), (1, 1, 500, 6), (3, 3, 100, 2), (2, 1, 72, 10)])
+@pytest.mark.parametrize("form", ["head", "row", "normaliser"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("news", [[39, 1, 16, 5], [1, 1, 1, 1]])
+def test_recurrence_of_few_columns_over_all_lanes(heads, groups, n, p, form, dtype, news):
+    _check_recurrence(heads, groups, n, p, form, dtype, news)
+
+
+def _check_recurrence(heads, groups, n, p, form, dtype, news):
     from kuiperllama_b200.csrc import ops
-    step = _step([0, 0, 0, 0], [39, 1, 16, 5])
+    step = _step([0] * len(news), news)
     rows = step.n_tokens
     g = torch.Generator(device=DEV).manual_seed(heads * n + p)
     rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
