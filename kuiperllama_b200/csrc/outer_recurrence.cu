@@ -254,7 +254,7 @@ outer_recurrence_slab_kernel(const OuterArgs A) {
     const int s = blockIdx.z, h = blockIdx.y;
     const int row0 = A.cu_tokens[s], n_new = A.cu_tokens[s + 1] - row0;
     if (n_new <= 0) return;
-    if (A.tile <= 8) pdl_launch_dependents();                  // a step of a few tokens
+    if (n_new <= 8) pdl_launch_dependents();                   // a few tokens; a walk over a prompt asks at its end, whatever its tile
     const int N = A.N, P = A.P, T = A.tile;
     const int threads = blockDim.x, lane = threadIdx.x & 31;
     const int rg = threadIdx.x % L, cg = threadIdx.x / L;      // the thread's lane along the rows, and its column pair in the CTA
