@@ -198,8 +198,8 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
                 const bool vis = r < nrows && pos <= i && (A.window == 0 || i - pos < A.window || pos < keep);
                 float v = S[n][e] * A.scale;
                 if (A.softcap > 0.f) {                                     // v / cap, the quotient mended by its remainder
-                    const float x = v * inv_cap;
-                    v = A.softcap * tanhf(fmaf(fmaf(-x, A.softcap, v), inv_cap, x));
+                    const float x = v * inv_cap;                           // (an infinite score has none, and tanh is 1 far before that)
+                    v = A.softcap * tanhf(fabsf(x) < 64.f ? fmaf(fmaf(-x, A.softcap, v), inv_cap, x) : x);
                 }
                 if (A.r1 != nullptr) v -= bias[(e >> 1) * MX_BIAS + r + (MX_CH - 1) - key];
                 S[n][e] = vis ? v : -INFINITY;

@@ -195,6 +195,29 @@ def test_mixed_heads_on_the_tensor_cores(H, G, d, window, keep):
                 assert bool((off <= 2.0 ** -8 * ref.abs() + 2e-5 * bound + 1e-30).all()), (full, starts, tiled, float((off / (bound + 1e-30)).max()))
 
 
+@pytest.mark.parametrize("H,G,d", [(32, 8, 64), (16, 2, 32)])
+def test_mixed_heads_with_scores_that_overflow(H, G, d):
+    """Keys and queries whose products pass the largest float32: the soft cap takes infinite scores to +-cap, as in the tiled kernel."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator().manual_seed(d)
+    dt, T = torch.bfloat16, 100
+    table = torch.tensor([[1, 0]], dtype=torch.int32, device=DEV)
+    kc, vc = torch.randn(2, G, 64, d, generator=g).to(dt).to(DEV), torch.randn(2, G, 64, d, generator=g).to(dt).to(DEV)
+    q, talk = torch.randn(T, H * d, generator=g).to(dt).to(DEV), (torch.eye(H) + 0.2 * torch.randn(H, H, generator=g)).to(DEV)
+    kc[1, :, 3] = kc[1, :, 40] = 3e19                       # one sign a row: a score is +-inf, never inf - inf
+    q[10:60] = 2e19
+    q[60:] = q[60:].abs()
+    q[20] = -2e19
+    step, got = _step([0], [T]), []
+    for tiled in (None, True):
+        out = torch.full((T, H * d), 9.0, dtype=dt, device=DEV)
+        ops.attention_mixed(q, None, out, kc, vc, table, step, H, G, d, d, 1.0, 20.0, None, None, talk, 0, 0, 1.0, tiled=tiled)
+        got.append(out.float())
+    assert bool(torch.isfinite(got[1]).all())
+    # both round to bfloat16 sums of 32-bit weights of at most sum |talk| of order one
+    assert bool(((got[0] - got[1]).abs() <= 2.0 ** -7 * got[1].abs() + 1e-3).all())
+
+
 @pytest.mark.parametrize("H,KV,hd,vd", [(4, 2, 64, 64), (2, 1, 128, 128), (3, 3, 20, 20), (4, 1, 48, 32)])
 def test_float32_attention_of_runs_has_the_same_bits(H, KV, hd, vd):
     """Tiles of eight rows, a CTA per row, and the plain kernel (which a distance bias of zeros asks for): prompts, portions, single tokens
