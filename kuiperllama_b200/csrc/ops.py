@@ -1279,7 +1279,8 @@ def attention_mixed(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Te
     if tiled is None and splits is None and q.dtype == torch.bfloat16 and max_new > 1:
         M = lib("attention_mixed_mma")
         if (M.kl_attention_mixed_mma_fits(heads, kv_heads, dim, vdim, BF16, max_new) and q.stride(0) % 2 == 0 and out.stride(0) % 2 == 0
-                and (q.data_ptr() | out.data_ptr()) % 4 == 0 and (talk is None or talk.data_ptr() % 8 == 0)):
+                and (q.data_ptr() | out.data_ptr()) % 4 == 0 and (talk is None or talk.data_ptr() % 8 == 0)
+                and (k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0):
             ml = torch.empty((n, heads, 2), dtype=torch.float32, device=q.device)
             _check(M.kl_attention_mixed_mma(
                 _ptr(q), ctypes.c_longlong(q.stride(0)), _ptr(gate), ctypes.c_longlong(gate.stride(0) if gate is not None else 0), _ptr(out),

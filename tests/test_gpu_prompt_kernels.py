@@ -218,6 +218,26 @@ def test_mixed_heads_with_scores_that_overflow(H, G, d):
     assert bool(((got[0] - got[1]).abs() <= 2.0 ** -7 * got[1].abs() + 1e-3).all())
 
 
+@pytest.mark.parametrize("which", ["keys", "values"])
+def test_mixed_heads_of_caches_on_eight_bytes(which):
+    """A cache that starts between two 16-byte boundaries is served as before, by the kernel that copies smaller pieces."""
+    from kuiperllama_b200.csrc import ops
+    H, G, d, T, dt = 16, 4, 64, 70, torch.bfloat16
+    g = torch.Generator().manual_seed(1)
+    rand = lambda *s: torch.randn(*s, generator=g).to(dt).to(DEV)
+    table, step = torch.tensor([[1, 0]], dtype=torch.int32, device=DEV), _step([0], [T])
+    q, caches = rand(T, H * d), {"keys": rand(2, G, 64, d), "values": rand(2, G, 64, d)}
+    outs = []
+    for shift in (0, 4):
+        c = dict(caches)
+        room = torch.empty(c[which].numel() + 8, dtype=dt, device=DEV)
+        c[which] = room[shift:shift + c[which].numel()].view(2, G, 64, d).copy_(caches[which])
+        out = torch.empty(T, H * d, dtype=dt, device=DEV)
+        ops.attention_mixed(q, None, out, c["keys"], c["values"], table, step, H, G, d, d, 0.125, 0.0, None, None, None, 0, 0, 1.0)
+        outs.append(out.float())
+    assert bool(((outs[0] - outs[1]).abs() <= 2.0 ** -7 * outs[0].abs() + 1e-4).all())
+
+
 @pytest.mark.parametrize("H,KV,hd,vd", [(4, 2, 64, 64), (2, 1, 128, 128), (3, 3, 20, 20), (4, 1, 48, 32)])
 def test_float32_attention_of_runs_has_the_same_bits(H, KV, hd, vd):
     """Tiles of eight rows, a CTA per row, and the plain kernel (which a distance bias of zeros asks for): prompts, portions, single tokens
