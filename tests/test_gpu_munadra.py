@@ -469,6 +469,43 @@ def test_long_decoding_from_graphs(models, dtype):
     assert_logits(torch.cat(rows), oracle_logits(folder, toks), dtype, "long decoding")
 
 
+def test_padding_rows_of_a_replayed_step_stay_defined(models, monkeypatch):
+    """A small step captured with exactly 64 tokens has no padding; replayed with 40 it has 24 rows that no kernel writes.  With
+    NaN in every buffer that a latent layer leaves uninitialised, those rows of its result are finite all the same, and the real
+    rows agree with the plain implementation."""
+    import kuiperllama_b200.parts.latent_attention as module
+
+    class Marked:
+        def __getattr__(self, name):
+            return getattr(torch, name)
+
+        @staticmethod
+        def empty(*a, **kw):
+            return torch.empty(*a, **kw).fill_(float("nan"))
+
+    made, forward = [], module.LatentAttentionMixer.forward
+
+    def spy(self, x, step, cache):
+        made.append(forward(self, x, step, cache))
+        return made[-1]
+
+    monkeypatch.setattr(module, "torch", Marked())
+    monkeypatch.setattr(module.LatentAttentionMixer, "forward", spy)
+    model, folder = models("mixed", "float32", seed=1)
+    toks = [tokens(n, CONFIGS["mixed"]["vocab"], seed=80 + n) for n in (64, 40)]
+    eng = _engine(model, use_graphs=True)
+    with torch.inference_mode():
+        for t in toks:
+            slot = eng.alloc_slot()
+            row = eng.step([_inputs(slot, t, [len(t) - 1])]).clone()
+            assert_logits(row, oracle_logits(folder, t)[-1:], "float32", f"{len(t)} tokens through the captured step")
+    eng.check_device_errors()
+    layers = len(made) // 2                                                # every latent layer once eagerly and once captured
+    assert layers == sum(x["type"] == "latent_attention" for x in CONFIGS["mixed"]["layers"]) and len(eng._step_graphs) == 1
+    for out in made[layers:]:
+        assert out.shape[0] == 64 and bool(torch.isfinite(out).all())
+
+
 # ----------------------------------------------------------------------------- the entry points
 
 @pytest.mark.parametrize("dtype", DTYPES)
