@@ -86,8 +86,11 @@ def _places(want: Sequence[int], n: int, slot: int) -> np.ndarray:
             return np.arange(want.start, want.stop, want.step, dtype=np.int32)
         want = bad
     a = np.asarray(want)
-    if a.ndim != 1:
-        a = np.asarray([w for w in want])
+    if a.ndim != 1:                                       # no plain sequence of places (a set, nested lists): looked at one by one, and
+        for w in want:                                    # taken if it is one to numpy too
+            if not 0 <= w < n:
+                raise StepError(f"slot {slot}: wanted place {w} is outside its {n} tokens")
+        return np.asarray(want, dtype=np.int32)
     bad = np.flatnonzero(~((a >= 0) & (a < n)))
     if bad.size:
         raise StepError(f"slot {slot}: wanted place {a[bad[0]]} is outside its {n} tokens")

@@ -18,3 +18,10 @@ def test_places_outside_are_refused(want, first):
     from kuiperllama_b200.engine.step import StepError, _places
     with pytest.raises(StepError, match=f"slot 3: wanted place {first} is outside its 5 tokens"):
         _places(want, 5, 3)
+
+
+@pytest.mark.parametrize("want", [{0, 2}, {1: 0}, [[0], [1]], [[0, 1]], ["1"], [None]])
+def test_what_is_no_sequence_of_places_is_refused(want):
+    from kuiperllama_b200.engine.step import _places
+    with pytest.raises(TypeError):
+        _places(want, 5, 3)
