@@ -88,11 +88,14 @@ gemm_rows_kernel(const float* __restrict__ A, int lda, const float* __restrict__
     const int m0 = blockIdx.y * MT;
     const int nb = (K + BLOCK - 1) / BLOCK, spans = (nb + GR_LANES - 1) / GR_LANES;
     const int mine = first < spans ? (spans - 1 - first) / wb + 1 : 0;        // spans of this warp
+    // chunks of a span: the last one stops where its first block does (64 columns of 64 in one chunk: 2 us, 15 with all eight or sixteen)
+    const int last_parts = min(R::PER, (K - (spans - 1) * GR_SPAN + R::CHUNK - 1) / R::CHUNK);
+    auto parts = [&](int span) { return span == spans - 1 ? last_parts : R::PER; };
     float* ring = gr_smem + warp * GR_STAGES * R::STAGE;
     float* sums = gr_smem + GR_WARPS * GR_STAGES * R::STAGE;                  // two of [blocks][MT][rows_item]
     const int sums_floats = spans * GR_LANES * MT * rows_item;
     const int n_items = (int)blockIdx.x < items ? (items - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    const int chunks = mine * R::PER * n_items;
+    const int chunks = mine > 0 ? ((mine - 1) * R::PER + parts(first + (mine - 1) * wb)) * n_items : 0;
 
     constexpr int Q = R::CHUNK / 4, RSTEP = 32 / Q;
     const int q = lane % Q, r0 = lane / Q;
@@ -100,7 +103,7 @@ gemm_rows_kernel(const float* __restrict__ A, int lda, const float* __restrict__
     Place pw = {(int)blockIdx.x, first, 0}, pa = pw;
     auto next = [&](Place& p) {
         p.k += R::CHUNK;
-        if (p.k == BLOCK) {
+        if (p.k == parts(p.span) * R::CHUNK) {
             p.k = 0;
             p.span += wb;
             if (p.span >= spans) { p.span = first; p.item += gridDim.x; }
@@ -147,7 +150,7 @@ gemm_rows_kernel(const float* __restrict__ A, int lda, const float* __restrict__
             float acc[MT];
 #pragma unroll
             for (int m = 0; m < MT; ++m) acc[m] = 0.f;
-            for (int part = 0; part < R::PER; ++part, ++c) {
+            for (int part = parts(first + sp * wb); part > 0; --part, ++c) {
                 if (c + GR_STAGES - 1 < chunks) {
                     const int to = slot == 0 ? GR_STAGES - 1 : slot - 1;
                     load_w(to);

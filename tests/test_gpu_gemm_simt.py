@@ -9,8 +9,9 @@ pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda:0")
 
 
-# K: below, at and above blocks of 512 and spans of 2,048; one block over 16 (no cluster); N: remainders of 8, 32 and 128
-@pytest.mark.parametrize("n,k", [(7, 4), (100, 172), (130, 512), (129, 516), (260, 2048), (65, 2052), (2100, 1028), (70, 8704)])
+# K: below, at and above blocks of 512, spans of 2,048 and chunks of 32 and 64 at a span's end; one block over 16 (no cluster); N: remainders of 8, 32 and 128
+@pytest.mark.parametrize("n,k", [(7, 4), (100, 172), (130, 512), (129, 516), (260, 2048), (65, 2052), (2100, 1028), (70, 8704),
+                                 (70, 32), (33, 36), (64, 64), (40, 68), (24, 500), (24, 2080), (9, 6212)])
 def test_outputs_do_not_depend_on_the_kernel(n, k):
     from kuiperllama_b200.csrc import ops
     g = torch.Generator(device=DEV).manual_seed(n * k)
