@@ -228,34 +228,62 @@ gemm_tile_kernel(const TI* __restrict__ A, int lda, const TI* __restrict__ W, in
     const int k_lo = rank * per * BLOCK, k_hi = min(K, (rank + 1) * per * BLOCK);
     const int steps = k_hi > k_lo ? (k_hi - k_lo + GT_BK - 1) / GT_BK : 0;
 
-    auto load = [&](int s) {
+    static_assert(T::BN * GT_BK % (4 * GT_THREADS) == 0 && T::BM * GT_BK % GT_THREADS == 0, "whole rounds of copies");
+    auto load = [&](int s) {                                     // VEC: a step's copies on their way
         float* sa = gt_smem + (s % T::STAGES) * T::STAGE;
         float* sw = sa + T::A_FLOATS;
         const int kb = k_lo + s * GT_BK;
-        if constexpr (VEC) {
-            constexpr int COPIES = T::BN * (GT_BK / 4);
+        constexpr int COPIES = T::BN * (GT_BK / 4);
 #pragma unroll
-            for (int i = 0; i < COPIES / GT_THREADS; ++i) {
-                const int e = tid + GT_THREADS * i, q = e % (GT_BK / 4), r = e / (GT_BK / 4), k = kb + 4 * q;
-                const bool ok = n0 + r < N && k < k_hi;
-                cp_async<16>(sw + r * T::W_ROW + 4 * q, ok ? W + (size_t)(n0 + r) * ldw + k : W, ok);
-            }
-            static_assert(COPIES % GT_THREADS == 0 && T::BM * GT_BK % GT_THREADS == 0, "whole rounds of copies");
-            // a warp copies 8 k (a sector) of four rows: 32 banks of A's transposed place
+        for (int i = 0; i < COPIES / GT_THREADS; ++i) {
+            const int e = tid + GT_THREADS * i, q = e % (GT_BK / 4), r = e / (GT_BK / 4), k = kb + 4 * q;
+            const bool ok = n0 + r < N && k < k_hi;
+            cp_async<16>(sw + r * T::W_ROW + 4 * q, ok ? W + (size_t)(n0 + r) * ldw + k : W, ok);
+        }
+        // a warp copies 8 k (a sector) of four rows: 32 banks of A's transposed place
 #pragma unroll
-            for (int i = 0; i < T::BM * GT_BK / GT_THREADS; ++i) {
-                const int e = tid + GT_THREADS * i, r = e % 4 + e / 32 % (T::BM / 4) * 4, q = e / 4 % 8 + e / (8 * T::BM) * 8, k = kb + q;
-                const bool ok = m0 + r < M && k < k_hi;
-                cp_async<4>(sa + q * T::A_ROW + r, ok ? A + (size_t)(m0 + r) * lda + k : A, ok);
+        for (int i = 0; i < T::BM * GT_BK / GT_THREADS; ++i) {
+            const int e = tid + GT_THREADS * i, r = e % 4 + e / 32 % (T::BM / 4) * 4, q = e / 4 % 8 + e / (8 * T::BM) * 8, k = kb + q;
+            const bool ok = m0 + r < M && k < k_hi;
+            cp_async<4>(sa + q * T::A_ROW + r, ok ? A + (size_t)(m0 + r) * lda + k : A, ok);
+        }
+    };
+    // Else (bfloat16, or rows on no 16-byte boundary) GROUP steps are fetched into registers while the GROUP before is worked, and laid
+    // down behind it: 64 x 64 x 172 of bfloat16 8.4 us, 18.2 when every step
+    // waited for its own elements.
+    constexpr int GROUP = VEC ? 1 : T::STAGES >= 8 ? 4 : 1, WE = VEC ? 1 : T::BN * GT_BK / GT_THREADS, AE = VEC ? 1 : T::BM * GT_BK / GT_THREADS;
+    static_assert(VEC || T::STAGES >= 2 * GROUP, "the group that is worked and the next one");
+    TI rw[GROUP][WE], ra[GROUP][AE];
+    auto fetch = [&](int s0) {
+#pragma unroll
+        for (int u = 0; u < GROUP; ++u) {
+            const int kb = k_lo + (s0 + u) * GT_BK;
+#pragma unroll
+            for (int i = 0; i < WE; ++i) {
+                const int e = tid + GT_THREADS * i, q = e % GT_BK, r = e / GT_BK;
+                rw[u][i] = n0 + r < N && kb + q < k_hi ? W[(size_t)(n0 + r) * ldw + kb + q] : from_f32<TI>(0.f);
             }
-        } else {
-            for (int e = tid; e < T::BN * GT_BK; e += GT_THREADS) {
-                const int q = e % GT_BK, r = e / GT_BK;
-                sw[r * T::W_ROW + q] = n0 + r < N && kb + q < k_hi ? to_f32(W[(size_t)(n0 + r) * ldw + kb + q]) : 0.f;
+#pragma unroll
+            for (int i = 0; i < AE; ++i) {
+                const int e = tid + GT_THREADS * i, q = e % GT_BK, r = e / GT_BK;
+                ra[u][i] = m0 + r < M && kb + q < k_hi ? A[(size_t)(m0 + r) * lda + kb + q] : from_f32<TI>(0.f);
             }
-            for (int e = tid; e < T::BM * GT_BK; e += GT_THREADS) {
-                const int q = e % GT_BK, r = e / GT_BK;
-                sa[q * T::A_ROW + r] = m0 + r < M && kb + q < k_hi ? to_f32(A[(size_t)(m0 + r) * lda + kb + q]) : 0.f;
+        }
+    };
+    auto lay = [&](int s0) {
+#pragma unroll
+        for (int u = 0; u < GROUP; ++u) {
+            float* sa = gt_smem + ((s0 + u) % T::STAGES) * T::STAGE;
+            float* sw = sa + T::A_FLOATS;
+#pragma unroll
+            for (int i = 0; i < WE; ++i) {
+                const int e = tid + GT_THREADS * i;
+                sw[e / GT_BK * T::W_ROW + e % GT_BK] = to_f32(rw[u][i]);
+            }
+#pragma unroll
+            for (int i = 0; i < AE; ++i) {
+                const int e = tid + GT_THREADS * i;
+                sa[e % GT_BK * T::A_ROW + e / GT_BK] = to_f32(ra[u][i]);
             }
         }
     };
@@ -265,16 +293,7 @@ gemm_tile_kernel(const TI* __restrict__ A, int lda, const TI* __restrict__ W, in
     for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = 0;
-#pragma unroll
-    for (int s = 0; s < T::STAGES - 1; ++s) {
-        if (s < steps) load(s);
-        cp_commit();
-    }
-    for (int s = 0; s < steps; ++s) {
-        cp_wait<T::STAGES - 2>();
-        __syncthreads();                                         // step s is here, and everyone has read step s - 1
-        if (s + T::STAGES - 1 < steps) load(s + T::STAGES - 1);
-        cp_commit();
+    auto work = [&](int s) {
         const float* as = gt_smem + (s % T::STAGES) * T::STAGE + ty * 4;
         const float* ws = gt_smem + (s % T::STAGES) * T::STAGE + T::A_FLOATS + tx * T::W_ROW;
 #pragma unroll
@@ -315,6 +334,31 @@ gemm_tile_kernel(const TI* __restrict__ A, int lda, const TI* __restrict__ W, in
                     *p2 = add ? *p2 + v.y : v.y;
                     acc[i][j] = 0;
                 }
+        }
+    };
+    if constexpr (VEC) {
+#pragma unroll
+        for (int s = 0; s < T::STAGES - 1; ++s) {
+            if (s < steps) load(s);
+            cp_commit();
+        }
+        for (int s = 0; s < steps; ++s) {
+            cp_wait<T::STAGES - 2>();
+            __syncthreads();                                     // step s is here, and everyone has read step s - 1
+            if (s + T::STAGES - 1 < steps) load(s + T::STAGES - 1);
+            cp_commit();
+            work(s);
+        }
+    } else if (steps > 0) {
+        fetch(0);
+        lay(0);
+        for (int s0 = 0; s0 < steps; s0 += GROUP) {
+            __syncthreads();                                     // this group is here, and everyone has read the one before
+            const bool more = s0 + GROUP < steps;
+            if (more) fetch(s0 + GROUP);
+#pragma unroll 1
+            for (int s = s0; s < min(s0 + GROUP, steps); ++s) work(s);
+            if (more) lay(s0 + GROUP);
         }
     }
 

@@ -31,3 +31,19 @@ def test_outputs_do_not_depend_on_the_kernel(n, k):
             ops.gemm_simt(rows, w, out[:m])
             assert torch.equal(out[:m], whole[:m]), f"{m} rows"
             assert bool((out[m] == 5.0).all())
+
+
+# steps of 16 columns in groups of four (small tiles) or one by one (large ones): below a step, at and past a group and two groups
+@pytest.mark.parametrize("n,k", [(5, 3), (33, 16), (40, 60), (64, 64), (31, 66), (96, 172), (130, 1030), (40, 2051)])
+def test_bfloat16_operands_give_the_bits_of_their_float32_copies(n, k):
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(n * k)
+    a, w = torch.randn(4100, k, device=DEV, generator=g).bfloat16(), torch.randn(n, k, device=DEV, generator=g).bfloat16()
+    for m in (1, 9, 64, 65, 4100):                              # small tiles, and (130 features) large ones
+        want, got = torch.empty(m, n, device=DEV), torch.full((m + 1, n), 5.0, device=DEV)
+        ops.gemm_simt(a[:m].float(), w.float(), want)
+        ops.gemm_simt(a[:m], w, got[:m])
+        assert torch.equal(got[:m], want) and bool((got[m] == 5.0).all()), m
+        rounded = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+        ops.gemm_simt(a[:m], w, rounded)
+        assert torch.equal(rounded, want.bfloat16()), m
