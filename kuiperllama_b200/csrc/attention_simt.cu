@@ -13,11 +13,15 @@
 // round-robin, so the order of every sum depends only on the token's own position: the
 // result does not change with the way tokens are cut into steps or batched.
 //
+// attention_simt_kernel reads keys and values where they lie and hides the latency with many CTAs an SM and with loads in batches: 128
+// bytes of a key's row, then the values of eight keys, are on their way together (one load at a time made a chunk wait for every 16
+// bytes: one token of 300 keys, 32 heads of 64 on 8, 27.3 us, now 10.7; 64 such tokens 116, now 57).
+//
 // attention_simt_tile_kernel does the same for float32 rows without a window, chunks or distance bias (key and value sizes up to 128):
-// a warp copies its chunk of keys and values to shared memory first (a row per lane straight from L2 waits for every 16 bytes of
-// every row: 55 us for one token of 300 keys, now 15), and a CTA takes eight neighbouring rows of a prompt, which share the copies.
-// Every token's sums are the same operations in the same order as in the kernel above, so its result has the same bits.  One prompt of
-// 777 tokens, 32 heads of 64 on 8: 483 us, 1,066 with a CTA per token.
+// a warp copies its chunk of keys and values to shared memory first, as whole lines, and a CTA takes eight neighbouring rows of a
+// prompt, which share the copies (TQ = 8), or one row (TQ = 1).  Every token's sums are the same operations in the same order as in the
+// kernel above, so its result has the same bits.  Its shared memory leaves one to five CTAs an SM, so it runs only where that is
+// no loss (simt_rows_of_a_tile).  One prompt of 777 tokens, 32 heads of 64 on 8: 480 us, 757 with a CTA per token.
 //
 // Options beyond KuiperLLama's attention: values of another size than the keys (`vd` columns of rows
 // that are `v_ld` apart; with v_cache == k_cache and v_ld == hd the values are the leading columns of
@@ -52,7 +56,15 @@ template <>
 __device__ __forceinline__ float dot_row<float>(const float* __restrict__ k, const float* __restrict__ q, int hd) {
     if (hd & 3) return dot_row_scalar(k, q, hd);
     float s = 0.f;
-    for (int i = 0; i < hd; i += 4) {
+    int i = 0;
+    for (; i + 32 <= hd; i += 32) {                                  // 128 bytes of the row on their way at a time
+        float4 kv[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) kv[u] = *reinterpret_cast<const float4*>(k + i + 4 * u);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += dot4(kv[u], *reinterpret_cast<const float4*>(q + i + 4 * u));
+    }
+    for (; i < hd; i += 4) {
         const float4 kv = *reinterpret_cast<const float4*>(k + i);
         s += dot4(kv, *reinterpret_cast<const float4*>(q + i));
     }
@@ -129,7 +141,22 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
         for (int i = 0; i < PL; ++i) acc[i] *= corr;
         const int j_lo = max(lo - base, 0), j_hi = min(pos - base, 31);
         const T* vbase = v_cache + (((size_t)page * KV + g) * PAGE + (base % PAGE)) * (size_t)v_ld;
-        for (int j = j_lo; j <= j_hi; ++j) {
+        constexpr int U = PL <= 4 ? 8 : 32 / PL;                     // keys whose values are requested together
+        int j = j_lo;
+        for (; j + U - 1 <= j_hi; j += U) {
+            float v[U][PL];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int i = 0; i < PL; ++i) v[u][i] = lane + 32 * i < vd ? to_f32(vbase[(size_t)(j + u) * v_ld + lane + 32 * i]) : 0.f;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const float pj = __shfl_sync(0xffffffffu, p, j + u);
+#pragma unroll
+                for (int i = 0; i < PL; ++i) acc[i] = fmaf(pj, v[u][i], acc[i]);
+            }
+        }
+        for (; j <= j_hi; ++j) {
             const float pj = __shfl_sync(0xffffffffu, p, j);
             const T* vrow = vbase + (size_t)j * v_ld;
 #pragma unroll
@@ -306,11 +333,32 @@ attention_simt_tile_kernel(const float* __restrict__ q, int q_stride, float* __r
     }
 }
 
+static size_t simt_tile_smem(int TQ, int hd, int vd) {
+    return (size_t)(TQ * hd + 2 * ATT_WARPS * TQ + ATT_WARPS * TQ * vd + ATT_WARPS * 32 * (hd + vd + 8) + ATT_WARPS * TQ * 32) * sizeof(float);
+}
+
+// Rows of a tile: 8, 1, or 0 for the row kernel.  us with the row kernel / one row a tile / eight (heads on key heads, size of keys):
+//   eight, a prompt of many keys whose tiles give most SMs a CTA (fewer when heads are long):
+//     777 tokens, 32 on 8 of 64 757 / - / 480, of 128 1,409 / - / 1,009, 6 on 2 of 32 99 / - / 68; 64 tokens after 1,000, 32 on 8 of 64 168 / - / 98;
+//     but 16 tokens after 500 of 8 on 2 of 64 22 / - / 46, 8 prompts of 128 of 32 on 8 203 / - / 259, heads of 16 never
+//   one, where every CTA is resident at once and most SMs have two or more:
+//     8 tokens of 300 keys, 32 on 8 of 64 22 / 16 / -; 64 of 1,500 keys, 8 on 2 of 64 106 / 60 / -; 16 after 500, 12 on 4 of 96 46 / 31 / -;
+//     but one token of 300 keys, 32 on 8 of 64 10.7 / 13.3 / -, a prompt of five 4.0 / 5.6 / - (runs < 0: few keys), and 64 tokens of 20 keys
+//     10.4 / 30 / -
+static int simt_rows_of_a_tile(int n_tokens, int H, int hd, int vd, int runs) {
+    const int sms = sm_count();
+    if (hd < 32 || sms <= 0 || runs < 0) return 0;
+    const long long rows = (long long)n_tokens * H, tiles = (long long)(n_tokens + 7) / 8 * H;
+    if (runs > 0 && tiles >= (hd > 64 ? 64 : sms)) return 8;
+    const long long resident = (228 * 1024) / (long long)(simt_tile_smem(1, hd, vd) + 1024);       // CTAs that an SM's shared memory holds
+    return rows > sms && rows <= resident * sms ? 1 : 0;
+}
+
 template <int PL, int TQ>
 static int launch_simt_tiles(const float* q, int q_stride, float* out, const float* k_cache, const float* v_cache, const int* block_table,
                              int blocks_per_seq, const int* positions, const int* token_slot, int n_tokens, int H, int KV, int hd, float scale,
                              int vd, int v_ld, const float* sink, cudaStream_t stream) {
-    const size_t smem = (size_t)(TQ * hd + 2 * ATT_WARPS * TQ + ATT_WARPS * TQ * vd + ATT_WARPS * 32 * (hd + vd + 8) + ATT_WARPS * TQ * 32) * sizeof(float);
+    const size_t smem = simt_tile_smem(TQ, hd, vd);
     KL_CUDA(cudaFuncSetAttribute(attention_simt_tile_kernel<PL, TQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     launch_kernel(attention_simt_tile_kernel<PL, TQ>, dim3((n_tokens + TQ - 1) / TQ, H), ATT_WARPS * 32, smem, stream, q, q_stride, out, k_cache, v_cache,
                   block_table, blocks_per_seq, positions, token_slot, n_tokens, H, KV, hd, scale, vd, v_ld, sink);
@@ -324,7 +372,8 @@ using namespace kl;
 
 // q: rows of q_stride elements, head h at column h * hd.  out: [tokens, H * vd].  vd <= 0 means values like
 // keys (vd = v_ld = hd).  sink: float32 [H] or null.  chunk: positions per chunk (0: none).  rel: float32 [H, rel_n] or null.
-// runs: most rows follow the row before them in the same sequence (a prompt): tiles of eight of them.
+// runs: 1, most rows follow the row before them in the same sequence and read hundreds of keys (a long prompt); -1, no row reads more
+// than a few dozen keys; 0, unknown.  The results are the same.
 KL_API int kl_attention_simt(const void* q, int q_stride, void* out, const void* k_cache, const void* v_cache,
                              const int* block_table, int blocks_per_seq, const int* positions,
                              const int* token_slot, int n_tokens, int H, int KV, int hd, float scale, int window,
@@ -335,10 +384,15 @@ KL_API int kl_attention_simt(const void* q, int q_stride, void* out, const void*
     if (vd > ATT_MAX_VALUE_DIM || hd <= 0 || v_ld < vd || KV <= 0 || H % KV) return KL_ERR_BAD_SIZE;
     if (H > 65535 || chunk < 0 || (rel != nullptr && rel_n < 1)) return KL_ERR_BAD_SIZE;
     if (dtype == KL_F32 && window <= 0 && chunk == 0 && rel == nullptr && hd % 4 == 0 && vd % 4 == 0 && v_ld % 4 == 0 && hd <= 128 && vd <= 128 &&
-        ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0)
-        return (runs ? (vd <= 64 ? launch_simt_tiles<2, 8> : launch_simt_tiles<4, 8>) : (vd <= 64 ? launch_simt_tiles<2, 1> : launch_simt_tiles<4, 1>))(
-            (const float*)q, q_stride, (float*)out, (const float*)k_cache, (const float*)v_cache, block_table, blocks_per_seq, positions, token_slot,
-            n_tokens, H, KV, hd, scale, vd, v_ld, sink, stream);
+        ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0) {
+#define KL_TILES(PL, TQ)                                                                                                                   \
+    launch_simt_tiles<PL, TQ>((const float*)q, q_stride, (float*)out, (const float*)k_cache, (const float*)v_cache, block_table, blocks_per_seq, \
+                              positions, token_slot, n_tokens, H, KV, hd, scale, vd, v_ld, sink, stream)
+        const int tq = simt_rows_of_a_tile(n_tokens, H, hd, vd, runs);
+        if (tq == 8) return vd <= 64 ? KL_TILES(2, 8) : KL_TILES(4, 8);
+        if (tq == 1) return vd <= 64 ? KL_TILES(2, 1) : KL_TILES(4, 1);
+#undef KL_TILES
+    }
     const dim3 grid(n_tokens, H);
     const size_t smem = (size_t)(hd + 2 * ATT_WARPS + ATT_WARPS * vd) * sizeof(float);
     if (smem > 200 * 1024) return KL_ERR_BAD_SIZE;
@@ -349,9 +403,14 @@ KL_API int kl_attention_simt(const void* q, int q_stride, void* out, const void*
                       (const T*)k_cache, (const T*)v_cache, block_table, blocks_per_seq, positions, token_slot, H, KV, hd,    \
                       scale, window, vd, v_ld, sink, chunk, rel, rel_n);                                                                         \
     } while (0)
-    if (dtype == KL_F32) { if (vd <= 256) KL_ATT(float, 8); else KL_ATT(float, 16); }
-    else if (dtype == KL_BF16) { if (vd <= 256) KL_ATT(bf16, 8); else KL_ATT(bf16, 16); }
+#define KL_ATT_T(T)                                                                                                           \
+    do {                                                                                                                      \
+        if (vd <= 64) KL_ATT(T, 2); else if (vd <= 128) KL_ATT(T, 4); else if (vd <= 256) KL_ATT(T, 8); else KL_ATT(T, 16);   \
+    } while (0)
+    if (dtype == KL_F32) KL_ATT_T(float);
+    else if (dtype == KL_BF16) KL_ATT_T(bf16);
     else return KL_ERR_BAD_DTYPE;
+#undef KL_ATT_T
 #undef KL_ATT
     KL_LAUNCH_CHECK();
     return KL_OK;

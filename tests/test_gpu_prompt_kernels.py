@@ -264,6 +264,37 @@ def test_float32_attention_of_runs_has_the_same_bits(H, KV, hd, vd):
             assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2]) and bool(torch.isfinite(got[0]).all()) and bool((got[0][-3:] == 3.0).all())
 
 
+# rows x heads on both sides of what tiles of eight rows, tiles of one row and a CTA per row each take; rows of 32 columns read at a time
+# and a remainder; values in one to sixteen columns a lane
+@pytest.mark.parametrize("H,KV,hd,vd,starts,news", [(8, 2, 64, 64, [0, 200], [390, 56]), (4, 4, 128, 128, [0], [256]), (4, 1, 36, 32, [5, 0], [240, 250]),
+                                                    (32, 8, 64, 64, [250, 30, 63], [1, 1, 1]), (32, 8, 64, 64, [100] * 3, [4, 5, 6]), (40, 8, 100, 96, [90], [6]),
+                                                    (64, 1, 128, 64, [300, 20], [1, 2]), (16, 2, 32, 20, [0], [30])])
+def test_float32_attention_by_tiles_and_by_rows_has_the_same_bits(H, KV, hd, vd, starts, news):
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator().manual_seed(H + hd)
+    pages = 8
+    table = torch.randperm(len(news) * pages, generator=g).to(torch.int32).view(len(news), pages).to(DEV)
+    kc, vc = torch.randn(len(news) * pages, KV, 64, hd, generator=g).to(DEV), torch.randn(len(news) * pages, KV, 64, vd, generator=g).to(DEV)
+    pos = torch.tensor([a + t for a, n in zip(starts, news) for t in range(n)], dtype=torch.int32, device=DEV)
+    slot = torch.tensor([s for s, n in enumerate(news) for _ in range(n)], dtype=torch.int32, device=DEV)
+    q, got = torch.randn(len(pos), H * hd, generator=g).to(DEV), []
+    for runs, zeros in ((False, None), (True, None), (False, torch.zeros(H, 1, device=DEV))):
+        out = torch.full((len(pos), H * vd), 3.0, device=DEV)
+        ops.attention_simt(q, H * hd, out, kc, vc, table, pos, slot, len(pos), H, KV, hd, 0.2, value_dim=vd, distance_bias=zeros, runs=runs)
+        got.append(out)
+    assert torch.equal(got[0], got[2]) and torch.equal(got[1], got[2])
+    flat = lambda c, s: c[table[s].long()].permute(1, 0, 2, 3).reshape(KV, pages * 64, -1).double().repeat_interleave(H // KV, 0)
+    for s in range(len(news)):
+        mine = slot == s
+        sc = torch.einsum("thd,hjd->thj", q[mine].double().view(-1, H, hd), flat(kc, s)) * 0.2
+        sc = sc.masked_fill(torch.arange(pages * 64, device=DEV)[None, None] > pos[mine][:, None, None], float("-inf"))
+        w, v = torch.softmax(sc, -1), flat(vc, s)
+        want, most = torch.einsum("thj,hjd->thd", w, v), torch.einsum("thj,hjd->thd", w, v.abs())
+        # a score is off by hd roundings of its largest partial sum, which the exponential passes on; the sums by one rounding a key
+        score = 0.2 * torch.einsum("thd,hjd->thj", q[mine].double().abs().view(-1, H, hd), flat(kc, s).abs()).amax()
+        assert bool(((got[0][mine].double().view(want.shape) - want).abs() <= (2 * (hd + 4) * score + 512 + 32) * U * most).all())
+
+
 @pytest.mark.parametrize("H,G,d,dv", [(4, 2, 16, 24), (2, 1, 32, 8), (4, 4, 64, 48), (2, 1, 100, 36), (3, 1, 256, 20)])
 def test_delta_rule_has_the_same_bits_however_a_prompt_is_cut(H, G, d, dv):
     """Whole tiles of eight tokens and tokens one by one, over every number of lanes a column is cut into."""
