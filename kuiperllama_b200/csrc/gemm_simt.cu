@@ -406,10 +406,12 @@ int tiles(const TI* A, int lda, const TI* W, int ldw, TO* C, int ldc, int M, int
     const int sms = sm_count() > 0 ? sm_count() : 1, nb = (K + BLOCK - 1) / BLOCK;
     const long long big = (long long)((N + Big::BN - 1) / Big::BN) * ((M + Big::BM - 1) / Big::BM);
     // Where the tiles do not fill the device four times, the blocks of K are dealt to a cluster (at most two a CTA: a block's sums take 32 KB).
+    // Where they do, a CTA keeps one running sum (77 KB, three CTAs an SM instead of two, and no sums to exchange): us with a cluster / without,
+    // 777 x 16,384 x 2,048 1,367 / 1,257, 777 x 28,672 x 4,096 4,759 / 4,117, 777 x 9,000 x 1,100 804 / 410.
     int ranks = 1;
-    if (nb <= 16)
+    if (nb <= 16 && big < 4LL * sms)
         while (ranks < 8 && ranks < nb && (big * ranks < 4LL * sms || (nb + ranks - 1) / ranks > 2)) ranks *= 2;
-    if ((nb + ranks - 1) / ranks > 2) ranks = 1;
+    if (ranks > 1 && (nb + ranks - 1) / ranks > 2) ranks = 1;
     if (2 * big * ranks >= 3LL * sms)
         return launch_tiles<TI, TO, VEC, 8, 8, 16>(A, lda, W, ldw, C, ldc, M, N, K, ranks, stream);
     return launch_tiles<TI, TO, VEC, 4, 4, 8>(A, lda, W, ldw, C, ldc, M, N, K, ranks, stream);
