@@ -17,8 +17,8 @@
 //       lanes' sums are added by shuffles.  Tokens are walked in order from the slot's state, so a result does not
 //       depend on how a prompt was cut.
 //   outer_recurrence_slab_kernel<TI, R, L, MODE>   the form that runs where the sizes allow: R x 2 of S per thread (see there).
-//   outer_recurrence_single_kernel<TI, CL>   a step of single tokens, bound by reading and writing S once: neighbouring lanes hold
-//       neighbouring columns of a row, eight rows a thread on their way at a time.
+//   outer_recurrence_few_kernel<TI, V, CL, T>   a step of at most eight tokens a sequence, bound by reading and writing S once:
+//       neighbouring lanes hold neighbouring columns of a row, four or eight rows a thread on their way at a time.
 //   decay_softplus_kernel     dt = softplus(raw + bias), a = exp(-exp(A_log) dt) per (token, head), 32-bit.
 //   decay_lowrank_kernel      a = sigmoid(z)^(1 / tau) = exp(-softplus(-z) / tau), z = W2 r + b with r a short row per
 //                             token (the first of two projections, made with the mixer's other projections), 32-bit.
@@ -440,80 +440,124 @@ outer_recurrence_slab_kernel(const OuterArgs A) {
     }
 }
 
-// One token per sequence.  A CTA takes 4 CL columns of S of one (sequence, head); CL lanes hold four columns each and
-// OS_THREADS / CL groups of lanes share the rows.
-constexpr int OS_THREADS = 256;
-template <typename TI, int CL>
+// At most T tokens per sequence (a step of single tokens: T = 1).  A CTA takes V CL columns of S of one (sequence, head); CL lanes hold
+// V = 4 or 2 columns each and OS_THREADS / CL groups of lanes share the rows.  A row of S is read once, takes its tokens in order and is
+// written once.  The slab form reads a column pair per lane, rows apart: 64 sequences of 2 tokens, us with slabs / here, 64 heads of
+// 128 x 64 111 / 65, 8 heads of 256 x 256 with the normaliser 172 / 56; of 8 tokens 131 / 115 and 210 / 103.
+constexpr int OS_THREADS = 256, OS_TOKENS = 8;
+template <int V> struct OsCols;
+template <> struct OsCols<4> { typedef float4 type; };
+template <> struct OsCols<2> { typedef float2 type; };
+template <typename TI, int V, int CL, int T>
 __global__ void __launch_bounds__(OS_THREADS)
-outer_recurrence_single_kernel(const OuterArgs A) {
+outer_recurrence_few_kernel(const OuterArgs A) {
     pdl_launch_dependents();
     pdl_wait();
-    constexpr int RG = OS_THREADS / CL, U = 8;
+    constexpr int RG = OS_THREADS / CL, U = T <= 2 ? 8 : 4;
+    constexpr int PG = T > 1 && CL == 16 ? RG / 2 : RG;        // groups whose sums meet in shared memory (a warp's two add theirs first)
     extern __shared__ __align__(16) float sm[];
     __shared__ float scratch[33];
     const int s = blockIdx.z, h = blockIdx.y, N = A.N, P = A.P;
-    if (A.cu_tokens[s + 1] <= A.cu_tokens[s]) return;
-    const size_t row = (size_t)A.cu_tokens[s];
+    const size_t row0 = (size_t)A.cu_tokens[s];
+    const int nt = T == 1 ? min(1, A.cu_tokens[s + 1] - A.cu_tokens[s]) : min(T, A.cu_tokens[s + 1] - A.cu_tokens[s]);
+    if (nt <= 0) return;
     const int g = h / (A.heads / A.groups);
-    float* kk = sm;                                            // [N] times c
-    float* qq = kk + N;                                        // [N] times q_scale
-    float* aa = qq + N;                                        // [N]
-    float* part = aa + N;                                      // [RG][4 CL]; N is a multiple of 4
+    float4* kqa = reinterpret_cast<float4*>(sm);               // [T][N]: k times c, q times q_scale, a
+    float* part = sm + 4 * T * N;                              // [PG][T][V CL]
     const int cl = threadIdx.x % CL, rg = threadIdx.x / CL;
-    const int col = (blockIdx.x * CL + cl) * 4;
-    const bool live = col < P;                                 // P is a multiple of 4
+    const int col = (blockIdx.x * CL + cl) * V;
+    const bool live = col < P;                                 // P is a multiple of V
+    typedef typename OsCols<V>::type Cols;
     float* S = A.state + (size_t)A.seq_slots[s] * A.ld_state + (size_t)h * N * P + col;
-    const float c = A.c != nullptr ? A.c[row * A.ld_c + h] : 1.f;
-    for (int n = threadIdx.x; n < N; n += OS_THREADS) {
-        kk[n] = to_f32(((const TI*)A.k)[row * A.ld_k + A.k_col + (size_t)g * N + n]) * c;
-        qq[n] = to_f32(((const TI*)A.q)[row * A.ld_q + A.q_col + (size_t)g * N + n]) * A.q_scale;
-        aa[n] = A.a_per_row ? A.a[row * A.ld_a + (size_t)h * N + n] : A.a[row * A.ld_a + h];
+    for (int idx = threadIdx.x; idx < nt * N; idx += OS_THREADS) {
+        const int t = T == 1 ? 0 : idx / N, n = idx - t * N;
+        const size_t row = row0 + t;
+        kqa[idx] = make_float4(to_f32(((const TI*)A.k)[row * A.ld_k + A.k_col + (size_t)g * N + n]) * (A.c != nullptr ? A.c[row * A.ld_c + h] : 1.f),
+                               to_f32(((const TI*)A.q)[row * A.ld_q + A.q_col + (size_t)g * N + n]) * A.q_scale,
+                               A.a_per_row ? A.a[row * A.ld_a + (size_t)h * N + n] : A.a[row * A.ld_a + h], 0.f);
     }
-    float v[4] = {0.f, 0.f, 0.f, 0.f}, acc[4] = {0.f, 0.f, 0.f, 0.f};
-    if (live) {
+    float v[T][V], acc[T][V];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = to_f32(((const TI*)A.v)[row * A.ld_v + A.v_col + (size_t)h * P + col + j]);
-    }
+    for (int t = 0; t < T; ++t)
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            v[t][j] = live && t < nt ? to_f32(((const TI*)A.v)[(row0 + t) * A.ld_v + A.v_col + (size_t)h * P + col + j]) : 0.f;
+            acc[t][j] = 0.f;
+        }
     __syncthreads();
     for (int n0 = rg; n0 < N && live; n0 += RG * U) {
-        float4 x[U];
+        float x[U][V];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int n = n0 + u * RG;
-            x[u] = n < N ? *reinterpret_cast<const float4*>(S + (size_t)n * P) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const Cols w = n < N ? *reinterpret_cast<const Cols*>(S + (size_t)n * P) : Cols{};
+#pragma unroll
+            for (int j = 0; j < V; ++j) x[u][j] = reinterpret_cast<const float*>(&w)[j];
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int n = n0 + u * RG;
             if (n >= N) break;
-            const float kn = kk[n], qn = qq[n], an = aa[n];
-            x[u].x = fmaf(an, x[u].x, kn * v[0]); x[u].y = fmaf(an, x[u].y, kn * v[1]);
-            x[u].z = fmaf(an, x[u].z, kn * v[2]); x[u].w = fmaf(an, x[u].w, kn * v[3]);
-            acc[0] = fmaf(x[u].x, qn, acc[0]); acc[1] = fmaf(x[u].y, qn, acc[1]);
-            acc[2] = fmaf(x[u].z, qn, acc[2]); acc[3] = fmaf(x[u].w, qn, acc[3]);
-            *reinterpret_cast<float4*>(S + (size_t)n * P) = x[u];
+#pragma unroll
+            for (int t = 0; t < T; ++t) {
+                if (T > 1 && t >= nt) break;
+                const float4 w = kqa[t * N + n];
+#pragma unroll
+                for (int j = 0; j < V; ++j) {
+                    x[u][j] = fmaf(w.z, x[u][j], w.x * v[t][j]);
+                    acc[t][j] = fmaf(x[u][j], w.y, acc[t][j]);
+                }
+            }
+            Cols w;
+#pragma unroll
+            for (int j = 0; j < V; ++j) reinterpret_cast<float*>(&w)[j] = x[u][j];
+            *reinterpret_cast<Cols*>(S + (size_t)n * P) = w;
         }
     }
-    *reinterpret_cast<float4*>(part + (size_t)rg * 4 * CL + 4 * cl) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        if constexpr (PG < RG) {
+#pragma unroll
+            for (int j = 0; j < V; ++j) acc[t][j] += __shfl_xor_sync(0xffffffffu, acc[t][j], 16);
+        }
+        if (PG == RG || rg % 2 == 0) {
+#pragma unroll
+            for (int j = 0; j < V; ++j) part[(size_t)((PG < RG ? rg / 2 : rg) * T + t) * V * CL + V * cl + j] = acc[t][j];
+        }
+    }
     __syncthreads();
-    if (threadIdx.x < 4 * CL && blockIdx.x * 4 * CL + threadIdx.x < P) {
-        const int at = blockIdx.x * 4 * CL + threadIdx.x;
+    for (int e = threadIdx.x; e < nt * V * CL; e += OS_THREADS) {
+        const int t = e / (V * CL), at = blockIdx.x * V * CL + e % (V * CL);
+        if (at >= P) continue;
         float y = 0.f;
 #pragma unroll
-        for (int r = 0; r < RG; ++r) y += part[r * 4 * CL + threadIdx.x];
+        for (int r = 0; r < PG; ++r) y += part[(size_t)(r * T) * V * CL + e];
+        const size_t row = row0 + t;
         if (A.skip != nullptr) y = fmaf(A.skip[h], to_f32(((const TI*)A.v)[row * A.ld_v + A.v_col + (size_t)h * P + at]), y);
         A.y[row * A.ld_y + (size_t)h * P + at] = y;
     }
     if (A.norm_state != nullptr && blockIdx.x == 0) {          // the normaliser: the first columns' CTA
         float* z = A.norm_state + (size_t)A.seq_slots[s] * A.ld_state + (size_t)h * N;
-        float dot = 0.f;
+        float dot[T];
+#pragma unroll
+        for (int t = 0; t < T; ++t) dot[t] = 0.f;
         for (int n = threadIdx.x; n < N; n += OS_THREADS) {
-            const float x = fmaf(aa[n], z[n], kk[n]);
+            float x = z[n];
+#pragma unroll
+            for (int t = 0; t < T; ++t) {
+                if (t >= nt) break;
+                const float4 w = kqa[t * N + n];
+                x = fmaf(w.z, x, w.x);
+                dot[t] = fmaf(x, w.y, dot[t]);
+            }
             z[n] = x;
-            dot = fmaf(x, qq[n], dot);
         }
-        dot = block_sum(dot, scratch);
-        if (threadIdx.x == 0) A.den[row * A.heads + h] = or_den(A, row, h, dot);
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            if (t >= nt) break;
+            const float d = block_sum(dot[t], scratch);
+            if (threadIdx.x == 0) A.den[(row0 + t) * A.heads + h] = or_den(A, row0 + t, h, d);
+        }
     }
 }
 
@@ -613,21 +657,37 @@ KL_API int kl_outer_recurrence(const void* q, long long ld_q, int q_col, const v
     A.a_per_row = a_per_row ? 1 : 0; A.q_scale = q_scale;
     A.norm_state = norm_state; A.floor = floor; A.den = den; A.den_eps = den_eps;
     A.vec_state = ((uintptr_t)state % 16 == 0 && ld_state % 4 == 0 && P % 4 == 0) ? 1 : 0;
-    // single tokens: S read and written once
-    if (max_new == 1 && A.vec_state && N % 4 == 0 && N <= 1024) {
+    // a few tokens: S read and written once
+    // (by slabs all the same: several tokens of narrow S, of which few lanes would have columns, 64 sequences of 4 heads of 16 x 8 by two 3.1 / 2.6
+    // us; of few CTAs, one sequence of 4 heads of 500 x 64 by two 7.3 / 5.2; five and more tokens of small S, whose reading is not what takes
+    // the time, 64 sequences of 32 heads of 64 x 64 by eight 32 / 28)
+    const int vec = A.vec_state ? 4 : (uintptr_t)state % 8 == 0 && ld_state % 2 == 0 && P % 2 == 0 && P >= 16 ? 2 : 0;     // columns to a lane
+    if (max_new <= OS_TOKENS && vec != 0 &&
+        (max_new <= 1 || (P >= 8 * vec && (long long)((P + 63) / 64) * heads * n_seqs >= 16 && (max_new <= 4 || N * P > 4096)))) {
         // 64 columns a CTA where S has no more (128 leave half of the threads idle: 64 sequences of 64 heads of 128 x 64, 268 MB, 78 us
         // against 53) or where CTAs are few
         const bool narrow = P <= 64 || (long long)((P + 127) / 128) * heads * n_seqs < 2LL * sms;
-        const int cols = narrow ? 64 : 128;
+        const int cols = vec == 2 ? 32 : narrow ? 64 : 128, T = max_new <= 1 && vec == 4 ? 1 : max_new <= 2 ? 2 : max_new <= 4 ? 4 : 8;
         const dim3 grid((P + cols - 1) / cols, heads, n_seqs);
-        const size_t smem = (size_t)(3 * N + 4 * OS_THREADS) * sizeof(float);
-        if (in_dtype == KL_F32) {
-            if (narrow) launch_kernel(outer_recurrence_single_kernel<float, 16>, grid, OS_THREADS, smem, stream, A);
-            else launch_kernel(outer_recurrence_single_kernel<float, 32>, grid, OS_THREADS, smem, stream, A);
-        } else {
-            if (narrow) launch_kernel(outer_recurrence_single_kernel<bf16, 16>, grid, OS_THREADS, smem, stream, A);
-            else launch_kernel(outer_recurrence_single_kernel<bf16, 32>, grid, OS_THREADS, smem, stream, A);
-        }
+        const size_t smem = (size_t)T * (4 * N + vec * OS_THREADS) * sizeof(float);
+#define KL_FEW(TI, V, CL, T_)                                                                                        \
+    do {                                                                                                            \
+        if (smem > 47 * 1024)                                                                                       \
+            KL_CUDA(cudaFuncSetAttribute(outer_recurrence_few_kernel<TI, V, CL, T_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        launch_kernel(outer_recurrence_few_kernel<TI, V, CL, T_>, grid, OS_THREADS, smem, stream, A);               \
+    } while (0)
+#define KL_FEW_T(TI, V, CL)                                                                                          \
+    do {                                                                                                            \
+        if (V == 4 && T == 1) KL_FEW(TI, 4, CL, 1); else if (T == 2) KL_FEW(TI, V, CL, 2); else if (T == 4) KL_FEW(TI, V, CL, 4); else KL_FEW(TI, V, CL, 8); \
+    } while (0)
+#define KL_FEW_V(TI)                                                                                                 \
+    do {                                                                                                            \
+        if (vec == 2) KL_FEW_T(TI, 2, 16); else if (narrow) KL_FEW_T(TI, 4, 16); else KL_FEW_T(TI, 4, 32);          \
+    } while (0)
+        if (in_dtype == KL_F32) KL_FEW_V(float); else KL_FEW_V(bf16);
+#undef KL_FEW_V
+#undef KL_FEW_T
+#undef KL_FEW
         KL_LAUNCH_CHECK();
         return KL_OK;
     }

@@ -54,6 +54,17 @@ def test_recurrence_of_few_columns_over_all_lanes(heads, groups, n, p, form, dty
     _check_recurrence(heads, groups, n, p, form, dtype, news)
 
 
+# at most one, two, four and eight tokens a sequence: columns of S in fours and in twos (S read and written once) and what goes by slabs; a
+# remainder of a CTA's columns, one and several CTAs of columns, more rows than a round of a CTA's threads
+@pytest.mark.parametrize("heads,groups,n,p", [(2, 1, 4, 4), (3, 3, 64, 68), (2, 2, 128, 132), (40, 8, 20, 200), (1, 1, 1000, 12), (2, 1, 130, 8), (2, 1, 24, 10),
+                                               (8, 1, 32, 30), (4, 2, 21, 50), (6, 3, 64, 130), (16, 16, 7, 18), (40, 8, 90, 66)])
+@pytest.mark.parametrize("form", ["head", "row", "normaliser"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_recurrence_of_a_few_tokens(heads, groups, n, p, form, dtype):
+    for news in ([1, 1, 1, 1], [2, 1, 2, 2], [4, 3, 1, 4], [8, 5, 7, 8]):
+        _check_recurrence(heads, groups, n, p, form, dtype, news)
+
+
 def _check_recurrence(heads, groups, n, p, form, dtype, news):
     from kuiperllama_b200.csrc import ops
     step = _step([0] * len(news), news)
