@@ -45,7 +45,7 @@ struct OuterArgs {
     int heads, groups, N, P, L, a_per_row;
     int tile;                                        // tokens per shared-memory tile (the lane form; OR_TILE unless the rows are long)
     int vec_state;                                   // every row piece of four columns of S is 16-byte aligned
-    int vec_in;                                      // k, q and a can be read four elements at a time
+    int piece;                                       // elements of k, q and v to an asynchronous copy: four, what four bytes hold, or 0 (one by one)
     float q_scale;
     float* norm_state;                               // the slot's n at norm_state + slot * ld_state, [heads, N], or null
     const float* floor;                              // [rows, heads]
@@ -282,23 +282,41 @@ outer_recurrence_slab_kernel(const OuterArgs A) {
                 const float* src = A.a + row * A.ld_a + (size_t)h * N + c;
                 for (int tt = 0; tt < T; ++tt, to += tok, src += A.ld_a) {
                     if (tt >= nt) *reinterpret_cast<float4*>(to) = make_float4(1.f, 1.f, 1.f, 1.f);      // a token past the end leaves S as it is
-                    else if (A.vec_in) or_copy<16>(to, n > 0 ? src : A.a, n > 0);
+                    else if (A.piece == 4) or_copy<16>(to, n > 0 ? src : A.a, n > 0);
                     else
-                        for (int u = 0; u < 4; ++u) reinterpret_cast<float*>(to)[u] = u < n ? src[u] : 0.f;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) or_copy<4>(to + 4 * u, u < n ? src + u : A.a, u < n);
                 }
                 continue;
             }
             const TI* base = (const TI*)(which == 0 ? A.k : which == 1 ? A.q : A.v);
             const long long ld = which == 0 ? A.ld_k : which == 1 ? A.ld_q : A.ld_v;
             const TI* src = base + row * ld + (which == 0 ? A.k_col + (size_t)g * N : which == 1 ? A.q_col + (size_t)g * N : A.v_col + (size_t)h * P) + c;
-            if (A.vec_in) {                                                        // N and P are multiples of four
+            if (A.piece == 4) {                                                    // N and P are multiples of four
                 for (int tt = 0; tt < T; ++tt, to += tok, src += ld) {
                     const bool in = n > 0 && tt < nt;
                     or_copy<4 * ES>(to, in ? src : base, in);
                 }
-            } else {
+            } else if (A.piece > 0) {                                              // of what four bytes hold
+                constexpr int W = 4 / ES;
                 for (int tt = 0; tt < T; ++tt, to += tok, src += ld)
-                    for (int u = 0; u < 4; ++u) reinterpret_cast<TI*>(to)[u] = tt < nt && u < n ? src[u] : from_f32<TI>(0.f);
+#pragma unroll
+                    for (int u = 0; u < 4; u += W) {
+                        const bool in = tt < nt && u < n;
+                        or_copy<4>(to + u * ES, in ? src + u : base, in);
+                    }
+            } else {
+                for (int t4 = 0; t4 < T; t4 += 4) {                                // T is a multiple of four: sixteen loads on their way together
+                    TI x[4][4];
+#pragma unroll
+                    for (int tt = 0; tt < 4; ++tt)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) x[tt][u] = t4 + tt < nt && u < n ? src[(t4 + tt) * ld + u] : from_f32<TI>(0.f);
+#pragma unroll
+                    for (int tt = 0; tt < 4; ++tt)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) reinterpret_cast<TI*>(to + (t4 + tt) * tok)[u] = x[tt][u];
+                }
             }
         }
         for (int t = threadIdx.x; t < 2 * T; t += threads) {
@@ -712,9 +730,13 @@ KL_API int kl_outer_recurrence(const void* q, long long ld_q, int q_col, const v
         threads = threads > OSL_THREADS ? OSL_THREADS : threads;
         while (threads % (2 * fewest) == 0 && (long long)((pairs * L + threads - 1) / threads) * heads * n_seqs < sms) threads >>= 1;
         const int cols = threads / L * 2, Np = R * L, tok = (2 * Np * es + (mode == 1 ? Np * 4 : 0) + cols * es + 15) / 16 * 16;
-        auto quad = [&](const void* p, long long ld, int col) { return (uintptr_t)p % (4 * es) == 0 && ld % 4 == 0 && col % 4 == 0; };
-        A.vec_in = (N % 4 == 0 && P % 4 == 0 && quad(q, ld_q, q_col) && quad(k, ld_k, k_col) && quad(v, ld_v, v_col) &&
-                    (!a_per_row || ((uintptr_t)a % 16 == 0 && ld_a % 4 == 0))) ? 1 : 0;
+        // the widest asynchronous copies that every row of k, q and v (and a) allows (8 heads of 20 x 50, bfloat16, 512 tokens: 213 us copied
+        // element by element, 133 in pairs)
+        auto whole = [&](int w) {
+            auto rows = [&](const void* p, long long ld, int col) { return (uintptr_t)p % (w * es) == 0 && ld % w == 0 && col % w == 0; };
+            return N % w == 0 && P % w == 0 && rows(q, ld_q, q_col) && rows(k, ld_k, k_col) && rows(v, ld_v, v_col);
+        };
+        A.piece = whole(4) && (!a_per_row || ((uintptr_t)a % 16 == 0 && ld_a % 4 == 0)) ? 4 : whole(4 / es) ? 4 / es : 0;
         A.tile = max_new <= 4 ? 4 : max_new <= 8 || Np > 256 ? 8 : 16;       // (a prompt of long rows of S: 8)
         A.L = L;
         const size_t smem = (size_t)2 * ((A.tile * tok + 2 * A.tile * 4 + 15) / 16 * 16);
@@ -754,7 +776,7 @@ KL_API int kl_outer_recurrence(const void* q, long long ld_q, int q_col, const v
     long long warps = (long long)n_seqs * heads * P * L / 32;
     while (L < 32 && (N + L - 1) / L > 2 && warps < 24LL * sms) { L <<= 1; warps <<= 1; }
     const int npt = (N + L - 1) / L;
-    A.L = L; A.vec_in = 0;
+    A.L = L;
     // the largest CTA that still leaves two CTAs per SM (a CTA loads a tile of tokens, waits, and computes: another one
     // fills the wait), and no wider than the columns of S
     int threads = OR_THREADS;
