@@ -625,8 +625,9 @@ KL_API int kl_head_rmsnorm_gate(const float* x, const void* gate, long long gate
 #define KL_HR(T, TH)                                                                                                                     \
     launch_kernel(head_rmsnorm_gate_row_kernel<T, TH>, (int)items, TH, 0, stream, x, (const T*)gate, gate_ld, w, (T*)out, out_ld, out_scale, \
                   heads, dim, eps, gate_first, wide_weight, divisor, sigmoid)
-            if (dtype == KL_F32) { if (dim <= 4096) KL_HR(float, 256); else KL_HR(float, 512); }
-            else { if (dim <= 4096) KL_HR(bf16, 256); else KL_HR(bf16, 512); }
+            // threads of at most 16 elements, and not many with none: 2,048 heads of 1,028 13.2 us with 256 threads, 7.6 with 128 (two passes 11.6)
+            if (dtype == KL_F32) { if (dim <= 2048) KL_HR(float, 128); else if (dim <= 4096) KL_HR(float, 256); else KL_HR(float, 512); }
+            else { if (dim <= 2048) KL_HR(bf16, 128); else if (dim <= 4096) KL_HR(bf16, 256); else KL_HR(bf16, 512); }
 #undef KL_HR
             KL_LAUNCH_CHECK();
             return KL_OK;
