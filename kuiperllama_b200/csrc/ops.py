@@ -1571,8 +1571,12 @@ def gemm_skinny_stream(w: torch.Tensor, a: torch.Tensor, row_scale=None, sink=No
 #   32 tokens:  3,072 x 2,048 8.3 / 7.0, 1,024 x 4,096 14.1 / 7.7
 # (``tokens_first``: the lines of K where tokens as rows win while their tiles run at once.)  The gate/up product cannot cut
 # its K range (its epilogue needs whole sums):
-#   16,384 x 2,048: 16 tokens 18.1 / 14.5, 32 tokens 14.0 / 16.5, 64 tokens 14.1 / 21.4
-#   8,192 x 1,024:  16 tokens 8.2 / 7.8, 32 tokens 8.0 / 9.8, 128 tokens 7.2 / 23.5
+#   16,384 x 2,048: 16 tokens 17.8 / 14.3, 17 19.2 / 15.1, 31 17.1 / 16.3, 32 13.5 / 16.3, 64 14.1 / 21.4
+#   8,192 x 2,048:  17 tokens 13.5 / 11.3, 31 14.0 / 12.4, 32 9.8 / 12.5
+#   8,192 x 4,096:  8 tokens 25.3 / 15.8, 16 16.7 / 16.6, 17 16.8 / 17.3
+#   8,192 x 1,024:  17 tokens 8.0 / 8.2, 32 7.7 / 9.5, 128 7.2 / 23.5; 16,384 x 1,024: 17 10.5 / 10.2, 31 10.2 / 11.3
+# (tokens as rows are slow while the tokens' own rows hold less than 64K elements, 128 KB, that all CTAs fetch at the same time, the more
+# so the more CTAs there are; the line is measured, its cause in the memory system is not known)
 #   28,672 x 4,096: 16 tokens 41.1 / 39.4, 32 tokens 41.5 / 41.0, 48 tokens 41.8 / 45.7 (more tiles than SMs)
 # The pieces of a cut product that its consumer adds itself (``gemm_skinny_partials``) stay 32-bit numbers: there weights as
 # rows run up to the number of tokens at which the tiles of 128 x 256 reach 0.6 of the SMs.
@@ -1587,9 +1591,9 @@ def one_wave(M: int, N: int) -> bool:
     return ((M + 127) // 128) * ((N + 127) // 128) <= sm_count()
 
 
-def weights_as_rows(M: int, N: int, swiglu: bool = False) -> bool:
+def weights_as_rows(M: int, N: int, swiglu: bool = False, K: Optional[int] = None) -> bool:
     if swiglu:
-        return M <= 16 or (M <= SWIGLU_WEIGHT_ROWS_MAX and not one_wave(M, N))
+        return M <= 16 or (M <= SWIGLU_WEIGHT_ROWS_MAX and (not one_wave(M, N) or (K is not None and N >= 8192 and K >= 1536 and M * K < 65536)))
     if M <= 64:
         return True
     if M > SKINNY_MAX_ROWS:
@@ -1802,7 +1806,7 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 
 def matmul_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, activation="silu") -> None:
     """out[M, I] = act(a @ gate^T) * (a @ up^T) in one kernel; ``w_gate_up`` from ``interleave_gate_up``."""
-    if weights_as_rows(a.shape[0], w_gate_up.shape[0], swiglu=True):
+    if weights_as_rows(a.shape[0], w_gate_up.shape[0], swiglu=True, K=w_gate_up.shape[1]):
         gemm_skinny(a, w_gate_up, out, swiglu=True, activation=activation)
     else:
         gemm_tcgen05(a, w_gate_up, out, swiglu=True, activation=activation)

@@ -357,7 +357,7 @@ def test_tiles_of_128_features_give_the_sums_of_the_larger_tiles(M, N, K, f32_ou
 
 
 @pytest.mark.parametrize("M", [16, 17, 32, 33, 128, 129, 512, 513])
-@pytest.mark.parametrize("N,K", [(256, 2048), (256, 2056), (2048, 4096), (1280, 4104), (19072, 256)])
+@pytest.mark.parametrize("N,K", [(256, 2048), (256, 2056), (2048, 4096), (1280, 4104), (19072, 256), (8192, 2048)])
 def test_products_on_both_sides_of_the_lines_between_the_ways_round(M, N, K):
     from kuiperllama_b200.csrc import ops
     a, w = _rand(M, K, seed=M), _rand(N, K, seed=K)
