@@ -341,17 +341,18 @@ static size_t simt_tile_smem(int TQ, int hd, int vd) {
 //   eight, a prompt of many keys whose tiles give most SMs a CTA (fewer when heads are long):
 //     777 tokens, 32 on 8 of 64 757 / - / 480, of 128 1,409 / - / 1,009, 6 on 2 of 32 99 / - / 68; 64 tokens after 1,000, 32 on 8 of 64 168 / - / 98;
 //     but 16 tokens after 500 of 8 on 2 of 64 22 / - / 46, 8 prompts of 128 of 32 on 8 203 / - / 259, heads of 16 never
-//   one, where every CTA is resident at once and most SMs have two or more:
+//   one, where every CTA is resident at once: a decode step finds its keys in memory, not in a cache, and a tile has a chunk's keys and values
+//   on their way together, the row kernel one batch after another (a step of one sequence of 300 keys through two layers of width 2,048:
+//   191 us by rows, 182 by tiles):
 //     8 tokens of 300 keys, 32 on 8 of 64 22 / 16 / -; 64 of 1,500 keys, 8 on 2 of 64 106 / 60 / -; 16 after 500, 12 on 4 of 96 46 / 31 / -;
-//     but one token of 300 keys, 32 on 8 of 64 10.7 / 13.3 / -, a prompt of five 4.0 / 5.6 / - (runs < 0: few keys), and 64 tokens of 20 keys
-//     10.4 / 30 / -
+//     but a prompt of five, 32 on 8 of 64 4.0 / 5.6 / - (runs < 0: few keys), and, with more CTAs, 64 tokens of 20 keys 10.4 / 30 / -
 static int simt_rows_of_a_tile(int n_tokens, int H, int hd, int vd, int runs) {
     const int sms = sm_count();
-    if (hd < 32 || sms <= 0 || runs < 0) return 0;
+    if (sms <= 0 || runs < 0) return 0;
     const long long rows = (long long)n_tokens * H, tiles = (long long)(n_tokens + 7) / 8 * H;
-    if (runs > 0 && tiles >= (hd > 64 ? 64 : sms)) return 8;
+    if (runs > 0 && hd >= 32 && tiles >= (hd > 64 ? 64 : sms)) return 8;
     const long long resident = (228 * 1024) / (long long)(simt_tile_smem(1, hd, vd) + 1024);       // CTAs that an SM's shared memory holds
-    return rows > sms && rows <= resident * sms ? 1 : 0;
+    return rows <= resident * sms ? 1 : 0;
 }
 
 template <int PL, int TQ>
