@@ -75,7 +75,8 @@ struct Rows {
 
 // Warp w of a CTA: rows 8 * (w / wb) .. of an item's 8 * (4 / wb), spans of four blocks w % wb, + wb, ...; lane = row + 8 * block.
 // Items (sets of rows) blockIdx.x, + gridDim.x, ...
-template <int MT>
+// FULL: the last span's first block is a whole one, so that every span has the same number of chunks.
+template <int MT, bool FULL>
 __global__ void __launch_bounds__(GR_WARPS * 32)
 gemm_rows_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C, int ldc,
                  int M, int N, int K, int wb) {
@@ -89,8 +90,8 @@ gemm_rows_kernel(const float* __restrict__ A, int lda, const float* __restrict__
     const int nb = (K + BLOCK - 1) / BLOCK, spans = (nb + GR_LANES - 1) / GR_LANES;
     const int mine = first < spans ? (spans - 1 - first) / wb + 1 : 0;        // spans of this warp
     // chunks of a span: the last one stops where its first block does (64 columns of 64 in one chunk: 2 us, 15 with all eight or sixteen)
-    const int last_parts = min(R::PER, (K - (spans - 1) * GR_SPAN + R::CHUNK - 1) / R::CHUNK);
-    auto parts = [&](int span) { return span == spans - 1 ? last_parts : R::PER; };
+    const int last_parts = FULL ? R::PER : min(R::PER, (K - (spans - 1) * GR_SPAN + R::CHUNK - 1) / R::CHUNK);
+    auto parts = [&](int span) { return FULL || span < spans - 1 ? R::PER : last_parts; };
     float* ring = gr_smem + warp * GR_STAGES * R::STAGE;
     float* sums = gr_smem + GR_WARPS * GR_STAGES * R::STAGE;                  // two of [blocks][MT][rows_item]
     const int sums_floats = spans * GR_LANES * MT * rows_item;
@@ -423,9 +424,13 @@ int rows(const float* A, int lda, const float* W, int ldw, float* C, int ldc, in
     const int nb = (K + BLOCK - 1) / BLOCK, spans = (nb + GR_LANES - 1) / GR_LANES;
     const int wb = spans >= 4 ? 4 : spans >= 2 ? 2 : 1, rows_item = GR_ROWS * (GR_WARPS / wb), items = (N + rows_item - 1) / rows_item;
     const size_t smem = (size_t)(GR_WARPS * GR_STAGES * R::STAGE + 2 * spans * GR_LANES * MT * rows_item) * sizeof(float);
-    KL_CUDA(cudaFuncSetAttribute(gemm_rows_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int most = 2 * (sm_count() > 0 ? sm_count() : 1);      // two CTAs fit an SM
-    launch_kernel(gemm_rows_kernel<MT>, dim3(items < most ? items : most, (M + MT - 1) / MT), dim3(GR_WARPS * 32), smem, stream, A, lda, W, ldw,
+    const auto kernel = K - (spans - 1) * GR_SPAN > BLOCK - R::CHUNK ? gemm_rows_kernel<MT, true> : gemm_rows_kernel<MT, false>;
+    KL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // Two CTAs an SM, although shared memory holds one (118 KB for one row; two for three and four rows): the second ones start where the
+    // first ones end.  us with this grid / with one CTA an SM, one row: 16,384 x 2,048 30.2 / 32.0, 32,000 x 2,048 59.5 / 59.5, 4,096 x 4,096
+    // 16.3 / 15.7, 2,048 x 8,192 15.0 / 13.5; eight rows: 64.2 / 66.1, 2,048 x 8,192 33.1 / 29.9.
+    const int most = 2 * (sm_count() > 0 ? sm_count() : 1);
+    launch_kernel(kernel, dim3(items < most ? items : most, (M + MT - 1) / MT), dim3(GR_WARPS * 32), smem, stream, A, lda, W, ldw,
                   C, ldc, M, N, K, wb);
     return KL_OK;
 }
