@@ -11,18 +11,18 @@
 // the call has or which kernel takes it: K is cut into blocks of 512; a block is one chain of fused multiply-adds in ascending k,
 // and the output is the sum of its blocks in ascending order.
 //
-// * gemm_rows_kernel (few rows of A: a decode step) is bound by reading W once.  A warp takes 8 rows of W and four blocks of K, a
-//   lane one row and one block; the warp copies its weights by 16-byte cp.async into a ring of its own, two chunks (17 KB a warp, 139 KB
-//   an SM) ahead of the arithmetic, without a break between one set of rows and the next, the first ones before the kernel ahead has
-//   finished.  W of 16,384 x 2,048: 28.7 us for one row of A (4.7 TB/s), 68 for eight (the shared-memory reads of A bind); a decode step
-//   of one sequence through two layers of width 2,048: 183 us, 4,051 with 64 x 64 tiles of which one row was used.
+// * gemm_rows_kernel (few rows of A: a decode step) is bound by reading W once.  A warp takes 8 rows of W and four blocks of K,
+//   a lane one row and one block; the warp copies its weights by 16-byte cp.async into a ring of its own, two chunks (17 KB a
+//   warp, 70 KB an SM) ahead of the arithmetic, without a break between one set of rows and the next, the first ones before the
+//   kernel ahead has finished.  W of 16,384 x 2,048: 30 us for one row of A (4.4 TB/s), 64 for eight (the shared-memory reads
+//   of A bind); 2,048 x 2,048 7 and 17 us.
 // * gemm_tile_kernel (everything else) is bound by the FMA pipe.  128 threads make a tile of 64 x 128 outputs, 8 x 8 each, as
 //   packed pairs of rows of A (fma.rn.f32x2: the same two results in one instruction, whose operands come from both register
-//   banks; scalar multiply-adds of this form stay at 39 TFLOP/s whatever the tile and the occupancy).  A lies in shared memory with the row
-//   innermost (4-byte cp.async), W with k innermost (16-byte cp.async); the sums of blocks live in shared memory.  The blocks of
-//   K are dealt to a cluster of CTAs where the tiles alone leave multiprocessors idle; its CTAs add each other's sums through
-//   distributed shared memory, in order.  Tiles of 64 x 32 where even that is less than three CTAs for two SMs.  777 x 16,384 x 2,048: 1.36 ms (38 TFLOP/s; 72 is what the
-//   pipe gives register operands), 777 x 2,048 x 8,192: 0.78 ms; 64 x 64 tiles of scalar multiply-adds ran the prompt's products at 16.
+//   banks).  A lies in shared memory with the row innermost (4-byte cp.async), W with k innermost (16-byte cp.async); the sums of
+//   blocks live in shared memory.  The blocks of K are dealt to a cluster of CTAs where the tiles alone leave multiprocessors
+//   idle; its CTAs add each other's sums through distributed shared memory, in order.  Tiles of 64 x 32 where even that is less
+//   than three CTAs for two SMs.  777 x 16,384 x 2,048: 1.26 ms (41 TFLOP/s; 72 is what the pipe gives register operands),
+//   777 x 2,048 x 8,192: 0.77 ms.
 #include <cooperative_groups.h>
 #include "common.cuh"
 

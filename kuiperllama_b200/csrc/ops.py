@@ -1583,7 +1583,7 @@ def gemm_skinny_stream(w: torch.Tensor, a: torch.Tensor, row_scale=None, sink=No
 SKINNY_MAX_ROWS = 512
 
 
-SWIGLU_WEIGHT_ROWS_MAX = 32     # tokens up to which the gate/up product takes the weights as tile rows (16 where the other way's tiles run at once)
+SWIGLU_WEIGHT_ROWS_MAX = 32     # tokens up to which the gate/up product takes the weights as tile rows (16 where the other way is faster, see above)
 
 
 def one_wave(M: int, N: int) -> bool:
