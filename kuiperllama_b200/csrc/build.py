@@ -45,6 +45,7 @@ SOURCES: Dict[str, str] = {
     "linear_recurrence": "linear_recurrence.cu",
     "short_conv": "short_conv.cu",
     "outer_recurrence": "outer_recurrence.cu",
+    "outer_chunked": "outer_chunked.cu",
     "mlstm": "mlstm.cu",
     "mlstm_chunked": "mlstm_chunked.cu",
     "attention_mixed": "attention_mixed.cu",

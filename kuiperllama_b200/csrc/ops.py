@@ -31,6 +31,9 @@ _libs: Dict[str, ctypes.CDLL] = {}
 _lock = threading.Lock()
 
 
+_LONG_RESULTS = {"outer_chunked": ("kl_outer_chunked_scratch",)}      # entry points that return a long long
+
+
 def lib(name: str) -> ctypes.CDLL:
     """The loaded shared library of one kernel module."""
     got = _libs.get(name)
@@ -40,7 +43,10 @@ def lib(name: str) -> ctypes.CDLL:
         if name not in _libs:
             path = build.ensure_built(name)
             try:
-                _libs[name] = ctypes.CDLL(path)
+                loaded = ctypes.CDLL(path)
+                for entry in _LONG_RESULTS.get(name, ()):
+                    getattr(loaded, entry).restype = ctypes.c_longlong
+                _libs[name] = loaded
             except OSError as e:
                 raise ExtensionError(f"cannot load {path}: {e}") from None
         return _libs[name]
@@ -1121,16 +1127,24 @@ def decay_lowrank(r1: torch.Tensor, W2: torch.Tensor, b: Optional[torch.Tensor],
                                                     ctypes.c_float(tau), n_rows, C, _ptr(a), dtype_code(r1.dtype), _stream()), "decay_lowrank")
 
 
+# A step takes the chunked form from this many tokens of its longest sequence on, with at least so many rows for every sequence: a chunk costs
+# the same for one token as for 32.  us walked / in chunks: 64 heads of 128 x 64, one sequence of 33 tokens 13.7 / 11.6, 64 18.8 / 11.7, 2,048
+# 416 / 151, eight of 40 43 / 57, eight of 64 62 / 57, one of 64 beside 31 single tokens 59 / 160; 16 heads of 64 x 128 with a decay per row, one
+# of 33 9.4 / 11.9, 64 13.8 / 12.0, 2,048 374 / 114, eight of 40 18 / 23, eight of 64 26 / 23; 32 heads of 128 x 64, 48 tokens 10.4 / 11.6.
+OUTER_CHUNKED_FROM, OUTER_CHUNKED_ROWS = 64, 48
+
+
 def outer_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tensor, state: torch.Tensor, y: torch.Tensor, step,
                      heads: int, groups: int, N: int, P: int, c: Optional[torch.Tensor] = None, skip: Optional[torch.Tensor] = None,
-                     q_scale: float = 1.0, *, normaliser: Optional[tuple] = None) -> None:
+                     q_scale: float = 1.0, *, normaliser: Optional[tuple] = None, chunked: Optional[bool] = None) -> None:
     """S_t = diag(a_t) S_(t-1) + (c_t k_t) v_t^T and y_t = S_t^T (q_scale q_t) + skip v_t per head over a ragged step, from and
     into ``state`` float32 [slots, >= heads * N * P] (S as [heads, N, P]).  ``q``, ``k`` [rows, groups * N] and ``v``
     [rows, heads * P] share one dtype (float32 or the compute dtype) and may be column slices; ``a`` float32 [rows, heads]
     (one decay per head) or [rows, heads * N] (one per row of S); ``c`` float32 [rows, heads] or None; ``skip`` float32
     [heads] or None; ``y`` float32 [rows, heads * P].  ``normaliser`` = (n, floor, den, eps): beside S a vector
     n_t = diag(a_t) n_(t-1) + c_t k_t per head (``n`` float32 [slots, heads * N], rows as far apart as ``state``'s), and
-    den_t = max(|n_t . q_scale q_t|, floor_t) + eps; ``floor`` and ``den`` float32 [rows, heads]."""
+    den_t = max(|n_t . q_scale q_t|, floor_t) + eps; ``floor`` and ``den`` float32 [rows, heads].  ``chunked``: True for chunks on the
+    tensor cores (outer_chunked.cu), False for token by token, None by the sizes."""
     _cuda(q, k, v, a, state, y, c, skip)
     n_state = floor = den = None
     den_eps = 0.0
@@ -1154,6 +1168,22 @@ def outer_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch
     _need(state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1 and state.shape[1] >= heads * N * P, "outer_recurrence: state")
     _need(y.dtype == torch.float32 and y.dim() == 2 and y.stride(1) == 1 and y.shape[0] >= n and y.shape[1] == heads * P, "outer_recurrence: y")
     _need(heads % groups == 0 and N <= 1024, "outer_recurrence: heads in equal groups, at most 1,024 rows of state")
+    if chunked or (chunked is None and step.max_new >= OUTER_CHUNKED_FROM and n >= OUTER_CHUNKED_ROWS * step.n_seqs):
+        # what the chunked form takes: see kl_outer_chunked_scratch; rows of q and k (and of a, with a decay per row) on 16-byte boundaries
+        aligned = lambda t: t.data_ptr() % 16 == 0 and t.stride(0) * t.element_size() % 16 == 0
+        need = -1
+        if normaliser is None and aligned(q) and aligned(k) and (not per_row or aligned(a)):
+            need = lib("outer_chunked").kl_outer_chunked_scratch(n, step.n_seqs, int(step.max_new), heads, groups, N, P, int(per_row), dtype_code(q.dtype))
+        if need >= 0:
+            scratch = torch.empty(need, dtype=torch.uint8, device=q.device)
+            _check(lib("outer_chunked").kl_outer_chunked(
+                _ptr(q), ctypes.c_longlong(q.stride(0)), _ptr(k), ctypes.c_longlong(k.stride(0)), _ptr(v), ctypes.c_longlong(v.stride(0)),
+                _ptr(a), ctypes.c_longlong(a.stride(0)), int(per_row), _ptr(c), ctypes.c_longlong(c.stride(0) if c is not None else 0), _ptr(skip),
+                _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(y), ctypes.c_longlong(y.stride(0)), _ptr(scratch), _ptr(step.cu_tokens),
+                _ptr(step.seq_slots), n, step.n_seqs, int(step.max_new), heads, groups, N, P, ctypes.c_float(q_scale), dtype_code(q.dtype),
+                _stream()), "outer_recurrence", 2)
+            return
+        _need(not chunked, "outer_recurrence: the chunked form does not run these operands")
     _check(lib("outer_recurrence").kl_outer_recurrence(
         _ptr(q), ctypes.c_longlong(q.stride(0)), 0, _ptr(k), ctypes.c_longlong(k.stride(0)), 0, _ptr(v), ctypes.c_longlong(v.stride(0)), 0,
         _ptr(a), ctypes.c_longlong(a.stride(0)), int(per_row), _ptr(c), ctypes.c_longlong(c.stride(0) if c is not None else 0), _ptr(skip),

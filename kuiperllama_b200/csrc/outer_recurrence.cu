@@ -14,11 +14,11 @@
 //   outer_recurrence_kernel<TI, NPT>   a CTA per (sequence, head, block of columns of S).  A column of S is cut over
 //       L lanes of one warp, lane l holding rows l, l + L, ... (NPT of them, in registers); tokens arrive in tiles
 //       through shared memory; per token every thread decays and updates its rows, multiplies them by q and the
-//       lanes' sums are added by shuffles.  Tokens are walked in order from the slot's state, so a result does not
-//       depend on how a prompt was cut.
+//       lanes' sums are added by shuffles.  Tokens are walked in order from the slot's state.
 //   outer_recurrence_slab_kernel<TI, R, L, MODE>   the form that runs where the sizes allow: R x 2 of S per thread (see there).
 //   outer_recurrence_few_kernel<TI, V, CL, T>   a step of at most eight tokens a sequence, bound by reading and writing S once:
 //       neighbouring lanes hold neighbouring columns of a row, four or eight rows a thread on their way at a time.
+//   Prompts of 64 tokens and more go in chunks on the tensor cores where the sizes allow (outer_chunked.cu).
 //   decay_softplus_kernel     dt = softplus(raw + bias), a = exp(-exp(A_log) dt) per (token, head), 32-bit.
 //   decay_lowrank_kernel      a = sigmoid(z)^(1 / tau) = exp(-softplus(-z) / tau), z = W2 r + b with r a short row per
 //                             token (the first of two projections, made with the mixer's other projections), 32-bit.

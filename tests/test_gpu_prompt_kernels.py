@@ -103,6 +103,105 @@ def _check_recurrence(heads, groups, n, p, form, dtype, news):
         assert torch.equal(state[:, size:], state0[:, size:])
 
 
+# rows of S on both sides of 64 and 128, columns of one 16, of a remainder of a CTA's 32 and of several CTAs; chunks of one token, of the first
+# block alone, whole ones and remainders; operands as they come and as columns of wider rows
+@pytest.mark.parametrize("heads,groups,n,p", [(2, 1, 8, 16), (4, 2, 64, 48), (3, 3, 72, 32), (6, 2, 128, 64), (5, 5, 128, 16)])
+@pytest.mark.parametrize("form", ["head", "row"])
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("near", [False, True])
+def test_recurrence_in_chunks(heads, groups, n, p, form, wide, near):
+    from kuiperllama_b200.csrc import ops
+    news = [64, 1, 97, 16, 33, 300]
+    step = _step([0] * len(news), news)
+    rows, dtype = step.n_tokens, torch.float32 if form == "head" else torch.bfloat16
+    g = torch.Generator(device=DEV).manual_seed(heads * n + p)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+
+    def placed(x):
+        if not wide:
+            return x
+        room = torch.full((rows, x.shape[1] + 24), float("nan"), dtype=dtype, device=DEV)
+        room[:, 8:8 + x.shape[1]] = x
+        return room[:, 8:8 + x.shape[1]]
+
+    q, k, v = (placed(x.to(dtype)) for x in (rand(rows, groups * n), 0.3 * rand(rows, groups * n), rand(rows, heads * p)))
+    a = torch.rand(rows, heads * n if form == "row" else heads, device=DEV, generator=g)
+    a = a ** 0.0625 if near else a ** 4                    # decays near one, and ones whose products underflow within a chunk
+    a[3] = 0.0
+    c, skip = torch.rand(rows, heads, device=DEV, generator=g), rand(heads)
+    size = heads * n * p
+    state0 = 0.1 * rand(len(news), size + 4)
+    state, y = state0.clone(), torch.full((rows, heads * p), 7.0, device=DEV)
+    ops.outer_recurrence(q, k, v, a, state, y, step, heads, groups, n, p, c=c, skip=skip, q_scale=0.7, chunked=True)
+    spread = lambda x: x.double().reshape(rows, groups, n).repeat_interleave(heads // groups, dim=1)
+    args = [spread(q), spread(k), v.double().reshape(rows, heads, p), a.double().view(rows, heads, -1), c.double(), skip.double(),
+            state0[:, :size].double().view(len(news), heads, n, p)]
+    want, S = _recurrence(*args, step.cu, 0.7)
+    most, S_most = _recurrence(*[x.abs() for x in args], step.cu, 0.7)
+    # within a chunk a term takes at most 36 roundings of decays and factors and a few for its pieces; a sum of n terms one for every 16 and
+    # a few; S four a chunk
+    chunks = 300 / 32
+    assert bool(((y.double().view(want.shape) - want).abs() <= (36 + n / 16 + 4 * chunks + 16) * U * most).all())
+    assert bool(((state[:, :size].double().view(S.shape) - S).abs() <= (36 + 4 * chunks + 16) * U * S_most).all())
+    assert torch.equal(state[:, size:], state0[:, size:])
+    walked = torch.empty_like(y)
+    ops.outer_recurrence(q, k, v, a, state0.clone(), walked, step, heads, groups, n, p, c=c, skip=skip, q_scale=0.7, chunked=False)
+    off = lambda x: float((x.double().view(want.shape) - want).norm() / want.norm())
+    assert off(y) <= 1.5 * off(walked) + U                 # no less exact than token by token
+
+
+@pytest.mark.parametrize("form", ["head", "row"])
+@pytest.mark.parametrize("what", ["v", "q", "k", "a", "c", "state", "grows", "huge"])
+def test_recurrence_in_chunks_keeps_what_is_not_finite_where_it_arises(form, what):
+    """NaN, infinities, numbers too large for the products and decays above one: the same places are not finite as token by token, and the
+    others are as close as sums in another order are."""
+    from kuiperllama_b200.csrc import ops
+    heads, n, p = 4, 64, 48
+    groups, dtype = (1, torch.float32) if form == "head" else (heads, torch.bfloat16)
+    step = _step([0, 0], [100, 70])
+    g = torch.Generator(device=DEV).manual_seed(1)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    q, k, v = rand(170, groups * n).to(dtype), (0.3 * rand(170, groups * n)).to(dtype), rand(170, heads * p).to(dtype)
+    a, c = torch.rand(170, heads * n if form == "row" else heads, device=DEV, generator=g) ** 0.1, torch.rand(170, heads, device=DEV, generator=g)
+    state0 = 0.1 * rand(2, heads * n * p)
+    if what in ("v", "q", "k", "a", "c"):
+        {"v": v, "q": q, "k": k, "a": a, "c": c}[what][40, 2], {"v": v, "q": q, "k": k, "a": a, "c": c}[what][120, 1] = float("nan"), float("inf")
+    elif what == "state":
+        state0[1, 100], state0[0, 7] = float("inf"), 1e30
+    elif what == "grows":
+        a[20:30] = 1.5
+    else:
+        v[50], k[90] = 1e12, 1e9
+    got = []
+    for chunked in (False, True):
+        state, y = state0.clone(), torch.empty(170, heads * p, device=DEV)
+        ops.outer_recurrence(q, k, v, a, state, y, step, heads, groups, n, p, c=c, q_scale=0.7, chunked=chunked)
+        got += [y, state]
+    for x, z in ((got[0], got[2]), (got[1], got[3])):
+        fine = torch.isfinite(x)
+        assert torch.equal(fine, torch.isfinite(z))
+        assert bool(((x - z)[fine].abs() <= 1e-4 * x[fine].abs() + 1e-5 * x[fine].abs().median()).all()) or what in ("huge", "state"), what
+        assert float((x - z)[fine].double().norm()) <= 2e-6 * float(x[fine].double().norm()), what
+
+
+def test_recurrence_of_steps_that_the_chunks_do_not_take():
+    """Rows between 16-byte boundaries, odd sizes, a normaliser and many short sequences go token by token."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator(device=DEV).manual_seed(2)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    for n, p, shift, news in ((64, 32, 1, [80]), (20, 32, 0, [80]), (64, 20, 0, [80]), (136, 32, 0, [80]), (64, 32, 0, [64] + [1] * 40)):
+        step = _step([0] * len(news), news)
+        rows = step.n_tokens
+        wide = rand(rows, 4 * n + 4)
+        q, k, v, a = wide[:, shift:shift + 2 * n], wide[:, 2 * n:4 * n], rand(rows, 2 * p), torch.rand(rows, 2, device=DEV, generator=g)
+        out = []
+        for chunked in (None, False):
+            state, y = torch.zeros(len(news), 2 * n * p, device=DEV), torch.empty(rows, 2 * p, device=DEV)
+            ops.outer_recurrence(q, k, v, a, state, y, step, 2, 2, n, p, chunked=chunked)
+            out.append((y, state))
+        assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
 @pytest.mark.parametrize("channels", [4, 36, 512, 1028])
 @pytest.mark.parametrize("dtype,out_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
 def test_four_taps_in_tiles(channels, dtype, out_dtype):
