@@ -20,6 +20,18 @@
 // reference was set, which is rare after the first blocks.  While one tile is in the softmax
 // the tensor core works on the other tile's products.
 //
+// Options (EXTRA): a window (a row sees the keys of its last `window` positions; blocks of keys are counted from the page that holds the
+// first key the CTA's first row sees, so no earlier page is touched) and a sink (a number per head that joins the denominator as
+// exp(sink)).
+//
+// Attention over a shared latent (LATENT) for whole prompts: a key/value head per query head.  A head's keys are its own `dim` columns, made
+// from the latent by one product for all heads, then the rotated columns that all heads share, which are read where they lie in the latent's cache;
+// its values come from the same product.  Scores over (dim + rot) and values over vdim columns cost a third of what the latent's own
+// rows do (288 and 256 columns a head): 2,048 tokens of 32 heads of 64 + 32 | 64 with all that goes before and behind take 79 us so, 459 over the latent
+// on mma.sync.  With a window of 1,024, 32 heads of 64 on 8, prompts of 6,000 tokens: 113 us, 200 on mma.sync.  A sequence's
+// rows of that product start at a multiple of 64 rows (padded_first_row), zeros between, so no row of another sequence meets a product.
+// The result may be multiplied by sigmoid of a number per (row, head).
+//
 // Every wait is bounded, as in gemm_tcgen05.cu.
 #include "tcgen05.cuh"
 #include "tma_host.cuh"
@@ -110,23 +122,32 @@ struct AttnArgs {
     int H, KV, Gp;
     float scale_log2;
     int* status;
+    int window;                // 0: none
+    const float* sink;         // [H] or null
+    // LATENT: columns of a head's own keys and of its values in the rows of `map_k` (all heads' keys, then all heads' values), the column of the
+    // shared keys in the latent's cache, the gate's rows or null
+    int dim, rank;
+    const bf16* gate;
+    long long gate_stride;
 };
 
-// HD: head size, 64 or 128 (one or two 64-wide slabs per row of queries, keys and values).
-template <int HD>
+// KS: steps of 16 columns of the scores' product (the slabs behind the last one are not multiplied); VS: slabs of 64 columns of the values;
+// BP: pages of a block of keys.
+template <int KS, int VS, int BP, bool EXTRA, bool LATENT>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                          const __grid_constant__ CUtensorMap map_v, AttnArgs args) {
-    constexpr int AT_HD = HD;
-    constexpr int SLABS = HD / 64;
+    constexpr int AT_VD = VS * 64;
+    constexpr int SLABS = (KS + 3) / 4;
+    constexpr uint32_t PAGE_BYTES = PAGE * 128, KV_SLAB = BP * PAGE_BYTES;
     constexpr uint32_t AT_Q_BYTES = SLABS * AT_SLAB;      // one tile's queries
-    constexpr uint32_t AT_K_BYTES = SLABS * AT_SLAB;      // [128 keys][HD dims] as 64-wide slabs
+    constexpr uint32_t AT_K_BYTES = SLABS * KV_SLAB, AT_V_BYTES = VS * KV_SLAB;      // a block's keys and values as 64-wide slabs
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* q_sm = smem;                                 // [2 tiles]
     uint8_t* k_sm = q_sm + 2 * AT_Q_BYTES;                // [2 stages]
     uint8_t* v_sm = k_sm + 2 * AT_K_BYTES;                // [2 stages]
-    uint64_t* bars = (uint64_t*)(v_sm + 2 * AT_K_BYTES);
+    uint64_t* bars = (uint64_t*)(v_sm + 2 * AT_V_BYTES);
     uint64_t* q_full = bars;
     uint64_t* kv_full = bars + 1;                         // [2 stages] a key block has landed
     uint64_t* kv_empty = bars + 3;                        // [2 stages] every product that reads it is done
@@ -148,16 +169,17 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     if (t0 >= T) return;
     const int n_tiles = t0 + BT < T ? 2 : 1;
     const int start = args.seq_starts[b], slot = args.seq_slots[b], row0 = args.cu_tokens[b];
-    // pages and key blocks (two pages) that each tile reads: tile 1 reads at least as many as tile 0
+    // pages (from page `pf` on) and key blocks (BP pages) that each tile reads: tile 1 reads at least as many as tile 0
+    const int pf = EXTRA && args.window > 0 ? max(0, start + t0 - args.window + 1) / PAGE : 0;
     int n_pages[2], n_blocks[2];
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         const int max_pos = start + min(T, t0 + (t + 1) * BT) - 1;
-        n_pages[t] = t < n_tiles ? max_pos / PAGE + 1 : 0;
-        n_blocks[t] = (n_pages[t] + 1) / 2;
+        n_pages[t] = t < n_tiles ? max_pos / PAGE + 1 - pf : 0;
+        n_blocks[t] = (n_pages[t] + BP - 1) / BP;
     }
     const int all_pages = n_pages[n_tiles - 1], all_blocks = n_blocks[n_tiles - 1];
-    const int* table = args.block_table + (size_t)slot * args.blocks_per_seq;
+    const int* table = args.block_table + (size_t)slot * args.blocks_per_seq + pf;
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
@@ -189,13 +211,21 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             for (int j = 0; j < all_blocks; ++j) {
                 const int s = j & 1;
                 if (j >= 2 && !mbar_wait(&kv_empty[s], ((j >> 1) - 1) & 1, abort_flag, args.status, 11)) break;
-                const int pages = min(2, all_pages - 2 * j);
-                mbar_expect_tx(&kv_full[s], pages * 2 * SLABS * (PAGE * 128));
+                const int pages = min(BP, all_pages - BP * j);
+                mbar_expect_tx(&kv_full[s], pages * (SLABS + VS) * PAGE_BYTES);
                 for (int pg = 0; pg < pages; ++pg) {
-                    const int y = (table[2 * j + pg] * KV + g) * PAGE;
-                    for (int h = 0; h < SLABS; ++h) {
-                        tma_load_2d(k_sm + s * AT_K_BYTES + h * AT_SLAB + pg * (PAGE * 128), &map_k, &kv_full[s], h * 64, y);
-                        tma_load_2d(v_sm + s * AT_K_BYTES + h * AT_SLAB + pg * (PAGE * 128), &map_v, &kv_full[s], h * 64, y);
+                    uint8_t *kd = k_sm + s * AT_K_BYTES + pg * PAGE_BYTES, *vd = v_sm + s * AT_V_BYTES + pg * PAGE_BYTES;
+                    if constexpr (LATENT) {
+                        const int y = padded_first_row(row0, b) + (pf + BP * j + pg) * PAGE;
+                        for (int h = 0; h < args.dim / 64; ++h) tma_load_2d(kd + h * KV_SLAB, &map_k, &kv_full[s], g * args.dim + h * 64, y);
+                        tma_load_2d(kd + (SLABS - 1) * KV_SLAB, &map_v, &kv_full[s], args.rank, table[BP * j + pg] * PAGE);
+                        for (int h = 0; h < VS; ++h) tma_load_2d(vd + h * KV_SLAB, &map_k, &kv_full[s], H * args.dim + g * AT_VD + h * 64, y);
+                    } else {
+                        const int y = (table[BP * j + pg] * KV + g) * PAGE;
+                        for (int h = 0; h < SLABS; ++h) {
+                            tma_load_2d(kd + h * KV_SLAB, &map_k, &kv_full[s], h * 64, y);
+                            tma_load_2d(vd + h * KV_SLAB, &map_v, &kv_full[s], h * 64, y);
+                        }
                     }
                 }
                 issued = j + 1;
@@ -212,14 +242,12 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 const int s = j & 1;
                 if (!mbar_wait(&kv_full[s], (j >> 1) & 1, abort_flag, args.status, 13)) return false;
                 tc_fence_after();
-                const int keys = min(2, n_pages[t] - 2 * j) * PAGE;
+                const int keys = min(BP, n_pages[t] - BP * j) * PAGE;
                 const uint32_t idesc = umma_idesc_ab(keys, 0);
 #pragma unroll
-                for (int ks = 0; ks < AT_HD / 16; ++ks) {
-                    const uint32_t off = (ks >> 2) * AT_SLAB + (ks & 3) * 32;
-                    umma_bf16(tmem_base + t * 128, smem_desc_sw128(smem_u32(q_sm + t * AT_Q_BYTES + off)),
-                              smem_desc_sw128(smem_u32(k_sm + s * AT_K_BYTES + off)), idesc, ks > 0 ? 1u : 0u);
-                }
+                for (int ks = 0; ks < KS; ++ks)
+                    umma_bf16(tmem_base + t * 128, smem_desc_sw128(smem_u32(q_sm + t * AT_Q_BYTES + (ks >> 2) * AT_SLAB + (ks & 3) * 32)),
+                              smem_desc_sw128(smem_u32(k_sm + s * AT_K_BYTES + (ks >> 2) * KV_SLAB + (ks & 3) * 32)), idesc, ks > 0 ? 1u : 0u);
                 umma_commit(&s_full[t]);
                 return true;
             };
@@ -231,11 +259,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     ok = mbar_wait(&p_ready[t], j & 1, abort_flag, args.status, 14);
                     if (!ok) break;
                     tc_fence_after();
-                    const int keys = min(2, n_pages[t] - 2 * j) * PAGE;
-                    const uint32_t idesc = umma_idesc_ab(AT_HD, 1);
+                    const int keys = min(BP, n_pages[t] - BP * j) * PAGE;
+                    const uint32_t idesc = umma_idesc_ab(AT_VD, 1);
                     for (int kk = 0; kk < keys / 16; ++kk)     // O_t += P_t V_j: P from tensor memory, 8 columns per 16 keys
                         umma_bf16_ta(tmem_base + 256 + t * 128, tmem_base + t * 128 + kk * 8,
-                                     smem_desc_sw128_mn(smem_u32(v_sm + s * AT_K_BYTES + kk * 2048), AT_SLAB), idesc,
+                                     smem_desc_sw128_mn(smem_u32(v_sm + s * AT_V_BYTES + kk * 2048), KV_SLAB), idesc,
                                      (j > 0 || kk > 0) ? 1u : 0u);
                     umma_commit(&o_done[t]);
                     if (t == n_tiles - 1) umma_commit(&kv_empty[s]);      // the last product that reads this stage
@@ -262,17 +290,18 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             ok = mbar_wait(&s_full[tile], j & 1, abort_flag, args.status, 15);
             if (!ok) break;
             tc_fence_after();
-            const int keys = min(2, n_pages[tile] - 2 * j) * PAGE;      // 64 or 128, the same for the whole tile
-            const int key0 = 2 * j * PAGE;
+            const int keys = min(BP, n_pages[tile] - BP * j) * PAGE;    // 64 or 128, the same for the whole tile
+            const int key0 = (pf + BP * j) * PAGE;
             const int limit = pos - key0;                               // scores 0..limit of this block are visible
+            const int low = EXTRA && args.window > 0 ? limit - args.window + 1 : 0;       // and, with a window, none before this one
             // The same for all lanes of the warp: the tensor-memory loads and stores below are warp-wide
             // instructions and must not sit in branches that lanes take differently.
-            const bool need_mask = __any_sync(0xffffffffu, limit < keys - 1);
+            const bool need_mask = __any_sync(0xffffffffu, limit < keys - 1 || (EXTRA && low > 0));
             // two passes over the scores, 64 at a time (tensor-memory loads are cheap, registers are not)
             uint32_t sc[2][32];
             float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains: a warp has little else to hide latency behind
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+            for (int h = 0; h < BP; ++h)
                 if (h * 64 < keys) {
                     tmem_ld32(s_addr + h * 64, sc[0]);
                     tmem_ld32(s_addr + h * 64 + 32, sc[1]);
@@ -282,7 +311,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                         for (int q = 0; q < 2; ++q)
 #pragma unroll
                             for (int e = 0; e < 32; ++e)
-                                mx4[e & 3] = fmaxf(mx4[e & 3], h * 64 + q * 32 + e <= limit ? __uint_as_float(sc[q][e]) : -INFINITY);
+                                mx4[e & 3] = fmaxf(mx4[e & 3], h * 64 + q * 32 + e <= limit && (!EXTRA || h * 64 + q * 32 + e >= low) ? __uint_as_float(sc[q][e]) : -INFINITY);
                     } else {
 #pragma unroll
                         for (int q = 0; q < 2; ++q)
@@ -302,7 +331,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             uint64_t sum4[4] = {0ull, 0ull, 0ull, 0ull};                  // four chains of float32 pairs
             const uint64_t scale2 = pack2(args.scale_log2, args.scale_log2), shift2 = pack2(-muse, -muse);
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+            for (int h = 0; h < BP; ++h)
                 if (h * 64 < keys) {
                     tmem_ld32(s_addr + h * 64, sc[0]);
                     tmem_ld32(s_addr + h * 64 + 32, sc[1]);
@@ -316,8 +345,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                             unpack2(fma2(pack2(__uint_as_float(sc[q][e]), __uint_as_float(sc[q][e + 1])), scale2, shift2), x0, x1);
                             float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
                             if (need_mask) {
-                                if (h * 64 + q * 32 + e > limit) p0 = 0.f;
-                                if (h * 64 + q * 32 + e + 1 > limit) p1 = 0.f;
+                                if (h * 64 + q * 32 + e > limit || (EXTRA && h * 64 + q * 32 + e < low)) p0 = 0.f;
+                                if (h * 64 + q * 32 + e + 1 > limit || (EXTRA && h * 64 + q * 32 + e + 1 < low)) p1 = 0.f;
                             }
                             sum4[(e >> 1) & 3] = add2(sum4[(e >> 1) & 3], pack2(p0, p1));
                             __nv_bfloat162 pr = __floats2bfloat162_rn(p0, p1);
@@ -339,7 +368,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 if (__any_sync(0xffffffffu, factor != 1.f)) {
                     uint32_t c32[32];
 #pragma unroll
-                    for (int c = 0; c < AT_HD; c += 32) {
+                    for (int c = 0; c < AT_VD; c += 32) {
                         tmem_ld32(o_addr + c, c32);
                         tmem_ld_wait();
 #pragma unroll
@@ -358,10 +387,21 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             if (ok) {
                 tc_fence_after();
                 uint32_t c32[32];
-                const float inv = 1.f / l;
-                bf16* orow = args.out + ((size_t)(row0 + tl) * H + (g * G + hh)) * AT_HD;
+                float inv = 1.f / l;
+                if constexpr (EXTRA) {
+                    if (valid) {
+                        if (args.sink != nullptr) {
+                            const float sk = args.sink[g * G + hh] * 1.4426950408889634f;      // in the exp2 domain, as the scores are
+                            const float top = fmaxf(m_ref, sk), w = fast_exp2(m_ref - top);
+                            inv = w / (l * w + fast_exp2(sk - top));
+                        }
+                        if (LATENT && args.gate != nullptr)
+                            inv *= 1.f / (1.f + expf(-__bfloat162float(args.gate[(size_t)(row0 + tl) * args.gate_stride + g * G + hh])));
+                    }
+                }
+                bf16* orow = args.out + ((size_t)(row0 + tl) * H + (g * G + hh)) * AT_VD;
 #pragma unroll
-                for (int c = 0; c < AT_HD; c += 32) {
+                for (int c = 0; c < AT_VD; c += 32) {
                     tmem_ld32(o_addr + c, c32);
                     tmem_ld_wait();
                     if (valid) {
@@ -391,30 +431,28 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 using namespace kl;
 
 namespace kl {
-template <int HD>
+template <int KS, int VS, int BP, bool EXTRA, bool LATENT>
 static int launch_attention_tcgen05(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnArgs& args,
                                     dim3 grid, cudaStream_t stream) {
-    constexpr size_t smem = (size_t)(2 + 4) * (HD / 64) * AT_SLAB + 11 * 8 + 16 + 1024;     // two query tiles, two stages of keys and of values
-    static bool configured = false;
-    if (!configured) {
-        KL_CUDA(cudaFuncSetAttribute(attention_tcgen05_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured = true;
-    }
-    launch_kernel(attention_tcgen05_kernel<HD>, grid, AT_THREADS, smem, stream, mq, mk, mv, args);
+    // two query tiles, two stages of keys and of values
+    constexpr size_t smem = (size_t)2 * ((KS + 3) / 4) * AT_SLAB + (size_t)2 * ((KS + 3) / 4 + VS) * BP * PAGE * 128 + 11 * 8 + 16 + 1024;
+    static_assert(smem <= 227 * 1024, "attention_tcgen05_kernel: shared memory");
+    KL_CUDA(cudaFuncSetAttribute(attention_tcgen05_kernel<KS, VS, BP, EXTRA, LATENT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    launch_kernel(attention_tcgen05_kernel<KS, VS, BP, EXTRA, LATENT>, grid, AT_THREADS, smem, stream, mq, mk, mv, args);
     KL_LAUNCH_CHECK();
     return KL_OK;
 }
 }  // namespace kl
 
 // Prefill attention of a ragged batch (see kl_attention_mma for the arguments' meaning).  Head
-// sizes 64 and 128, group sizes that divide 128, no window; q rows 16-byte aligned.  Others:
+// sizes 64 and 128, group sizes that divide 128; q rows 16-byte aligned.  window: keys a row sees (0: all); sink: float32 [H] or null.  Others:
 // KL_ERR_BAD_SIZE / KL_ERR_BAD_ALIGN, and the caller takes the mma.sync kernel.
 KL_API int kl_attention_tcgen05(const void* q, int q_stride, void* out, const void* k_cache, const void* v_cache,
                                 long long n_cache_rows, const int* block_table, int blocks_per_seq, const int* cu_tokens,
                                 const int* seq_slots, const int* seq_starts, const int* seq_new, int n_seqs, int max_new,
-                                int n_rows, int H, int KV, int hd, float scale, int* status, cudaStream_t stream) {
+                                int n_rows, int H, int KV, int hd, float scale, int window, const float* sink, int* status, cudaStream_t stream) {
     if (n_seqs <= 0 || max_new <= 0) return KL_OK;
-    if ((hd != 64 && hd != 128) || KV <= 0 || H % KV) return KL_ERR_BAD_SIZE;
+    if ((hd != 64 && hd != 128) || KV <= 0 || H % KV || window < 0) return KL_ERR_BAD_SIZE;
     const int G = H / KV;
     int Gp = 1;
     while (Gp < G) Gp <<= 1;
@@ -435,9 +473,58 @@ KL_API int kl_attention_tcgen05(const void* q, int q_stride, void* out, const vo
         if ((rc = tma_make_map(&mv, v_cache, 2, dims, strides, box)) != KL_OK) return rc;
     }
     AttnArgs args{(bf16*)out, block_table, blocks_per_seq, cu_tokens, seq_slots, seq_starts, seq_new, H, KV, Gp,
-                  scale * 1.4426950408889634f, status};
+                  scale * 1.4426950408889634f, status, window, sink, 0, 0, nullptr, 0};
     const dim3 grid(KV, n_seqs, (max_new + 2 * BT - 1) / (2 * BT));          // two tiles of BT tokens per CTA
     if (grid.y > 65535 || grid.z > 65535) return KL_ERR_BAD_SIZE;
-    return hd == 128 ? launch_attention_tcgen05<128>(mq, mk, mv, args, grid, stream)
-                     : launch_attention_tcgen05<64>(mq, mk, mv, args, grid, stream);
+    const bool extra = window > 0 || sink != nullptr;
+    if (hd == 128) return extra ? launch_attention_tcgen05<8, 2, 2, true, false>(mq, mk, mv, args, grid, stream)
+                                : launch_attention_tcgen05<8, 2, 2, false, false>(mq, mk, mv, args, grid, stream);
+    return extra ? launch_attention_tcgen05<4, 1, 2, true, false>(mq, mk, mv, args, grid, stream)
+                 : launch_attention_tcgen05<4, 1, 2, false, false>(mq, mk, mv, args, grid, stream);
+}
+
+// Attention over a shared latent for prompts that start at position 0.  q: [rows, H, dim + rot] bfloat16, rows q_stride apart, rotated parts last;
+// kv: [kv_rows, H * (dim + vdim)] (all heads' keys, then all heads' values), a sequence from row padded_first_row on; cache: the latent's pages
+// [pages, 64, rank + rot]; out: [rows, H * vdim], times sigmoid(gate[row, h]) with a gate.  dim + rot | vdim: 64 + 16, 32, 48 or 64 | 64 and
+// 128 + 16, 32, 48 or 64 | 128.
+KL_API int kl_attention_tcgen05_latent(const void* q, long long q_stride, int q_rows, void* out, const void* kv, int kv_rows, const void* cache,
+                                       long long n_cache_rows, const int* block_table, int blocks_per_seq, const int* cu_tokens, const int* seq_slots,
+                                       const int* seq_starts, const int* seq_new, int n_seqs, int max_new, int H, int dim, int rot, int vdim,
+                                       int rank, float scale, int window, const float* sink, const void* gate, long long gate_stride, int* status,
+                                       cudaStream_t stream) {
+    if (n_seqs <= 0 || max_new <= 0) return KL_OK;
+    if (H <= 0 || (dim != 64 && dim != 128) || vdim != dim || rot <= 0 || rot > 64 || rot % 16 || rank <= 0 || window < 0) return KL_ERR_BAD_SIZE;
+    if (q_stride % 8 || rank % 8 || (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)cache | (uintptr_t)out) & 15)) return KL_ERR_BAD_ALIGN;
+    CUtensorMap mq, mk, mr;
+    int rc;
+    {
+        const long long dims[3] = {dim + rot, H, q_rows}, strides[2] = {dim + rot, q_stride};
+        const int box[3] = {64, 1, AT_ROWS};
+        if ((rc = tma_make_map(&mq, q, 3, dims, strides, box)) != KL_OK) return rc;
+    }
+    const int box[2] = {64, PAGE};
+    {
+        const long long dims[2] = {(long long)H * (dim + vdim), kv_rows}, strides[1] = {(long long)H * (dim + vdim)};
+        if ((rc = tma_make_map(&mk, kv, 2, dims, strides, box)) != KL_OK) return rc;
+    }
+    {
+        const long long dims[2] = {rank + rot, n_cache_rows}, strides[1] = {rank + rot};
+        if ((rc = tma_make_map(&mr, cache, 2, dims, strides, box)) != KL_OK) return rc;
+    }
+    AttnArgs args{(bf16*)out, block_table, blocks_per_seq, cu_tokens, seq_slots, seq_starts, seq_new, H, H, 1,
+                  scale * 1.4426950408889634f, status, window, sink, dim, rank, (const bf16*)gate, gate_stride};
+    const dim3 grid(H, n_seqs, (max_new + 2 * AT_ROWS - 1) / (2 * AT_ROWS));
+    if (grid.y > 65535 || grid.z > 65535) return KL_ERR_BAD_SIZE;
+#define KL_AT(STEPS)                                                                                                  \
+    case STEPS:                                                                                                      \
+        return dim == 64 ? launch_attention_tcgen05<4 + STEPS, 1, 2, true, true>(mq, mk, mr, args, grid, stream)     \
+                         : launch_attention_tcgen05<8 + STEPS, 2, 1, true, true>(mq, mk, mr, args, grid, stream)
+    switch (rot / 16) {
+        KL_AT(1);
+        KL_AT(2);
+        KL_AT(3);
+        KL_AT(4);
+    }
+#undef KL_AT
+    return KL_ERR_BAD_SIZE;
 }

@@ -187,4 +187,8 @@ __device__ __forceinline__ size_t cache_row_offset(const int* __restrict__ block
     return (((size_t)page * kv_heads + kv_head) * PAGE + (pos % PAGE)) * (size_t)head_dim;
 }
 
+// Where a step's sequences lie when each starts at a multiple of PAGE rows: the row at which sequence b, whose first row in the step is `cu`,
+// begins.  Sequences follow one another and no two share a block of PAGE rows; all of them take at most (rows / PAGE + sequences) * PAGE rows.
+__host__ __device__ inline int padded_first_row(int cu, int b) { return (cu / PAGE + b) * PAGE; }
+
 }  // namespace kl

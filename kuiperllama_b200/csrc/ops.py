@@ -946,20 +946,25 @@ def moe_combine(results: torch.Tensor, pair_pos: torch.Tensor, weight: torch.Ten
 
 def latent_prepare(proj: torch.Tensor, q_col: int, kv_col: Optional[int], norm_weight: Optional[torch.Tensor], eps: float,
                    inv_freq: Optional[torch.Tensor], rot_dims: int, mscale: float, interleaved: bool, positions: torch.Tensor,
-                   token_slot: torch.Tensor, block_table: Optional[torch.Tensor], cache: Optional[torch.Tensor], qfull: torch.Tensor,
-                   n_tokens: int, heads: int, dim: int, rot_dim: int, kv_rank: int, q: Optional[torch.Tensor] = None) -> None:
+                   token_slot: torch.Tensor, block_table: Optional[torch.Tensor], cache: Optional[torch.Tensor], qfull: Optional[torch.Tensor],
+                   n_tokens: int, heads: int, dim: int, rot_dim: int, kv_rank: int, q: Optional[torch.Tensor] = None,
+                   rows: Optional[torch.Tensor] = None, step=None) -> None:
     """Per token: the normed latent and the rotated shared key part into the cache row (unless ``kv_col`` is
     None: the layer reads another layer's cache), and every head's rotated query part into the last
     ``rot_dim`` columns of its [kv_rank + rot_dim] slice of ``qfull`` (see latent.cu).  ``q``: the matrix that holds the
-    queries from column ``q_col`` on, where that is not ``proj`` (queries that came through a latent of their own)."""
-    _cuda(proj, norm_weight, inv_freq, positions, token_slot, block_table, cache, qfull, q)
+    queries from column ``q_col`` on, where that is not ``proj`` (queries that came through a latent of their own).  ``qfull`` None: the
+    queries are rotated where they lie.  ``rows`` [.., kv_rank] takes the latent too, the sequences of ``step`` as ``latent_expanded``
+    wants them."""
+    _cuda(proj, norm_weight, inv_freq, positions, token_slot, block_table, cache, qfull, q, rows)
     qsrc = proj if q is None else q
     _need(qsrc.dim() == 2 and qsrc.stride(1) == 1 and qsrc.dtype == proj.dtype and qsrc.shape[0] >= n_tokens, "latent_prepare: queries")
     _i32(positions, "positions"); _i32(token_slot, "token_slot"); _i32(block_table, "block_table")
     Dk = kv_rank + rot_dim
     _need(proj.dim() == 2 and proj.stride(1) == 1 and q_col + heads * (dim + rot_dim) <= qsrc.shape[1], "latent_prepare: projections")
-    _need(qfull.is_contiguous() and qfull.dtype == proj.dtype and qfull.shape[0] >= n_tokens and qfull.shape[1] == heads * Dk,
+    _need(qfull is None or (qfull.is_contiguous() and qfull.dtype == proj.dtype and qfull.shape[0] >= n_tokens and qfull.shape[1] == heads * Dk),
           "latent_prepare: query buffer")
+    _need(rows is None or (kv_col is not None and rows.is_contiguous() and rows.dtype == proj.dtype and rows.shape[1] == kv_rank
+                           and rows.shape[0] >= latent_rows(step)), "latent_prepare: rows of the latent")
     if kv_col is not None:
         _need(kv_col + Dk <= proj.shape[1], "latent_prepare: the down-projection's columns")
         _need(cache is not None and cache.is_contiguous() and cache.dtype == proj.dtype and tuple(cache.shape[1:]) == (1, PAGE, Dk),
@@ -972,7 +977,59 @@ def latent_prepare(proj: torch.Tensor, q_col: int, kv_col: Optional[int], norm_w
         _ptr(norm_weight), ctypes.c_float(eps),
         _ptr(inv_freq), rot_dims, ctypes.c_float(mscale), int(bool(interleaved)), _ptr(positions), _ptr(token_slot),
         _ptr(block_table), 0 if block_table is None else block_table.shape[1], _ptr(cache if kv_col is not None else None), _ptr(qfull),
-        n_tokens, heads, dim, rot_dim, kv_rank, dtype_code(proj.dtype), _stream()), "latent_prepare")
+        n_tokens, heads, dim, rot_dim, kv_rank, _ptr(rows), _ptr(step.cu_tokens if rows is not None else None),
+        0 if rows is None else step.n_seqs, dtype_code(proj.dtype), _stream()), "latent_prepare")
+
+
+def latent_rows(step) -> int:
+    """Rows that hold the sequences of ``step`` with each starting at a multiple of PAGE rows (padded_first_row in common.cuh)."""
+    return (step.n_tokens // PAGE + step.n_seqs) * PAGE
+
+
+# Tokens of the longest sequence from which prompts take keys and values of every head's own, and rows for every sequence (one of fewer rows
+# than its 64 pays for all of them).  us over the latent / so, 32 heads of 64 + 32 | 64, rank 256: one prompt of 20 tokens 54 / 15, 64 32 / 15, 512 78 /
+# 31, 2,048 459 / 79, eight of 64 43 / 26, one of 128 beside 31 single tokens 39 / 59; heads of 128 + 64 | 128: 64 35 / 17, 2,048 491 / 116, eight
+# of 64 52 / 32, one of 128 beside 31 single tokens 44 / 73.
+LATENT_EXPANDED_FROM = LATENT_EXPANDED_ROWS = 16
+
+
+def latent_expandable(dtype: torch.dtype, dim: int, rot_dim: int, value_dim: int, kv_rank: int, scale: float) -> bool:
+    """Whether ``latent_expanded`` runs these sizes: bfloat16, 64 or 128 columns for a head's own keys and values alike beside 16 to 64
+    rotated ones."""
+    return dtype == torch.bfloat16 and dim in (64, 128) and value_dim == dim and rot_dim in (16, 32, 48, 64) and kv_rank % 8 == 0 and scale > 0
+
+
+def latent_expands(step, q: torch.Tensor) -> bool:
+    """Whether a step's prompts take it: all start at position 0, and the step is launched for itself alone (a captured one is replayed
+    for others); rows of ``q`` on 16-byte boundaries."""
+    return (LATENT_KERNEL == "mma" and step.max_new >= LATENT_EXPANDED_FROM and step.n_tokens >= LATENT_EXPANDED_ROWS * step.n_seqs
+            and not step.captured and not step.padded and not any(step.host_starts) and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
+
+
+def latent_expanded(q: torch.Tensor, kv: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, step, heads: int,
+                    dim: int, rot_dim: int, value_dim: int, kv_rank: int, scale: float, sink: Optional[torch.Tensor] = None, window: int = 0,
+                    gate: Optional[torch.Tensor] = None) -> None:
+    """Causal attention of prompts over a shared latent with keys and values of every head's own: ``q`` [rows, heads * (dim + rot_dim)]
+    (rotated parts last), ``kv`` [latent_rows(step), heads * (dim + value_dim)] (all heads' keys, then all heads' values, made from the rows of
+    ``latent_prepare``), the shared rotated keys in the latent's ``cache``; out [rows, heads * value_dim], times sigmoid(gate[row, h])."""
+    _cuda(q, kv, out, cache, block_table, sink, gate)
+    _i32(block_table, "block_table")
+    n, bf = step.n_tokens, torch.bfloat16
+    _need(q.dtype == kv.dtype == out.dtype == cache.dtype == bf and latent_expandable(q.dtype, dim, rot_dim, value_dim, kv_rank, scale)
+          and latent_expands(step, q), "latent_expanded: this step")
+    _columns(q, n, heads * (dim + rot_dim), "latent_expanded: q")
+    _need(kv.is_contiguous() and kv.shape[0] >= latent_rows(step) and kv.shape[1] == heads * (dim + value_dim), "latent_expanded: keys and values")
+    _need(out.is_contiguous() and out.shape[0] >= n and out.shape[1] == heads * value_dim, "latent_expanded: out shape")
+    _need(cache.is_contiguous() and tuple(cache.shape[1:]) == (1, PAGE, kv_rank + rot_dim), "latent_expanded: cache layout")
+    _need(sink is None or (sink.dtype == torch.float32 and sink.is_contiguous() and sink.numel() == heads), "latent_expanded: sink")
+    if gate is not None:
+        _columns(gate, n, heads, "latent_expanded: gate")
+        _need(gate.dtype == bf, "latent_expanded: gate")
+    _check(lib("attention_tcgen05").kl_attention_tcgen05_latent(
+        _ptr(q), ctypes.c_longlong(q.stride(0)), n, _ptr(out), _ptr(kv), kv.shape[0], _ptr(cache), ctypes.c_longlong(cache.shape[0] * PAGE),
+        _ptr(block_table), block_table.shape[1], _ptr(step.cu_tokens), _ptr(step.seq_slots), _ptr(step.seq_starts), _ptr(step.seq_new), step.n_seqs,
+        int(step.max_new), heads, dim, rot_dim, value_dim, kv_rank, ctypes.c_float(scale), int(window or 0), _ptr(sink), _ptr(gate),
+        ctypes.c_longlong(gate.stride(0) if gate is not None else 0), _status_ptr(q.device), _stream()), "latent_expanded")
 
 
 def latent_decode_splits(n_seqs: int, heads: int, context_class: int) -> int:
@@ -1845,9 +1902,10 @@ def matmul_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, a
 def attention_tcgen05(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                       block_table: torch.Tensor, cu_tokens: torch.Tensor, seq_slots: torch.Tensor, seq_starts: torch.Tensor,
                       seq_new: torch.Tensor, n_seqs: int, max_new: int, n_rows: int, num_heads: int, num_kv_heads: int,
-                      head_dim: int, scale: float) -> None:
-    """Prefill attention with both products on tcgen05 (bfloat16, head size 64 or 128, no window)."""
-    _cuda(q, out, k_cache, v_cache, block_table, cu_tokens, seq_slots, seq_starts, seq_new)
+                      head_dim: int, scale: float, window: int = 0, sink: Optional[torch.Tensor] = None) -> None:
+    """Prefill attention with both products on tcgen05 (bfloat16, head size 64 or 128).  ``window``: a token reads the keys of the last
+    so many positions only (0: all); ``sink`` (float32 [heads]): exp(sink) joins the softmax's denominator."""
+    _cuda(q, out, k_cache, v_cache, block_table, cu_tokens, seq_slots, seq_starts, seq_new, sink)
     for t, nm in ((block_table, "block_table"), (cu_tokens, "cu_tokens"), (seq_slots, "seq_slots"),
                   (seq_starts, "seq_starts"), (seq_new, "seq_new")):
         _i32(t, nm)
@@ -1857,12 +1915,34 @@ def attention_tcgen05(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache
     _need(k_cache.is_contiguous() and v_cache.is_contiguous()
           and tuple(k_cache.shape[1:]) == (num_kv_heads, PAGE, head_dim), "attention_tcgen05: cache layout")
     _need(q.shape[0] >= n_rows, "attention_tcgen05: q rows")
+    _need(scale > 0 and (sink is None or (sink.dtype == torch.float32 and sink.is_contiguous() and sink.numel() == num_heads)),
+          "attention_tcgen05: a positive scale, a sink per head")
     cache_rows = k_cache.shape[0] * num_kv_heads * PAGE
     _check(lib("attention_tcgen05").kl_attention_tcgen05(
         _ptr(q), q_stride, _ptr(out), _ptr(k_cache), _ptr(v_cache), ctypes.c_longlong(cache_rows), _ptr(block_table),
         block_table.shape[1], _ptr(cu_tokens), _ptr(seq_slots), _ptr(seq_starts), _ptr(seq_new), n_seqs, max_new,
-        q.shape[0], num_heads, num_kv_heads, head_dim, ctypes.c_float(scale), _status_ptr(q.device), _stream()),
+        q.shape[0], num_heads, num_kv_heads, head_dim, ctypes.c_float(scale), int(window or 0), _ptr(sink), _status_ptr(q.device), _stream()),
         "attention_tcgen05")
+
+
+# Keys that a token sees from which a step with a window or a sink takes tcgen05 with heads of 64, in groups of two and more heads / alone; heads
+# of 128 take it from the first on.  us on mma.sync / tcgen05, 32 heads: of 64 on 8, window 1,024, prompts of 6,000 tokens 200 / 113, 32 tokens
+# after 500 16.7 / 14.9, one prompt of 128 6.0 / 8.0, of 32 4.4 / 5.1; window 128, 2,048 tokens 26 / 22, prompts of 6,000 63 / 57; window 16, 41 /
+# 46; of 128 on 8, window 1,024, prompts of 6,000 341 / 136, 128 tokens 9.4 / 9.8, 32 tokens 6.5 / 5.8; 16 heads of 64 on 16, window 1,024,
+# 2,048 tokens 49 / 36, 32 tokens after 500 16.5 / 18.7, 64 after 1,000 35.0 / 34.2, window 128, prompts of 6,000 36 / 47.
+TCGEN05_WINDOW_KEYS = (512, 1024)
+
+
+def prefill_on_tcgen05(q: torch.Tensor, q_stride: int, step, num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: int = 0,
+                       sink: Optional[torch.Tensor] = None) -> bool:
+    """Whether a step's softmax attention takes ``attention_tcgen05``: bfloat16 prompts, head sizes of 64 and 128, rows on 16-byte boundaries;
+    with a window or a sink where it is the faster one."""
+    group = num_heads // num_kv_heads
+    if not (q.dtype == torch.bfloat16 and not step.is_decode and PREFILL_KERNEL == "tcgen05" and head_dim in (64, 128) and group <= 128
+            and q_stride % 8 == 0 and q.data_ptr() % 16 == 0 and step.max_new >= 8 and scale > 0):
+        return False
+    keys = min(window or step.max_context, step.max_context)
+    return (not window and sink is None) or head_dim == 128 or keys >= TCGEN05_WINDOW_KEYS[0 if group > 1 else 1]
 
 
 # Which kernel prefill steps of the bfloat16 path use for head sizes 64 and 128: "tcgen05", or "mma"
@@ -1973,10 +2053,9 @@ def attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.
     sizes, the split-KV kernel; float32 and everything else takes the plain kernel."""
     bf = q.dtype == torch.bfloat16
     group = num_heads // num_kv_heads
-    if (bf and not step.is_decode and PREFILL_KERNEL == "tcgen05" and head_dim in (64, 128) and not window and group <= 128
-            and q_stride % 8 == 0 and q.data_ptr() % 16 == 0 and step.max_new >= 8):
+    if prefill_on_tcgen05(q, q_stride, step, num_heads, num_kv_heads, head_dim, scale, window):
         attention_tcgen05(q, q_stride, out, k_cache, v_cache, block_table, step.cu_tokens, step.seq_slots, step.seq_starts,
-                          step.seq_new, step.n_seqs, step.max_new, step.n_tokens, num_heads, num_kv_heads, head_dim, scale)
+                          step.seq_new, step.n_seqs, step.max_new, step.n_tokens, num_heads, num_kv_heads, head_dim, scale, window)
     elif (bf and head_dim in MMA_HEAD_DIMS and group <= 16 and (not step.is_decode or DECODE_KERNEL == "mma")
           and q_stride % 2 == 0 and q.data_ptr() % 4 == 0):
         splits = 1

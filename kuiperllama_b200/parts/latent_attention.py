@@ -26,8 +26,10 @@ class LatentAttentionMixer(Mixer):
 
     The scores are computed as (W_uk[h]^T q_n) . c + q_r . k_r and the values as W_uv[h] (sum_j p_j c_j),
     so the kernels see attention of H query heads over ONE key head whose rows [c | k_r] are read from
-    the cache as they lie there, values being the rows' first ``kv_rank`` columns; nothing per head is
-    ever built for a cached token.  W_uk^T and W_uv are applied by one grouped product each.  A layer
+    the cache as they lie there, values being the rows' first ``kv_rank`` columns.  W_uk^T and W_uv are applied by one grouped
+    product each.  bfloat16 prompts of ``ops.LATENT_EXPANDED_FROM`` tokens and more that start at position 0 go the
+    other way round (``ops.latent_expands``): one product makes every head's keys and values of the step's tokens, and the scores and sums run
+    over those; nothing per head is kept.  A layer
     with ``own_latent`` False has no W_dkv and reads the rows that the execution named by the
     schedule's ``cache_from`` wrote.
 
@@ -92,7 +94,12 @@ class LatentAttentionMixer(Mixer):
         # W_uk^T per head, [H, kv_rank, dim]: the product that takes a query's unrotated part to the latent's side
         uk = tensors[prefix + n["uk"]].to(device=dev, dtype=dt).reshape(self.H, self.d, self.r)
         self.uk_t = uk.transpose(1, 2).contiguous()
-        self.uv = tensors[prefix + n["uv"]].to(device=dev, dtype=dt).reshape(self.H, self.dv, self.r).contiguous()
+        uv = tensors[prefix + n["uv"]].to(device=dev, dtype=dt).reshape(self.H * self.dv, self.r)
+        # W_uk and W_uv one above the other: the product that makes every head's own keys and values of a prompt from its latent
+        self.expand = None
+        if self.own and self.gate_kind == "head" and ops.latent_expandable(dt, self.d, self.rd, self.dv, self.r, self.scale):
+            self.expand = Linear(torch.cat([uk.reshape(self.H * self.d, self.r), uv]).contiguous(), runtime)
+        self.uv_alone = uv.contiguous() if self.expand is None else None
         self.o = Linear(tensors[prefix + n["o"]], runtime)
         rot = position.rotary() if position is not None else None
         self.inv_freq, self.rot_dims = rot if rot is not None else (None, 0)
@@ -100,6 +107,11 @@ class LatentAttentionMixer(Mixer):
             raise ValueError(f"{self.rot_dims} rotated dimensions do not fit the rotated part of {self.rd}")
         self.magnitude = float(getattr(position, "magnitude", 1.0)) if position is not None else 1.0
         self.interleaved = getattr(position, "pairing", "half") == "interleaved"
+
+    @property
+    def uv(self) -> torch.Tensor:
+        """W_uv, [H, vdim, kv_rank]."""
+        return (self.uv_alone if self.expand is None else self.expand.weight[self.H * self.d:]).view(self.H, self.dv, self.r)
 
     def kv_request(self) -> Optional[KVRequest]:
         return KVRequest(kv_heads=1, head_dim=self.Dk, kind="keys", window=self.window)
@@ -118,6 +130,16 @@ class LatentAttentionMixer(Mixer):
             qsrc, q_col = self.uq.forward(cq), 0
         else:
             qsrc, q_col = proj, self.inputs.column("q")
+        q = qsrc[:, q_col:q_col + self.H * (self.d + self.rd)]
+        if self.expand is not None and ops.latent_expands(step, q):
+            rows = torch.zeros((ops.latent_rows(step), self.r), dtype=dt, device=dev)
+            ops.latent_prepare(proj, q_col, self.inputs.column("dkv"), self.norm_weight, self.eps, self.inv_freq, self.rot_dims, self.magnitude,
+                               self.interleaved, step.positions, step.token_slot, cache.block_table, cache.k, None, n, self.H, self.d, self.rd,
+                               self.r, q=qsrc, rows=rows, step=step)
+            attn = torch.empty((n, self.H * self.dv), dtype=dt, device=dev)
+            ops.latent_expanded(q, self.expand.forward(rows), attn, cache.k, cache.block_table, step, self.H, self.d, self.rd, self.dv, self.r,
+                                self.scale, self.sink, int(self.window or 0), self.inputs.view("g") if self.gated else None)
+            return self.o.forward(attn, allow_partials=True)
         # rows that belong to no sequence (a small step's padding) are not written by the kernels: keep them defined
         make = torch.zeros if step.padded else torch.empty
         qfull = make((n, self.H * self.Dk), dtype=dt, device=dev)

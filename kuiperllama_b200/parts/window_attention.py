@@ -213,9 +213,13 @@ class WindowAttentionMixer(Mixer):
         window = int(self.window or 0)
         if self.weights == "softmax" and not self.pool and self.sink is None and self.vd == self.hd:
             ops.attention(q, proj.stride(0), attn, cache.k, cache.v, cache.block_table, step, self.H, self.KV, self.hd, self.scale, window)
+        elif (self.KERNEL == "mma" and self.weights == "softmax" and not self.pool and self.vd == self.hd
+              and ops.prefill_on_tcgen05(q, proj.stride(0), step, self.H, self.KV, self.hd, self.scale, window, self.sink)):
+            ops.attention_tcgen05(q, proj.stride(0), attn, cache.k, cache.v, cache.block_table, step.cu_tokens, step.seq_slots, step.seq_starts,
+                                  step.seq_new, step.n_seqs, step.max_new, n, self.H, self.KV, self.hd, self.scale, window, self.sink)
         elif (dt == torch.bfloat16 and self.KERNEL == "mma" and self.vd == self.hd and self.hd in ops.MMA_HEAD_DIMS and self.H // self.KV <= 16
               and proj.stride(0) % 2 == 0 and q.data_ptr() % 4 == 0):
-            # the tensor cores: sink, sigmoid weights and pooled rows are options of the windowed kernel
+            # sink, sigmoid weights and pooled rows are options of the windowed kernel on mma.sync
             splits = 1
             if step.is_decode:
                 splits = ops.decode_attention_splits(step.n_seqs, self.KV, self.hd, getattr(step, "context_class", 0))

@@ -476,3 +476,110 @@ def test_products_on_both_sides_of_the_lines_between_the_ways_round(M, N, K):
     # |d silu / dg| <= 1.1; the two units' exponential and quotient are good to about 2^-20; one rounding to 8 bits
     bound = 1.1 * dg * u.abs() + (g * torch.sigmoid(g)).abs() * du + want.abs() * (2.0 ** -8 + 2.0 ** -18) + 1e-30
     assert bool(((gated.double() - want).abs() <= bound + 1e-6).all())
+
+
+def _softmax_over_keys(sc, hidden, sink):
+    """[T, heads, keys] scores in float64 -> weights; a sink joins the denominator."""
+    sc = sc.masked_fill(hidden, float("-inf"))
+    top = sc.amax(-1, keepdim=True)
+    if sink is not None:
+        top = torch.maximum(top, sink.double()[None, :, None])
+    e = torch.exp(sc - top)
+    return e / (e.sum(-1, keepdim=True) + (0.0 if sink is None else torch.exp(sink.double()[None, :, None] - top)))
+
+
+# heads on key/value heads in groups of 1 to 16; windows of one key, inside a page, over pages and longer than the prompts; portions that
+# start in the middle of a page, whose earlier pages have gone back to the pool
+@pytest.mark.parametrize("H,KV,hd", [(8, 8, 64), (8, 2, 64), (4, 1, 128), (16, 1, 64), (6, 2, 128)])
+@pytest.mark.parametrize("window", [1, 40, 64, 130, 1000, 0])
+@pytest.mark.parametrize("with_sink", [False, True])
+def test_attention_tcgen05_with_windows_and_sinks(H, KV, hd, window, with_sink):
+    """Outputs are off by their own rounding (2^-9) and by the weights' (2^-9 of each): 2^-8 of sum w |v|, and 2^-8 of the result."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator().manual_seed(H + hd + window)
+    bf, pages = torch.bfloat16, 8
+    table = torch.randperm(3 * pages, generator=g).to(torch.int32).view(3, pages)
+    kc, vc = (torch.randn(3 * pages, KV, 64, hd, generator=g).to(bf) for _ in range(2))
+    sink = torch.randn(H, generator=g) * 3 if with_sink else None
+    for starts, news in (([0, 0, 0], [300, 8, 129]), ([100, 63, 200], [30, 12, 256]), ([0, 250, 64], [512, 9, 64])):
+        step = _step(starts, news)
+        q = (2 * torch.randn(step.n_tokens, H * hd + 16, generator=g)).to(bf)
+        k, v, used = kc.clone(), vc.clone(), table.clone()
+        for s, (a, n) in enumerate(zip(starts, news)):
+            before = max(0, a - window + 1) // 64 if window else 0
+            for b in range(before):                        # what a window leaves behind belongs to others now
+                k[int(table[s, b])] = v[int(table[s, b])] = float("nan")
+                used[s, b] = -1
+        out = torch.full((step.n_tokens, H * hd), 9.0, dtype=bf, device=DEV)
+        ops.attention_tcgen05(q.to(DEV)[:, :H * hd], H * hd + 16, out, k.to(DEV), v.to(DEV), used.to(DEV), step.cu_tokens, step.seq_slots, step.seq_starts,
+                              step.seq_new, 3, step.max_new, step.n_tokens, H, KV, hd, hd ** -0.5, window, None if sink is None else sink.to(DEV))
+        ops.check_status(out.device)
+        for s, (a, n) in enumerate(zip(starts, news)):
+            flat = lambda c: c[table[s].long()].permute(1, 0, 2, 3).reshape(KV, pages * 64, hd).double().repeat_interleave(H // KV, 0).to(DEV)
+            i, j = torch.arange(a, a + n, device=DEV)[:, None], torch.arange(pages * 64, device=DEV)[None]
+            hidden = (j > i) | ((i - j >= window) if window else torch.zeros(n, pages * 64, dtype=torch.bool, device=DEV))
+            rows = slice(step.cu[s], step.cu[s + 1])
+            sc = torch.einsum("thd,hjd->thj", q[rows, :H * hd].double().view(n, H, hd).to(DEV), flat(kc)) * hd ** -0.5
+            w = _softmax_over_keys(sc, hidden[:, None], None if sink is None else sink.to(DEV))
+            want, most = torch.einsum("thj,hjd->thd", w, flat(vc)), torch.einsum("thj,hjd->thd", w, flat(vc).abs())
+            off = (out[rows].double().view(n, H, hd) - want).abs()
+            assert bool((off <= 2.0 ** -8 * (want.abs() + most)).all()), (s, float((off / most).max()))
+
+
+# a head's own 64 or 128 columns beside 16 to 64 rotated ones, ranks on both sides of a slab of 64, one to several tiles of 128 rows
+@pytest.mark.parametrize("H,d,rd,r", [(3, 64, 32, 256), (2, 64, 16, 72), (2, 64, 64, 64), (2, 128, 64, 256), (1, 128, 48, 512), (5, 64, 48, 128)])
+@pytest.mark.parametrize("window,with_sink,with_gate", [(0, True, True), (0, False, False), (70, True, False), (300, False, True)])
+def test_latent_attention_with_keys_of_every_heads_own(H, d, rd, r, window, with_sink, with_gate):
+    """Rotation, norm, the rows of the latent, and scores and sums over every head's own keys and values; one prompt's latent is not
+    finite and no other prompt notices.  Keys, values, weights and results are rounded to bfloat16 (2^-9 each); scores are at most a few units, whose
+    errors of 2^-9 from keys and queries the weights pass on."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator().manual_seed(H + d + r + window)
+    bf, news, bad = torch.bfloat16, [300, 128, 7, 200], 2
+    step = _step([0, 0, 0, 0], news)
+    step.host_starts, step.captured, step.padded = [0, 0, 0, 0], False, False
+    n, width = step.n_tokens, H * (d + rd)
+    proj = torch.randn(n, width + r + rd + 8, generator=g).to(bf)
+    proj[step.cu[bad]:step.cu[bad + 1], width:] = float("inf")
+    w_norm, freq = 1 + 0.1 * torch.randn(r, generator=g), torch.rand(rd // 2, generator=g)
+    w = (torch.randn(2 * H * d, r, generator=g) * r ** -0.5).to(bf)
+    sink, gate = torch.randn(H, generator=g), torch.randn(n, H + 8, generator=g).to(bf)
+    table = torch.randperm(24, generator=g).to(torch.int32).view(4, 6).to(DEV)
+    cache = torch.zeros(24, 1, 64, r + rd, dtype=bf, device=DEV)
+    p = proj.to(DEV)
+    q = p[:, :width]
+    assert ops.latent_expands(step, q) and ops.latent_expandable(bf, d, rd, d, r, 0.1)
+    rows = torch.zeros(ops.latent_rows(step), r, dtype=bf, device=DEV)
+    ops.latent_prepare(p, 0, width, w_norm.to(DEV), 1e-6, freq.to(DEV), rd, 1.25, True, step.positions, step.token_slot, table, cache, None, n, H, d, rd, r,
+                       rows=rows, step=step)
+    # against the kernel that leaves the queries where they lie: the same cache, the same rotated parts
+    qfull, other = torch.zeros(n, H * (r + rd), dtype=bf, device=DEV), torch.zeros_like(cache)
+    ops.latent_prepare(proj.to(DEV), 0, width, w_norm.to(DEV), 1e-6, freq.to(DEV), rd, 1.25, True, step.positions, step.token_slot, table, other, qfull, n, H, d, rd, r)
+    same = lambda x, y: torch.equal(x.view(torch.int16), y.view(torch.int16))
+    assert same(cache, other) and same(q.reshape(n, H, d + rd)[..., d:].contiguous(), qfull.view(n, H, r + rd)[..., r:].contiguous())
+    assert same(q.reshape(n, H, d + rd)[..., :d].contiguous(), proj[:, :width].to(DEV).reshape(n, H, d + rd)[..., :d].contiguous())
+    kv = torch.empty(rows.shape[0], 2 * H * d, dtype=bf, device=DEV)
+    ops.matmul(rows, w.to(DEV), kv)
+    scale, out = 0.3 * (d + rd) ** -0.5, torch.full((n, H * d), 9.0, dtype=bf, device=DEV)
+    ops.latent_expanded(q, kv, out, cache, table, step, H, d, rd, d, r, scale, sink.to(DEV) if with_sink else None, window,
+                        gate.to(DEV)[:, 4:4 + H] if with_gate else None)
+    ops.check_status(out.device)
+    for s, m in enumerate(news):
+        if s == bad:
+            continue
+        mine = slice(step.cu[s], step.cu[s + 1])
+        flat = cache[table[s].long()].reshape(-1, r + rd)[:m].double()
+        k, v = (flat[:, :r] @ x.to(DEV).double().T for x in (w[:H * d], w[H * d:]))
+        k = torch.cat([k.view(m, H, d), flat[:, None, r:].expand(m, H, rd)], -1)
+        i, j = torch.arange(m, device=DEV)[:, None], torch.arange(m, device=DEV)[None]
+        hidden = (j > i) | ((i - j >= window) if window else torch.zeros(m, m, dtype=torch.bool, device=DEV))
+        sc = torch.einsum("thd,jhd->thj", q[mine].double().view(m, H, d + rd), k) * scale
+        weight = _softmax_over_keys(sc, hidden[:, None], sink.to(DEV) if with_sink else None)
+        f = torch.sigmoid(gate[mine, 4:4 + H].to(DEV).double())[..., None] if with_gate else 1.0
+        want = torch.einsum("thj,jhd->thd", weight, v.view(m, H, d)) * f
+        most = torch.einsum("thj,jhd->thd", weight, v.view(m, H, d).abs()) * f
+        # a score's error: 2^-9 of |q| |k| over the own columns of k, in root mean square over d terms a few times less
+        err = scale * 2.0 ** -9 * torch.einsum("thd,jhd->thj", q[mine].double().view(m, H, d + rd).abs()[..., :d], k.abs()[..., :d]).amax()
+        off = (out[mine].double().view(m, H, d) - want).abs()
+        assert bool((off <= 2.0 ** -8 * want.abs() + (2.0 ** -7 + 2 * float(err)) * most).all()), (s, float((off / most).max()))
+        assert float((out[mine].double().view(m, H, d) - want).norm() / want.norm()) <= 6e-3
