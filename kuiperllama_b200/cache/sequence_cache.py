@@ -143,6 +143,7 @@ class PagedGroup:
         # so the host may rewrite a row (a slot that is reused) while an earlier step's copy
         # is still queued on the device.
         self.table_host = torch.zeros((n_slots, blocks_per_seq), dtype=torch.int32)
+        self.table_rows = self.table_host.numpy()
         self.table = torch.zeros((n_slots, blocks_per_seq), dtype=torch.int32, device=device)
         # a sequence's pages by block index; a block below the window that was given back is -1
         self.slot_pages: List[List[int]] = [[] for _ in range(n_slots)]
@@ -167,9 +168,8 @@ class PagedGroup:
         need = pages_for(new_length, PAGE)
         if need > len(have):
             fresh = self.pages.take_many(need - len(have))
-            for p in fresh:
-                self.table_host[slot, len(have)] = p
-                have.append(p)
+            self.table_rows[slot, len(have):need] = fresh          # (100 pages one by one into a tensor's elements: 280 us)
+            have.extend(fresh)
             self.dirty.add(slot)
 
     def first_needed(self, old_length: int) -> int:
@@ -249,6 +249,7 @@ class PooledWindowGroup(PagedGroup):
         self.pool_k = torch.zeros(shape + (request.head_dim,), dtype=dtype, device=device)
         self.pool_v = torch.zeros(shape + (request.value_dim or request.head_dim,), dtype=dtype, device=device)
         self.pool_table_host = torch.zeros((n_slots, self.pool_blocks_per_seq), dtype=torch.int32)
+        self.pool_table_rows = self.pool_table_host.numpy()
         self.pool_table = torch.zeros((n_slots, self.pool_blocks_per_seq), dtype=torch.int32, device=device)
         self.pool_slot_pages: List[List[int]] = [[] for _ in range(n_slots)]
         self.pool_dirty: set = set()
@@ -270,9 +271,9 @@ class PooledWindowGroup(PagedGroup):
         have = self.pool_slot_pages[slot]
         need = pages_for(new_length // self.request.pool, PAGE)
         if need > len(have):
-            for p in self.pool_pages.take_many(need - len(have)):
-                self.pool_table_host[slot, len(have)] = p
-                have.append(p)
+            fresh = self.pool_pages.take_many(need - len(have))
+            self.pool_table_rows[slot, len(have):need] = fresh
+            have.extend(fresh)
             self.pool_dirty.add(slot)
 
     def release(self, slot: int) -> None:

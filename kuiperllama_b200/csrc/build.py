@@ -15,6 +15,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -55,6 +56,7 @@ SOURCES: Dict[str, str] = {
     "attention_pooled": "attention_pooled.cu",
     "qkv_conv": "qkv_conv.cu",
     "streams": "streams.cu",
+    "host_tokens": "host_tokens.cpp",
 }
 HEADERS: List[str] = ["common.cuh", "attention_mma.cuh", "tcgen05.cuh", "tma_host.cuh", "attention_decode_noalloc.h"]
 
@@ -67,6 +69,11 @@ NVCC_FLAGS += os.environ.get("KL_NVCC_FLAGS", "").split()
 
 class ExtensionError(RuntimeError):
     """The CUDA extension is missing and cannot be built, or failed to load."""
+
+
+def _host_flags(name: str) -> List[str]:
+    """More flags for a source that talks to the interpreter: its headers."""
+    return ["-I", sysconfig.get_paths()["include"]] if SOURCES[name].endswith(".cpp") else []
 
 
 def find_nvcc() -> str:
@@ -91,6 +98,8 @@ def _source_hash(name: str) -> str:
             h.update(f.encode())
             h.update(fh.read())
     h.update(" ".join(NVCC_FLAGS).encode())
+    if SOURCES[name].endswith(".cpp"):
+        h.update(sys.version.encode())
     return h.hexdigest()
 
 
@@ -136,7 +145,7 @@ def ensure_built(name: str, quiet: bool = False) -> str:
     out_dir = _writable_dir()
     out = os.path.join(out_dir, f"{name}.so")
     tmp = os.path.join(out_dir, f".{name}.{os.getpid()}.{threading.get_ident()}.so")
-    cmd = [nvcc] + NVCC_FLAGS + ["-I", CSRC, "-o", tmp, os.path.join(CSRC, SOURCES[name])]
+    cmd = [nvcc] + NVCC_FLAGS + _host_flags(name) + ["-I", CSRC, "-o", tmp, os.path.join(CSRC, SOURCES[name])]
     if not quiet:
         _say(f"compiling {SOURCES[name]} for sm_100a (first use) ...")
     t0 = time.time()

@@ -13,6 +13,7 @@ buffers, launched as one graph per batch size.
 """
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass, field
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -20,6 +21,7 @@ import numpy as np
 import torch
 
 from ..cache import PAGE, CacheError, SequenceCache
+from ..csrc import build
 from ..parts.base import StepContext
 from .model import DecoderModel
 
@@ -97,6 +99,27 @@ def _places(want: Sequence[int], n: int, slot: int) -> np.ndarray:
     return a.astype(np.int32)
 
 
+_host_tokens = None            # the native routine; False where it cannot be built
+
+
+def _token_ids(tokens: Sequence[int], n: int) -> Tuple[np.ndarray, int, int]:
+    """A sequence's ids as int32 with the smallest and the largest.  Lists and tuples of plain ints go through host_tokens.cpp;
+    whatever it does not take (arrays, other integers) through numpy."""
+    global _host_tokens
+    if _host_tokens is None:
+        try:
+            _host_tokens = ctypes.PyDLL(build.ensure_built("host_tokens")).kl_host_tokens
+            _host_tokens.argtypes = [ctypes.py_object, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_void_p]
+        except (build.ExtensionError, OSError):
+            _host_tokens = False
+    if _host_tokens and type(tokens) in (list, tuple):
+        out, ends = np.empty(n, dtype=np.int32), np.empty(2, dtype=np.int64)
+        if _host_tokens(tokens, out.ctypes.data, n, ends.ctypes.data) == 0:
+            return out, int(ends[0]), int(ends[1])
+    toks = np.asarray(tokens, dtype=np.int64)
+    return toks.astype(np.int32), int(toks.min()), int(toks.max())
+
+
 def context_class(max_context: int) -> int:
     """The class of a step by its longest sequence: 0 up to 16 cache pages, then one class per
     doubling.  A captured decode step is replayed only for steps of its own class, so a part may
@@ -161,11 +184,10 @@ class Engine:
             if n < 1:
                 raise StepError(f"the sequence in slot {s.slot} brings no token")
             places.append(_places(s.want, n, s.slot) if len(s.want) else None)
-            toks = np.asarray(s.tokens, dtype=np.int64)
-            lo, hi = int(toks.min()), int(toks.max())
+            toks, lo, hi = _token_ids(s.tokens, n)
             if lo < 0 or hi >= vocab:
                 raise StepError(f"slot {s.slot}: token id {lo if lo < 0 else hi} is outside the vocabulary of {vocab}")
-            token_arrays.append(toks.astype(np.int32))
+            token_arrays.append(toks)
             slots.append(s.slot)
             starts.append(self.cache.lengths[s.slot])
             news.append(n)

@@ -25,3 +25,30 @@ def test_what_is_no_sequence_of_places_is_refused(want):
     from kuiperllama_b200.engine.step import _places
     with pytest.raises(TypeError):
         _places(want, 5, 3)
+
+
+@pytest.mark.parametrize("tokens", [[5], [3, 0, 127999, 2], (7, 8), [-1, 4], [2 ** 31, 1], [-2 ** 40, 2 ** 40], [True, 2], [1.5, 2], range(4), np.array([3, 9]),
+                                    np.array([4, 5], dtype=np.int32), [np.int64(6), 7], [2 ** 63, 0], ["a", 1], [[1], [2]], [None]])
+def test_token_ids_are_what_numpy_makes_of_them(tokens):
+    """Lists and tuples of plain ints take a routine of their own; everything else, and every refusal, is numpy's."""
+    from kuiperllama_b200.engine import step
+
+    def by_numpy():
+        a = np.asarray(tokens, dtype=np.int64)
+        return a.astype(np.int32), int(a.min()), int(a.max())
+
+    try:
+        want = by_numpy()
+    except Exception as e:
+        with pytest.raises(type(e)):
+            step._token_ids(tokens, len(tokens))
+        return
+    got = step._token_ids(tokens, len(tokens))
+    assert got[0].dtype == np.int32 and np.array_equal(got[0], want[0]) and got[1:] == want[1:]
+
+
+def test_token_ids_of_a_long_prompt():
+    from kuiperllama_b200.engine import step
+    tokens = [(i * 7919) % 128256 for i in range(5000)]
+    ids, lo, hi = step._token_ids(tokens, len(tokens))
+    assert ids.tolist() == tokens and (lo, hi) == (min(tokens), max(tokens)) and step._host_tokens
