@@ -47,6 +47,7 @@ SOURCES: Dict[str, str] = {
     "short_conv": "short_conv.cu",
     "outer_recurrence": "outer_recurrence.cu",
     "outer_chunked": "outer_chunked.cu",
+    "delta_chunked": "delta_chunked.cu",
     "mlstm": "mlstm.cu",
     "mlstm_chunked": "mlstm_chunked.cu",
     "attention_mixed": "attention_mixed.cu",
@@ -58,7 +59,7 @@ SOURCES: Dict[str, str] = {
     "streams": "streams.cu",
     "host_tokens": "host_tokens.cpp",
 }
-HEADERS: List[str] = ["common.cuh", "attention_mma.cuh", "tcgen05.cuh", "tma_host.cuh", "attention_decode_noalloc.h"]
+HEADERS: List[str] = ["common.cuh", "attention_mma.cuh", "tcgen05.cuh", "pieces.cuh", "tma_host.cuh", "attention_decode_noalloc.h"]
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared", "--expt-relaxed-constexpr", "--extended-lambda"]

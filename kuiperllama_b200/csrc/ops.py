@@ -31,7 +31,7 @@ _libs: Dict[str, ctypes.CDLL] = {}
 _lock = threading.Lock()
 
 
-_LONG_RESULTS = {"outer_chunked": ("kl_outer_chunked_scratch",)}      # entry points that return a long long
+_LONG_RESULTS = {"outer_chunked": ("kl_outer_chunked_scratch",), "delta_chunked": ("kl_delta_chunked_scratch",)}      # entry points that return a long long
 
 
 def lib(name: str) -> ctypes.CDLL:
@@ -419,13 +419,21 @@ def mingru_scan(proj: torch.Tensor, z_col: int, x_col: int, g_col: int, bias_z: 
                                            dtype_code(proj.dtype), _stream()), "mingru_scan", launches)
 
 
+# A bfloat16 step takes the chunked form from this many tokens of its longest sequence on, with at least so many rows for every sequence.  us
+# walked / in chunks, 16 heads of 128 x 128 on 4: one sequence of 64 tokens 25.1 / 28.5, 96 31.0 / 29.9, 128 37.5 / 32.0, 512 120 / 56, 2,048 444 / 169,
+# eight of 64 80 / 67, one of 64 beside 31 single tokens 42 / 150; 32 heads of 64 x 64 on 8, 64 21.6 / 25.6, 128 32.9 / 30.2, 32 of 64 134 / 162;
+# 4 heads of 128 x 128, eight of 64 29.6 / 34.1.
+DELTA_CHUNKED_FROM, DELTA_CHUNKED_ROWS = 96, 64
+
+
 def gated_delta_rule(proj: torch.Tensor, conv_col: int, b_col: int, a_col: int, conv_weight: torch.Tensor, A_log: torch.Tensor,
                      dt_bias: torch.Tensor, state: torch.Tensor, conv_off: int, out: torch.Tensor, step, heads: int, kv_heads: int,
-                     dim: int, vdim: int, q_scale: float, unit_eps: float) -> None:
+                     dim: int, vdim: int, q_scale: float, unit_eps: float, *, chunked: Optional[bool] = None) -> None:
     """The gated delta rule over a ragged step (see recurrent.cu).  ``proj`` holds q | k | v at
     ``conv_col`` and the projections of beta and of the decay at ``b_col`` and ``a_col``;
     ``conv_weight`` float32 [2 G d + H dv, taps]; ``state`` float32 [slots, S | convolution state];
-    ``out`` float32 [rows, H * dv]."""
+    ``out`` float32 [rows, H * dv].  ``chunked``: True for chunks on the tensor cores (delta_chunked.cu, bfloat16 ``proj``), False for token by
+    token, None by the sizes."""
     _cuda(proj, conv_weight, A_log, dt_bias, state, out)
     C = 2 * kv_heads * dim + heads * vdim
     taps = conv_weight.shape[1]
@@ -438,6 +446,19 @@ def gated_delta_rule(proj: torch.Tensor, conv_col: int, b_col: int, a_col: int, 
           and state.shape[1] >= conv_off + (taps - 1) * C and conv_off >= heads * vdim * dim, "gated_delta_rule: state")
     _need(out.dtype == torch.float32 and out.is_contiguous() and out.shape[0] >= n and out.shape[1] == heads * vdim, "gated_delta_rule: out")
     _need(dim <= 256, f"gated_delta_rule: key size {dim} is above 256")
+    if chunked or (chunked is None and step.max_new >= DELTA_CHUNKED_FROM and n >= DELTA_CHUNKED_ROWS * step.n_seqs):
+        need = -1
+        if proj.dtype == torch.bfloat16 and proj.data_ptr() % 8 == 0 and proj.stride(0) % 4 == 0 and conv_col % 4 == 0:
+            need = lib("delta_chunked").kl_delta_chunked_scratch(n, step.n_seqs, heads, kv_heads, dim, vdim, taps)
+        if need >= 0:
+            scratch = torch.empty(need, dtype=torch.uint8, device=proj.device)
+            _check(lib("delta_chunked").kl_delta_chunked(
+                _ptr(proj), ctypes.c_longlong(proj.stride(0)), conv_col, b_col, a_col, _ptr(conv_weight), taps, _ptr(A_log), _ptr(dt_bias),
+                _ptr(state), ctypes.c_longlong(state.stride(0)), ctypes.c_longlong(conv_off), _ptr(out), _ptr(scratch), _ptr(step.cu_tokens),
+                _ptr(step.seq_slots), n, step.n_seqs, int(step.max_new), heads, kv_heads, dim, vdim, ctypes.c_float(q_scale), ctypes.c_float(unit_eps),
+                _stream()), "gated_delta_rule", 3)
+            return
+        _need(not chunked, "gated_delta_rule: the chunked form does not run these operands")
     prep = torch.empty((n, C), dtype=torch.float32, device=proj.device)
     bg = torch.empty((n, 2 * heads + kv_heads), dtype=torch.float32, device=proj.device)
     _check(lib("recurrent").kl_gated_delta_rule(

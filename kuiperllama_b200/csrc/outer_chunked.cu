@@ -28,7 +28,7 @@
 // 2,222 tokens of the former 585 / 266.  Error of y against 64 bits, one sequence of 200 tokens: 1.08e-7 / 1.06e-7 and 1.06e-7 / 1.17e-7.
 //
 // ExiledOfCode/KuiperLLama has no recurrent mixer (its mixer is mha_kernel.cu:61,74-106).
-#include "tcgen05.cuh"
+#include "pieces.cuh"
 
 namespace kl {
 
@@ -64,82 +64,7 @@ constexpr int OC_PROD = OC * OC_MS + 4, OC_FACS = OC * OC_FAC + 4;             /
 template <int NP> constexpr int oc_k_bytes() { return 3 * OC * NP * 2; }
 template <int NP, int MODE> constexpr int oc_q_bytes() { return oc_k_bytes<NP>() + (MODE == 1 ? 3 * OC * OC * 2 + NP * 4 + 256 : 0); }
 
-// `bytes` (a multiple of 16) that lie together, counted by a barrier
-__device__ __forceinline__ void oc_bulk(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void oc_ldm4(uint32_t a, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
-}
-__device__ __forceinline__ void oc_ldm4t(uint32_t a, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
-}
-__device__ __forceinline__ void oc_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// the same from zero
-__device__ __forceinline__ void oc_mma0(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
-}
-// two numbers as three packed pairs of bfloat16 that add up to them
-__device__ __forceinline__ void oc_split(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    float2 f = __bfloat1622float2(h);
-    x -= f.x; y -= f.y;
-    const __nv_bfloat162 m = __floats2bfloat162_rn(x, y);
-    f = __bfloat1622float2(m);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(x - f.x, y - f.y);
-    a = *reinterpret_cast<const uint32_t*>(&h);
-    b = *reinterpret_cast<const uint32_t*>(&m);
-    c = *reinterpret_cast<const uint32_t*>(&l);
-}
-// the place of 16-byte piece c of row r in a tile of rows of W elements: neighbouring rows' pieces fall on different banks
-template <int W> __device__ __forceinline__ int oc_at(int r, int c) {
-    constexpr int P = W / 8;
-    if constexpr (P >= 8) return r * W + ((c ^ (r & 7)) << 3);
-    else return r * W + ((c ^ ((r / (8 / P)) & (P - 1))) << 3);
-}
 __device__ __forceinline__ bool oc_wild(float x) { return !(fabsf(x) <= OC_MOST); }      // too large, infinite or NaN
-// Operands of three pieces each: d is the leading product, the five others down to 2^-16 of it, smallest first, are added to e.  A product of
-// the tensor cores cuts its sum off where it does not fit 32 bits, so no sum is carried through many of them (8e-7 of y, 1e-7 as it is): d starts
-// from zero and is added with rounding.
-template <int NT, bool FIRST>
-__device__ __forceinline__ void oc_mma33(float (&d)[NT][4], float (&e)[NT][4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][NT][2]) {
-#pragma unroll
-    for (int sum = 2; sum >= 1; --sum)
-#pragma unroll
-        for (int x = sum; x >= 0; --x)
-#pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                if (FIRST && sum == 2 && x == 2) oc_mma0(e[n], a[x], b[sum - x][n][0], b[sum - x][n][1]);
-                else oc_mma(e[n], a[x], b[sum - x][n][0], b[sum - x][n][1]);
-            }
-#pragma unroll
-    for (int n = 0; n < NT; ++n) oc_mma0(d[n], a[0], b[0][n][0], b[0][n][1]);
-}
-template <int NT>
-__device__ __forceinline__ void oc_zero(float (&d)[NT][4]) {
-#pragma unroll
-    for (int n = 0; n < NT; ++n) d[n][0] = d[n][1] = d[n][2] = d[n][3] = 0.f;
-}
-template <int NT>
-__device__ __forceinline__ void oc_add(float (&d)[NT][4], const float (&e)[NT][4]) {
-#pragma unroll
-    for (int n = 0; n < NT; ++n) { d[n][0] += e[n][0]; d[n][1] += e[n][1]; d[n][2] += e[n][2]; d[n][3] += e[n][3]; }
-}
-// B fragments of NT tiles of 8 rows (the columns of the product) for the 16 columns from piece p on; rows of W elements
-template <int W, int NT>
-__device__ __forceinline__ void oc_rows(const bf16* tile, int row0, int p, int lane, uint32_t (&b)[NT][2]) {
-#pragma unroll
-    for (int n = 0; n < NT; n += 2) {
-        uint32_t r[4];
-        oc_ldm4(smem_u32(tile + oc_at<W>(row0 + n * 8 + (lane & 7) + ((lane >> 4) << 3), p + ((lane >> 3) & 1))), r);
-        b[n][0] = r[0]; b[n][1] = r[1]; b[n + 1][0] = r[2]; b[n + 1][1] = r[3];
-    }
-}
 
 // ------------------------------------------------------------------------------------------ what does not depend on S
 // One decay per head.  blockIdx.y < groups: k and q of a group in three pieces, and the products q_scale q_i . k_j of the chunk's tokens.
@@ -217,16 +142,16 @@ oc_group_kernel(const OuterChunkArgs A) {
             for (int u = 0; u < 2; ++u) {
                 const float4 v = x[i][u];
                 wild = wild || oc_wild(v.x) || oc_wild(v.y) || oc_wild(v.z) || oc_wild(v.w);
-                oc_split(v.x, v.y, w[0][2 * u], w[1][2 * u], w[2][2 * u]);
-                oc_split(v.z, v.w, w[0][2 * u + 1], w[1][2 * u + 1], w[2][2 * u + 1]);
+                pc_split(v.x, v.y, w[0][2 * u], w[1][2 * u], w[2][2 * u]);
+                pc_split(v.z, v.w, w[0][2 * u + 1], w[1][2 * u + 1], w[2][2 * u + 1]);
             }
             bf16* tile = which ? Ks : Qs;
             bf16* out = which ? kp : qp;
 #pragma unroll
             for (int y = 0; y < 3; ++y) {
                 const uint4 v = make_uint4(w[y][0], w[y][1], w[y][2], w[y][3]);
-                *reinterpret_cast<uint4*>(tile + y * OC * NP + oc_at<NP>(r, p)) = v;
-                *reinterpret_cast<uint4*>(out + y * OC * NP + oc_at<NP>(r, p)) = v;
+                *reinterpret_cast<uint4*>(tile + y * OC * NP + pc_at<NP>(r, p)) = v;
+                *reinterpret_cast<uint4*>(out + y * OC * NP + pc_at<NP>(r, p)) = v;
             }
         }
     }
@@ -234,8 +159,8 @@ oc_group_kernel(const OuterChunkArgs A) {
     if (threadIdx.x == 0) reinterpret_cast<int*>(prod + OC * OC_MS)[0] = any;
     const int rt = warp & 1, ct = warp >> 1;               // 16 tokens by 16 tokens a warp; nothing above the diagonal is asked for
     float d[2][4], small[2][4];
-    oc_zero<2>(d);
-    oc_zero<2>(small);
+    pc_zero<2>(d);
+    pc_zero<2>(small);
     if (ct <= rt) {
 #pragma unroll 2
         for (int ks = 0; ks < NP / 16; ++ks) {
@@ -243,13 +168,13 @@ oc_group_kernel(const OuterChunkArgs A) {
             float main[2][4];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                oc_ldm4(smem_u32(Qs + i * OC * NP + oc_at<NP>(rt * 16 + (lane & 15), ks * 2 + (lane >> 4))), a[i]);
-                oc_rows<NP, 2>(Ks + i * OC * NP, ct * 16, ks * 2, lane, b[i]);
+                pc_ldm4(smem_u32(Qs + i * OC * NP + pc_at<NP>(rt * 16 + (lane & 15), ks * 2 + (lane >> 4))), a[i]);
+                pc_rows<NP, 2>(Ks + i * OC * NP, ct * 16, ks * 2, lane, b[i]);
             }
-            oc_mma33<2, false>(main, small, a, b);
-            oc_add<2>(d, main);
+            pc_mma33<2, false>(main, small, a, b);
+            pc_add<2>(d, main);
         }
-        oc_add<2>(d, small);
+        pc_add<2>(d, small);
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -355,8 +280,8 @@ oc_row_kernel(const OuterChunkArgs A) {
     __syncthreads();
     if (warp == 0 && live > 16) {                          // between the blocks
         float d[2][4], small[2][4];
-        oc_zero<2>(d);
-        oc_zero<2>(small);
+        pc_zero<2>(d);
+        pc_zero<2>(small);
         const int r = lane >> 2, kc = 2 * (lane & 3);
 #pragma unroll 2
         for (int kk = 0; kk < NP / 16; ++kk) {
@@ -365,14 +290,14 @@ oc_row_kernel(const OuterChunkArgs A) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float2 x = *reinterpret_cast<const float2*>(qs + (16 + r + 8 * (e & 1)) * RS + kk * 16 + kc + 8 * (e >> 1));
-                oc_split(x.x, x.y, a[0][e], a[1][e], a[2][e]);
+                pc_split(x.x, x.y, a[0][e], a[1][e], a[2][e]);
                 const float2 z = *reinterpret_cast<const float2*>(as + (r + 8 * (e & 1)) * RS + kk * 16 + kc + 8 * (e >> 1));
-                oc_split(z.x, z.y, b[0][e & 1][e >> 1], b[1][e & 1][e >> 1], b[2][e & 1][e >> 1]);
+                pc_split(z.x, z.y, b[0][e & 1][e >> 1], b[1][e & 1][e >> 1], b[2][e & 1][e >> 1]);
             }
-            oc_mma33<2, false>(main, small, a, b);
-            oc_add<2>(d, main);
+            pc_mma33<2, false>(main, small, a, b);
+            pc_add<2>(d, main);
         }
-        oc_add<2>(d, small);
+        pc_add<2>(d, small);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             float* o = ms + (16 + r + 8 * i) * OC_MS + kc;
@@ -391,10 +316,10 @@ oc_row_kernel(const OuterChunkArgs A) {
         for (int u = 0; u < 4; ++u) {
             float x = src[2 * u], z = src[2 * u + 1];
             if (f != nullptr) { x *= f[p * 8 + 2 * u]; z *= f[p * 8 + 2 * u + 1]; }
-            oc_split(x, z, w[0][u], w[1][u], w[2][u]);
+            pc_split(x, z, w[0][u], w[1][u], w[2][u]);
         }
 #pragma unroll
-        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(out + i * OC * NP + oc_at<NP>(r, p)) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(out + i * OC * NP + pc_at<NP>(r, p)) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
     }
     float* alpha = reinterpret_cast<float*>(qm + 3 * OC * NP * 2 + 3 * OC * OC * 2);
     for (int n = threadIdx.x; n < NP; n += OC_THREADS) alpha[n] = pre[n] * pre[NP + n];
@@ -405,9 +330,9 @@ oc_row_kernel(const OuterChunkArgs A) {
         bf16* out = reinterpret_cast<bf16*>(qm + 3 * OC * NP * 2);
         uint32_t w[3][4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) oc_split(m[2 * u], m[2 * u + 1], w[0][u], w[1][u], w[2][u]);
+        for (int u = 0; u < 4; ++u) pc_split(m[2 * u], m[2 * u + 1], w[0][u], w[1][u], w[2][u]);
 #pragma unroll
-        for (int x = 0; x < 3; ++x) *reinterpret_cast<uint4*>(out + x * OC * OC + oc_at<OC>(i, q4)) = make_uint4(w[x][0], w[x][1], w[x][2], w[x][3]);
+        for (int x = 0; x < 3; ++x) *reinterpret_cast<uint4*>(out + x * OC * OC + pc_at<OC>(i, q4)) = make_uint4(w[x][0], w[x][1], w[x][2], w[x][3]);
     }
 }
 
@@ -500,16 +425,16 @@ oc_walk_kernel(const OuterChunkArgs A) {
         if (threadIdx.x == 0 && c < chunks) {
             const int b = c & 1;
             mbar_expect_tx(bars + b, L::Q_BYTES + L::K_BYTES);
-            oc_bulk(oc_raw + b * L::Q_BYTES, A.qp + ((entry0 + c) * units + unit) * L::Q_BYTES, L::Q_BYTES, bars + b);
-            oc_bulk(oc_raw + L::K + b * L::K_BYTES, A.kp + ((entry0 + c) * units + unit) * L::K_BYTES, L::K_BYTES, bars + b);
+            pc_bulk(oc_raw + b * L::Q_BYTES, A.qp + ((entry0 + c) * units + unit) * L::Q_BYTES, L::Q_BYTES, bars + b);
+            pc_bulk(oc_raw + L::K + b * L::K_BYTES, A.kp + ((entry0 + c) * units + unit) * L::K_BYTES, L::K_BYTES, bars + b);
         }
     };
     auto copy_factors = [&](int c) {
         if (MODE == 0 && threadIdx.x == 0 && c < chunks) {
             const int b = c & 1;
             mbar_expect_tx(bars + 2 + b, L::F_BYTES);
-            oc_bulk(oc_raw + L::F + b * L::F_BYTES, A.prod + ((entry0 + c) * A.groups + g) * OC_PROD, OC_PROD * 4, bars + 2 + b);
-            oc_bulk(oc_raw + L::F + b * L::F_BYTES + OC_PROD * 4, A.fac + ((entry0 + c) * A.heads + h) * OC_FACS, OC_FACS * 4, bars + 2 + b);
+            pc_bulk(oc_raw + L::F + b * L::F_BYTES, A.prod + ((entry0 + c) * A.groups + g) * OC_PROD, OC_PROD * 4, bars + 2 + b);
+            pc_bulk(oc_raw + L::F + b * L::F_BYTES + OC_PROD * 4, A.fac + ((entry0 + c) * A.heads + h) * OC_FACS, OC_FACS * 4, bars + 2 + b);
         }
     };
     // A copy of this CTA's own always arrives; the limit is there so that no wait is without one (a chunk whose wait ran out goes token by token).
@@ -561,10 +486,10 @@ oc_walk_kernel(const OuterChunkArgs A) {
                 w.w = y.w * (near ? f.w : from * to[3 * OC_FAC]);
             }
             uint32_t pc[3][2];
-            oc_split(w.x, w.y, pc[0][0], pc[1][0], pc[2][0]);
-            oc_split(w.z, w.w, pc[0][1], pc[1][1], pc[2][1]);
+            pc_split(w.x, w.y, pc[0][0], pc[1][0], pc[2][0]);
+            pc_split(w.z, w.w, pc[0][1], pc[1][1], pc[2][1]);
 #pragma unroll
-            for (int y = 0; y < 3; ++y) *reinterpret_cast<uint2*>(Mp + y * OC * OC + oc_at<OC>(i, j0 >> 3) + (j0 & 7)) = make_uint2(pc[y][0], pc[y][1]);
+            for (int y = 0; y < 3; ++y) *reinterpret_cast<uint2*>(Mp + y * OC * OC + pc_at<OC>(i, j0 >> 3) + (j0 & 7)) = make_uint2(pc[y][0], pc[y][1]);
             const float* f = Fs + (nq * 8 + kc) * OC_FAC;
             const float to0 = f[19], to1 = f[OC_FAC + 19];
             next.from[0] = A.q_scale * f[16];
@@ -573,8 +498,8 @@ oc_walk_kernel(const OuterChunkArgs A) {
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 uint32_t p[3], d[3];
-                oc_split(x[e].x, x[e].y, p[0], p[1], p[2]);
-                oc_split(x[e].x * to0, x[e].y * to1, d[0], d[1], d[2]);
+                pc_split(x[e].x, x[e].y, p[0], p[1], p[2]);
+                pc_split(x[e].x * to0, x[e].y * to1, d[0], d[1], d[2]);
 #pragma unroll
                 for (int y = 0; y < 3; ++y) { mine[y * 128 + e] = p[y]; mine[768 + y * 128 + e] = d[y]; }
             }
@@ -620,7 +545,7 @@ oc_walk_kernel(const OuterChunkArgs A) {
     // where a lane reads pieces of q (rows of tokens) and k (rows of tokens, turned): the piece of a step by exclusive or
     const uint32_t q_lane = smem_u32(oc_raw) + ((lane & 7) + ((lane >> 4) << 3)) * NP * 2 + ((((lane >> 3) & 1) ^ (lane & 7)) << 4);
     const uint32_t k_lane = smem_u32(oc_raw + L::K) + (lane & 15) * NP * 2 + (((lane >> 4) ^ (lane & 7)) << 4);
-    const uint32_t m_lane = smem_u32(oc_raw + (MODE == 1 ? oc_k_bytes<NP>() : L::M)) + oc_at<OC>(nq * 8 + (lane & 7), lane >> 3) * 2;
+    const uint32_t m_lane = smem_u32(oc_raw + (MODE == 1 ? oc_k_bytes<NP>() : L::M)) + pc_at<OC>(nq * 8 + (lane & 7), lane >> 3) * 2;
     float mine[4], from[2] = {1.f, 1.f};                   // of the chunk before
     bool left = false;                                     // its y is to be finished
 
@@ -659,21 +584,21 @@ oc_walk_kernel(const OuterChunkArgs A) {
                     uint32_t a[3][4], f[3][4][2];
                     float more[4][4];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) oc_split(S[2 * ks + (e >> 1)][2 * (e & 1)], S[2 * ks + (e >> 1)][2 * (e & 1) + 1], a[0][e], a[1][e], a[2][e]);
+                    for (int e = 0; e < 4; ++e) pc_split(S[2 * ks + (e >> 1)][2 * (e & 1)], S[2 * ks + (e >> 1)][2 * (e & 1) + 1], a[0][e], a[1][e], a[2][e]);
                     const uint32_t at = (q_lane + b * L::Q_BYTES) ^ ((nq * KT + ks) << 5);
 #pragma unroll
                     for (int x = 0; x < 3; ++x)
 #pragma unroll
                         for (int n = 0; n < 4; n += 2) {
                             uint32_t w[4];
-                            oc_ldm4(at + (x * OC + n * 8) * NP * 2, w);
+                            pc_ldm4(at + (x * OC + n * 8) * NP * 2, w);
                             f[x][n][0] = w[0]; f[x][n][1] = w[1]; f[x][n + 1][0] = w[2]; f[x][n + 1][1] = w[3];
                         }
                     if (ks == 0) {
-                        oc_mma33<4, true>(Y, small, a, f);
+                        pc_mma33<4, true>(Y, small, a, f);
                     } else {
-                        oc_mma33<4, false>(more, small, a, f);
-                        oc_add<4>(Y, more);
+                        pc_mma33<4, false>(more, small, a, f);
+                        pc_add<4>(Y, more);
                     }
                 }
                 float4* share = shares(b) + warp * 4 * 32;
@@ -694,7 +619,7 @@ oc_walk_kernel(const OuterChunkArgs A) {
 #pragma unroll
                         for (int x = 0; x < 3; ++x) {
                             uint32_t w[4];
-                            oc_ldm4t(at + (x * OC + ks * 16) * NP * 2, w);
+                            pc_ldm4t(at + (x * OC + ks * 16) * NP * 2, w);
                             f[x][n][0] = w[0]; f[x][n][1] = w[1]; f[x][n + 1][0] = w[2]; f[x][n + 1][1] = w[3];
                         }
                     }
@@ -704,11 +629,11 @@ oc_walk_kernel(const OuterChunkArgs A) {
                         const uint32_t a[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                         for (int n = 0; n < ST; ++n)
-                            if (ks == 0) oc_mma0(small[n], a, f[2][n][0], f[2][n][1]); else oc_mma(small[n], a, f[2][n][0], f[2][n][1]);
+                            if (ks == 0) pc_mma0(small[n], a, f[2][n][0], f[2][n][1]); else pc_mma(small[n], a, f[2][n][0], f[2][n][1]);
 #pragma unroll
-                        for (int n = 0; n < ST; ++n) oc_mma(small[n], a, f[1][n][0], f[1][n][1]);
+                        for (int n = 0; n < ST; ++n) pc_mma(small[n], a, f[1][n][0], f[1][n][1]);
 #pragma unroll
-                        for (int n = 0; n < ST; ++n) oc_mma0(ks ? more[n] : main[n], a, f[0][n][0], f[0][n][1]);
+                        for (int n = 0; n < ST; ++n) pc_mma0(ks ? more[n] : main[n], a, f[0][n][0], f[0][n][1]);
                     } else {
                         uint32_t a[3][4];
 #pragma unroll
@@ -716,9 +641,9 @@ oc_walk_kernel(const OuterChunkArgs A) {
                             const uint4 w = V[(ks * 3 + x) * 32];
                             a[x][0] = w.x; a[x][1] = w.y; a[x][2] = w.z; a[x][3] = w.w;
                         }
-                        if (ks == 0) oc_mma33<ST, true>(main, small, a, f); else oc_mma33<ST, false>(more, small, a, f);
+                        if (ks == 0) pc_mma33<ST, true>(main, small, a, f); else pc_mma33<ST, false>(more, small, a, f);
                     }
-                    if (ks) oc_add<ST>(main, more);
+                    if (ks) pc_add<ST>(main, more);
                 }
 #pragma unroll
                 for (int n = 0; n < ST; ++n) {
@@ -735,7 +660,7 @@ oc_walk_kernel(const OuterChunkArgs A) {
                 const uint32_t at = m_lane + b * (MODE == 1 ? L::Q_BYTES : L::M_BYTES);
                 uint32_t m[3][4];
 #pragma unroll
-                for (int x = 0; x < 3; ++x) oc_ldm4(at + x * OC * OC * 2, m[x]);
+                for (int x = 0; x < 3; ++x) pc_ldm4(at + x * OC * OC * 2, m[x]);
                 float own[4], lo[4], hi[4] = {0.f, 0.f, 0.f, 0.f}, more[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) {
@@ -747,16 +672,16 @@ oc_walk_kernel(const OuterChunkArgs A) {
                             a[x][0] = w.x; a[x][1] = w.y; a[x][2] = w.z; a[x][3] = w.w;
                         }
                         if constexpr (MODE == 1) {
-                            if (ks == 0) oc_mma0(lo, a[0], m[2][0], m[2][1]); else oc_mma(lo, a[0], m[2][2], m[2][3]);
-                            oc_mma(hi, a[0], m[1][2 * ks], m[1][2 * ks + 1]);
-                            oc_mma0(ks ? more : own, a[0], m[0][2 * ks], m[0][2 * ks + 1]);
+                            if (ks == 0) pc_mma0(lo, a[0], m[2][0], m[2][1]); else pc_mma(lo, a[0], m[2][2], m[2][3]);
+                            pc_mma(hi, a[0], m[1][2 * ks], m[1][2 * ks + 1]);
+                            pc_mma0(ks ? more : own, a[0], m[0][2 * ks], m[0][2 * ks + 1]);
                         } else {
-                            if (ks == 0) oc_mma0(lo, a[2], m[0][0], m[0][1]); else oc_mma(lo, a[2], m[0][2], m[0][3]);
-                            oc_mma(hi, a[1], m[0][2 * ks], m[0][2 * ks + 1]);
-                            oc_mma0(ks ? more : own, a[0], m[0][2 * ks], m[0][2 * ks + 1]);
-                            oc_mma(lo, a[1], m[1][2 * ks], m[1][2 * ks + 1]);
-                            oc_mma(hi, a[0], m[1][2 * ks], m[1][2 * ks + 1]);
-                            oc_mma(lo, a[0], m[2][2 * ks], m[2][2 * ks + 1]);
+                            if (ks == 0) pc_mma0(lo, a[2], m[0][0], m[0][1]); else pc_mma(lo, a[2], m[0][2], m[0][3]);
+                            pc_mma(hi, a[1], m[0][2 * ks], m[0][2 * ks + 1]);
+                            pc_mma0(ks ? more : own, a[0], m[0][2 * ks], m[0][2 * ks + 1]);
+                            pc_mma(lo, a[1], m[1][2 * ks], m[1][2 * ks + 1]);
+                            pc_mma(hi, a[0], m[1][2 * ks], m[1][2 * ks + 1]);
+                            pc_mma(lo, a[0], m[2][2 * ks], m[2][2 * ks + 1]);
                         }
                     }
                 }

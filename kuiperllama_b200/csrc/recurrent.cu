@@ -9,7 +9,7 @@
 // Both run over a ragged batch (sequence i owns rows cu_tokens[i] .. cu_tokens[i + 1] of the step,
 // in time order) from the state that the cache keeps per slot, and leave the state after the
 // step's last token there: a prompt in one step, in pieces, or token by token gives the same
-// sums in the same order.  State, gates, decays and unit norms are 32-bit; the projections come
+// sums in the same order (bfloat16 prompts of the delta rule go in chunks: delta_chunked.cu).  State, gates, decays and unit norms are 32-bit; the projections come
 // in the compute dtype as column slices of one stacked product (row stride `ld`).
 // ExiledOfCode/KuiperLLama has no recurrent mixer; its one sequence-mixing op is attention over
 // a cache (mha_kernel.cu:61,74-106).

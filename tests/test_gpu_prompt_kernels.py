@@ -583,3 +583,95 @@ def test_latent_attention_with_keys_of_every_heads_own(H, d, rd, r, window, with
         off = (out[mine].double().view(m, H, d) - want).abs()
         assert bool((off <= 2.0 ** -8 * want.abs() + (2.0 ** -7 + 2 * float(err)) * most).all()), (s, float((off / most).max()))
         assert float((out[mine].double().view(m, H, d) - want).norm() / want.norm()) <= 6e-3
+
+
+def _delta_inputs(H, G, d, dv, rows, n_seqs, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    C = 2 * G * d + H * dv
+    room = torch.full((rows, -(-(C + 2 * H + 12) // 4) * 4), float("nan"), dtype=torch.bfloat16, device=DEV)
+    room[:, 4:4 + C + 2 * H] = rand(rows, C + 2 * H)
+    A_log, dt_bias = torch.log(1 + 15 * torch.rand(H, device=DEV, generator=g)), rand(H) - 4.0
+    return dict(proj=room, taps=0.5 * rand(C, 4), A_log=A_log, dt_bias=dt_bias, state=0.1 * rand(n_seqs, H * d * dv + 3 * C + 4), C=C)
+
+
+def _delta(x, step, H, G, d, dv, chunked, scale=0.1):
+    from kuiperllama_b200.csrc import ops
+    state, out = x["state"].clone(), torch.full((step.n_tokens, H * dv), 7.0, device=DEV)
+    ops.gated_delta_rule(x["proj"], 4, 4 + x["C"], 4 + x["C"] + H, x["taps"], x["A_log"], x["dt_bias"], state, H * d * dv, out, step, H, G, d, dv, scale, 1e-6,
+                         chunked=chunked)
+    return out, state
+
+
+# keys of one slab of 64 and of two, with a remainder; values of one 16 and of more than 128; heads that share keys; chunks of one token, of the
+# first block alone, whole ones and remainders
+@pytest.mark.parametrize("H,G,d,dv", [(4, 1, 128, 128), (3, 3, 64, 32), (2, 1, 40, 144), (6, 2, 128, 16), (2, 2, 72, 48)])
+@pytest.mark.parametrize("news", [[200, 1, 33, 64], [96]])
+def test_delta_rule_in_chunks(H, G, d, dv, news):
+    """As exact as token by token, with the convolution from and into its state; both are off by sums of float32 numbers of order one: a few
+    units of 2^-24 a token at most, whose effect the rule itself damps."""
+    step = _step([0] * len(news), news)
+    x = _delta_inputs(H, G, d, dv, step.n_tokens, len(news), d + dv)
+    C, wide, S, want = x["C"], x["proj"].double(), [], []
+    for s in range(len(news)):
+        rows = slice(step.cu[s], step.cu[s + 1])
+        past = x["state"][s, H * d * dv:H * d * dv + 3 * C].double().view(3, C)
+        pad = torch.cat([past, wide[rows, 4:4 + C]])
+        y = sum(pad[j:j + news[s]] * x["taps"].double()[:, j] for j in range(4))
+        y = y * torch.sigmoid(y)
+        q, k, v = y[:, :G * d].view(-1, G, d), y[:, G * d:2 * G * d].view(-1, G, d), y[:, 2 * G * d:].view(-1, H, dv)
+        q, k = ((z / torch.sqrt((z * z).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(H // G, 1) for z in (q, k))
+        beta = torch.sigmoid(wide[rows, 4 + C:4 + C + H])
+        decay = torch.exp(-torch.exp(x["A_log"].double()) * torch.nn.functional.softplus(wide[rows, 4 + C + H:4 + C + 2 * H] + x["dt_bias"].double()))
+        M = x["state"][s, :H * d * dv].double().view(H, d, dv).clone()
+        for t in range(news[s]):
+            M = M * decay[t][:, None, None]
+            M = M + k[t][:, :, None] * (beta[t][:, None] * (v[t] - torch.einsum("hd,hdv->hv", k[t], M)))[:, None]
+            want.append(0.1 * torch.einsum("hd,hdv->hv", q[t], M))
+        S.append(M)
+    want, S = torch.stack(want), torch.stack(S)
+    off = lambda r: (float((r[0].double().view(want.shape) - want).norm() / want.norm()), float((r[1][:, :H * d * dv].double().view(S.shape) - S).norm() / S.norm()))
+    walked, chunked = _delta(x, step, H, G, d, dv, False), _delta(x, step, H, G, d, dv, True)
+    for a, b in zip(off(chunked), off(walked)):
+        assert a <= 1.5 * b + 2 * U and a <= 64 * U
+    assert torch.equal(walked[1][:, H * d * dv:], chunked[1][:, H * d * dv:])              # the convolution's state, and what lies behind it
+    again = _delta(x, step, H, G, d, dv, True)
+    assert torch.equal(again[0], chunked[0]) and torch.equal(again[1], chunked[1])
+
+
+@pytest.mark.parametrize("what", ["q", "k", "v", "beta", "decay", "state", "large"])
+def test_delta_rule_in_chunks_keeps_what_is_not_finite_where_it_arises(what):
+    H, G, d, dv, news = 4, 2, 64, 32, [100, 70]
+    step = _step([0, 0], news)
+    x = _delta_inputs(H, G, d, dv, 170, 2, 3)
+    C, p = x["C"], x["proj"]
+    bad = float("nan")
+    if what == "state":
+        x["state"][1, 77] = float("inf")
+    elif what == "large":
+        p[50, 4 + 2 * G * d + 3] = 1e9
+    else:
+        col = {"q": 4 + 5, "k": 4 + G * d + 70, "v": 4 + 2 * G * d + 40, "beta": 4 + C + 1, "decay": 4 + C + H + 2}[what]
+        p[40, col], p[130, col] = bad, float("inf") if what != "v" else bad
+    (a, sa), (b, sb) = _delta(x, step, H, G, d, dv, False), _delta(x, step, H, G, d, dv, True)
+    for y, z in ((a, b), (sa, sb)):
+        fine = torch.isfinite(y)
+        assert torch.equal(fine, torch.isfinite(z))
+        assert float((y - z)[fine].double().norm()) <= 4e-6 * float(y[fine].double().norm())
+
+
+def test_delta_rule_of_steps_that_the_chunks_do_not_take():
+    """float32 rows (whose bits do not depend on how a prompt is cut), odd sizes, rows between 8-byte boundaries and short sequences go token by token."""
+    from kuiperllama_b200.csrc import ops
+    for d, dv, dtype, shift, news in ((64, 32, torch.float32, 4, [130]), (20, 32, torch.bfloat16, 4, [130]), (64, 20, torch.bfloat16, 4, [130]),
+                                      (64, 32, torch.bfloat16, 3, [130]), (64, 32, torch.bfloat16, 4, [90]), (64, 32, torch.bfloat16, 4, [100, 1, 1, 1])):
+        step = _step([0] * len(news), news)
+        x = _delta_inputs(2, 1, d, dv, step.n_tokens, len(news), d)
+        proj = x["proj"].nan_to_num(0.0).to(dtype)
+        got = []
+        for chunked in (None, False):
+            state, out = x["state"].clone(), torch.empty(step.n_tokens, 2 * dv, device=DEV)
+            ops.gated_delta_rule(proj, shift, shift + x["C"], shift + x["C"] + 2, x["taps"], x["A_log"], x["dt_bias"], state, 2 * d * dv, out, step, 2, 1, d, dv, 0.1,
+                                 1e-6, chunked=chunked)
+            got.append((out, state))
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
