@@ -18,14 +18,15 @@
 //
 // Nothing is rounded to 16 bits.  A 32-bit number enters a product as the sum of three bfloat16 numbers (24 bits of mantissa); of two such
 // operands the six products down to 2^-16 of the leading one are added, smallest first; a bfloat16 operand enters as it is.  Products of
-// decays are made as products (no logarithms, no quotients), at most 32 factors long.
+// decays are made as products (no logarithms, no quotients), at most 32 factors long and rounded once.
 // A chunk in which something is not finite, larger than OC_MOST, or whose decays leave [0, 1], is walked token by token (oc_tokens), so that
 // infinities and NaN stay where they arise: a masked product would pass them on to the tokens before them.
 //
 // What bounds it: a chunk's chain of instructions (2.3 us where the products of mma.m16n8k16, six where there was one, take 0.9 of the tensor
 // cores' time: 38 % busy, 0.33 instructions a cycle and scheduler).  One prompt of 2,048 tokens, us token by token / in chunks: 64 heads of
 // 128 x 64 (state-space) 416 / 151, 16 heads of 64 x 128 with a decay per row (gated linear attention) 374 / 114; three prompts of 446, 1,333 and
-// 2,222 tokens of the former 585 / 266.  Error of y against 64 bits, one sequence of 200 tokens: 1.08e-7 / 1.06e-7 and 1.06e-7 / 1.17e-7.
+// 2,222 tokens of the former 585 / 266.  Error against 64 bits, one sequence of 500 tokens with decays as such layers have: y 1.11e-7 / 1.00e-7 and
+// 1.01e-7 / 1.04e-7, S 7.6e-8 / 6.1e-8 and 7.8e-8 / 6.6e-8.
 //
 // ExiledOfCode/KuiperLLama has no recurrent mixer (its mixer is mha_kernel.cu:61,74-106).
 #include "pieces.cuh"
@@ -90,28 +91,30 @@ oc_group_kernel(const OuterChunkArgs A) {
         float* fac = A.fac + (entry * A.heads + h) * OC_FACS;
         if (lane == 0) reinterpret_cast<int*>(fac + OC * OC_FAC)[0] = any != 0;
         const int t = lane & 15;
-        float pre = a, suf = a;                            // from the block's start to here; from here to its end
+        // (running products in 64 bits: a product of 32 decays is rounded once)
+        double pre = a, suf = a;                           // from the block's start to here; from here to its end
 #pragma unroll
         for (int o = 1; o < 16; o <<= 1) {
-            const float up = __shfl_up_sync(0xffffffffu, pre, o, 16), down = __shfl_down_sync(0xffffffffu, suf, o, 16);
+            const double up = __shfl_up_sync(0xffffffffu, pre, o, 16), down = __shfl_down_sync(0xffffffffu, suf, o, 16);
             if (t >= o) pre *= up;
             if (t + o < 16) suf *= down;
         }
         suf = __shfl_down_sync(0xffffffffu, suf, 1, 16);   // without this token's own
-        if (t == 15) suf = 1.f;
-        const float first = __shfl_sync(0xffffffffu, pre, 15), second = __shfl_sync(0xffffffffu, pre, 31);
-        float d[16], r = 1.f;                              // c_j times the decays from the block's token j (exclusive) to here
+        if (t == 15) suf = 1.0;
+        const double first = __shfl_sync(0xffffffffu, pre, 15), second = __shfl_sync(0xffffffffu, pre, 31);
+        float d[16];                                       // c_j times the decays from the block's token j (exclusive) to here
+        double r = 1.0;
 #pragma unroll
         for (int j = 15; j >= 0; --j) {
             const float aj = __shfl_sync(0xffffffffu, a, j, 16), cj = __shfl_sync(0xffffffffu, c, j, 16);
-            d[j] = j <= t ? cj * r : 0.f;
-            r = j <= t ? r * aj : 1.f;
+            d[j] = j <= t ? (float)(cj * r) : 0.f;
+            r = j <= t ? r * aj : 1.0;
         }
         float4* f = reinterpret_cast<float4*>(fac + lane * OC_FAC);
         const bool in = lane < live;
 #pragma unroll
         for (int j = 0; j < 16; j += 4) f[j / 4] = in ? make_float4(d[j], d[j + 1], d[j + 2], d[j + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
-        f[4] = in ? make_float4(lane < 16 ? pre : first * pre, pre, c * suf, c * (lane < 16 ? suf * second : suf)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        f[4] = in ? make_float4((float)(lane < 16 ? pre : first * pre), (float)pre, (float)(c * suf), (float)(c * (lane < 16 ? suf * second : suf))) : make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
     const int g = blockIdx.y, N = A.N;
@@ -269,13 +272,14 @@ oc_row_kernel(const OuterChunkArgs A) {
     }
     __syncthreads();
     // the decays' products along the tokens of a block: q times those from its start, in as k times those to its end
+    // (running products in 64 bits: a product of 16 decays is rounded once)
     for (int idx = threadIdx.x; idx < 2 * NP; idx += OC_THREADS) {
         const int b = idx / NP, n = idx % NP;
-        float r = 1.f;
-        for (int t = b * 16; t < b * 16 + 16; ++t) { r *= as[t * RS + n]; qs[t * RS + n] *= r; }
-        pre[idx] = r;
-        float f = 1.f;
-        for (int t = b * 16 + 15; t >= b * 16; --t) { const float a = as[t * RS + n]; as[t * RS + n] = ks[t * RS + n] * f; f *= a; }
+        double r = 1.0;
+        for (int t = b * 16; t < b * 16 + 16; ++t) { r *= as[t * RS + n]; qs[t * RS + n] = (float)(qs[t * RS + n] * r); }
+        pre[idx] = (float)r;
+        double f = 1.0;
+        for (int t = b * 16 + 15; t >= b * 16; --t) { const float a = as[t * RS + n]; as[t * RS + n] = (float)(ks[t * RS + n] * f); f *= a; }
     }
     __syncthreads();
     if (warp == 0 && live > 16) {                          // between the blocks
