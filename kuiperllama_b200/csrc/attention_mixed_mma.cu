@@ -14,8 +14,11 @@
 //
 // talk, p and w are 32-bit numbers.  They enter the products as the sum of three bfloat16 numbers (24 bits of mantissa); of two such
 // operands the six products down to 2^-16 of the leading one are added, smallest first, so nothing is rounded to 16 bits.
-// One prompt of 2,048 tokens (32 heads of 64 on 8, window 1,024, 64 kept keys): phase 0 205 us, phase 1 365 us; 950 and 1,292 us with 32-bit
-// multiply-adds throughout (attention_mixed_tiled.cu).
+// What bounds it is the instructions of a score outside the products: 76 of phase 0's with a tanh for every size of x, an exact quotient and a mask
+// for every score, 56 now (0.72 of them a cycle and scheduler; phase 1 98, 0.50), and the tiles' uneven numbers of chunks, which several CTAs share
+// (`splits0` and `splits1`; phase 1's sums then meet in a third launch).  One prompt (32 heads of 64 on 8, window 1,024, 64 kept keys), us: 2,048 tokens 571
+// before, 414 now; 1,024 349 and 163; 64 tokens after 1,500 301 in one piece each and 67 in 16.  With 32-bit multiply-adds throughout
+// (attention_mixed_tiled.cu) 2,242 for 2,048.
 //
 // ExiledOfCode/KuiperLLama's attention is mha_kernel.cu:61,74-106 (one sequence, one query, no window, no bias).
 #include "common.cuh"
@@ -35,10 +38,26 @@ struct MixedMmaArgs {
     const int* block_table; int blocks_per_seq;
     const int* cu_tokens; const int* seq_slots; const int* seq_starts;
     const float* r1; const float* r2; const float* talk;
-    float* ml;                                    // [rows, heads, 2]
+    float* ml;                                    // [splits, rows, heads, 2]
+    float* part;                                  // [splits, rows, heads * dim]: phase 1 in several pieces, or null
+    int rows, splits0, splits1;                   // pieces that a tile's chunks are dealt to, in phase 0 and in phase 1
     int kv_heads, window, keep_first;
     float scale, softcap, out_scale;
+    float scale_cap;                              // scale / softcap
 };
+
+// tanh(x) for |x| <= MX_SMALL: x + x^3 R(x^2) with R of degree four, the best one for the relative error of tanh (2.8e-9 of it; in 32 bits 0.76
+// units in the last place).  Scores under a soft cap lie there as a rule, and this takes seven instructions and no branch.
+constexpr float MX_SMALL = 0.6f;
+__device__ __forceinline__ float mx_tanh(float x) {
+    const float u = x * x;
+    float r = fmaf(-5.895158275961876e-3f, u, 2.0795971155166626e-2f);
+    r = fmaf(r, u, -5.3783830255270004e-2f);
+    r = fmaf(r, u, 0.13331924378871918f);
+    r = fmaf(r, u, -0.33333298563957214f);
+    return fmaf(x * u, r, x);
+}
+
 
 __device__ __forceinline__ uint32_t mx_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mx_ldm4(uint32_t a, uint32_t (&r)[4]) {
@@ -82,6 +101,7 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
     pdl_wait();
     extern __shared__ __align__(128) unsigned char mx_raw[];
     const int s = blockIdx.y, tile = gridDim.x - 1 - blockIdx.x;           // late tiles see the most keys: they start first
+    const int pieces = PHASE == 0 ? A.splits0 : A.splits1, piece = blockIdx.z;
     const int row0 = A.cu_tokens[s] + tile * MX_TQ;
     const int nrows = min(MX_TQ, A.cu_tokens[s + 1] - row0);
     if (nrows <= 0) return;
@@ -102,9 +122,9 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
     float* Ps = reinterpret_cast<float*>(Vs + (PHASE == 1 ? tile_elems : 0)) + WARPS * 2 * MX_BIAS;      // [H][MX_PH] (phase 1)
     bf16* Ts = reinterpret_cast<bf16*>(Ps + H * MX_PH);                    // [3][H][H + 8]: talk in three pieces (phase 1)
 
-    // chunks that neither the window nor the kept first keys reach are skipped
+    // chunks that neither the window nor the kept first keys reach are skipped; this piece has every `pieces`-th
     auto next_chunk = [&](int c) {
-        for (++c; c < n_chunks; ++c)
+        for (c += pieces; c < n_chunks; c += pieces)
             if (c * MX_CH + MX_CH - 1 >= lo_tile || c * MX_CH < keep) break;
         return c;
     };
@@ -120,7 +140,7 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
     };
     auto commit = [&]() { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
-    int c = next_chunk(-1);
+    int c = next_chunk(piece - pieces);
     if (c < n_chunks) copy_chunk(Ks, A.k_cache, c);
     commit();
     if (PHASE == 1 && A.talk != nullptr)
@@ -146,14 +166,18 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
     if (PHASE == 1) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            const float2 x = *reinterpret_cast<const float2*>(A.ml + ((size_t)(row0 + min(r, nrows - 1)) * H + h0 + e) * 2);
-            m[e] = x.x;
-            l[e] = x.y > 0.f ? 1.0f / x.y : 0.f;
+            const float* ml = A.ml + ((size_t)(row0 + min(r, nrows - 1)) * H + h0 + e) * 2;
+            for (int z = 0; z < A.splits0; ++z) m[e] = fmaxf(m[e], ml[(size_t)z * A.rows * H * 2]);
+            for (int z = 0; z < A.splits0; ++z) {          // (a piece that saw nothing: its maximum is -inf, its sum 0)
+                const float2 x = *reinterpret_cast<const float2*>(ml + (size_t)z * A.rows * H * 2);
+                if (x.y > 0.f) l[e] += x.y * expf(x.x - m[e]);
+                else if (!(x.y == 0.f)) l[e] = x.y;        // NaN stays
+            }
+            l[e] = l[e] > 0.f ? 1.0f / l[e] : 0.f;
         }
     }
     const float r1[2] = {A.r1 != nullptr ? A.r1[h0] : 0.f, A.r1 != nullptr ? A.r1[h0 + 1] : 0.f};
     const float r2[2] = {A.r1 != nullptr ? A.r2[h0] : 0.f, A.r1 != nullptr ? A.r2[h0 + 1] : 0.f};
-    const float inv_cap = A.softcap > 0.f ? 1.0f / A.softcap : 0.f;
     const int i = i0 + r;
     float O[PHASE == 1 ? D / 8 : 1][4];
 #pragma unroll
@@ -190,20 +214,51 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
             }
             __syncwarp();
         }
+        if (A.softcap > 0.f) {
+            float most = 0.f;
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+            for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int key = n * 8 + kc + (e & 1), pos = j0 + key;
-                const bool vis = r < nrows && pos <= i && (A.window == 0 || i - pos < A.window || pos < keep);
-                float v = S[n][e] * A.scale;
-                if (A.softcap > 0.f) {                                     // v / cap, the quotient mended by its remainder
-                    const float x = v * inv_cap;                           // (an infinite score has none, and tanh is 1 far before that)
-                    v = A.softcap * tanhf(fabsf(x) < 64.f ? fmaf(fmaf(-x, A.softcap, v), inv_cap, x) : x);
+                for (int e = 0; e < 4; ++e) {
+                    S[n][e] *= A.scale_cap;
+                    most = fmaxf(most, fabsf(S[n][e]));
                 }
-                if (A.r1 != nullptr) v -= bias[(e >> 1) * MX_BIAS + r + (MX_CH - 1) - key];
-                S[n][e] = vis ? v : -INFINITY;
+            if (__any_sync(0xffffffffu, most > MX_SMALL)) {                // (rows past the end repeat the last one's query)
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) S[n][e] = tanhf(S[n][e]);
+            } else {
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) S[n][e] = mx_tanh(S[n][e]);
             }
+        }
+        const float factor = A.softcap > 0.f ? A.softcap : A.scale;
+        if (A.r1 != nullptr) {
+            const float* at = bias + r + (MX_CH - 1) - kc;
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[n][e] = fmaf(S[n][e], factor, -at[(e >> 1) * MX_BIAS - n * 8 - (e & 1)]);
+        } else {
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[n][e] *= factor;
+        }
+        // (a chunk that every token of a whole tile sees has no masks)
+        const bool inside = nrows == MX_TQ && j0 + MX_CH - 1 <= i0 && (A.window == 0 || i_last - j0 < A.window || j0 + MX_CH <= keep);
+        if (!inside)
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int pos = j0 + n * 8 + kc + (e & 1);
+                    const bool vis = r < nrows && pos <= i && (A.window == 0 || i - pos < A.window || pos < keep);
+                    S[n][e] = vis ? S[n][e] : -INFINITY;
+                }
         if constexpr (PHASE == 0) {
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
@@ -311,7 +366,14 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
         for (int e = 0; e < 2; ++e) {
             l[e] += __shfl_xor_sync(0xfu << (lane & ~3), l[e], 1);
             l[e] += __shfl_xor_sync(0xfu << (lane & ~3), l[e], 2);
-            if ((lane & 3) == 0) *reinterpret_cast<float2*>(A.ml + (row * H + h0 + e) * 2) = make_float2(m[e], l[e]);
+            if ((lane & 3) == 0) *reinterpret_cast<float2*>(A.ml + (((size_t)piece * A.rows + row) * H + h0 + e) * 2) = make_float2(m[e], l[e]);
+        }
+    } else if (pieces > 1) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            float* o = A.part + ((size_t)piece * A.rows + row) * H * D + (size_t)(h0 + e) * D + kc;
+#pragma unroll
+            for (int n = 0; n < D / 8; ++n) *reinterpret_cast<float2*>(o + n * 8) = make_float2(O[n][2 * e], O[n][2 * e + 1]);
         }
     } else {
 #pragma unroll
@@ -325,11 +387,32 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
     }
 }
 
+// The pieces of phase 1 put together: four neighbouring columns of a row a thread, pieces in ascending order.
+__global__ void __launch_bounds__(256)
+attention_mixed_mma_reduce_kernel(const MixedMmaArgs A, const int* __restrict__ token_slot, int heads, int dim) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int width = heads * dim / 4;
+    const int idx = blockIdx.x * 256 + threadIdx.x, row = idx / width, c = (idx - row * width) * 4;
+    if (row >= A.rows || token_slot[row] < 0) return;              // (a padding row has no sums)
+    const float* p = A.part + (size_t)row * heads * dim + c;
+    float4 y = *reinterpret_cast<const float4*>(p);
+    for (int z = 1; z < A.splits1; ++z) {
+        const float4 x = *reinterpret_cast<const float4*>(p + (size_t)z * A.rows * heads * dim);
+        y.x += x.x; y.y += x.y; y.z += x.z; y.w += x.w;
+    }
+    float f = A.out_scale;
+    if (A.gate != nullptr) f *= 1.0f / (1.0f + expf(-to_f32(A.gate[row * A.gate_stride + c / dim])));
+    bf16* o = A.out + row * A.out_stride + c;
+    *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(y.x * f, y.y * f);
+    *reinterpret_cast<__nv_bfloat162*>(o + 2) = __floats2bfloat162_rn(y.z * f, y.w * f);
+}
+
 template <int H, int D, int PHASE>
 static int launch_mixed_mma(const MixedMmaArgs& A, dim3 grid, cudaStream_t stream) {
     const size_t smem = mx_smem_bytes(H, D, A.kv_heads, PHASE);
     KL_CUDA(cudaFuncSetAttribute(attention_mixed_mma_kernel<H, D, PHASE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    launch_kernel(attention_mixed_mma_kernel<H, D, PHASE>, grid, H * 16, smem, stream, A);
+    launch_kernel(attention_mixed_mma_kernel<H, D, PHASE>, dim3(grid.x, grid.y, PHASE == 0 ? A.splits0 : A.splits1), H * 16, smem, stream, A);
     KL_LAUNCH_CHECK();
     return KL_OK;
 }
@@ -346,15 +429,17 @@ KL_API int kl_attention_mixed_mma_fits(int heads, int kv_heads, int dim, int vdi
            (dim == 32 || dim == 64) && max_new > 4 && mx_smem_bytes(heads, dim, kv_heads, 1) <= 227 * 1024;
 }
 
-// ml: float32 [rows, heads, 2].  q and out: rows and heads on 4-byte boundaries; the caches on 16-byte ones.
+// ml: float32 [splits0, rows, heads, 2]; part: float32 [splits1, rows, heads * dim] on a 16-byte boundary where splits1 > 1.  q and out: rows and
+// heads on 4-byte boundaries; the caches on 16-byte ones.
 KL_API int kl_attention_mixed_mma(const void* q, long long q_stride, const void* gate, long long gate_stride, void* out, long long out_stride,
                                   const void* k_cache, const void* v_cache, const int* block_table, int blocks_per_seq, const int* cu_tokens,
-                                  const int* seq_slots, const int* seq_starts, int rows, int n_seqs, int max_new, int heads, int kv_heads, int dim,
-                                  float scale, float softcap, const float* r1, const float* r2, const float* talk, int window, int keep_first,
-                                  float out_scale, float* ml, cudaStream_t stream) {
+                                  const int* seq_slots, const int* seq_starts, const int* token_slot, int rows, int n_seqs, int max_new, int heads,
+                                  int kv_heads, int dim, float scale, float softcap, const float* r1, const float* r2, const float* talk, int window,
+                                  int keep_first, float out_scale, int splits0, int splits1, float* ml, float* part, cudaStream_t stream) {
     if (rows <= 0 || n_seqs <= 0 || max_new <= 0) return KL_OK;
     if (!kl_attention_mixed_mma_fits(heads, kv_heads, dim, dim, KL_BF16, max_new) || window < 0 || keep_first < 0 || n_seqs > 65535) return KL_ERR_BAD_SIZE;
-    if ((r1 == nullptr) != (r2 == nullptr) || ml == nullptr) return KL_ERR_BAD_SIZE;
+    if ((r1 == nullptr) != (r2 == nullptr) || ml == nullptr || splits0 < 1 || splits1 < 1 || splits0 > 64 || splits1 > 64) return KL_ERR_BAD_SIZE;
+    if (splits1 > 1 && (part == nullptr || (uintptr_t)part % 16)) return KL_ERR_BAD_ALIGN;
     if (((uintptr_t)q | (uintptr_t)out) % 4 || q_stride % 2 || out_stride % 2 || ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 || (uintptr_t)talk % 8 ||
         (uintptr_t)ml % 8) return KL_ERR_BAD_ALIGN;
     MixedMmaArgs A;
@@ -362,15 +447,22 @@ KL_API int kl_attention_mixed_mma(const void* q, long long q_stride, const void*
     A.k_cache = (const bf16*)k_cache; A.v_cache = (const bf16*)v_cache; A.block_table = block_table; A.blocks_per_seq = blocks_per_seq;
     A.cu_tokens = cu_tokens; A.seq_slots = seq_slots; A.seq_starts = seq_starts; A.r1 = r1; A.r2 = r2; A.talk = talk; A.ml = ml;
     A.kv_heads = kv_heads; A.window = window; A.keep_first = keep_first; A.scale = scale; A.softcap = softcap; A.out_scale = out_scale;
+    A.scale_cap = softcap > 0.f ? (float)((double)scale / (double)softcap) : 0.f;
+    A.rows = rows; A.splits0 = splits0; A.splits1 = splits1; A.part = part;
     const dim3 grid((max_new + MX_TQ - 1) / MX_TQ, n_seqs);
+    int err = KL_OK;
 #define KL_MX(H_, D_)                                                                       \
     do {                                                                                    \
-        const int err = launch_mixed_mma<H_, D_, 0>(A, grid, stream);                       \
-        return err != KL_OK ? err : launch_mixed_mma<H_, D_, 1>(A, grid, stream);           \
+        err = launch_mixed_mma<H_, D_, 0>(A, grid, stream);                                 \
+        if (err == KL_OK) err = launch_mixed_mma<H_, D_, 1>(A, grid, stream);               \
     } while (0)
     if (heads == 32 && dim == 64) KL_MX(32, 64);
-    if (heads == 32) KL_MX(32, 32);
-    if (dim == 64) KL_MX(16, 64);
-    KL_MX(16, 32);
+    else if (heads == 32) KL_MX(32, 32);
+    else if (dim == 64) KL_MX(16, 64);
+    else KL_MX(16, 32);
 #undef KL_MX
+    if (err != KL_OK || splits1 == 1) return err;
+    launch_kernel(attention_mixed_mma_reduce_kernel, (int)(((long long)rows * heads * dim / 4 + 255) / 256), 256, 0, stream, A, token_slot, heads, dim);
+    KL_LAUNCH_CHECK();
+    return KL_OK;
 }

@@ -1359,6 +1359,24 @@ def mixed_attention_splits(n_seqs: int, context_class: int, window: int, keep_fi
     return max(1, min(chunks, want, 32))
 
 
+MIXED_SPLITS = None             # (phase 0, phase 1): fixed numbers of pieces, for comparisons
+
+
+def mixed_prompt_splits(step, window: int, keep_first: int):
+    """(phase 0, phase 1): into how many pieces a prompt's tiles of 8 tokens cut the 32-key chunks that they see, so that few tiles, or tiles of
+    few and of many chunks, still fill the device: about 300 CTAs, twice that many for the light phase 0, never more pieces than chunks.
+    us with one piece each / with these, 32 heads of 64 on 8, window 1,024 and 64 kept keys: 64 tokens 26 / 20, 150 53 / 26, 300 98 / 43, 600 162 / 82,
+    1,024 266 / 163, 2,048 469 / 414, 64 after 1,500 301 / 67, four prompts of 500 216 / 185; 16 heads on 4, 300 tokens 58 / 29, 2,048 247 / 222."""
+    if MIXED_SPLITS is not None:
+        return MIXED_SPLITS
+    chunks = -(-int(step.max_context) // 32)
+    if window:
+        chunks = min(chunks, (int(window) + 31) // 32 + 1 + (int(keep_first or 0) + 31) // 32)
+    tiles = step.n_tokens // 8 + step.n_seqs
+    s1 = max(1, min(chunks, 16, -(-300 // tiles)))
+    return max(1, min(chunks, 16, 2 * s1)), s1
+
+
 def attention_mixed(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                     block_table: torch.Tensor, step, heads: int, kv_heads: int, dim: int, vdim: int, scale: float, softcap: float = 0.0,
                     r1: Optional[torch.Tensor] = None, r2: Optional[torch.Tensor] = None, talk: Optional[torch.Tensor] = None,
@@ -1390,13 +1408,15 @@ def attention_mixed(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Te
         if (M.kl_attention_mixed_mma_fits(heads, kv_heads, dim, vdim, BF16, max_new) and q.stride(0) % 2 == 0 and out.stride(0) % 2 == 0
                 and (q.data_ptr() | out.data_ptr()) % 4 == 0 and (talk is None or talk.data_ptr() % 8 == 0)
                 and (k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0):
-            ml = torch.empty((n, heads, 2), dtype=torch.float32, device=q.device)
+            s0, s1 = mixed_prompt_splits(step, window, keep_first)
+            ml = torch.empty((s0, n, heads, 2), dtype=torch.float32, device=q.device)
+            part = torch.empty((s1, n, heads * dim), dtype=torch.float32, device=q.device) if s1 > 1 else None
             _check(M.kl_attention_mixed_mma(
                 _ptr(q), ctypes.c_longlong(q.stride(0)), _ptr(gate), ctypes.c_longlong(gate.stride(0) if gate is not None else 0), _ptr(out),
                 ctypes.c_longlong(out.stride(0)), _ptr(k_cache), _ptr(v_cache), _ptr(block_table), block_table.shape[1], _ptr(step.cu_tokens),
-                _ptr(step.seq_slots), _ptr(step.seq_starts), n, step.n_seqs, max_new, heads, kv_heads, dim, ctypes.c_float(scale),
-                ctypes.c_float(softcap or 0.0), _ptr(r1), _ptr(r2), _ptr(talk), int(window or 0), int(keep_first or 0),
-                ctypes.c_float(out_scale), _ptr(ml), _stream()), "attention_mixed_mma", 2)
+                _ptr(step.seq_slots), _ptr(step.seq_starts), _ptr(step.token_slot), n, step.n_seqs, max_new, heads, kv_heads, dim,
+                ctypes.c_float(scale), ctypes.c_float(softcap or 0.0), _ptr(r1), _ptr(r2), _ptr(talk), int(window or 0), int(keep_first or 0),
+                ctypes.c_float(out_scale), s0, s1, _ptr(ml), _ptr(part), _stream()), "attention_mixed_mma", 2 if s1 == 1 else 3)
             return
     L = lib("attention_mixed_tiled")
     fits = L.kl_attention_mixed_tiled_fits(heads, kv_heads, dim, vdim, dtype_code(q.dtype), int(talk is not None), max_new)

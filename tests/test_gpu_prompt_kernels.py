@@ -19,7 +19,7 @@ def _step(starts, news):
     for n in news:
         cu.append(cu[-1] + n)
     return SimpleNamespace(n_tokens=cu[-1], n_seqs=len(news), cu_tokens=i32(cu), seq_slots=i32(list(range(len(news)))), seq_starts=i32(starts),
-                           seq_new=i32(news), max_new=max(news), token_slot=i32([s for s, n in enumerate(news) for _ in range(n)]),
+                           seq_new=i32(news), max_new=max(news), max_context=max(a + n for a, n in zip(starts, news)), token_slot=i32([s for s, n in enumerate(news) for _ in range(n)]),
                            positions=i32([a + t for a, n in zip(starts, news) for t in range(n)]), host_new=news, cu=cu)
 
 
@@ -326,6 +326,43 @@ def test_mixed_heads_with_scores_that_overflow(H, G, d):
     assert bool(torch.isfinite(got[1]).all())
     # both round to bfloat16 sums of 32-bit weights of at most sum |talk| of order one
     assert bool(((got[0] - got[1]).abs() <= 2.0 ** -7 * got[1].abs() + 1e-3).all())
+
+
+@pytest.mark.parametrize("H,G,d", [(32, 8, 64), (16, 2, 32)])
+@pytest.mark.parametrize("splits", [(1, 1), (3, 1), (2, 3), (16, 16)])
+def test_mixed_heads_in_pieces(monkeypatch, H, G, d, splits):
+    """However many pieces a tile's chunks are dealt to, also pieces without a chunk, and scores on both sides of where tanh is a polynomial
+    (0.6 of the cap): float64 within what the test above allows."""
+    from kuiperllama_b200.csrc import ops
+    monkeypatch.setattr(ops, "MIXED_SPLITS", splits)
+    g = torch.Generator().manual_seed(H + splits[0])
+    bf, T = torch.bfloat16, 200
+    table = torch.tensor([[3, 0, 2, 1]], dtype=torch.int32, device=DEV)
+    k, v = (torch.randn(T, G, d, generator=g).to(bf).to(DEV) for _ in range(2))
+    kc, vc = torch.zeros(4, G, 64, d, dtype=bf, device=DEV), torch.zeros(4, G, 64, d, dtype=bf, device=DEV)
+    for p in range(T):
+        kc[int(table[0, p // 64]), :, p % 64], vc[int(table[0, p // 64]), :, p % 64] = k[p], v[p]
+    q, gate = torch.randn(T, H, d, generator=g).to(bf).to(DEV), torch.randn(T, H, generator=g).to(bf).to(DEV)
+    q[:100:3] *= 6                                         # (the tiles of the other tokens see small scores alone)
+    r1, r2 = (torch.rand(H, generator=g) * 0.5 + 0.1).to(DEV), (torch.rand(H, generator=g) + 0.05).to(DEV)
+    talk = (torch.eye(H) + 0.3 * torch.randn(H, H, generator=g)).to(DEV)
+    i, j = torch.arange(T, device=DEV)[:, None], torch.arange(T, device=DEV)[None]
+    for starts, news, window, keep in (([0], [T], 0, 0), ([0], [T], 70, 20), ([130], [70], 70, 0), ([195], [5], 0, 0)):
+        step = _step(starts, news)
+        rows = slice(starts[0], T)
+        hidden = (j > i) | ((i - j >= window) & (j >= keep) if window else torch.zeros(T, T, dtype=torch.bool, device=DEV))
+        sc = torch.einsum("ihd,jhd->hij", q.double(), k.double().repeat_interleave(H // G, 1)) * 0.2
+        assert float(sc[:, 104:].abs().max()) < 0.6 * 20 < float(sc[:, :100:3].abs().max())
+        sc = 20.0 * torch.tanh(sc / 20.0) - r1.double()[:, None, None] * torch.log1p(r2.double()[:, None, None] * (i - j).clamp(min=0).double())
+        w = torch.softmax(sc.masked_fill(hidden, float("-inf")), -1)
+        f = torch.sigmoid(gate.double())[..., None]
+        values = v.double().repeat_interleave(H // G, 1)
+        want = (torch.einsum("hg,gij,jhd->ihd", talk.double(), w, values) * f)[rows]
+        most = (torch.einsum("hg,gij,jhd->ihd", talk.double().abs(), w, values.abs()) * f)[rows]
+        out = torch.full((news[0], H * d), 9.0, dtype=bf, device=DEV)
+        ops.attention_mixed(q[rows].reshape(news[0], -1).contiguous(), gate[rows].contiguous(), out, kc, vc, table, step, H, G, d, d, 0.2, 20.0, r1, r2, talk, window, keep, 1.0)
+        off = (out.double().view(want.shape) - want).abs()
+        assert bool((off <= 2.0 ** -8 * want.abs() + 2e-5 * most + 1e-30).all()), (splits, starts, float((off / most).max()))
 
 
 @pytest.mark.parametrize("which", ["keys", "values"])
