@@ -53,6 +53,7 @@ SOURCES: Dict[str, str] = {
     "attention_mixed": "attention_mixed.cu",
     "attention_mixed_tiled": "attention_mixed_tiled.cu",
     "attention_mixed_mma": "attention_mixed_mma.cu",
+    "attention_mixed_token": "attention_mixed_token.cu",
     "qk_prepare": "qk_prepare.cu",
     "attention_pooled": "attention_pooled.cu",
     "qkv_conv": "qkv_conv.cu",

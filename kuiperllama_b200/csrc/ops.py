@@ -1359,6 +1359,22 @@ def mixed_attention_splits(n_seqs: int, context_class: int, window: int, keep_fi
     return max(1, min(chunks, want, 32))
 
 
+def mixed_token_ranks(n_seqs: int, context_class: int, window: int, keep_first: int):
+    """(CTAs a sequence, chunks of 32 keys that each of them is planned for) of attention_mixed_token.cu: 8, 4 or 2 CTAs as long as every sequence's
+    cluster is resident at once with one CTA an SM (of 148 SMs 15 clusters of eight, 33 of four, 74 of two: a cluster stays within its part of the
+    chip), and more where a CTA would otherwise have more than 40 chunks, whose scores it computes twice.  us with 1 / 2 / 4 / 8 CTAs a sequence, 32
+    heads of 64 on 8: 15 sequences of 200 keys 22.5 / 16.8 / 12.7 / 11.2, 16 22.6 / 16.6 / 12.6 / 20.8, 33 22.8 / 16.6 / 12.9 / 31.3, 34 22.7 / 16.6 /
+    22.2 / 31.7, 74 22.7 / 17.0 / 34.5 / 53.4; 160 of 4,000 506 / 413 / 332 / 400."""
+    chunks = (16 << max(0, int(context_class))) * (PAGE // 32)
+    if window:
+        chunks = min(chunks, (int(window) + 31) // 32 + 1 + (int(keep_first or 0) + 31) // 32)
+    sms, n = sm_count(), int(n_seqs)
+    ranks = 8 if 8 * n <= sms - 28 else 4 if 4 * n <= sms - 16 else 2 if 2 * n <= sms else 1
+    while ranks < 8 and chunks > 40 * ranks:
+        ranks *= 2
+    return ranks, -(-chunks // ranks)
+
+
 MIXED_SPLITS = None             # (phase 0, phase 1): fixed numbers of pieces, for comparisons
 
 
@@ -1386,9 +1402,9 @@ def attention_mixed(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Te
     r1_h ln(1 + r2_h (i - j)) taken off, a sliding window that also keeps the first ``keep_first`` keys, the heads' softmax
     weights mixed by ``talk`` [heads, heads], and head h's result times out_scale * sigmoid(gate[t, h]) (see
     attention_mixed.cu).  ``q`` [rows, heads * dim], ``gate`` [rows, heads], ``out`` [rows, heads * vdim]: the compute dtype,
-    any row stride.  Prompts of bfloat16 rows run on the tensor cores where the sizes allow (attention_mixed_mma.cu); else the
-    tiled kernel (attention_mixed_tiled.cu) runs where its shared memory holds the sizes (``tiled=True`` asks for it), else the
-    plain one; ``tiled=False`` asks for the plain one, and ``splits`` (1 to 32) sets into how many pieces a step of single
+    any row stride.  bfloat16 rows run on the tensor cores where the sizes allow: prompts by attention_mixed_mma.cu, steps of single tokens by
+    attention_mixed_token.cu.  Else the tiled kernel (attention_mixed_tiled.cu) runs where its shared memory holds the sizes (``tiled=True`` asks
+    for it), else the plain one; ``tiled=False`` asks for the plain one, and ``splits`` (1 to 32) sets into how many pieces a step of single
     tokens cuts each sequence's keys instead of ``mixed_attention_splits``."""
     _cuda(q, gate, out, k_cache, v_cache, block_table, r1, r2, talk)
     _i32(block_table, "block_table")
@@ -1417,6 +1433,19 @@ def attention_mixed(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Te
                 _ptr(step.seq_slots), _ptr(step.seq_starts), _ptr(step.token_slot), n, step.n_seqs, max_new, heads, kv_heads, dim,
                 ctypes.c_float(scale), ctypes.c_float(softcap or 0.0), _ptr(r1), _ptr(r2), _ptr(talk), int(window or 0), int(keep_first or 0),
                 ctypes.c_float(out_scale), s0, s1, _ptr(ml), _ptr(part), _stream()), "attention_mixed_mma", 2 if s1 == 1 else 3)
+            return
+    if tiled is None and splits is None and q.dtype == torch.bfloat16 and max_new == 1:
+        M = lib("attention_mixed_token")
+        if (M.kl_attention_mixed_token_fits(heads, kv_heads, dim, vdim, int(talk is not None)) and q.stride(0) % 2 == 0 and out.stride(0) % 2 == 0
+                and (q.data_ptr() | out.data_ptr()) % 4 == 0 and (k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0 and step.n_seqs <= 65535):
+            ranks, chunks = mixed_token_ranks(step.n_seqs, getattr(step, "context_class", 0), window, keep_first)
+            _check(M.kl_attention_mixed_token(
+                _ptr(q), ctypes.c_longlong(q.stride(0)), _ptr(gate), ctypes.c_longlong(gate.stride(0) if gate is not None else 0), _ptr(out),
+                ctypes.c_longlong(out.stride(0)), _ptr(k_cache), _ptr(v_cache), ctypes.c_longlong(k_cache.shape[0]), _ptr(block_table),
+                block_table.shape[1], _ptr(step.cu_tokens), _ptr(step.seq_slots), _ptr(step.seq_starts), step.n_seqs, heads, kv_heads, dim, ctypes.c_float(scale), ctypes.c_float(softcap or 0.0),
+                _ptr(r1), _ptr(r2), _ptr(talk), int(window or 0), int(keep_first or 0), ctypes.c_float(out_scale), ranks, chunks,
+                _status_ptr(q.device), _stream()),
+                "attention_mixed_token")
             return
     L = lib("attention_mixed_tiled")
     fits = L.kl_attention_mixed_tiled_fits(heads, kv_heads, dim, vdim, dtype_code(q.dtype), int(talk is not None), max_new)

@@ -365,6 +365,81 @@ def test_mixed_heads_in_pieces(monkeypatch, H, G, d, splits):
         assert bool((off <= 2.0 ** -8 * want.abs() + 2e-5 * most + 1e-30).all()), (splits, starts, float((off / most).max()))
 
 
+@pytest.mark.parametrize("H,G,d,n,longest,window,keep", [
+    (32, 8, 64, 3, 2500, 0, 0), (32, 8, 64, 40, 97, 0, 0), (5, 5, 32, 2, 65, 40, 3), (24, 3, 128, 20, 300, 100, 40), (64, 8, 64, 2, 700, 0, 0),
+    (16, 16, 64, 150, 64, 0, 0), (40, 8, 32, 1, 1, 1, 0)])
+def test_mixed_heads_of_single_tokens(H, G, d, n, longest, window, keep):
+    """Clusters of eight, four, two and one CTAs, CTAs without a chunk, chunks with one key and with all, scores in rounds (more chunks than a CTA
+    is planned for), heads that are no whole tiles, NaN in the cache past the last key and in pages of others: float64 within a result's
+    rounding and 2e-5 of the sum's largest terms (32-bit sums of 32-bit numbers)."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator().manual_seed(H + n)
+    bf = torch.bfloat16
+    contexts = [max(1, longest - 31 * (i % 5) - i % 2) for i in range(n)]
+    pages = -(-longest // 64)
+    table = torch.randperm(n * pages, generator=g).to(torch.int32).view(n, pages).to(DEV)
+    kc, vc = (torch.full((n * pages, G, 64, d), float("nan"), dtype=bf, device=DEV) for _ in range(2))
+    ks, vs = [], []
+    for b, c in enumerate(contexts):
+        for cache, kept in ((kc, ks), (vc, vs)):
+            x = torch.full((pages * 64, G, d), float("nan"))
+            x[:c] = torch.randn(c, G, d, generator=g)
+            x = x.to(bf).to(DEV)
+            cache[table[b].long()] = x.view(pages, 64, G, d).transpose(1, 2)
+            kept.append(x[:c].double().repeat_interleave(H // G, 1))
+    q, gate = torch.randn(n, H, d, generator=g).to(bf).to(DEV), torch.randn(n, H, generator=g).to(bf).to(DEV)
+    q[::2] *= 6                                            # (scores on both sides of where tanh is a polynomial)
+    r1, r2 = (torch.rand(H, generator=g) * 0.5 + 0.1).to(DEV), (torch.rand(H, generator=g) + 0.05).to(DEV)
+    talk = (torch.eye(H) + 0.3 * torch.randn(H, H, generator=g)).to(DEV)
+    step = _step([c - 1 for c in contexts], [1] * n)
+    for full in (True, False):
+        out = torch.full((n, H * d), 9.0, dtype=bf, device=DEV)
+        ops.attention_mixed(q.view(n, -1), gate if full else None, out, kc, vc, table, step, H, G, d, d, 0.2, 20.0 if full else 0.0, r1 if full else None,
+                            r2 if full else None, talk if full else None, window, keep, 1.5)
+        for b, c in enumerate(contexts):
+            away = torch.arange(c - 1, -1, -1, device=DEV).double()
+            sc = torch.einsum("hd,jhd->hj", q[b].double(), ks[b]) * 0.2
+            if full:
+                sc = 20.0 * torch.tanh(sc / 20.0) - r1.double()[:, None] * torch.log1p(r2.double()[:, None] * away)
+            if window:
+                sc = sc.masked_fill((away >= window) & (torch.arange(c, device=DEV) >= keep), float("-inf"))
+            w, f = torch.softmax(sc, -1), torch.full((H, 1), 1.5, dtype=torch.float64, device=DEV)
+            mixed, mass = (talk.double() @ w, talk.double().abs() @ w) if full else (w, w)
+            if full:
+                f = f * torch.sigmoid(gate[b].double())[:, None]
+            want, most = torch.einsum("hj,jhd->hd", mixed, vs[b]) * f, torch.einsum("hj,jhd->hd", mass, vs[b].abs()) * f
+            off = (out[b].double().view(H, d) - want).abs()
+            assert bool((off <= 2.0 ** -8 * want.abs() + 2e-5 * most + 1e-30).all()), (b, c, full, float((off / most).max()))
+
+
+@pytest.mark.parametrize("what", ["value inf", "value nan", "key nan", "key inf", "all keys -inf", "talk inf"])
+def test_mixed_heads_of_single_tokens_not_finite(what):
+    """Infinities and NaN come out where the kernel of 32-bit multiply-adds has them, as the same."""
+    from kuiperllama_b200.csrc import ops
+    H, G, d, n, T, bf = 8, 2, 32, 2, 150, torch.bfloat16
+    g = torch.Generator().manual_seed(3)
+    table = torch.tensor([[4, 1, 3], [0, 5, 2]], dtype=torch.int32, device=DEV)
+    kc, vc = (torch.randn(6, G, 64, d, generator=g).to(bf).to(DEV) for _ in range(2))
+    q = torch.rand(n, H * d, generator=g).add(0.1).to(bf).to(DEV)
+    talk = (torch.eye(H) + 0.3 * torch.rand(H, H, generator=g)).to(DEV)
+    if what == "value inf": vc[1, 0, 9, 5] = float("inf")
+    elif what == "value nan": vc[1, 0, 9, 5] = float("nan")
+    elif what == "key nan": kc[4, 1, 7, 3] = float("nan")
+    elif what == "key inf": kc[4, 1, 7, 3] = float("inf")
+    elif what == "all keys -inf": kc[..., 2] = float("-inf")
+    else: talk[3, 2] = float("inf")
+    step, outs = _step([T - 1, T - 2], [1, 1]), []
+    for tiled in (None, True):
+        for mix in (talk, None):
+            out = torch.full((n, H * d), 9.0, dtype=bf, device=DEV)
+            ops.attention_mixed(q, None, out, kc, vc, table, step, H, G, d, d, 0.1, 0.0, None, None, mix, 60 if what == "key inf" else 0, 8, 1.0, tiled=tiled)
+            outs.append(out.float())
+    for new, old in zip(outs[:2], outs[2:]):
+        assert bool((new.isnan() == old.isnan()).all()) and bool((new.isinf() == old.isinf()).all())
+        assert bool(((new - old).abs()[new.isfinite()] <= 2.0 ** -7 * old.abs()[new.isfinite()] + 1e-3).all())
+        assert bool((new[new.isinf()] == old[new.isinf()]).all())
+
+
 @pytest.mark.parametrize("which", ["keys", "values"])
 def test_mixed_heads_of_caches_on_eight_bytes(which):
     """A cache that starts between two 16-byte boundaries is served as before, by the kernel that copies smaller pieces."""
