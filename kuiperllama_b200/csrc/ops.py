@@ -515,10 +515,10 @@ def attention_simt(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: t
                    block_table: torch.Tensor, positions: torch.Tensor, token_slot: torch.Tensor, n_tokens: int,
                    num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: int = 0,
                    value_dim: Optional[int] = None, sink: Optional[torch.Tensor] = None, *, chunk: int = 0,
-                   distance_bias: Optional[torch.Tensor] = None, runs: bool = False, few_keys: bool = False) -> None:
-    """out[t, h] = softmax(scale * q[t, h] . K[slot_t, lo..pos_t]) V over the paged cache.  ``runs``: most rows follow the row
-    before them in the same sequence and read hundreds of keys, as a long prompt's do; ``few_keys``: no
-    row reads more than a few dozen (the same results, faster for such rows).  ``value_dim``: the
+                   distance_bias: Optional[torch.Tensor] = None, runs: int = 0, few_keys: bool = False) -> None:
+    """out[t, h] = softmax(scale * q[t, h] . K[slot_t, lo..pos_t]) V over the paged cache.  ``runs``: about so many rows follow one
+    another in a sequence, as a prompt's do (True: many, 0: unknown); ``few_keys``: no row reads more than a few dozen
+    keys (the same results, faster for such rows).  ``value_dim``: the
     values are the first so many columns of ``v_cache``'s rows (which may be the key cache itself);
     ``sink``: float32 [heads], exp(sink[h]) joins head h's denominator; ``chunk``: a token reads the keys of its own chunk of so
     many positions (0: no chunks); ``distance_bias``: float32 [heads, n], column min(pos - key, n - 1) is added to the score."""
@@ -534,11 +534,13 @@ def attention_simt(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: t
     _need(0 < vd <= 512, f"attention: value size {vd} must be at most 512")
     _need(num_heads % num_kv_heads == 0, "attention: heads must be a multiple of kv heads")
     _need(sink is None or (sink.dtype == torch.float32 and sink.is_contiguous() and sink.numel() == num_heads), "attention: sink")
+    run = 1 << 20 if runs is True else int(runs)
+    run = -max(run, 1) if few_keys else run
     _check(lib("attention_simt").kl_attention_simt(_ptr(q), q_stride, _ptr(out), _ptr(k_cache), _ptr(v_cache),
                                                    _ptr(block_table), block_table.shape[1], _ptr(positions),
                                                    _ptr(token_slot), n_tokens, num_heads, num_kv_heads, head_dim,
                                                    ctypes.c_float(scale), int(window or 0), vd, int(v_cache.shape[3]), _ptr(sink), int(chunk or 0),
-                                                   _ptr(distance_bias), 0 if distance_bias is None else distance_bias.shape[1], -1 if few_keys else int(bool(runs)),
+                                                   _ptr(distance_bias), 0 if distance_bias is None else distance_bias.shape[1], run,
                                                    dtype_code(q.dtype), _stream()), "attention_simt")
 
 
@@ -2138,8 +2140,11 @@ def attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.
         attention_decode(q, q_stride, out, k_cache, v_cache, block_table, step.positions, step.token_slot, step.n_tokens,
                          num_heads, num_kv_heads, head_dim, scale, window)
     else:
-        # tiles of eight rows: not for short runs (a tile that holds rows of several sequences walks them one after the other: 8 runs of 2
-        # tokens after 500, 32 heads of 64, 210 us against 37) nor for few keys (one prompt of 256 / 777 tokens 96 / 480 us against 97 / 757)
+        # rows together: not where a sequence brings fewer than four (a CTA walks the runs that its rows fall into one after the other: 8 runs of 3
+        # tokens after 500, 32 heads of 64, 136 us against 42 by rows), unless they are few among many
+        runs = step.n_tokens // step.n_seqs
+        if min(step.host_new) < 4 and not (runs >= 16 and step.max_context >= 384):
+            runs = 0
         attention_simt(q, q_stride, out, k_cache, v_cache, block_table, step.positions, step.token_slot, step.n_tokens,
-                       num_heads, num_kv_heads, head_dim, scale, window, runs=step.n_tokens >= 16 * step.n_seqs and step.max_context >= 384,
+                       num_heads, num_kv_heads, head_dim, scale, window, runs=runs,
                        few_keys=step.max_new > 1 and step.max_context <= 64)

@@ -486,6 +486,31 @@ def test_float32_attention_of_runs_has_the_same_bits(H, KV, hd, vd):
             assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2]) and bool(torch.isfinite(got[0]).all()) and bool((got[0][-3:] == 3.0).all())
 
 
+# four and two rows a lane of the kernel of prompts, four, two and one heads together, runs that end within a CTA's rows, single rows between them
+@pytest.mark.parametrize("H,KV,hd,vd,starts,news", [(32, 8, 64, 64, [3, 70, 0], [600, 1, 9]), (16, 8, 32, 28, [0], [619]), (12, 4, 96, 96, [0, 40], [500, 333]),
+                                                    (32, 8, 128, 128, [100, 0], [130, 20]), (20, 10, 36, 64, [0, 5], [90, 100]), (5, 5, 64, 32, [0, 33], [250, 250])])
+def test_float32_attention_of_long_prompts_has_the_same_bits(H, KV, hd, vd, starts, news):
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator().manual_seed(H * hd)
+    pages = 11
+    table = torch.randperm(len(news) * pages, generator=g).to(torch.int32).view(len(news), pages).to(DEV)
+    kc, vc = torch.randn(len(news) * pages, KV, 64, hd, generator=g).to(DEV), torch.randn(len(news) * pages, KV, 64, vd, generator=g).to(DEV)
+    for s, (a, n) in enumerate(zip(starts, news)):
+        for p in range(a + n, pages * 64):
+            kc[int(table[s, p // 64]), :, p % 64], vc[int(table[s, p // 64]), :, p % 64] = float("inf"), float("nan")
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    pos = i32([a + t for a, n in zip(starts, news) for t in range(n)] + [0, 0])
+    slot = i32([s for s, n in enumerate(news) for _ in range(n)] + [-1, -1])
+    q, sink = torch.randn(len(pos), H * hd, generator=g).to(DEV), torch.randn(H, generator=g).to(DEV)
+    for sink in (None, sink):
+        got = []
+        for runs, zeros in ((True, None), (0, torch.zeros(H, 1, device=DEV))):
+            out = torch.full((len(pos), H * vd), 3.0, device=DEV)
+            ops.attention_simt(q, H * hd, out, kc, vc, table, pos, slot, len(pos), H, KV, hd, 0.2, value_dim=vd, sink=sink, distance_bias=zeros, runs=runs)
+            got.append(out)
+        assert torch.equal(got[0], got[1]) and bool(torch.isfinite(got[0]).all()) and bool((got[0][-2:] == 3.0).all())
+
+
 # rows x heads on both sides of what tiles of eight rows, tiles of one row and a CTA per row each take; rows of 32 columns read at a time
 # and a remainder; values in one to sixteen columns a lane
 @pytest.mark.parametrize("H,KV,hd,vd,starts,news", [(8, 2, 64, 64, [0, 200], [390, 56]), (4, 4, 128, 128, [0], [256]), (4, 1, 36, 32, [5, 0], [240, 250]),
