@@ -338,74 +338,93 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const int row = tile_a * TC_BM + quarter * 32 + lane;              // row of the A operand
         const uint32_t taddr = tmem_base + buf * ACC_COLS + ((uint32_t)(quarter * 32) << 16);
         if constexpr (WEIGHT_ROWS) {
+            // A CTA runs this once, with four warps, and nothing hides it: the next 16 tokens come out of tensor memory while these are written, and
+            // what holds for a whole chunk (no factor, every token there, which activation) is asked once for it, not for every number.  With the
+            // questions for every number and each load waited for / so, us: 2,048 x 2,048 in four pieces 64 tokens 6.05 / 4.14, 8 tokens 3.73 / 3.26; 2,048 x
+            // 8,192 in sixteen 10.0 / 8.1; 2,048 x 2,048 whole in bfloat16 64 tokens 10.4 / 8.5.  The loop stays rolled: unrolled for 64 tokens
+            // most of its time went to instruction fetches.
+            const int first = tile_b * BN, tokens = min(BN, args.rows_b - first);
+            auto walk = [&](auto&& use) {
+                uint32_t r[16];
+                if (nkb > 0) tmem_ld16(taddr, r);
+#pragma unroll 1
+                for (int c = 0; c < tokens; c += 16) {
+                    float v[16];
+                    if (nkb > 0) {
+                        tmem_ld16_wait(r);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+                        if (c + 16 < tokens) tmem_ld16(taddr + c + 16, r);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] = 0.f;
+                    }
+                    if (args.scale_ss != nullptr)
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] *= inv_rms[c + j];
+                    use(c, v);
+                }
+                if (nkb > 0) tmem_ld_wait();
+            };
+            // 16 numbers of a feature (column `column` of the output) for tokens first + c ..
+            auto put_bf16 = [&](int c, int column, const float (&v)[16]) {
+                __nv_bfloat16* o = (__nv_bfloat16*)args.out + (size_t)(first + c) * args.ld_out + column;
+                if (c + 16 <= tokens) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j, o += args.ld_out) *o = __float2bfloat16_rn(v[j]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j, o += args.ld_out)
+                        if (c + j < tokens) *o = __float2bfloat16_rn(v[j]);
+                }
+            };
             if (args.swiglu) {
                 // Tile rows 0..63 are gate features, 64..127 the up rows of the same features.  The
                 // warps that hold the up rows pass them through shared memory (the stages are
                 // free: every MMA has read them) to the warps that hold the gate rows.
                 float* xch = reinterpret_cast<float*>(tiles_a);            // [BN tokens][64 features]
                 const int f = (quarter & 1) * 32 + lane;                   // feature within the tile
-                uint32_t r[16];
-                if (ok && quarter >= 2) {
-                    // The loops over the chunks of 16 tokens stay rolled: a CTA runs its epilogue once, and
-                    // unrolled for 64 tokens most of its time went to instruction fetches (64 sequences of the
-                    // 8B shape: 4.94 ms per decode step unrolled, 4.53 ms rolled).
-#pragma unroll 1
-                    for (int c = 0; c < BN; c += 16) {
-                        if (nkb > 0) { tmem_ld16(taddr + c, r); tmem_ld_wait(); }
-                        else {
+                if (ok && quarter >= 2)
+                    walk([&](int c, const float (&v)[16]) {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) r[j] = 0u;
-                        }
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) xch[(c + j) * 64 + f] = __uint_as_float(r[j]) * inv_rms[c + j];
-                    }
-                }
+                        for (int j = 0; j < 16; ++j) xch[(c + j) * 64 + f] = v[j];
+                    });
                 asm volatile("bar.sync 1, 128;" ::: "memory");             // the four epilogue warps, whatever happened
                 if (ok && quarter < 2) {
                     const int feature = tile_a * 64 + f;
-                    __nv_bfloat16* outb = (__nv_bfloat16*)args.out;
-#pragma unroll 1
-                    for (int c = 0; c < BN; c += 16) {
-                        if (nkb > 0) { tmem_ld16(taddr + c, r); tmem_ld_wait(); }
-                        else {
+                    walk([&](int c, float (&v)[16]) {
+                        if (!args.act_custom) {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) r[j] = 0u;
-                        }
-                        if (feature < args.rows_a / 2) {
+                            for (int j = 0; j < 16; ++j) v[j] = silu_mul(v[j], xch[(c + j) * 64 + f]);
+                        } else {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const int m = c + j, token = tile_b * BN + m;
-                                if (token < args.rows_b)
-                                    outb[(size_t)token * args.ld_out + feature] =
-                                        __float2bfloat16_rn(gated_mul(args, __uint_as_float(r[j]) * inv_rms[m], xch[m * 64 + f]));
-                            }
+                            for (int j = 0; j < 16; ++j) v[j] = gated_mul(args, v[j], xch[(c + j) * 64 + f]);
                         }
-                    }
+                        if (feature < args.rows_a / 2) put_bf16(c, feature, v);
+                    });
                 }
             } else if (ok) {
                 // tile rows are output features n, tile columns are tokens m: out[z][m][n]
-                float* out = (float*)args.out + (size_t)blockIdx.z * args.split_stride;
-                __nv_bfloat16* outb = (__nv_bfloat16*)args.out;
-                uint32_t r[16];
-#pragma unroll 1
-                for (int c = 0; c < BN; c += 16) {
-                    if (nkb > 0) { tmem_ld16(taddr + c, r); tmem_ld_wait(); }
-                    else {
+                walk([&](int c, float (&v)[16]) {
+                    if (row >= args.rows_a) return;
+                    if (args.out_f32) {
+                        float* o = (float*)args.out + (size_t)blockIdx.z * args.split_stride + (size_t)(first + c) * args.ld_out + row;
+                        if (c + 16 <= tokens) {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) r[j] = 0u;
+                            for (int j = 0; j < 16; ++j, o += args.ld_out) *o = v[j];
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j, o += args.ld_out)
+                                if (c + j < tokens) *o = v[j];
+                        }
+                        return;
                     }
-                    const int token0 = tile_b * BN + c;
-                    if (row < args.rows_a && args.out_f32) {
+                    if (args.act_plain == 1) {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (token0 + j < args.rows_b) out[(size_t)(token0 + j) * args.ld_out + row] = __uint_as_float(r[j]) * inv_rms[c + j];
-                    } else if (row < args.rows_a) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (token0 + j < args.rows_b)
-                                outb[(size_t)(token0 + j) * args.ld_out + row] = __float2bfloat16_rn(plain_act(args, __uint_as_float(r[j]) * inv_rms[c + j]));
+                        for (int j = 0; j < 16; ++j) v[j] = plain_act(args, v[j]);
                     }
-                }
+                    put_bf16(c, row, v);
+                });
             }
             if (args.sink != nullptr) {
                 // The last CTA of this row tile (over the k cuts) adds all pieces, in ascending order, into

@@ -1614,15 +1614,18 @@ def sm_count(device: Optional[torch.device] = None) -> int:
 
 
 def skinny_splits(N: int, K: int, M: int = 1) -> int:
-    """Into how many pieces the K range is cut for a product with few tokens, so that about two
-    CTAs per SM stream weights: 128 output features per CTA, at least 4 k-blocks of 64 each.
-    Every piece is written as float32 [M, N] and read again by the kernel that adds the pieces, so
-    with many tokens and a short k range fewer pieces are better: their bytes stay under a quarter
-    of the weights' (pieces * M * 4 <= K * 2 / 4)."""
+    """Into how many pieces the K range is cut for a product with few tokens: up to two CTAs per SM that stream weights, 128 output
+    features per CTA, at least 4 k-blocks of 64 each.  Every piece is written as float32 [M, N] and read again by the kernel that adds
+    the pieces, so beyond eight pieces (of a product back to the width, N <= K, which a norm adds, beyond 16,384 columns of pieces, but four at
+    least) what the product gains the reader loses, and with many tokens and a short k range their bytes stay under half of
+    the weights' (pieces * M * 4 <= K * 2 / 2; a quarter beyond 64 tokens).  us with the norm that adds them, 4 / 6 / 8 / 16 pieces: 2,048 x 8,192 8
+    tokens 10.7 / 9.8 / 9.3 / 10.1, 64 12.1 / 10.8 / 11.3 / 12.2; 2,048 x 2,048 8 tokens 5.8 / 5.4 / 5.4 / 6.2; 4,096 x 4,096 8 tokens 9.6 / 9.6 / 10.2 / 14.3, 64
+    11.5 / 11.6 / 12.1 / 16.4; 1,024 x 4,096 24 tokens 7.7 / 7.2 / 6.7 / 6.9; without it 3,072 x 2,048 64 tokens 5.1 / 5.4 / 4.8 / 7.5."""
     tiles = ((N + 127) // 128) * max(1, (M + 127) // 128)    # CTAs per cut: weight tiles x token tiles (of 128 beyond 64 tokens)
     k_blocks = (K + 63) // 64
+    most = 8 if N > K else max(4, min(8, 16384 // N))
     # never more CTAs than the two per SM that are resident at once: one CTA too many is a second round
-    want = max(1, min((2 * sm_count()) // tiles, k_blocks // 4, 32, max(1, K // (8 * max(M, 1)))))
+    want = max(1, min((2 * sm_count()) // tiles, k_blocks // 4, most, max(1, K // ((4 if M <= 64 else 8) * max(M, 1)))))
     per = (k_blocks + want - 1) // want
     return (k_blocks + per - 1) // per
 
@@ -1724,25 +1727,19 @@ def gemm_skinny_stream(w: torch.Tensor, a: torch.Tensor, row_scale=None, sink=No
 # both operands are reused, but a product of 128 tokens and 4,096 features has 32 tiles for 148 SMs,
 # each of which walks all of K.  Measured per product, us with tokens / weights as rows (plain products
 # with their K cuts added up; features x K):
-#   48 tokens:  3,072 x 2,048 8.6 / 9.7, 1,024 x 1,024 5.3 / 7.4, 8,192 x 2,048 9.6 / 13.9, 4,096 x 4,096 14.8 / 13.0, 2,048 x 8,192 25.7 / 12.9
-#   128 tokens: 2,048 x 2,048 9.1 / 14.4, 8,192 x 2,048 10.3 / 21.1, 4,096 x 4,096 15.6 / 18.1, 1,024 x 4,096 14.7 / 13.1, 4,096 x 14,336 45.3 / 35.2
-#   256 tokens: 4,096 x 4,096 15.8 / 23.0, 1,024 x 4,096 14.7 / 17.2, 2,048 x 8,192 27.0 / 19.8
-#   32 tokens:  3,072 x 2,048 8.3 / 7.0, 1,024 x 4,096 14.1 / 7.7
-# (``tokens_first``: the lines of K where tokens as rows win while their tiles run at once.)  The gate/up product cannot cut
-# its K range (its epilogue needs whole sums):
-#   16,384 x 2,048: 16 tokens 17.8 / 14.3, 17 19.2 / 15.1, 31 17.1 / 16.3, 32 13.5 / 16.3, 64 14.1 / 21.4
-#   8,192 x 2,048:  17 tokens 13.5 / 11.3, 31 14.0 / 12.4, 32 9.8 / 12.5
-#   8,192 x 4,096:  8 tokens 25.3 / 15.8, 16 16.7 / 16.6, 17 16.8 / 17.3
-#   8,192 x 1,024:  17 tokens 8.0 / 8.2, 32 7.7 / 9.5, 128 7.2 / 23.5; 16,384 x 1,024: 17 10.5 / 10.2, 31 10.2 / 11.3
-# (tokens as rows are slow while the tokens' own rows hold less than 64K elements, 128 KB, that all CTAs fetch at the same time, the more
-# so the more CTAs there are; the line is measured, its cause in the memory system is not known)
-#   28,672 x 4,096: 16 tokens 41.1 / 39.4, 32 tokens 41.5 / 41.0, 48 tokens 41.8 / 45.7 (more tiles than SMs)
+#   24 tokens:  3,072 x 2,048 8.8 / 6.2, 1,024 x 4,096 14.4 / 5.8
+#   64 tokens:  3,072 x 2,048 9.3 / 7.8, 1,024 x 1,024 6.2 / 5.7, 8,192 x 2,048 10.3 / 13.2, 4,096 x 4,096 15.4 / 13.0, 2,048 x 8,192 26.6 / 11.8
+#   128 tokens: 2,048 x 2,048 9.8 / 10.4, 8,192 x 2,048 11.1 / 18.0, 4,096 x 4,096 16.2 / 15.1, 1,024 x 4,096 15.0 / 9.3, 4,096 x 14,336 46.0 / 30.3
+#   256 tokens: 4,096 x 4,096 16.5 / 19.8, 1,024 x 4,096 15.3 / 13.4, 2,048 x 8,192 27.3 / 16.6
+# (``tokens_first``: the lines where tokens as rows win while their tiles run at once.)  The gate/up product cannot cut
+# its K range (its epilogue needs whole sums); weights as rows to 32 tokens, and to 64 where the tiles of 128 x 128 need a second wave:
+#   16,384 x 2,048: 16 tokens 19.5 / 13.3, 24 18.5 / 14.1, 32 14.6 / 14.2, 33 14.5 / 14.9, 64 14.7 / 15.8
+#   8,192 x 2,048:  17 tokens 14.6 / 10.3, 32 10.8 / 10.3, 48 10.9 / 11.3;  2,048 x 1,024: 16 6.7 / 5.7, 24 6.7 / 6.7, 48 6.7 / 7.2
+#   8,192 x 4,096:  16 tokens 18.4 / 15.9, 32 18.1 / 16.7;  22,016 x 4,096: 32 36.9 / 32.9, 48 36.9 / 34.9, 64 37.2 / 36.0
+#   28,672 x 4,096: 16 tokens 42.7 / 38.7, 32 43.1 / 39.3, 64 43.3 / 42.1, 96 43.7 / 45.1 (more tiles than SMs)
 # The pieces of a cut product that its consumer adds itself (``gemm_skinny_partials``) stay 32-bit numbers: there weights as
 # rows run up to the number of tokens at which the tiles of 128 x 256 reach 0.6 of the SMs.
 SKINNY_MAX_ROWS = 512
-
-
-SWIGLU_WEIGHT_ROWS_MAX = 32     # tokens up to which the gate/up product takes the weights as tile rows (16 where the other way is faster, see above)
 
 
 def one_wave(M: int, N: int) -> bool:
@@ -1750,9 +1747,9 @@ def one_wave(M: int, N: int) -> bool:
     return ((M + 127) // 128) * ((N + 127) // 128) <= sm_count()
 
 
-def weights_as_rows(M: int, N: int, swiglu: bool = False, K: Optional[int] = None) -> bool:
+def weights_as_rows(M: int, N: int, swiglu: bool = False) -> bool:
     if swiglu:
-        return M <= 16 or (M <= SWIGLU_WEIGHT_ROWS_MAX and (not one_wave(M, N) or (K is not None and N >= 8192 and K >= 1536 and M * K < 65536)))
+        return M <= 32 or (M <= 64 and not one_wave(M, N))
     if M <= 64:
         return True
     if M > SKINNY_MAX_ROWS:
@@ -1762,7 +1759,7 @@ def weights_as_rows(M: int, N: int, swiglu: bool = False, K: Optional[int] = Non
 
 def tokens_first(M: int, N: int, K: int) -> bool:
     """Whether a product whose K cuts would be added by a kernel of their own runs with tokens as tile rows all the same."""
-    return M > 32 and one_wave(M, N) and (K <= 2048 or (M > 128 and K <= 4096) or skinny_splits(N, K, M) == 1)
+    return M > 32 and one_wave(M, N) and ((K <= 2048 and (M > 64 or N >= 6144)) or (M > 128 and K <= 4096) or skinny_splits(N, K, M) == 1)
 
 
 def gemm_skinny_partials(a: torch.Tensor, w: torch.Tensor, splits: Optional[int] = None) -> Optional[torch.Tensor]:
@@ -1965,7 +1962,7 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 
 def matmul_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, out: torch.Tensor, activation="silu") -> None:
     """out[M, I] = act(a @ gate^T) * (a @ up^T) in one kernel; ``w_gate_up`` from ``interleave_gate_up``."""
-    if weights_as_rows(a.shape[0], w_gate_up.shape[0], swiglu=True, K=w_gate_up.shape[1]):
+    if weights_as_rows(a.shape[0], w_gate_up.shape[0], swiglu=True):
         gemm_skinny(a, w_gate_up, out, swiglu=True, activation=activation)
     else:
         gemm_tcgen05(a, w_gate_up, out, swiglu=True, activation=activation)
