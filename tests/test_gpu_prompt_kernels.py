@@ -812,3 +812,36 @@ def test_delta_rule_of_steps_that_the_chunks_do_not_take():
                                  1e-6, chunked=chunked)
             got.append((out, state))
         assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+# both sides of where products of few tokens cut K, take the weights as tile rows, and need a second wave of tiles; chunks of 16 tokens with a remainder
+@pytest.mark.parametrize("M,N,K", [(33, 3072, 1024), (48, 6144, 512), (64, 200, 1024), (24, 520, 4096), (17, 1024, 264), (64, 2048, 2048)])
+def test_products_of_few_tokens(M, N, K):
+    """float64 within the rounding of the result and 2^-18 of the sum of the terms' magnitudes (32-bit sums of K terms in any order)."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator().manual_seed(M * N)
+    a, w = torch.randn(M, K, generator=g).bfloat16().to(DEV), torch.randn(N, K, generator=g).bfloat16().to(DEV)
+    want, most = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    ops.matmul(a, w, out)
+    pieces = ops.gemm_skinny_partials(a, w)
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * most).all())
+    assert pieces is None or bool(((pieces.double().sum(0) - want).abs() <= 2.0 ** -18 * most).all())
+
+
+@pytest.mark.parametrize("M,I,K", [(24, 256, 520), (32, 64, 128), (48, 9536, 64), (64, 9536, 72), (33, 512, 192)])
+@pytest.mark.parametrize("activation", ["silu", "relu"])
+def test_gate_up_products_of_few_tokens(M, I, K, activation):
+    """The same; the gate's factor has a slope of at most 1.1, so act(g) u is off by no more than 1.1 |u| dg + |act(g)| du beside the rounding of the
+    result, whose bound of 2^-8 is twice what rounding takes and holds the factor's own error (2^-17 where exp is large)."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator().manual_seed(M + I)
+    a = torch.randn(M, K, generator=g).bfloat16().to(DEV)
+    gate, up = (torch.randn(I, K, generator=g).bfloat16().to(DEV) for _ in range(2))
+    w = ops.interleave_gate_up(gate, up)
+    G, U = a.double() @ gate.double().T, a.double() @ up.double().T
+    dG, dU = (2.0 ** -18 * (a.double().abs() @ x.double().abs().T) for x in (gate, up))
+    act = torch.nn.functional.silu(G) if activation == "silu" else torch.relu(G)
+    out = torch.empty(M, I, dtype=torch.bfloat16, device=DEV)
+    ops.matmul_swiglu(a, w, out, activation)
+    assert bool(((out.double() - act * U).abs() <= 2.0 ** -8 * (act * U).abs() + 1.1 * U.abs() * dG + act.abs() * dU + dG * dU + 1e-30).all())
