@@ -214,16 +214,30 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
             }
             __syncwarp();
         }
+        // (a chunk that every token of a whole tile sees has no masks)
+        const bool inside = nrows == MX_TQ && j0 + MX_CH - 1 <= i0 && (A.window == 0 || i_last - j0 < A.window || j0 + MX_CH <= keep);
+        auto visible = [&](int n, int e) {
+            const int pos = j0 + n * 8 + kc + (e & 1);
+            return r < nrows && pos <= i && (A.window == 0 || i - pos < A.window || pos < keep);
+        };
         if (A.softcap > 0.f) {
-            float most = 0.f;
+            float most = 0.f;                                              // of the lane's visible scores, all of one token: its result does not depend on what it does not see
 #pragma unroll
             for (int n = 0; n < NT; ++n)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    S[n][e] *= A.scale_cap;
-                    most = fmaxf(most, fabsf(S[n][e]));
-                }
-            if (__any_sync(0xffffffffu, most > MX_SMALL)) {                // (rows past the end repeat the last one's query)
+                for (int e = 0; e < 4; ++e) S[n][e] *= A.scale_cap;
+            if (inside) {
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) most = fmaxf(most, fabsf(S[n][e]));
+            } else {
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) most = visible(n, e) ? fmaxf(most, fabsf(S[n][e])) : most;
+            }
+            if (most > MX_SMALL) {
 #pragma unroll
                 for (int n = 0; n < NT; ++n)
 #pragma unroll
@@ -248,17 +262,11 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) S[n][e] *= factor;
         }
-        // (a chunk that every token of a whole tile sees has no masks)
-        const bool inside = nrows == MX_TQ && j0 + MX_CH - 1 <= i0 && (A.window == 0 || i_last - j0 < A.window || j0 + MX_CH <= keep);
         if (!inside)
 #pragma unroll
             for (int n = 0; n < NT; ++n)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int pos = j0 + n * 8 + kc + (e & 1);
-                    const bool vis = r < nrows && pos <= i && (A.window == 0 || i - pos < A.window || pos < keep);
-                    S[n][e] = vis ? S[n][e] : -INFINITY;
-                }
+                for (int e = 0; e < 4; ++e) S[n][e] = visible(n, e) ? S[n][e] : -INFINITY;
         if constexpr (PHASE == 0) {
 #pragma unroll
             for (int e = 0; e < 2; ++e) {

@@ -248,7 +248,9 @@ attention_mixed_token_kernel(const __grid_constant__ CUtensorMap map_k, const __
             if (A.softcap > 0.f) {
                 v *= A.scale_cap;
                 v2 *= A.scale_cap;
-                if (__any_sync(0xffffffffu, fmaxf(fabsf(v), fabsf(v2)) > SMALL)) { v = tanhf(v); v2 = tanhf(v2); }
+                // (asked for every lane's own two scores: past the last key the page holds whatever was there before, and no visible score takes another
+                // form for it)
+                if (vis && fmaxf(fabsf(v), fabsf(v2)) > SMALL) { v = tanhf(v); v2 = tanhf(v2); }
                 else { v = mk_tanh(v); v2 = mk_tanh(v2); }
             }
             const float factor = A.softcap > 0.f ? A.softcap : A.scale;

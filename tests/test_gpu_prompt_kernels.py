@@ -440,6 +440,33 @@ def test_mixed_heads_of_single_tokens_not_finite(what):
         assert bool((new[new.isinf()] == old[new.isinf()]).all())
 
 
+@pytest.mark.parametrize("H,G,d", [(32, 8, 64), (16, 2, 32)])
+@pytest.mark.parametrize("single", [True, False])
+def test_mixed_heads_do_not_notice_keys_that_they_do_not_see(H, G, d, single):
+    """Rows past the last key hold what an earlier sequence left there, and a token's tile holds keys of the tokens after it: whatever those are, the
+    bits stay.  Every score is 1e5 and a little, so that its last bit is seen in the weights."""
+    from kuiperllama_b200.csrc import ops
+    g = torch.Generator().manual_seed(H)
+    bf, T = torch.bfloat16, 44
+    table = torch.zeros(1, 1, dtype=torch.int32, device=DEV)
+    kc, vc = (0.5 * torch.randn(1, G, 64, d, generator=g) for _ in range(2))
+    q = 0.5 * torch.randn(T, H, d, generator=g)
+    kc[..., 0], q[..., 0] = 316.0, 316.0
+    kc[:, :, T:], vc[:, :, T:] = 0.0, 0.0
+    outs = []
+    for far in (False, True):
+        k = kc.clone()
+        if far:
+            k[:, :, T - 1 if not single else T:] = 3000.0  # (scores past the cap)
+        step = _step([T - 1], [1]) if single else _step([0], [T])
+        rows = step.n_tokens
+        out = torch.empty(rows, H * d, dtype=bf, device=DEV)
+        ops.attention_mixed(q[-rows:].reshape(rows, -1).to(bf).to(DEV), None, out, k.to(bf).to(DEV), vc.to(bf).to(DEV), table, step, H, G, d, d, 1.0, 3e5,
+                            None, None, None, 0, 0, 1.0)
+        outs.append(out if single else out[:-1])
+    assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16)) and bool(torch.isfinite(outs[0]).all())
+
+
 @pytest.mark.parametrize("which", ["keys", "values"])
 def test_mixed_heads_of_caches_on_eight_bytes(which):
     """A cache that starts between two 16-byte boundaries is served as before, by the kernel that copies smaller pieces."""
