@@ -225,7 +225,10 @@ attention_mixed_token_kernel(const __grid_constant__ CUtensorMap map_k, const __
             for (int ks = 0; ks < D / 16; ++ks) {
                 uint32_t a[4];
                 pc_ldm4(smem_u32(k + mk_at<D>(half * 16 + (lane & 15), ks * 2 + (lane >> 4), box)), a);
-                pc_mma(c, a, *reinterpret_cast<const uint32_t*>(q + ks * 16), *reinterpret_cast<const uint32_t*>(q + ks * 16 + 8));
+                float more[4];                                             // (from zero and added with rounding: see pc_mma33)
+                pc_mma0(more, a, *reinterpret_cast<const uint32_t*>(q + ks * 16), *reinterpret_cast<const uint32_t*>(q + ks * 16 + 8));
+#pragma unroll
+                for (int e = 0; e < 4; ++e) c[e] += more[e];
             }
             float* p = Ps + (size_t)(g * per + h0 + t2) * J + o * MK_CH + half * 16 + gid;
             if (h0 + t2 < per) { p[0] = c[0]; p[8] = c[2]; }

@@ -467,6 +467,39 @@ def test_mixed_heads_do_not_notice_keys_that_they_do_not_see(H, G, d, single):
     assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16)) and bool(torch.isfinite(outs[0]).all())
 
 
+def _score_errors(H, G, d, q, k, cap, single, tiled):
+    """What a kernel's scores of q [H, d] and k [G, d] (bfloat16 numbers, products about 2^20) are off by.  Two keys: the first one's score less a
+    distance bias of the score itself, rounded to float32, is as good as zero, and so is the second one's; the first one's weight is its result."""
+    from kuiperllama_b200.csrc import ops
+    bf, T = torch.bfloat16, 2 if single else 8
+    kc, vc = torch.zeros(1, G, 64, d, dtype=bf, device=DEV), torch.zeros(1, G, 64, d, dtype=bf, device=DEV)
+    kc[0, :, 0], vc[0, :, 0] = k.to(bf).to(DEV), 1.0
+    step = _step([1], [1]) if single else _step([0], [T])
+    qs = torch.zeros(step.n_tokens, H, d, dtype=bf, device=DEV)
+    qs[0 if single else 1] = q.to(bf).to(DEV)
+    exact = (q.double() * k.double().repeat_interleave(H // G, 0)).sum(-1)
+    if cap:
+        exact = cap * torch.tanh(exact / cap)
+    bias = exact.float()
+    out = torch.empty(step.n_tokens, H * d, dtype=bf, device=DEV)
+    ops.attention_mixed(qs.view(step.n_tokens, -1), None, out, kc, vc, torch.zeros(1, 1, dtype=torch.int32, device=DEV), step, H, G, d, d, 1.0, cap,
+                        (bias * 2.0 ** 30).to(DEV), torch.full((H,), 2.0 ** -30, device=DEV), None, 0, 0, 1.0, tiled=tiled)
+    w = out.view(-1, H, d)[0 if single else 1, :, 0].double().cpu()
+    return torch.log(w / (1 - w)) + bias.double() - exact, exact
+
+
+def test_mixed_heads_of_single_tokens_add_scores_with_rounding():
+    """Sums of 128 products on the tensor cores are no less exact than the chain of 32-bit multiply-adds."""
+    g, H, G, d, off = torch.Generator().manual_seed(5), 24, 3, 128, {None: [], True: []}
+    for _ in range(40):
+        q, k = ((300.0 * torch.randn(n, d, generator=g)).bfloat16() for n in (H, G))
+        mass = (q.double() * k.double().repeat_interleave(H // G, 0)).abs().sum(-1)
+        for tiled, errors in off.items():
+            errors.append(_score_errors(H, G, d, q, k, 0.0, True, tiled)[0] / (U * mass))
+    rms = {tiled: float(torch.cat(errors).square().mean().sqrt()) for tiled, errors in off.items()}
+    assert rms[None] <= rms[True], rms
+
+
 @pytest.mark.parametrize("which", ["keys", "values"])
 def test_mixed_heads_of_caches_on_eight_bytes(which):
     """A cache that starts between two 16-byte boundaries is served as before, by the kernel that copies smaller pieces."""
