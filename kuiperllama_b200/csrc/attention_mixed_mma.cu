@@ -43,7 +43,7 @@ struct MixedMmaArgs {
     int rows, splits0, splits1;                   // pieces that a tile's chunks are dealt to, in phase 0 and in phase 1
     int kv_heads, window, keep_first;
     float scale, softcap, out_scale;
-    float scale_cap;                              // scale / softcap
+    float scale_cap, scale_cap_rest;              // scale / softcap as the sum of two numbers: a score times it is rounded once
 };
 
 // tanh(x) for |x| <= MX_SMALL: x + x^3 R(x^2) with R of degree four, the best one for the relative error of tanh (2.8e-9 of it; in 32 bits 0.76
@@ -57,7 +57,11 @@ __device__ __forceinline__ float mx_tanh(float x) {
     r = fmaf(r, u, -0.33333298563957214f);
     return fmaf(x * u, r, x);
 }
-
+// v * scale / softcap, rounded once; of an infinite or huge one the leading product (tanh is 1 far before that)
+__device__ __forceinline__ float mx_capped(float v, float c, float rest) {
+    const float x = v * c;
+    return fabsf(x) < 64.f ? fmaf(v, c, v * rest) : x;
+}
 
 __device__ __forceinline__ uint32_t mx_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mx_ldm4(uint32_t a, uint32_t (&r)[4]) {
@@ -222,10 +226,6 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
         };
         if (A.softcap > 0.f) {
             float most = 0.f;                                              // of the lane's visible scores, all of one token: its result does not depend on what it does not see
-#pragma unroll
-            for (int n = 0; n < NT; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) S[n][e] *= A.scale_cap;
             if (inside) {
 #pragma unroll
                 for (int n = 0; n < NT; ++n)
@@ -237,16 +237,16 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) most = visible(n, e) ? fmaxf(most, fabsf(S[n][e])) : most;
             }
-            if (most > MX_SMALL) {
+            if (most * fabsf(A.scale_cap) > MX_SMALL) {
 #pragma unroll
                 for (int n = 0; n < NT; ++n)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) S[n][e] = tanhf(S[n][e]);
+                    for (int e = 0; e < 4; ++e) S[n][e] = tanhf(mx_capped(S[n][e], A.scale_cap, A.scale_cap_rest));
             } else {
 #pragma unroll
                 for (int n = 0; n < NT; ++n)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) S[n][e] = mx_tanh(S[n][e]);
+                    for (int e = 0; e < 4; ++e) S[n][e] = mx_tanh(fmaf(S[n][e], A.scale_cap, S[n][e] * A.scale_cap_rest));
             }
         }
         const float factor = A.softcap > 0.f ? A.softcap : A.scale;
@@ -456,6 +456,7 @@ KL_API int kl_attention_mixed_mma(const void* q, long long q_stride, const void*
     A.cu_tokens = cu_tokens; A.seq_slots = seq_slots; A.seq_starts = seq_starts; A.r1 = r1; A.r2 = r2; A.talk = talk; A.ml = ml;
     A.kv_heads = kv_heads; A.window = window; A.keep_first = keep_first; A.scale = scale; A.softcap = softcap; A.out_scale = out_scale;
     A.scale_cap = softcap > 0.f ? (float)((double)scale / (double)softcap) : 0.f;
+    A.scale_cap_rest = softcap > 0.f ? (float)((double)scale / (double)softcap - (double)A.scale_cap) : 0.f;
     A.rows = rows; A.splits0 = splits0; A.splits1 = splits1; A.part = part;
     const dim3 grid((max_new + MX_TQ - 1) / MX_TQ, n_seqs);
     int err = KL_OK;

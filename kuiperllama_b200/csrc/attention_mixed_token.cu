@@ -44,7 +44,8 @@ struct MixedTokenArgs {
     int* status;
     int heads, kv_heads, window, keep_first;
     int slots, room;                              // slots of the ring; chunks whose scores shared memory holds
-    float scale, softcap, out_scale, scale_cap;   // scale_cap: scale / softcap
+    float scale, softcap, out_scale;
+    float scale_cap, scale_cap_rest;              // scale / softcap as the sum of two numbers
 };
 
 // byte offsets in shared memory
@@ -81,6 +82,11 @@ __device__ __forceinline__ float mk_tanh(float x) {
     r = fmaf(r, u, 0.13331924378871918f);
     r = fmaf(r, u, -0.33333298563957214f);
     return fmaf(x * u, r, x);
+}
+// v * scale / softcap, rounded once; of an infinite or huge one the leading product (tanh is 1 far before that)
+__device__ __forceinline__ float mx_capped(float v, float c, float rest) {
+    const float x = v * c;
+    return fabsf(x) < 64.f ? fmaf(v, c, v * rest) : x;
 }
 __device__ __forceinline__ void mk_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void mk_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -249,12 +255,15 @@ attention_mixed_token_kernel(const __grid_constant__ CUtensorMap map_k, const __
             float* p2 = p + (two ? (size_t)MK_WARPS * J : 0);
             float v = *p, v2 = *p2;
             if (A.softcap > 0.f) {
-                v *= A.scale_cap;
-                v2 *= A.scale_cap;
                 // (asked for every lane's own two scores: past the last key the page holds whatever was there before, and no visible score takes another
                 // form for it)
-                if (vis && fmaxf(fabsf(v), fabsf(v2)) > SMALL) { v = tanhf(v); v2 = tanhf(v2); }
-                else { v = mk_tanh(v); v2 = mk_tanh(v2); }
+                if (vis && fmaxf(fabsf(v), fabsf(v2)) * fabsf(A.scale_cap) > SMALL) {
+                    v = tanhf(mx_capped(v, A.scale_cap, A.scale_cap_rest));
+                    v2 = tanhf(mx_capped(v2, A.scale_cap, A.scale_cap_rest));
+                } else {
+                    v = mk_tanh(fmaf(v, A.scale_cap, v * A.scale_cap_rest));
+                    v2 = mk_tanh(fmaf(v2, A.scale_cap, v2 * A.scale_cap_rest));
+                }
             }
             const float factor = A.softcap > 0.f ? A.softcap : A.scale;
             if (A.r1 != nullptr) {
@@ -543,7 +552,8 @@ KL_API int kl_attention_mixed_token(const void* q, long long q_stride, const voi
     A.block_table = block_table; A.blocks_per_seq = blocks_per_seq;
     A.cu_tokens = cu_tokens; A.seq_slots = seq_slots; A.seq_starts = seq_starts; A.r1 = r1; A.r2 = r2; A.talk = talk; A.status = status;
     A.heads = heads; A.kv_heads = kv_heads; A.window = window; A.keep_first = keep_first; A.slots = P.slots; A.room = P.room;
-    A.scale = scale; A.softcap = softcap; A.out_scale = out_scale; A.scale_cap = softcap > 0.f ? scale / softcap : 0.f;
+    A.scale = scale; A.softcap = softcap; A.out_scale = out_scale; A.scale_cap = softcap > 0.f ? (float)((double)scale / (double)softcap) : 0.f;
+    A.scale_cap_rest = softcap > 0.f ? (float)((double)scale / (double)softcap - (double)A.scale_cap) : 0.f;
 #define KL_MK(DD, U)                                                                                                                          \
     do {                                                                                                                                      \
         KL_CUDA(cudaFuncSetAttribute(attention_mixed_token_kernel<DD, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));         \

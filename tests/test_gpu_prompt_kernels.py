@@ -500,6 +500,23 @@ def test_mixed_heads_of_single_tokens_add_scores_with_rounding():
     assert rms[None] <= rms[True], rms
 
 
+@pytest.mark.parametrize("single", [True, False])
+@pytest.mark.parametrize("lo,hi", [(0.3, 0.59), (0.61, 1.2)])
+def test_mixed_heads_divide_by_the_cap_as_exactly_as_before(single, lo, hi):
+    """A cap whose reciprocal float32 rounds by half a unit; one product a score, so that nothing else is rounded before the quotient.  On both sides of
+    where tanh is a polynomial, no further from float64 than the kernel that divides."""
+    g, H, G, d, cap, off = torch.Generator().manual_seed(6), 32, 8, 64, 2096640.0, {None: [], True: []}
+    for _ in range(30):
+        q, k = torch.zeros(H, d), torch.zeros(G, d)
+        k[:, 3] = (1000.0 * (1.0 + 0.01 * torch.rand(G, generator=g))).bfloat16().float()
+        q[:, 3] = ((lo + (hi - lo) * torch.rand(H, generator=g)) * cap / 1015.0).bfloat16().float()
+        for tiled, errors in off.items():
+            e, s = _score_errors(H, G, d, q, k, cap, single, tiled)
+            errors.append(e / (U * s))
+    rms = {tiled: float(torch.cat(errors).square().mean().sqrt()) for tiled, errors in off.items()}
+    assert rms[None] <= 1.02 * rms[True], rms              # (960 samples each)
+
+
 @pytest.mark.parametrize("which", ["keys", "values"])
 def test_mixed_heads_of_caches_on_eight_bytes(which):
     """A cache that starts between two 16-byte boundaries is served as before, by the kernel that copies smaller pieces."""
