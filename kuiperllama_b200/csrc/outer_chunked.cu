@@ -18,15 +18,16 @@
 //
 // Nothing is rounded to 16 bits.  A 32-bit number enters a product as the sum of three bfloat16 numbers (24 bits of mantissa); of two such
 // operands the six products down to 2^-16 of the leading one are added, smallest first; a bfloat16 operand enters as it is.  Products of
-// decays are made as products (no logarithms, no quotients), at most 32 factors long and rounded once.
+// decays are made as products (no logarithms, no quotients), at most 32 factors long, in 64 bits (those of 16 neighbouring tokens in 32, as the walk does).
 // A chunk in which something is not finite, larger than OC_MOST, or whose decays leave [0, 1], is walked token by token (oc_tokens), so that
 // infinities and NaN stay where they arise: a masked product would pass them on to the tokens before them.
 //
 // What bounds it: a chunk's chain of instructions (2.3 us where the products of mma.m16n8k16, six where there was one, take 0.9 of the tensor
 // cores' time: 38 % busy, 0.33 instructions a cycle and scheduler).  One prompt of 2,048 tokens, us token by token / in chunks: 64 heads of
 // 128 x 64 (state-space) 416 / 151, 16 heads of 64 x 128 with a decay per row (gated linear attention) 374 / 114; three prompts of 446, 1,333 and
-// 2,222 tokens of the former 585 / 266.  Error against 64 bits, one sequence of 500 tokens with decays as such layers have: y 1.11e-7 / 1.00e-7 and
-// 1.01e-7 / 1.04e-7, S 7.6e-8 / 6.1e-8 and 7.8e-8 / 6.6e-8.
+// 2,222 tokens of the former 585 / 266.  Error against 64 bits, one sequence of 500 tokens with decays as such layers have: y 7.5e-8 / 7.0e-8 and
+// 1.08e-7 / 8.8e-8, S 8.4e-8 / 6.7e-8 and 8.3e-8 / 5.3e-8.  With a decay per row and decays far from one (sigmoid(z) ** (1 / tau), tau 1 to 4) y 0.91 to
+// 0.998 of the walk's, and S, which the walk then rounds once and this three times, 3.0e-8 to 4.6e-8 / 4.7e-8 to 6.1e-8: within one unit of 2^-24 either way.
 //
 // ExiledOfCode/KuiperLLama has no recurrent mixer (its mixer is mha_kernel.cu:61,74-106).
 #include "pieces.cuh"
@@ -200,8 +201,8 @@ oc_row_kernel(const OuterChunkArgs A) {
     float* as = reinterpret_cast<float*>(oc_raw);          // [OC][RS]: decays, then c k with them
     float* qs = as + OC * RS;                              // q_scale q
     float* ks = qs + OC * RS;                              // c k
-    float* pre = ks + OC * RS;                             // [2][NP]: the blocks' whole products
-    float* ms = pre + 2 * NP;                              // [OC][OC_MS]: the weighted products
+    double* pre = reinterpret_cast<double*>(ks + OC * RS); // [2][NP]: the blocks' whole products
+    float* ms = reinterpret_cast<float*>(pre + 2 * NP);    // [OC][OC_MS]: the weighted products
     const int s = blockIdx.z, h = blockIdx.y, ch = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, N = A.N;
     const int row0 = A.cu_tokens[s] + ch * OC, live = min(OC, A.cu_tokens[s + 1] - row0);
     if (live <= 0) return;
@@ -241,7 +242,8 @@ oc_row_kernel(const OuterChunkArgs A) {
     }
     const int any = __syncthreads_or(wild);
     if (threadIdx.x == 0) reinterpret_cast<int*>(qm + oc_q_bytes<NP, 1>() - 16)[0] = any;
-    // inside a block: token j's c k, decayed from token to token, by the q of the tokens from j on.  Four lanes share the sum.
+    // inside a block: token j's c k, decayed from token to token, by the q of the tokens from j on.  Four lanes share the sum, each in eight parts
+    // (short chains of additions: with one of 32 y's error was up to 1.2 times the walk's).
     {
         constexpr int E = NP / 4;                          // elements a lane: fours, sixteen apart
         const int b0 = (threadIdx.x >> 6) * 16, j = (threadIdx.x >> 2) & 15, part = threadIdx.x & 3;
@@ -253,14 +255,16 @@ oc_row_kernel(const OuterChunkArgs A) {
         }
         for (int i = 0; i < 16; ++i) {
             const bool on = i >= j;
-            float sum = 0.f;
+            float parts[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int e = 0; e < E; e += 4) {
+                float* sums = parts + (e & 4);
                 const float4 x = *reinterpret_cast<const float4*>(qs + (b0 + i) * RS + e * 4 + part * 4);
                 const float4 d = *reinterpret_cast<const float4*>(as + (b0 + i) * RS + e * 4 + part * 4);
                 if (i > j) { r[e] *= d.x; r[e + 1] *= d.y; r[e + 2] *= d.z; r[e + 3] *= d.w; }
-                sum = fmaf(x.x, r[e], sum); sum = fmaf(x.y, r[e + 1], sum); sum = fmaf(x.z, r[e + 2], sum); sum = fmaf(x.w, r[e + 3], sum);
+                sums[0] = fmaf(x.x, r[e], sums[0]); sums[1] = fmaf(x.y, r[e + 1], sums[1]); sums[2] = fmaf(x.z, r[e + 2], sums[2]); sums[3] = fmaf(x.w, r[e + 3], sums[3]);
             }
+            float sum = ((parts[0] + parts[1]) + (parts[2] + parts[3])) + ((parts[4] + parts[5]) + (parts[6] + parts[7]));
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
             if (part == 0) {
@@ -270,16 +274,40 @@ oc_row_kernel(const OuterChunkArgs A) {
             }
         }
     }
-    __syncthreads();
-    // the decays' products along the tokens of a block: q times those from its start, in as k times those to its end
-    // (running products in 64 bits: a product of 16 decays is rounded once)
+    // the blocks' whole products of decays, in 64 bits as all of these products: what leaves here is rounded once
     for (int idx = threadIdx.x; idx < 2 * NP; idx += OC_THREADS) {
         const int b = idx / NP, n = idx % NP;
         double r = 1.0;
-        for (int t = b * 16; t < b * 16 + 16; ++t) { r *= as[t * RS + n]; qs[t * RS + n] = (float)(qs[t * RS + n] * r); }
-        pre[idx] = (float)r;
-        double f = 1.0;
-        for (int t = b * 16 + 15; t >= b * 16; --t) { const float a = as[t * RS + n]; as[t * RS + n] = (float)(ks[t * RS + n] * f); f *= a; }
+#pragma unroll
+        for (int t = 0; t < 16; ++t) r *= as[(b * 16 + t) * RS + n];
+        pre[idx] = r;
+    }
+    __syncthreads();
+    // Along the tokens of a block: q times the decays from the block's start, in `as` k times those to its end.  For the walk, which counts from the chunk's start
+    // and to its end, the other block's decays belong to q of the second block and to k of the first: those go to `ks`.
+    for (int idx = threadIdx.x; idx < 2 * NP; idx += OC_THREADS) {
+        const int b = idx / NP, n = idx % NP;
+        const double other = pre[(b ^ 1) * NP + n];
+        float whole[16];
+        const double before = b ? other : 1.0, behind = b ? 1.0 : other;
+        double r = 1.0, f = 1.0;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            const int at = (b * 16 + t) * RS + n;
+            r *= as[at];
+            const double q = qs[at] * r;
+            qs[at] = (float)q;
+            whole[t] = (float)(q * before);
+        }
+#pragma unroll
+        for (int t = 15; t >= 0; --t) {
+            const int at = (b * 16 + t) * RS + n;
+            const float a = as[at];
+            const double k = ks[at] * f;
+            as[at] = (float)k;
+            ks[at] = b ? whole[t] : (float)(k * behind);
+            f *= a;
+        }
     }
     __syncthreads();
     if (warp == 0 && live > 16) {                          // between the blocks
@@ -309,24 +337,21 @@ oc_row_kernel(const OuterChunkArgs A) {
             *reinterpret_cast<float2*>(o + 8) = make_float2(d[1][2 * i], d[1][2 * i + 1]);
         }
     }
-    // q and k for the walk: with the other block's decays (rows past the end are zeros: so are their k and q)
+    // q and k for the walk in pieces (rows past the end are zeros: so are their k and q)
     for (int idx = threadIdx.x; idx < OC * NP / 8 * 2; idx += OC_THREADS) {
         const int which = idx / (OC * NP / 8), e = idx % (OC * NP / 8), r = e / (NP / 8), p = e % (NP / 8);
-        const float* src = (which ? as : qs) + r * RS + p * 8;
-        const float* f = which ? (r < 16 ? pre + NP : nullptr) : (r >= 16 ? pre : nullptr);
+        const float* src = ((r < 16) == (which != 0) ? ks : which ? as : qs) + r * RS + p * 8;
         bf16* out = which ? kp : reinterpret_cast<bf16*>(qm);
         uint32_t w[3][4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            float x = src[2 * u], z = src[2 * u + 1];
-            if (f != nullptr) { x *= f[p * 8 + 2 * u]; z *= f[p * 8 + 2 * u + 1]; }
-            pc_split(x, z, w[0][u], w[1][u], w[2][u]);
+            pc_split(src[2 * u], src[2 * u + 1], w[0][u], w[1][u], w[2][u]);
         }
 #pragma unroll
         for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(out + i * OC * NP + pc_at<NP>(r, p)) = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
     }
     float* alpha = reinterpret_cast<float*>(qm + 3 * OC * NP * 2 + 3 * OC * OC * 2);
-    for (int n = threadIdx.x; n < NP; n += OC_THREADS) alpha[n] = pre[n] * pre[NP + n];
+    for (int n = threadIdx.x; n < NP; n += OC_THREADS) alpha[n] = (float)(pre[n] * pre[NP + n]);
     __syncthreads();
     {                                                      // the weighted products, eight of a row a thread
         const int i = threadIdx.x >> 2, q4 = threadIdx.x & 3;
@@ -713,7 +738,7 @@ oc_walk_kernel(const OuterChunkArgs A) {
 
 template <int NP, int MODE>
 static int launch_outer_chunked(const OuterChunkArgs& A, int n_seqs, cudaStream_t stream) {
-    const int pre = MODE == 0 ? 2 * 3 * OC * NP * 2 : (3 * OC * (NP + 4) + 2 * NP + OC * OC_MS) * 4;
+    const int pre = MODE == 0 ? 2 * 3 * OC * NP * 2 : (3 * OC * (NP + 4) + 4 * NP + OC * OC_MS) * 4;
     if constexpr (MODE == 0) {
         KL_CUDA(cudaFuncSetAttribute(oc_group_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, pre));
         launch_kernel(oc_group_kernel<NP>, dim3(A.max_chunks, A.groups + (A.heads + 3) / 4, n_seqs), OC_THREADS, pre, stream, A);

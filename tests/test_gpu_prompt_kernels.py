@@ -150,6 +150,27 @@ def test_recurrence_in_chunks(heads, groups, n, p, form, wide, near):
     assert off(y) <= 1.5 * off(walked) + U                 # no less exact than token by token
 
 
+# decays as the layers have them (sigmoid(z) ** (1 / tau)) and stronger ones; a few tokens behind a chunk and whole prompts
+@pytest.mark.parametrize("heads,n,p,tau", [(16, 64, 128, 16.0), (8, 64, 128, 4.0), (8, 64, 128, 2.0), (4, 128, 128, 4.0), (4, 128, 64, 8.0), (4, 128, 64, 16.0)])
+@pytest.mark.parametrize("news", [[33], [500]])
+def test_recurrence_in_chunks_is_as_exact_as_token_by_token(heads, n, p, tau, news):
+    from kuiperllama_b200.csrc import ops
+    step, g = _step([0], news), torch.Generator(device=DEV).manual_seed(5)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    q, k, v = (rand(news[0], heads * w).bfloat16() for w in (n, n, p))
+    a, state0 = torch.sigmoid(rand(news[0], heads * n)) ** (1 / tau), torch.zeros(1, heads * n * p, device=DEV)
+    one = torch.ones(news[0], heads, dtype=F64, device=DEV)
+    want, S = _recurrence(q.double().view(-1, heads, n), k.double().view(-1, heads, n), v.double().view(-1, heads, p), a.double().view(-1, heads, n), one,
+                          0 * one[0], state0.double().view(1, heads, n, p), step.cu, 0.125)
+    off = {}
+    for chunked in (False, True):
+        state, y = state0.clone(), torch.empty(news[0], heads * p, device=DEV)
+        ops.outer_recurrence(q, k, v, a, state, y, step, heads, heads, n, p, q_scale=0.125, chunked=chunked)
+        off[chunked] = float((y.double().view(want.shape) - want).norm() / want.norm()), float((state.double().view(S.shape) - S).norm() / S.norm())
+    assert off[True][0] <= off[False][0], off
+    assert off[True][1] <= max(off[False][1], U), off      # (of S one rounding of a sum's last bits: 2^-24 at most)
+
+
 @pytest.mark.parametrize("form", ["head", "row"])
 @pytest.mark.parametrize("what", ["v", "q", "k", "a", "c", "state", "grows", "huge"])
 def test_recurrence_in_chunks_keeps_what_is_not_finite_where_it_arises(form, what):
