@@ -13,6 +13,7 @@ from ..weights.loader import TensorDecl
 from .base import Mixer, NormedLazy, PositionEncoding, Runtime, StepContext, register_mixer
 from .composite import BranchMixer
 from .linear import Linear, StackedInput
+from .recurrent import in_chunks
 
 
 @register_mixer("mamba2")
@@ -29,8 +30,11 @@ class Mamba2Mixer(Mixer):
     the norm), times the norm's weight, and the output projection.  The convolution's sums, dt, the decay, S and y are
     32-bit; the slot's state is S as [heads, N, vdim], then the convolution's last conv - 1 inputs, float32.  Spec:
     ``hidden_size``, ``heads``, ``vdim``, ``state``, ``groups``, ``conv``, ``norm_groups``, ``norm_eps`` and ``names`` (in,
-    conv, conv_bias, dt_bias, A_log, D, norm, o).  KuiperLLama has no recurrent mixer (its mixer is
-    mha_kernel.cu:61,74-106)."""
+    conv, conv_bias, dt_bias, A_log, D, norm, o).  float32 runs walk their tokens, whose bits do not depend on how a prompt is cut or
+    what it is batched with; bfloat16 prompts go in chunks on the tensor cores (``ops.outer_recurrence``).  KuiperLLama has no recurrent
+    mixer (its mixer is mha_kernel.cu:61,74-106)."""
+
+    KERNEL = "chunked"            # "walk": token by token also for bfloat16 prompts
 
     @classmethod
     def manifest(cls, spec: PartSpec, prefix: str) -> Dict[str, TensorDecl]:
@@ -85,7 +89,7 @@ class Mamba2Mixer(Mixer):
         ops.decay_softplus(proj[:, inner + C:], self.dt_bias, self.A_log, n, dt, decay)
         y = make((n, inner), dtype=torch.float32, device=dev)
         ops.outer_recurrence(xbc[:, inner + GN:], xbc[:, inner:inner + GN], xbc[:, :inner], decay, cache.state, y, step,
-                             self.H, self.G, self.N, self.P, c=dt, skip=self.D)
+                             self.H, self.G, self.N, self.P, c=dt, skip=self.D, chunked=in_chunks(self))
         gated = torch.empty((n, inner), dtype=self.runtime.dtype, device=dev)
         ops.head_rmsnorm_gate(y, proj[:, :inner], self.norm_weight, gated, self.norm_groups, inner // self.norm_groups,
                               self.norm_eps, gate_first=True)
@@ -102,9 +106,11 @@ class GatedLinearAttentionMixer(BranchMixer):
         S_t = diag(alpha_t) S_(t-1) + k_t v_t^T;     o_t = S_t^T q_t
 
     then each head's o over its root mean square (over vdim) times a weight the heads share, times silu(Wg n), and the
-    output projection.  alpha, S, o and the norm are 32-bit; the slot's state is S as [heads, dim, vdim] float32.  Spec:
-    ``hidden_size``, ``heads``, ``dim``, ``vdim``, ``rank``, ``tau``, ``q_scale``, ``norm_eps`` and ``names`` (q, k, v, g, o, norm, a1,
-    a2, a2_bias).  KuiperLLama has no recurrent mixer (its mixer is mha_kernel.cu:61,74-106)."""
+    output projection.  alpha, S, o and the norm are 32-bit; the slot's state is S as [heads, dim, vdim] float32.  Prompts as in
+    ``Mamba2Mixer``.  Spec: ``hidden_size``, ``heads``, ``dim``, ``vdim``, ``rank``, ``tau``, ``q_scale``, ``norm_eps`` and ``names`` (q, k, v, g, o,
+    norm, a1, a2, a2_bias).  KuiperLLama has no recurrent mixer (its mixer is mha_kernel.cu:61,74-106)."""
+
+    KERNEL = "chunked"            # "walk": token by token also for bfloat16 prompts
 
     @classmethod
     def manifest(cls, spec: PartSpec, prefix: str) -> Dict[str, TensorDecl]:
@@ -146,7 +152,7 @@ class GatedLinearAttentionMixer(BranchMixer):
         make = torch.zeros if step.padded else torch.empty
         o = make((n, self.H * self.dv), dtype=torch.float32, device=dev)
         ops.outer_recurrence(stacked.view(tag + "q"), stacked.view(tag + "k"), stacked.view(tag + "v"), alpha, cache.state, o, step,
-                             self.H, self.H, self.d, self.dv, q_scale=self.q_scale)
+                             self.H, self.H, self.d, self.dv, q_scale=self.q_scale, chunked=in_chunks(self))
         ops.head_rmsnorm_gate(o, stacked.view(tag + "g"), self.norm_weight, out, self.H, self.dv, self.norm_eps, out_scale=out_scale)
 
 

@@ -13,6 +13,12 @@ from .base import Mixer, NormedLazy, PositionEncoding, Runtime, StepContext, reg
 from .linear import Linear, StackedInput
 
 
+def in_chunks(mixer: Mixer) -> Optional[bool]:
+    """What a recurrence's op is asked for: chunks where they are the faster ones (None), or token by token (False) in float32 runs and
+    for a mixer whose ``KERNEL`` says so."""
+    return None if mixer.KERNEL == "chunked" and mixer.runtime.dtype == torch.bfloat16 else False
+
+
 @register_mixer("mingru")
 class MinGRUMixer(Mixer):
     """A gated recurrence whose gates read only the current token:
@@ -74,8 +80,11 @@ class GatedDeltaMixer(Mixer):
     and out = Wo (o / rms(o) * w_norm * silu(Wg n)), the RMS over each head's dv values.  The slot's
     state is float32: S as [H, d, dv], then the last conv - 1 inputs of the convolution.  All of
     q, k, v, beta, decay and g come from one product.  Spec: ``hidden_size``, ``heads``,
-    ``kv_heads``, ``dim``, ``vdim``, ``conv``, ``norm_eps``, ``unit_eps``, ``q_scale`` and ``names``.
+    ``kv_heads``, ``dim``, ``vdim``, ``conv``, ``norm_eps``, ``unit_eps``, ``q_scale`` and ``names``.  float32 runs walk their tokens,
+    whose bits do not depend on how a prompt is cut; bfloat16 prompts go in chunks on the tensor cores (``ops.gated_delta_rule``).
     KuiperLLama has no recurrent mixer (its mixer is mha_kernel.cu:61,74-106)."""
+
+    KERNEL = "chunked"            # "walk": token by token also for bfloat16 prompts
 
     @classmethod
     def manifest(cls, spec: PartSpec, prefix: str) -> Dict[str, TensorDecl]:
@@ -131,7 +140,7 @@ class GatedDeltaMixer(Mixer):
         make = torch.zeros if step.padded else torch.empty
         o = make((n, self.H * self.dv), dtype=torch.float32, device=x.device)
         ops.gated_delta_rule(proj, col("qkv"), col("beta"), col("a"), self.conv_weight, self.A_log, self.dt_bias, cache.state,
-                             self.conv_off, o, step, self.H, self.G, self.d, self.dv, self.q_scale, self.unit_eps)
+                             self.conv_off, o, step, self.H, self.G, self.d, self.dv, self.q_scale, self.unit_eps, chunked=in_chunks(self))
         gated = torch.empty((n, self.H * self.dv), dtype=self.runtime.dtype, device=x.device)
         ops.head_rmsnorm_gate(o, self.inputs.view("g"), self.norm_weight, gated, self.H, self.dv, self.norm_eps)
         return self.o.forward(gated, allow_partials=True)
