@@ -40,7 +40,8 @@ struct MixedMmaArgs {
     const float* r1; const float* r2; const float* talk;
     float* ml;                                    // [splits, rows, heads, 2]
     float* part;                                  // [splits, rows, heads * dim]: phase 1 in several pieces, or null
-    int rows, splits0, splits1;                   // pieces that a tile's chunks are dealt to, in phase 0 and in phase 1
+    int* counts;                                  // [rows]: into how many pieces phase 1 cut the row's tile
+    int rows, n_seqs, splits0, splits1;           // pieces that a tile's chunks are dealt to at most, in phase 0 and in phase 1
     int kv_heads, window, keep_first;
     float scale, softcap, out_scale;
     float scale_cap, scale_cap_rest;              // scale / softcap as the sum of two numbers: a score times it is rounded once
@@ -98,6 +99,22 @@ inline size_t mx_smem_bytes(int H, int D, int G, int phase) {
            (phase == 1 ? (size_t)H * MX_PH * 4 + (size_t)3 * H * (H + 8) * 2 : 0);
 }
 
+// What a tile of tokens sees.  Its chunks are dealt to as many pieces as it has chunks, `splits` at most: the pieces follow from where a sequence stands
+// and not from what the host knew when it launched (or captured) the kernel.
+struct MixedTile {
+    int i0, nrows, lo, first, kept, visible;      // position of its first token, tokens, first key in the window, its chunk, chunks of kept keys, chunks in all
+    __device__ __forceinline__ MixedTile(const MixedMmaArgs& A, int s, int tile) {
+        nrows = min(MX_TQ, A.cu_tokens[s + 1] - A.cu_tokens[s] - tile * MX_TQ);
+        i0 = A.seq_starts[s] + tile * MX_TQ;
+        lo = A.window > 0 ? max(0, i0 - A.window + 1) : 0;
+        first = lo / MX_CH;
+        kept = A.window > 0 ? min(first, (A.keep_first + MX_CH - 1) / MX_CH) : 0;
+        visible = kept + (i0 + nrows - 1) / MX_CH + 1 - first;
+    }
+    __device__ __forceinline__ int pieces(int splits) const { return min(splits, visible); }
+    __device__ __forceinline__ int chunk(int v) const { return v < kept ? v : v - kept + first; }
+};
+
 template <int H, int D, int PHASE>
 __global__ void __launch_bounds__(H * 16, PHASE == 1 ? 1 : 512 / (H * 16) + 1)
 attention_mixed_mma_kernel(const MixedMmaArgs A) {
@@ -105,15 +122,14 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
     pdl_wait();
     extern __shared__ __align__(128) unsigned char mx_raw[];
     const int s = blockIdx.y, tile = gridDim.x - 1 - blockIdx.x;           // late tiles see the most keys: they start first
-    const int pieces = PHASE == 0 ? A.splits0 : A.splits1, piece = blockIdx.z;
-    const int row0 = A.cu_tokens[s] + tile * MX_TQ;
-    const int nrows = min(MX_TQ, A.cu_tokens[s + 1] - row0);
+    const MixedTile span(A, s, tile);
+    const int nrows = span.nrows, row0 = A.cu_tokens[s] + tile * MX_TQ, piece = blockIdx.z;
     if (nrows <= 0) return;
+    const int pieces = span.pieces(PHASE == 0 ? A.splits0 : A.splits1);
+    if (piece >= pieces) return;
     const int G = A.kv_heads;
-    const int i0 = A.seq_starts[s] + tile * MX_TQ, i_last = i0 + nrows - 1;
-    const int lo_tile = A.window > 0 ? max(0, i0 - A.window + 1) : 0;
+    const int i0 = span.i0, i_last = i0 + nrows - 1;
     const int keep = A.window > 0 ? A.keep_first : 0;
-    const int n_chunks = i_last / MX_CH + 1;
     const int* table = A.block_table + (size_t)A.seq_slots[s] * A.blocks_per_seq;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int h0 = 2 * warp, g = h0 / (H / G);
@@ -126,12 +142,6 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
     float* Ps = reinterpret_cast<float*>(Vs + (PHASE == 1 ? tile_elems : 0)) + WARPS * 2 * MX_BIAS;      // [H][MX_PH] (phase 1)
     bf16* Ts = reinterpret_cast<bf16*>(Ps + H * MX_PH);                    // [3][H][H + 8]: talk in three pieces (phase 1)
 
-    // chunks that neither the window nor the kept first keys reach are skipped; this piece has every `pieces`-th
-    auto next_chunk = [&](int c) {
-        for (c += pieces; c < n_chunks; c += pieces)
-            if (c * MX_CH + MX_CH - 1 >= lo_tile || c * MX_CH < keep) break;
-        return c;
-    };
     auto copy_chunk = [&](bf16* dst, const bf16* cache, int c) {
         const int j0 = c * MX_CH, valid = min(MX_CH, i_last - j0 + 1);
         const bf16* src = cache + ((size_t)table[j0 / PAGE] * G * PAGE + j0 % PAGE) * D;
@@ -144,8 +154,9 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
     };
     auto commit = [&]() { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
-    int c = next_chunk(piece - pieces);
-    if (c < n_chunks) copy_chunk(Ks, A.k_cache, c);
+    // chunks that neither the window nor the kept first keys reach are skipped; this piece has every `pieces`-th of the others
+    int v = piece;
+    copy_chunk(Ks, A.k_cache, span.chunk(v));
     commit();
     if (PHASE == 1 && A.talk != nullptr)
         for (int idx = threadIdx.x; idx < H * H / 2; idx += THREADS) {
@@ -171,8 +182,9 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const float* ml = A.ml + ((size_t)(row0 + min(r, nrows - 1)) * H + h0 + e) * 2;
-            for (int z = 0; z < A.splits0; ++z) m[e] = fmaxf(m[e], ml[(size_t)z * A.rows * H * 2]);
-            for (int z = 0; z < A.splits0; ++z) {          // (a piece that saw nothing: its maximum is -inf, its sum 0)
+            const int before = span.pieces(A.splits0);
+            for (int z = 0; z < before; ++z) m[e] = fmaxf(m[e], ml[(size_t)z * A.rows * H * 2]);
+            for (int z = 0; z < before; ++z) {             // (a piece that saw nothing: its maximum is -inf, its sum 0)
                 const float2 x = *reinterpret_cast<const float2*>(ml + (size_t)z * A.rows * H * 2);
                 if (x.y > 0.f) l[e] += x.y * expf(x.x - m[e]);
                 else if (!(x.y == 0.f)) l[e] = x.y;        // NaN stays
@@ -188,13 +200,13 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
     for (int n = 0; n < (PHASE == 1 ? D / 8 : 1); ++n) O[n][0] = O[n][1] = O[n][2] = O[n][3] = 0.f;
 
     int buf = 0;
-    while (c < n_chunks) {
-        const int j0 = c * MX_CH, cn = next_chunk(c);
+    for (; v < span.visible; v += pieces) {
+        const int c = span.chunk(v), j0 = c * MX_CH;
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                                                   // this chunk's keys are here; the chunk before is done with the buffers
         if (PHASE == 1) copy_chunk(Vs, A.v_cache, c);
         commit();
-        if (cn < n_chunks) copy_chunk(Ks + (buf ^ 1) * tile_elems, A.k_cache, cn);
+        if (v + pieces < span.visible) copy_chunk(Ks + (buf ^ 1) * tile_elems, A.k_cache, span.chunk(v + pieces));
         commit();
         // ---- scores: 8 tokens of two heads by 32 keys
         float S[NT][4];
@@ -363,7 +375,6 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
             __syncwarp();                                                  // the warp's rows of W are read before its next p are written there
         }
         buf ^= 1;
-        c = cn;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     pdl_launch_dependents();
@@ -376,7 +387,8 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
             l[e] += __shfl_xor_sync(0xfu << (lane & ~3), l[e], 2);
             if ((lane & 3) == 0) *reinterpret_cast<float2*>(A.ml + (((size_t)piece * A.rows + row) * H + h0 + e) * 2) = make_float2(m[e], l[e]);
         }
-    } else if (pieces > 1) {
+    } else if (A.splits1 > 1) {
+        if (piece == 0 && warp == 0 && (lane & 3) == 0) A.counts[row] = pieces;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             float* o = A.part + ((size_t)piece * A.rows + row) * H * D + (size_t)(h0 + e) * D + kc;
@@ -397,15 +409,16 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
 
 // The pieces of phase 1 put together: four neighbouring columns of a row a thread, pieces in ascending order.
 __global__ void __launch_bounds__(256)
-attention_mixed_mma_reduce_kernel(const MixedMmaArgs A, const int* __restrict__ token_slot, int heads, int dim) {
+attention_mixed_mma_reduce_kernel(const MixedMmaArgs A, int heads, int dim) {
     pdl_launch_dependents();
     pdl_wait();
     const int width = heads * dim / 4;
     const int idx = blockIdx.x * 256 + threadIdx.x, row = idx / width, c = (idx - row * width) * 4;
-    if (row >= A.rows || token_slot[row] < 0) return;              // (a padding row has no sums)
+    if (row >= A.cu_tokens[A.n_seqs]) return;                      // (a padding row has no sums)
+    const int pieces = A.counts[row];
     const float* p = A.part + (size_t)row * heads * dim + c;
     float4 y = *reinterpret_cast<const float4*>(p);
-    for (int z = 1; z < A.splits1; ++z) {
+    for (int z = 1; z < pieces; ++z) {
         const float4 x = *reinterpret_cast<const float4*>(p + (size_t)z * A.rows * heads * dim);
         y.x += x.x; y.y += x.y; y.z += x.z; y.w += x.w;
     }
@@ -437,17 +450,17 @@ KL_API int kl_attention_mixed_mma_fits(int heads, int kv_heads, int dim, int vdi
            (dim == 32 || dim == 64) && max_new > 4 && mx_smem_bytes(heads, dim, kv_heads, 1) <= 227 * 1024;
 }
 
-// ml: float32 [splits0, rows, heads, 2]; part: float32 [splits1, rows, heads * dim] on a 16-byte boundary where splits1 > 1.  q and out: rows and
+// ml: float32 [splits0, rows, heads, 2]; part: float32 [splits1, rows, heads * dim] on a 16-byte boundary, and counts: int32 [rows], where splits1 > 1.  q and out: rows and
 // heads on 4-byte boundaries; the caches on 16-byte ones.
 KL_API int kl_attention_mixed_mma(const void* q, long long q_stride, const void* gate, long long gate_stride, void* out, long long out_stride,
                                   const void* k_cache, const void* v_cache, const int* block_table, int blocks_per_seq, const int* cu_tokens,
-                                  const int* seq_slots, const int* seq_starts, const int* token_slot, int rows, int n_seqs, int max_new, int heads,
-                                  int kv_heads, int dim, float scale, float softcap, const float* r1, const float* r2, const float* talk, int window,
-                                  int keep_first, float out_scale, int splits0, int splits1, float* ml, float* part, cudaStream_t stream) {
+                                  const int* seq_slots, const int* seq_starts, int rows, int n_seqs, int max_new, int heads, int kv_heads,
+                                  int dim, float scale, float softcap, const float* r1, const float* r2, const float* talk, int window,
+                                  int keep_first, float out_scale, int splits0, int splits1, float* ml, float* part, int* counts, cudaStream_t stream) {
     if (rows <= 0 || n_seqs <= 0 || max_new <= 0) return KL_OK;
     if (!kl_attention_mixed_mma_fits(heads, kv_heads, dim, dim, KL_BF16, max_new) || window < 0 || keep_first < 0 || n_seqs > 65535) return KL_ERR_BAD_SIZE;
     if ((r1 == nullptr) != (r2 == nullptr) || ml == nullptr || splits0 < 1 || splits1 < 1 || splits0 > 64 || splits1 > 64) return KL_ERR_BAD_SIZE;
-    if (splits1 > 1 && (part == nullptr || (uintptr_t)part % 16)) return KL_ERR_BAD_ALIGN;
+    if (splits1 > 1 && (part == nullptr || counts == nullptr || (uintptr_t)part % 16)) return KL_ERR_BAD_ALIGN;
     if (((uintptr_t)q | (uintptr_t)out) % 4 || q_stride % 2 || out_stride % 2 || ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 || (uintptr_t)talk % 8 ||
         (uintptr_t)ml % 8) return KL_ERR_BAD_ALIGN;
     MixedMmaArgs A;
@@ -457,7 +470,7 @@ KL_API int kl_attention_mixed_mma(const void* q, long long q_stride, const void*
     A.kv_heads = kv_heads; A.window = window; A.keep_first = keep_first; A.scale = scale; A.softcap = softcap; A.out_scale = out_scale;
     A.scale_cap = softcap > 0.f ? (float)((double)scale / (double)softcap) : 0.f;
     A.scale_cap_rest = softcap > 0.f ? (float)((double)scale / (double)softcap - (double)A.scale_cap) : 0.f;
-    A.rows = rows; A.splits0 = splits0; A.splits1 = splits1; A.part = part;
+    A.rows = rows; A.n_seqs = n_seqs; A.splits0 = splits0; A.splits1 = splits1; A.part = part; A.counts = counts;
     const dim3 grid((max_new + MX_TQ - 1) / MX_TQ, n_seqs);
     int err = KL_OK;
 #define KL_MX(H_, D_)                                                                       \
@@ -471,7 +484,7 @@ KL_API int kl_attention_mixed_mma(const void* q, long long q_stride, const void*
     else KL_MX(16, 32);
 #undef KL_MX
     if (err != KL_OK || splits1 == 1) return err;
-    launch_kernel(attention_mixed_mma_reduce_kernel, (int)(((long long)rows * heads * dim / 4 + 255) / 256), 256, 0, stream, A, token_slot, heads, dim);
+    launch_kernel(attention_mixed_mma_reduce_kernel, (int)(((long long)rows * heads * dim / 4 + 255) / 256), 256, 0, stream, A, heads, dim);
     KL_LAUNCH_CHECK();
     return KL_OK;
 }

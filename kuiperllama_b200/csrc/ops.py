@@ -1380,19 +1380,19 @@ def mixed_token_ranks(n_seqs: int, context_class: int, window: int, keep_first: 
 MIXED_SPLITS = None             # (phase 0, phase 1): fixed numbers of pieces, for comparisons
 
 
-def mixed_prompt_splits(step, window: int, keep_first: int):
-    """(phase 0, phase 1): into how many pieces a prompt's tiles of 8 tokens cut the 32-key chunks that they see, so that few tiles, or tiles of
-    few and of many chunks, still fill the device: about 300 CTAs, twice that many for the light phase 0, never more pieces than chunks.
+def mixed_prompt_splits(step):
+    """(phase 0, phase 1): into how many pieces at most a prompt's tiles of 8 tokens cut the 32-key chunks that they see, so that few tiles, or tiles of
+    few and of many chunks, still fill the device: about 300 CTAs, twice that many for the light phase 0.  A tile of fewer chunks has as many pieces as
+    chunks, which the kernels count themselves: a captured step's plan holds wherever its replays stand.
     us with one piece each / with these, 32 heads of 64 on 8, window 1,024 and 64 kept keys: 64 tokens 26 / 20, 150 53 / 26, 300 98 / 43, 600 162 / 82,
     1,024 266 / 163, 2,048 469 / 414, 64 after 1,500 301 / 67, four prompts of 500 216 / 185; 16 heads on 4, 300 tokens 58 / 29, 2,048 247 / 222."""
     if MIXED_SPLITS is not None:
         return MIXED_SPLITS
-    chunks = -(-int(step.max_context) // 32)
-    if window:
-        chunks = min(chunks, (int(window) + 31) // 32 + 1 + (int(keep_first or 0) + 31) // 32)
-    tiles = step.n_tokens // 8 + step.n_seqs
-    s1 = max(1, min(chunks, 16, -(-300 // tiles)))
-    return max(1, min(chunks, 16, 2 * s1)), s1
+    s1 = max(1, min(16, -(-300 // (step.n_tokens // 8 + step.n_seqs))))
+    context = None if getattr(step, "captured", False) else getattr(step, "max_context", None)
+    if context is not None:                                # no piece that all tiles would leave out: the same pieces, fewer CTAs
+        s1 = min(s1, -(-int(context) // 32))
+    return min(16, 2 * s1), s1
 
 
 def attention_mixed(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
@@ -1426,15 +1426,16 @@ def attention_mixed(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Te
         if (M.kl_attention_mixed_mma_fits(heads, kv_heads, dim, vdim, BF16, max_new) and q.stride(0) % 2 == 0 and out.stride(0) % 2 == 0
                 and (q.data_ptr() | out.data_ptr()) % 4 == 0 and (talk is None or talk.data_ptr() % 8 == 0)
                 and (k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0):
-            s0, s1 = mixed_prompt_splits(step, window, keep_first)
+            s0, s1 = mixed_prompt_splits(step)
             ml = torch.empty((s0, n, heads, 2), dtype=torch.float32, device=q.device)
             part = torch.empty((s1, n, heads * dim), dtype=torch.float32, device=q.device) if s1 > 1 else None
+            counts = torch.empty(n, dtype=torch.int32, device=q.device) if s1 > 1 else None
             _check(M.kl_attention_mixed_mma(
                 _ptr(q), ctypes.c_longlong(q.stride(0)), _ptr(gate), ctypes.c_longlong(gate.stride(0) if gate is not None else 0), _ptr(out),
                 ctypes.c_longlong(out.stride(0)), _ptr(k_cache), _ptr(v_cache), _ptr(block_table), block_table.shape[1], _ptr(step.cu_tokens),
-                _ptr(step.seq_slots), _ptr(step.seq_starts), _ptr(step.token_slot), n, step.n_seqs, max_new, heads, kv_heads, dim,
-                ctypes.c_float(scale), ctypes.c_float(softcap or 0.0), _ptr(r1), _ptr(r2), _ptr(talk), int(window or 0), int(keep_first or 0),
-                ctypes.c_float(out_scale), s0, s1, _ptr(ml), _ptr(part), _stream()), "attention_mixed_mma", 2 if s1 == 1 else 3)
+                _ptr(step.seq_slots), _ptr(step.seq_starts), n, step.n_seqs, max_new, heads, kv_heads, dim, ctypes.c_float(scale),
+                ctypes.c_float(softcap or 0.0), _ptr(r1), _ptr(r2), _ptr(talk), int(window or 0), int(keep_first or 0),
+                ctypes.c_float(out_scale), s0, s1, _ptr(ml), _ptr(part), _ptr(counts), _stream()), "attention_mixed_mma", 2 if s1 == 1 else 3)
             return
     if tiled is None and splits is None and q.dtype == torch.bfloat16 and max_new == 1:
         M = lib("attention_mixed_token")
@@ -2000,6 +2001,10 @@ def attention_tcgen05(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache
 # 46; of 128 on 8, window 1,024, prompts of 6,000 341 / 136, 128 tokens 9.4 / 9.8, 32 tokens 6.5 / 5.8; 16 heads of 64 on 16, window 1,024,
 # 2,048 tokens 49 / 36, 32 tokens after 500 16.5 / 18.7, 64 after 1,000 35.0 / 34.2, window 128, prompts of 6,000 36 / 47.
 TCGEN05_WINDOW_KEYS = (512, 1024)
+# A captured step is replayed wherever its sequences stand by then, so it goes by its window and its rows alone.  us on mma.sync / tcgen05, window 1,024, 32
+# heads on 8: 64 rows at the start 4.1 / 5.5, after 1,500 31.5 / 29.1, 128 at the start 5.6 / 7.7, 256 after 1,500 39 / 29.5, 512 at the start 19 / 15, after
+# 1,500 43 / 30, eight of 64 after 700 30 / 21; 16 heads on 16: 256 after 1,500 32 / 37, 512 at the start 17.6 / 15.8, after 1,500 39.7 / 37.4.
+TCGEN05_CAPTURED_ROWS = (256, 512)
 
 
 def prefill_on_tcgen05(q: torch.Tensor, q_stride: int, step, num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: int = 0,
@@ -2010,8 +2015,12 @@ def prefill_on_tcgen05(q: torch.Tensor, q_stride: int, step, num_heads: int, num
     if not (q.dtype == torch.bfloat16 and not step.is_decode and PREFILL_KERNEL == "tcgen05" and head_dim in (64, 128) and group <= 128
             and q_stride % 8 == 0 and q.data_ptr() % 16 == 0 and step.max_new >= 8 and scale > 0):
         return False
-    keys = min(window or step.max_context, step.max_context)
-    return (not window and sink is None) or head_dim == 128 or keys >= TCGEN05_WINDOW_KEYS[0 if group > 1 else 1]
+    if (not window and sink is None) or head_dim == 128:
+        return True
+    alone, keys = int(group == 1), int(window or 1 << 30)
+    if getattr(step, "captured", False):
+        return step.max_new >= TCGEN05_CAPTURED_ROWS[alone] and keys >= TCGEN05_WINDOW_KEYS[alone]
+    return min(keys, step.max_context) >= TCGEN05_WINDOW_KEYS[alone]
 
 
 # Which kernel prefill steps of the bfloat16 path use for head sizes 64 and 128: "tcgen05", or "mma"
@@ -2138,9 +2147,12 @@ def attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.
                          num_heads, num_kv_heads, head_dim, scale, window)
     else:
         # rows together: not where a sequence brings fewer than four (a CTA walks the runs that its rows fall into one after the other: 8 runs of 3
-        # tokens after 500, 32 heads of 64, 136 us against 42 by rows), unless they are few among many
-        runs = step.n_tokens // step.n_seqs
-        if min(step.host_new) < 4 and not (runs >= 16 and step.max_context >= 384):
+        # tokens after 500, 32 heads of 64, 136 us against 42 by rows), unless they are few among many.  What a captured step's sequences
+        # bring in a replay is not known, nor what they hold by then.
+        runs = step.n_tokens // max(1, step.n_seqs)
+        news = None if getattr(step, "captured", False) else step.host_new
+        short = min(news) < 4 if news else step.n_seqs > 1
+        if short and not (runs >= 16 and (not news or step.max_context >= 384)):
             runs = 0
         attention_simt(q, q_stride, out, k_cache, v_cache, block_table, step.positions, step.token_slot, step.n_tokens,
                        num_heads, num_kv_heads, head_dim, scale, window, runs=runs,
