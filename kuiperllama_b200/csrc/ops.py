@@ -2020,7 +2020,7 @@ def prefill_on_tcgen05(q: torch.Tensor, q_stride: int, step, num_heads: int, num
     alone, keys = int(group == 1), int(window or 1 << 30)
     if getattr(step, "captured", False):
         return step.max_new >= TCGEN05_CAPTURED_ROWS[alone] and keys >= TCGEN05_WINDOW_KEYS[alone]
-    return min(keys, step.max_context) >= TCGEN05_WINDOW_KEYS[alone]
+    return min(keys, getattr(step, "max_context", keys)) >= TCGEN05_WINDOW_KEYS[alone]
 
 
 # Which kernel prefill steps of the bfloat16 path use for head sizes 64 and 128: "tcgen05", or "mma"
@@ -2150,7 +2150,7 @@ def attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.
         # tokens after 500, 32 heads of 64, 136 us against 42 by rows), unless they are few among many.  What a captured step's sequences
         # bring in a replay is not known, nor what they hold by then.
         runs = step.n_tokens // max(1, step.n_seqs)
-        news = None if getattr(step, "captured", False) else step.host_new
+        news = None if getattr(step, "captured", False) else getattr(step, "host_new", None)
         short = min(news) < 4 if news else step.n_seqs > 1
         if short and not (runs >= 16 and (not news or step.max_context >= 384)):
             runs = 0

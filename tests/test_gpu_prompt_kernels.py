@@ -19,7 +19,7 @@ def _step(starts, news):
     for n in news:
         cu.append(cu[-1] + n)
     return SimpleNamespace(n_tokens=cu[-1], n_seqs=len(news), cu_tokens=i32(cu), seq_slots=i32(list(range(len(news)))), seq_starts=i32(starts),
-                           seq_new=i32(news), max_new=max(news), max_context=max(a + n for a, n in zip(starts, news)), token_slot=i32([s for s, n in enumerate(news) for _ in range(n)]),
+                           seq_new=i32(news), max_new=max(news), token_slot=i32([s for s, n in enumerate(news) for _ in range(n)]),
                            positions=i32([a + t for a, n in zip(starts, news) for t in range(n)]), host_new=news, cu=cu)
 
 

@@ -1,4 +1,5 @@
-"""How a launch is planned from what a step says: what a captured step is replayed for does not depend on where its sequences stood when it was captured."""
+"""How a launch is planned from what a step says: steps that say less than the engine's are taken, and what a captured step is replayed for does not
+depend on where its sequences stood when it was captured."""
 from __future__ import annotations
 
 from types import SimpleNamespace
@@ -13,6 +14,13 @@ Q = torch.zeros(64, 64 * 32, dtype=torch.bfloat16)
 
 def _step(rows, seqs=1, **more):
     return SimpleNamespace(n_tokens=rows, n_seqs=seqs, max_new=rows, is_decode=False, **more)
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd", [(32, 8, 64), (16, 16, 64), (8, 2, 128)])
+def test_prompts_without_a_context_choose_a_kernel(heads, kv_heads, hd):
+    ask = lambda **k: ops.prefill_on_tcgen05(Q, 2048, _step(300), heads, kv_heads, hd, 0.125, **k)
+    assert ask() and ask(window=4096) and ask(sink=torch.zeros(heads))
+    assert ask(window=16) == (hd == 128)
 
 
 @pytest.mark.parametrize("heads,kv_heads", [(32, 8), (16, 16)])
@@ -42,7 +50,8 @@ def _runs(monkeypatch, step):
 def test_rows_that_float32_attention_takes_together(monkeypatch):
     places = dict(positions=None, token_slot=None)
     step = lambda rows, seqs, context, **more: _step(rows, seqs, max_context=context, **places, **more)
-    assert _runs(monkeypatch, step(24, 8, 500, host_new=[3] * 8)) == 0
+    assert _runs(monkeypatch, step(64, 1, 64)) == 64                                     # (no word of what each sequence brings)
+    assert _runs(monkeypatch, step(24, 8, 500)) == 0 and _runs(monkeypatch, step(24, 8, 500, host_new=[3] * 8)) == 0
     assert _runs(monkeypatch, step(64, 8, 500, host_new=[8] * 8)) == 8
     assert _runs(monkeypatch, step(64, 2, 100, host_new=[63, 1])) == 0 and _runs(monkeypatch, step(64, 2, 500, host_new=[63, 1])) == 32
     for rows, seqs in ((64, 1), (64, 8), (512, 8), (128, 2)):
