@@ -1617,14 +1617,16 @@ def sm_count(device: Optional[torch.device] = None) -> int:
 def skinny_splits(N: int, K: int, M: int = 1) -> int:
     """Into how many pieces the K range is cut for a product with few tokens: up to two CTAs per SM that stream weights, 128 output
     features per CTA, at least 4 k-blocks of 64 each.  Every piece is written as float32 [M, N] and read again by the kernel that adds
-    the pieces, so beyond eight pieces (of a product back to the width, N <= K, which a norm adds, beyond 16,384 columns of pieces, but four at
-    least) what the product gains the reader loses, and with many tokens and a short k range their bytes stay under half of
-    the weights' (pieces * M * 4 <= K * 2 / 2; a quarter beyond 64 tokens).  us with the norm that adds them, 4 / 6 / 8 / 16 pieces: 2,048 x 8,192 8
-    tokens 10.7 / 9.8 / 9.3 / 10.1, 64 12.1 / 10.8 / 11.3 / 12.2; 2,048 x 2,048 8 tokens 5.8 / 5.4 / 5.4 / 6.2; 4,096 x 4,096 8 tokens 9.6 / 9.6 / 10.2 / 14.3, 64
-    11.5 / 11.6 / 12.1 / 16.4; 1,024 x 4,096 24 tokens 7.7 / 7.2 / 6.7 / 6.9; without it 3,072 x 2,048 64 tokens 5.1 / 5.4 / 4.8 / 7.5."""
+    the pieces (up to ``STREAM_SINK_MAX_ROWS`` rows by the product's own last CTAs), so beyond eight pieces what the product gains the reader loses;
+    with more than 16 tokens a product back to the width (N <= K, whose pieces a norm adds) has up to 16,384 columns of pieces, but four at
+    least, and with many tokens and a short k range their bytes stay under half of the weights' (pieces * M * 4 <= K * 2 / 2; a quarter beyond
+    64 tokens).  us of a decode step of 16 layers of width 4,096 (4,096 x 4,096 and 4,096 x 14,336 in 4 / 8 pieces; four leave 20 of the 148 SMs without
+    a CTA): 1 token 1,402 / 1,322, 4 1,429 / 1,359, 8 1,422 / 1,370, 16 1,451 / 1,425, 24 1,508 / 1,512, 32 1,557 / 1,554, 48 1,674 / 1,693, 64 1,795 / 1,823; of
+    width 2,048 (2,048 x 8,192 in 8 / 16) 1 token 625 / 622, 8 662 / 671, 64 874 / 875; of width 1,024 (1,024 x 4,096 in 8 / 16) 1 token 457 / 466, 32
+    513 / 527."""
     tiles = ((N + 127) // 128) * max(1, (M + 127) // 128)    # CTAs per cut: weight tiles x token tiles (of 128 beyond 64 tokens)
     k_blocks = (K + 63) // 64
-    most = 8 if N > K else max(4, min(8, 16384 // N))
+    most = 8 if N > K or M <= 16 else max(4, min(8, 16384 // N))
     # never more CTAs than the two per SM that are resident at once: one CTA too many is a second round
     want = max(1, min((2 * sm_count()) // tiles, k_blocks // 4, most, max(1, K // ((4 if M <= 64 else 8) * max(M, 1)))))
     per = (k_blocks + want - 1) // want

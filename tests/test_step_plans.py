@@ -58,3 +58,12 @@ def test_rows_that_float32_attention_takes_together(monkeypatch):
         seen = {_runs(monkeypatch, step(rows, seqs, context, captured=True, host_new=news))
                 for context in (rows, 3000) for news in ([rows // seqs] * seqs, [rows - seqs + 1] + [1] * (seqs - 1))}
         assert len(seen) == 1, (rows, seqs, seen)
+
+
+@pytest.mark.parametrize("N,K", [(4096, 4096), (4096, 14336), (4096, 11008), (5120, 5120), (2048, 8192), (3072, 2048), (6144, 4096), (2560, 2560)])
+@pytest.mark.parametrize("M", [1, 4, 8, 16])
+def test_products_of_few_tokens_have_a_cta_for_every_sm(monkeypatch, N, K, M):
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
+    pieces = ops.skinny_splits(N, K, M)
+    assert 148 < pieces * -(-N // 128) <= 296 or pieces == 8 or pieces == -(-K // 64) // 4
+    assert pieces <= 8
