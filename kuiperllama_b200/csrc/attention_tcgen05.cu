@@ -441,7 +441,7 @@ static int launch_attention_tcgen05(const CUtensorMap& mq, const CUtensorMap& mk
 }  // namespace kl
 
 // Prefill attention of a ragged batch (see kl_attention_mma for the arguments' meaning).  Head
-// sizes 64 and 128, group sizes that divide 128; q rows 16-byte aligned.  window: keys a row sees (0: all); sink: float32 [H] or null.  Others:
+// sizes 64 and 128, group sizes that divide 128; q and out rows 16-byte aligned.  window: keys a row sees (0: all); sink: float32 [H] or null.  Others:
 // KL_ERR_BAD_SIZE / KL_ERR_BAD_ALIGN, and the caller takes the mma.sync kernel.
 KL_API int kl_attention_tcgen05(const void* q, int q_stride, void* out, const void* k_cache, const void* v_cache,
                                 long long n_cache_rows, const int* block_table, int blocks_per_seq, const int* cu_tokens,
@@ -453,7 +453,7 @@ KL_API int kl_attention_tcgen05(const void* q, int q_stride, void* out, const vo
     int Gp = 1;
     while (Gp < G) Gp <<= 1;
     if (Gp > 128) return KL_ERR_BAD_SIZE;
-    if (q_stride % 8 || ((uintptr_t)q & 15)) return KL_ERR_BAD_ALIGN;
+    if (q_stride % 8 || (((uintptr_t)q | (uintptr_t)out) & 15)) return KL_ERR_BAD_ALIGN;
     const int BT = AT_ROWS / Gp;
     CUtensorMap mq, mk, mv;
     int rc;

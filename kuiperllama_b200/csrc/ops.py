@@ -2010,12 +2010,12 @@ TCGEN05_CAPTURED_ROWS = (256, 512)
 
 
 def prefill_on_tcgen05(q: torch.Tensor, q_stride: int, step, num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: int = 0,
-                       sink: Optional[torch.Tensor] = None) -> bool:
-    """Whether a step's softmax attention takes ``attention_tcgen05``: bfloat16 prompts, head sizes of 64 and 128, rows on 16-byte boundaries;
-    with a window or a sink where it is the faster one."""
+                       sink: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> bool:
+    """Whether a step's softmax attention takes ``attention_tcgen05``: bfloat16 prompts, head sizes of 64 and 128, rows of queries and of results on
+    16-byte boundaries; with a window or a sink where it is the faster one."""
     group = num_heads // num_kv_heads
     if not (q.dtype == torch.bfloat16 and not step.is_decode and PREFILL_KERNEL == "tcgen05" and head_dim in (64, 128) and group <= 128
-            and q_stride % 8 == 0 and q.data_ptr() % 16 == 0 and step.max_new >= 8 and scale > 0):
+            and q_stride % 8 == 0 and q.data_ptr() % 16 == 0 and (out is None or out.data_ptr() % 16 == 0) and step.max_new >= 8 and scale > 0):
         return False
     if (not window and sink is None) or head_dim == 128:
         return True
@@ -2133,7 +2133,7 @@ def attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.
     sizes, the split-KV kernel; float32 and everything else takes the plain kernel."""
     bf = q.dtype == torch.bfloat16
     group = num_heads // num_kv_heads
-    if prefill_on_tcgen05(q, q_stride, step, num_heads, num_kv_heads, head_dim, scale, window):
+    if prefill_on_tcgen05(q, q_stride, step, num_heads, num_kv_heads, head_dim, scale, window, out=out):
         attention_tcgen05(q, q_stride, out, k_cache, v_cache, block_table, step.cu_tokens, step.seq_slots, step.seq_starts,
                           step.seq_new, step.n_seqs, step.max_new, step.n_tokens, num_heads, num_kv_heads, head_dim, scale, window)
     elif (bf and head_dim in MMA_HEAD_DIMS and group <= 16 and (not step.is_decode or DECODE_KERNEL == "mma")

@@ -214,7 +214,7 @@ class WindowAttentionMixer(Mixer):
         if self.weights == "softmax" and not self.pool and self.sink is None and self.vd == self.hd:
             ops.attention(q, proj.stride(0), attn, cache.k, cache.v, cache.block_table, step, self.H, self.KV, self.hd, self.scale, window)
         elif (self.KERNEL == "mma" and self.weights == "softmax" and not self.pool and self.vd == self.hd
-              and ops.prefill_on_tcgen05(q, proj.stride(0), step, self.H, self.KV, self.hd, self.scale, window, self.sink)):
+              and ops.prefill_on_tcgen05(q, proj.stride(0), step, self.H, self.KV, self.hd, self.scale, window, self.sink, attn)):
             ops.attention_tcgen05(q, proj.stride(0), attn, cache.k, cache.v, cache.block_table, step.cu_tokens, step.seq_slots, step.seq_starts,
                                   step.seq_new, step.n_seqs, step.max_new, n, self.H, self.KV, self.hd, self.scale, window, self.sink)
         elif (dt == torch.bfloat16 and self.KERNEL == "mma" and self.vd == self.hd and self.hd in ops.MMA_HEAD_DIMS and self.H // self.KV <= 16

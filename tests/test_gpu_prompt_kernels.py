@@ -761,6 +761,26 @@ def test_attention_tcgen05_with_windows_and_sinks(H, KV, hd, window, with_sink):
             assert bool((off <= 2.0 ** -8 * (want.abs() + most)).all()), (s, float((off / most).max()))
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("window", [1024, 0])
+def test_attention_into_rows_between_16_byte_boundaries(hd, window):
+    """Results that start on a 4-byte boundary are written by the kernel whose stores are that small; asked for by name, tcgen05 refuses them."""
+    from kuiperllama_b200.csrc import ops
+    g, bf, H, KV, T = torch.Generator().manual_seed(hd), torch.bfloat16, 8, 2, 700
+    kc, vc = (torch.randn(11, KV, 64, hd, generator=g).to(bf).to(DEV) for _ in range(2))
+    q, table = torch.randn(T, H * hd, generator=g).to(bf).to(DEV), torch.arange(11, dtype=torch.int32, device=DEV).view(1, 11)
+    step = _step([0], [T])
+    step.is_decode, step.max_context = False, T
+    room = torch.full((T * H * hd + 8,), 7.0, dtype=bf, device=DEV)
+    out, aligned = room[2:2 + T * H * hd].view(T, H * hd), torch.empty(T, H * hd, dtype=bf, device=DEV)
+    for o in (out, aligned):
+        ops.attention(q, H * hd, o, kc, vc, table, step, H, KV, hd, hd ** -0.5, window)
+    assert float((out.double() - aligned.double()).norm() / aligned.double().norm()) <= 2.0 ** -7      # (two kernels: weights and results rounded to 2^-9)
+    assert bool((room[:2] == 7.0).all()) and bool((room[2 + T * H * hd:] == 7.0).all())
+    with pytest.raises(ops.KernelError):
+        ops.attention_tcgen05(q, H * hd, out, kc, vc, table, step.cu_tokens, step.seq_slots, step.seq_starts, step.seq_new, 1, T, T, H, KV, hd, hd ** -0.5, window)
+
+
 # a head's own 64 or 128 columns beside 16 to 64 rotated ones, ranks on both sides of a slab of 64, one to several tiles of 128 rows
 @pytest.mark.parametrize("H,d,rd,r", [(3, 64, 32, 256), (2, 64, 16, 72), (2, 64, 64, 64), (2, 128, 64, 256), (1, 128, 48, 512), (5, 64, 48, 128)])
 @pytest.mark.parametrize("window,with_sink,with_gate", [(0, True, True), (0, False, False), (70, True, False), (300, False, True)])
