@@ -448,7 +448,8 @@ def gated_delta_rule(proj: torch.Tensor, conv_col: int, b_col: int, a_col: int, 
     _need(dim <= 256, f"gated_delta_rule: key size {dim} is above 256")
     if chunked or (chunked is None and step.max_new >= DELTA_CHUNKED_FROM and n >= DELTA_CHUNKED_ROWS * step.n_seqs):
         need = -1
-        if proj.dtype == torch.bfloat16 and proj.data_ptr() % 8 == 0 and proj.stride(0) % 4 == 0 and conv_col % 4 == 0:
+        # what the chunked form takes: see kl_delta_chunked_scratch and kl_delta_chunked
+        if proj.dtype == torch.bfloat16 and proj.data_ptr() % 8 == 0 and proj.stride(0) % 4 == 0 and conv_col % 4 == 0 and conv_weight.data_ptr() % 16 == 0:
             need = lib("delta_chunked").kl_delta_chunked_scratch(n, step.n_seqs, heads, kv_heads, dim, vdim, taps)
         if need >= 0:
             scratch = torch.empty(need, dtype=torch.uint8, device=proj.device)

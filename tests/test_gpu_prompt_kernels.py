@@ -932,6 +932,22 @@ def test_delta_rule_of_steps_that_the_chunks_do_not_take():
         assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+def test_delta_rule_with_taps_between_16_byte_boundaries():
+    """A contiguous view of the taps at another offset is served as before, token by token."""
+    from kuiperllama_b200.csrc import ops
+    H, G, d, dv = 2, 1, 64, 32
+    step = _step([0], [130])
+    x = _delta_inputs(H, G, d, dv, 130, 1, 4)
+    room = torch.empty(x["C"] * 4 + 4, device=DEV)
+    taps = room[1:1 + x["C"] * 4].view(x["C"], 4)
+    taps.copy_(x["taps"])
+    walked = _delta(x, step, H, G, d, dv, False)
+    got = _delta(dict(x, taps=taps), step, H, G, d, dv, None)
+    assert torch.equal(got[0], walked[0]) and torch.equal(got[1], walked[1])
+    with pytest.raises(ops.KernelError):
+        _delta(dict(x, taps=taps), step, H, G, d, dv, True)
+
+
 # both sides of where products of few tokens cut K, take the weights as tile rows, and need a second wave of tiles; chunks of 16 tokens with a remainder
 @pytest.mark.parametrize("M,N,K", [(33, 3072, 1024), (48, 6144, 512), (64, 200, 1024), (24, 520, 4096), (17, 1024, 264), (64, 2048, 2048)])
 def test_products_of_few_tokens(M, N, K):
