@@ -51,6 +51,7 @@ struct DeltaChunkArgs {
     unsigned char* wm;                     // [chunks, H]: W in three pieces [3][DC][NP], the weights in three pieces [3][DC][DC], the factors
     float* ub;                             // [chunks, H, dv / 16, DC, 16]: T (beta V)
     int H, G, d, dv;
+    int chunk0, span;                      // the chunks of every sequence that this launch works: `span` of them from chunk0 on (0: all)
     // the projections, and the convolution's state behind S, which moves on in the walk (see recurrent.cu)
     const bf16* proj; long long ld; int conv_col, b_col, a_col; long long conv_off;
 };
@@ -60,6 +61,9 @@ template <int NP> constexpr int dc_w_bytes() { return 3 * DC * NP * 2; }
 template <int NP> constexpr int dc_wm_bytes() { return dc_w_bytes<NP>() + 3 * DC * DC * 2 + DC_FACTORS * 4; }
 // The place of a chunk that starts at row `row0` of sequence s among all chunks: a sequence's chunks follow one another, and no two share one.
 __device__ __forceinline__ size_t dc_entry(int row0, int s) { return (size_t)(row0 / DC + s); }
+// The same in a portion of `span` chunks a sequence, from chunk0 on: first row of the portion's first chunk, and its place.
+__device__ __forceinline__ int dc_first(const DeltaChunkArgs& A, int s) { return A.cu_tokens[s] + A.chunk0 * DC; }
+__device__ __forceinline__ size_t dc_entry0(const DeltaChunkArgs& A, int s) { return A.span > 0 ? (size_t)s * A.span : dc_entry(A.cu_tokens[s], s); }
 __device__ __forceinline__ bool dc_wild(float x, float most) { return !(fabsf(x) <= most); }
 
 // ------------------------------------------------------------------------------------------ convolution, unit lengths, gates
@@ -207,9 +211,9 @@ dc_head_kernel(const DeltaChunkArgs A) {
           *Ts = reinterpret_cast<float*>(dc_raw + H::T), *sc = reinterpret_cast<float*>(dc_raw + H::SC);
     float *beta = sc, *from = sc + DC, *to = sc + 2 * DC, *bfrom = sc + 3 * DC;            // beta_t, G_t, A(t, C), beta_t G_t
     const int s = blockIdx.z, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int row0 = A.cu_tokens[s] + blockIdx.x * DC, live = min(DC, A.cu_tokens[s + 1] - row0);
+    const int row0 = dc_first(A, s) + blockIdx.x * DC, live = min(DC, A.cu_tokens[s + 1] - row0);
     if (live <= 0) return;
-    const size_t entry = dc_entry(row0, s);
+    const size_t entry = dc_entry0(A, s) + blockIdx.x;
     const int d = A.d, dv = A.dv, share = A.H / A.G, g = h / share, C = 2 * A.G * d + A.H * dv;
     unsigned char* wm = A.wm + (entry * A.H + h) * dc_wm_bytes<NP>();
     unsigned char* qk = h % share == 0 ? A.qk + (entry * A.G + g) * 2 * dc_w_bytes<NP>() : nullptr;
@@ -456,19 +460,19 @@ dc_walk_kernel(const DeltaChunkArgs A) {
     extern __shared__ __align__(256) unsigned char dc_raw[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(dc_raw + L::BARS);
     const int s = blockIdx.z, h = blockIdx.y, d = A.d, dv = A.dv, g = h / (A.H / A.G), C = 2 * A.G * d + A.H * dv;
-    const int first = A.cu_tokens[s], n_new = A.cu_tokens[s + 1] - first;
+    const int first = dc_first(A, s), rest = A.cu_tokens[s + 1] - first, n_new = A.span > 0 ? min(rest, A.span * DC) : rest;
     if (n_new <= 0) return;
     const int chunks = (n_new + DC - 1) / DC;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, kc = 2 * (lane & 3);
-    const size_t entry0 = dc_entry(first, s);
+    const size_t entry0 = dc_entry0(A, s);
     float* slot = A.state + (size_t)A.seq_slots[s] * A.ld_state;
-    {                                                      // the convolution's state moves on, a share of the channels a CTA
+    if (A.chunk0 == 0) {                                   // the convolution's state moves on, a share of the channels a CTA (nothing reads it any more)
         float* cs = slot + A.conv_off;
         const int n_ctas = gridDim.x * gridDim.y, mine = blockIdx.y * gridDim.x + blockIdx.x;
         for (int c = mine * THREADS + threadIdx.x; c < C; c += n_ctas * THREADS)
             for (int m = 0; m < DC_TAPS - 1; ++m) {         // ascending: an old entry is read before it is overwritten
-                const int tt = n_new - (DC_TAPS - 1) + m;
-                cs[(size_t)m * C + c] = tt >= 0 ? to_f32(A.proj[(size_t)(first + tt) * A.ld + A.conv_col + c]) : cs[(size_t)(n_new + m) * C + c];
+                const int tt = rest - (DC_TAPS - 1) + m;
+                cs[(size_t)m * C + c] = tt >= 0 ? to_f32(A.proj[(size_t)(first + tt) * A.ld + A.conv_col + c]) : cs[(size_t)(rest + m) * C + c];
             }
     }
     if (threadIdx.x == 0) {
@@ -666,12 +670,9 @@ dc_walk_kernel(const DeltaChunkArgs A) {
 }
 
 template <int NP>
-static int launch_delta_chunked(const DeltaChunkArgs& A, int n_seqs, int max_new, cudaStream_t stream) {
-    const int run = DC_RUN * (DC_THREADS / 32);
-    launch_kernel(dc_prepare_kernel, dim3((max_new + run - 1) / run, n_seqs, A.G + (A.H * A.dv + 127) / 128 + 1), DC_THREADS, 0, stream, A);
-    KL_LAUNCH_CHECK();
+static int launch_delta_chunked(const DeltaChunkArgs& A, int chunks, int n_seqs, cudaStream_t stream) {
     KL_CUDA(cudaFuncSetAttribute(dc_head_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, DcHead<NP>::BYTES));
-    launch_kernel(dc_head_kernel<NP>, dim3((max_new + DC - 1) / DC, A.H, n_seqs), DC_THREADS, DcHead<NP>::BYTES, stream, A);
+    launch_kernel(dc_head_kernel<NP>, dim3(chunks, A.H, n_seqs), DC_THREADS, DcHead<NP>::BYTES, stream, A);
     KL_LAUNCH_CHECK();
     KL_CUDA(cudaFuncSetAttribute(dc_walk_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, DcWalk<NP>::BYTES));
     launch_kernel_after(dc_walk_kernel<NP>, dim3(A.dv / DC_COLS, A.H, n_seqs), NP / 16 * 32, DcWalk<NP>::BYTES, stream, A);
@@ -682,38 +683,74 @@ static long long dc_round(long long bytes) { return (bytes + 255) / 256 * 256; }
 static long long dc_wm(int d) { return d <= 64 ? dc_wm_bytes<64>() : dc_wm_bytes<128>(); }
 static long long dc_qk(int d) { return 2 * (d <= 64 ? dc_w_bytes<64>() : dc_w_bytes<128>()); }
 
+// What a step's scratch holds: what is prepared of every row, and all chunks where they take up to `limit` bytes, else as many chunks of every sequence as
+// that (one at least), and the step is worked in portions of so many.
+struct DcPlan {
+    long long entries, bytes;
+    int chunks, span;                      // chunks of the longest sequence; of every sequence in a portion (0: all of them at once)
+    DcPlan(int rows, int n_seqs, int max_new, int H, int G, int d, int dv, long long limit) {
+        chunks = (max_new + DC - 1) / DC;
+        const long long one = (long long)G * dc_qk(d) + (long long)H * (dc_wm(d) + (long long)dv * DC * 4), C = 2LL * G * d + (long long)H * dv;
+        entries = rows / DC + n_seqs + 1;
+        span = 0;
+        if (entries * one > limit) {
+            const long long most = limit / one / n_seqs;
+            span = most < 1 ? 1 : most < chunks ? (int)most : chunks;
+            if ((long long)span * n_seqs < entries) entries = (long long)span * n_seqs;
+            else span = 0;
+        }
+        bytes = dc_round(entries * G * dc_qk(d)) + dc_round(entries * H * dc_wm(d)) + dc_round(entries * H * dv * DC * 4) + dc_round(rows * C * 4) + dc_round(2LL * rows * H * 4);
+    }
+    int portions() const { return span > 0 ? (chunks + span - 1) / span : 1; }
+};
+
 }  // namespace kl
 
 using namespace kl;
 
-// Bytes of scratch that kl_delta_chunked needs for these sizes, or -1 where it does not run them: keys a multiple of 8 up to 128, values one of
-// 16, four taps.
-KL_API long long kl_delta_chunked_scratch(int rows, int n_seqs, int H, int G, int d, int dv, int taps) {
-    if (rows <= 0 || n_seqs <= 0 || n_seqs > 65535 || H <= 0 || G <= 0 || H % G || H > 65535 || d <= 0 || d > 128 || d % 8 || dv <= 0 || dv % 16 || taps != DC_TAPS) return -1;
-    const long long entries = rows / DC + n_seqs + 1, C = 2LL * G * d + (long long)H * dv;
-    if (G + (C + 127) / 128 + 1 > 65535) return -1;
-    return dc_round(entries * G * dc_qk(d)) + dc_round(entries * H * dc_wm(d)) + dc_round(entries * H * dv * DC * 4) + dc_round(rows * C * 4) + dc_round(2LL * rows * H * 4);
+// 1 where the chunked form runs these sizes: keys a multiple of 8 up to 128, values one of 16, four taps.
+KL_API int kl_delta_chunked_fits(int n_seqs, int H, int G, int d, int dv, int taps) {
+    if (n_seqs <= 0 || n_seqs > 65535 || H <= 0 || G <= 0 || H % G || H > 65535 || d <= 0 || d > 128 || d % 8 || dv <= 0 || dv % 16 || taps != DC_TAPS) return 0;
+    return G + (2LL * G * d + (long long)H * dv + 127) / 128 + 1 <= 65535;
+}
+// Bytes of scratch that kl_delta_chunked needs, and in how many portions it works a step whose chunks keep to `limit` bytes (two launches each, and one before).
+KL_API long long kl_delta_chunked_scratch(int rows, int n_seqs, int max_new, int H, int G, int d, int dv, long long limit) {
+    return DcPlan(rows, n_seqs, max_new, H, G, d, dv, limit).bytes;
+}
+KL_API int kl_delta_chunked_portions(int rows, int n_seqs, int max_new, int H, int G, int d, int dv, long long limit) {
+    return DcPlan(rows, n_seqs, max_new, H, G, d, dv, limit).portions();
 }
 
 // What kl_gated_delta_rule does, for bfloat16 rows of proj whose q | k | v start on an 8-byte boundary, rows a multiple of four elements apart.
 // scratch: kl_delta_chunked_scratch bytes on a 16-byte boundary.
 KL_API int kl_delta_chunked(const void* proj, long long ld, int conv_col, int b_col, int a_col, const float* taps_w, int taps, const float* A_log,
-                            const float* dt_bias, float* state, long long ld_state, long long conv_off, float* out, void* scratch, const int* cu_tokens,
-                            const int* seq_slots, int rows, int n_seqs, int max_new, int H, int G, int d, int dv, float q_scale, float unit_eps,
-                            cudaStream_t stream) {
+                            const float* dt_bias, float* state, long long ld_state, long long conv_off, float* out, void* scratch, long long limit,
+                            const int* cu_tokens, const int* seq_slots, int rows, int n_seqs, int max_new, int H, int G, int d, int dv, float q_scale,
+                            float unit_eps, cudaStream_t stream) {
     if (rows <= 0 || n_seqs <= 0 || max_new <= 0) return KL_OK;
-    if (kl_delta_chunked_scratch(rows, n_seqs, H, G, d, dv, taps) < 0) return KL_ERR_BAD_SIZE;
+    if (!kl_delta_chunked_fits(n_seqs, H, G, d, dv, taps)) return KL_ERR_BAD_SIZE;
     if (((uintptr_t)scratch | (uintptr_t)taps_w) % 16 || (uintptr_t)proj % 8 || conv_col % 4 || ld % 4) return KL_ERR_BAD_ALIGN;
-    const long long entries = rows / DC + n_seqs + 1, C = 2LL * G * d + (long long)H * dv;
+    const long long C = 2LL * G * d + (long long)H * dv;
+    const DcPlan plan(rows, n_seqs, max_new, H, G, d, dv, limit);
     DeltaChunkArgs A;
     A.taps_w = taps_w; A.A_log = A_log; A.dt_bias = dt_bias; A.q_scale = q_scale; A.unit_eps = unit_eps;
     A.state = state; A.ld_state = ld_state; A.out = out; A.cu_tokens = cu_tokens; A.seq_slots = seq_slots; A.H = H; A.G = G; A.d = d; A.dv = dv;
     A.proj = (const bf16*)proj; A.ld = ld; A.conv_col = conv_col; A.b_col = b_col; A.a_col = a_col; A.conv_off = conv_off;
+    A.chunk0 = 0; A.span = plan.span;
     unsigned char* at = (unsigned char*)scratch;
-    A.qk = at; at += dc_round(entries * G * dc_qk(d));
-    A.wm = at; at += dc_round(entries * H * dc_wm(d));
-    A.ub = (float*)at; at += dc_round(entries * H * dv * DC * 4);
+    A.qk = at; at += dc_round(plan.entries * G * dc_qk(d));
+    A.wm = at; at += dc_round(plan.entries * H * dc_wm(d));
+    A.ub = (float*)at; at += dc_round(plan.entries * H * dv * DC * 4);
     A.prep = (float*)at; at += dc_round(rows * C * 4);
     A.bg = (float*)at;
-    return d <= 64 ? launch_delta_chunked<64>(A, n_seqs, max_new, stream) : launch_delta_chunked<128>(A, n_seqs, max_new, stream);
+    const int run = DC_RUN * (DC_THREADS / 32);
+    launch_kernel(dc_prepare_kernel, dim3((max_new + run - 1) / run, n_seqs, G + (H * dv + 127) / 128 + 1), DC_THREADS, 0, stream, A);
+    KL_LAUNCH_CHECK();
+    for (int i = 0; i < plan.portions(); ++i) {            // (S goes from one portion to the next through the slot, as the 32-bit numbers that it is)
+        A.chunk0 = i * plan.span;
+        const int chunks = plan.span > 0 ? (plan.span < plan.chunks - A.chunk0 ? plan.span : plan.chunks - A.chunk0) : plan.chunks;
+        const int rc = d <= 64 ? launch_delta_chunked<64>(A, chunks, n_seqs, stream) : launch_delta_chunked<128>(A, chunks, n_seqs, stream);
+        if (rc != KL_OK) return rc;
+    }
+    return KL_OK;
 }

@@ -424,6 +424,9 @@ def mingru_scan(proj: torch.Tensor, z_col: int, x_col: int, g_col: int, bias_z: 
 # eight of 64 80 / 67, one of 64 beside 31 single tokens 42 / 150; 32 heads of 64 x 64 on 8, 64 21.6 / 25.6, 128 32.9 / 30.2, 32 of 64 134 / 162;
 # 4 heads of 128 x 128, eight of 64 29.6 / 34.1.
 DELTA_CHUNKED_FROM, DELTA_CHUNKED_ROWS = 96, 64
+# Bytes that the operands of a step's chunks take at most, here and in ``outer_recurrence`` (30 KB a token with 16 heads of 128 x 128, 7 KB with 64 of 128 x
+# 64): longer steps are worked in portions, 8,900 tokens of the former in one, so what a step holds beside its rows does not grow with a prompt.
+CHUNK_SCRATCH = 256 << 20
 
 
 def gated_delta_rule(proj: torch.Tensor, conv_col: int, b_col: int, a_col: int, conv_weight: torch.Tensor, A_log: torch.Tensor,
@@ -447,17 +450,18 @@ def gated_delta_rule(proj: torch.Tensor, conv_col: int, b_col: int, a_col: int, 
     _need(out.dtype == torch.float32 and out.is_contiguous() and out.shape[0] >= n and out.shape[1] == heads * vdim, "gated_delta_rule: out")
     _need(dim <= 256, f"gated_delta_rule: key size {dim} is above 256")
     if chunked or (chunked is None and step.max_new >= DELTA_CHUNKED_FROM and n >= DELTA_CHUNKED_ROWS * step.n_seqs):
-        need = -1
-        # what the chunked form takes: see kl_delta_chunked_scratch and kl_delta_chunked
-        if proj.dtype == torch.bfloat16 and proj.data_ptr() % 8 == 0 and proj.stride(0) % 4 == 0 and conv_col % 4 == 0 and conv_weight.data_ptr() % 16 == 0:
-            need = lib("delta_chunked").kl_delta_chunked_scratch(n, step.n_seqs, heads, kv_heads, dim, vdim, taps)
-        if need >= 0:
-            scratch = torch.empty(need, dtype=torch.uint8, device=proj.device)
-            _check(lib("delta_chunked").kl_delta_chunked(
+        L = lib("delta_chunked")
+        # what the chunked form takes: see kl_delta_chunked_fits and kl_delta_chunked
+        if (proj.dtype == torch.bfloat16 and proj.data_ptr() % 8 == 0 and proj.stride(0) % 4 == 0 and conv_col % 4 == 0 and conv_weight.data_ptr() % 16 == 0
+                and n > 0 and L.kl_delta_chunked_fits(step.n_seqs, heads, kv_heads, dim, vdim, taps)):
+            limit = ctypes.c_longlong(CHUNK_SCRATCH)
+            sizes = (n, step.n_seqs, int(step.max_new), heads, kv_heads, dim, vdim)
+            scratch = torch.empty(L.kl_delta_chunked_scratch(*sizes, limit), dtype=torch.uint8, device=proj.device)
+            _check(L.kl_delta_chunked(
                 _ptr(proj), ctypes.c_longlong(proj.stride(0)), conv_col, b_col, a_col, _ptr(conv_weight), taps, _ptr(A_log), _ptr(dt_bias),
-                _ptr(state), ctypes.c_longlong(state.stride(0)), ctypes.c_longlong(conv_off), _ptr(out), _ptr(scratch), _ptr(step.cu_tokens),
-                _ptr(step.seq_slots), n, step.n_seqs, int(step.max_new), heads, kv_heads, dim, vdim, ctypes.c_float(q_scale), ctypes.c_float(unit_eps),
-                _stream()), "gated_delta_rule", 3)
+                _ptr(state), ctypes.c_longlong(state.stride(0)), ctypes.c_longlong(conv_off), _ptr(out), _ptr(scratch), limit, _ptr(step.cu_tokens),
+                _ptr(step.seq_slots), *sizes, ctypes.c_float(q_scale), ctypes.c_float(unit_eps),
+                _stream()), "gated_delta_rule", 1 + 2 * L.kl_delta_chunked_portions(*sizes, limit))
             return
         _need(not chunked, "gated_delta_rule: the chunked form does not run these operands")
     prep = torch.empty((n, C), dtype=torch.float32, device=proj.device)
@@ -1250,19 +1254,20 @@ def outer_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch
     _need(y.dtype == torch.float32 and y.dim() == 2 and y.stride(1) == 1 and y.shape[0] >= n and y.shape[1] == heads * P, "outer_recurrence: y")
     _need(heads % groups == 0 and N <= 1024, "outer_recurrence: heads in equal groups, at most 1,024 rows of state")
     if chunked or (chunked is None and step.max_new >= OUTER_CHUNKED_FROM and n >= OUTER_CHUNKED_ROWS * step.n_seqs):
-        # what the chunked form takes: see kl_outer_chunked_scratch; rows of q and k (and of a, with a decay per row) on 16-byte boundaries
+        # what the chunked form takes: see kl_outer_chunked_fits; rows of q and k (and of a, with a decay per row) on 16-byte boundaries
         aligned = lambda t: t.data_ptr() % 16 == 0 and t.stride(0) * t.element_size() % 16 == 0
-        need = -1
-        if normaliser is None and aligned(q) and aligned(k) and (not per_row or aligned(a)):
-            need = lib("outer_chunked").kl_outer_chunked_scratch(n, step.n_seqs, int(step.max_new), heads, groups, N, P, int(per_row), dtype_code(q.dtype))
-        if need >= 0:
-            scratch = torch.empty(need, dtype=torch.uint8, device=q.device)
-            _check(lib("outer_chunked").kl_outer_chunked(
+        L = lib("outer_chunked")
+        if (normaliser is None and aligned(q) and aligned(k) and (not per_row or aligned(a)) and n > 0
+                and L.kl_outer_chunked_fits(step.n_seqs, heads, groups, N, P, int(per_row), dtype_code(q.dtype))):
+            limit = ctypes.c_longlong(CHUNK_SCRATCH)
+            plan = (n, step.n_seqs, int(step.max_new), heads, groups, N, int(per_row), limit)
+            scratch = torch.empty(L.kl_outer_chunked_scratch(*plan), dtype=torch.uint8, device=q.device)
+            _check(L.kl_outer_chunked(
                 _ptr(q), ctypes.c_longlong(q.stride(0)), _ptr(k), ctypes.c_longlong(k.stride(0)), _ptr(v), ctypes.c_longlong(v.stride(0)),
                 _ptr(a), ctypes.c_longlong(a.stride(0)), int(per_row), _ptr(c), ctypes.c_longlong(c.stride(0) if c is not None else 0), _ptr(skip),
-                _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(y), ctypes.c_longlong(y.stride(0)), _ptr(scratch), _ptr(step.cu_tokens),
+                _ptr(state), ctypes.c_longlong(state.stride(0)), _ptr(y), ctypes.c_longlong(y.stride(0)), _ptr(scratch), limit, _ptr(step.cu_tokens),
                 _ptr(step.seq_slots), n, step.n_seqs, int(step.max_new), heads, groups, N, P, ctypes.c_float(q_scale), dtype_code(q.dtype),
-                _stream()), "outer_recurrence", 2)
+                _stream()), "outer_recurrence", 2 * L.kl_outer_chunked_portions(*plan))
             return
         _need(not chunked, "outer_recurrence: the chunked form does not run these operands")
     _check(lib("outer_recurrence").kl_outer_recurrence(

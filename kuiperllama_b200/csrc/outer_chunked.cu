@@ -56,12 +56,16 @@ struct OuterChunkArgs {
     unsigned char* kp;                     // [chunks, units]: k in three pieces [3][OC][NP]
     float* prod;                           // [chunks, groups] (one decay per head): the products of the chunk's tokens [OC][OC_MS] and whether it goes token by token [4]
     float* fac;                            // [chunks, heads] (one decay per head): [OC][OC_FAC] and the same [4]
-    int heads, groups, N, P, max_chunks;
+    int heads, groups, N, P;
+    int chunk0, span;                      // the chunks of every sequence that this launch works: `span` of them from chunk0 on (0: all)
     float q_scale;
 };
 
 // The place of a chunk that starts at row `row0` of sequence s among all chunks: a sequence's chunks follow one another, and no two share one.
 __device__ __forceinline__ size_t oc_entry(int row0, int s) { return (size_t)(row0 / OC + s); }
+// The same in a portion of `span` chunks a sequence, from chunk0 on: first row of the portion's first chunk, and its place.
+__device__ __forceinline__ int oc_first(const OuterChunkArgs& A, int s) { return A.cu_tokens[s] + A.chunk0 * OC; }
+__device__ __forceinline__ size_t oc_entry0(const OuterChunkArgs& A, int s) { return A.span > 0 ? (size_t)s * A.span : oc_entry(A.cu_tokens[s], s); }
 constexpr int OC_PROD = OC * OC_MS + 4, OC_FACS = OC * OC_FAC + 4;             // floats of a piece of `prod` and of `fac`
 template <int NP> constexpr int oc_k_bytes() { return 3 * OC * NP * 2; }
 template <int NP, int MODE> constexpr int oc_q_bytes() { return oc_k_bytes<NP>() + (MODE == 1 ? 3 * OC * OC * 2 + NP * 4 + 256 : 0); }
@@ -78,9 +82,9 @@ oc_group_kernel(const OuterChunkArgs A) {
     pdl_wait();
     extern __shared__ __align__(256) unsigned char oc_raw[];
     const int s = blockIdx.z, ch = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int row0 = A.cu_tokens[s] + ch * OC, live = min(OC, A.cu_tokens[s + 1] - row0);
+    const int row0 = oc_first(A, s) + ch * OC, live = min(OC, A.cu_tokens[s + 1] - row0);
     if (live <= 0) return;
-    const size_t entry = oc_entry(row0, s);
+    const size_t entry = oc_entry0(A, s) + ch;
     if ((int)blockIdx.y >= A.groups) {
         const int h = (blockIdx.y - A.groups) * 4 + warp;
         if (h >= A.heads) return;
@@ -204,10 +208,10 @@ oc_row_kernel(const OuterChunkArgs A) {
     double* pre = reinterpret_cast<double*>(ks + OC * RS); // [2][NP]: the blocks' whole products
     float* ms = reinterpret_cast<float*>(pre + 2 * NP);    // [OC][OC_MS]: the weighted products
     const int s = blockIdx.z, h = blockIdx.y, ch = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, N = A.N;
-    const int row0 = A.cu_tokens[s] + ch * OC, live = min(OC, A.cu_tokens[s + 1] - row0);
+    const int row0 = oc_first(A, s) + ch * OC, live = min(OC, A.cu_tokens[s + 1] - row0);
     if (live <= 0) return;
     const int g = h / (A.heads / A.groups);
-    const size_t entry = oc_entry(row0, s);
+    const size_t entry = oc_entry0(A, s) + ch;
     unsigned char* qm = A.qp + (entry * A.heads + h) * oc_q_bytes<NP, 1>();
     bf16* kp = reinterpret_cast<bf16*>(A.kp + (entry * A.heads + h) * oc_k_bytes<NP>());
     bool wild = false;
@@ -433,14 +437,14 @@ oc_walk_kernel(const OuterChunkArgs A) {
         }
         s = __ffs(__ballot_sync(0xffffffffu, lane < gridDim.z && longer == (int)blockIdx.z)) - 1;
     }
-    const int first = A.cu_tokens[s], n_new = A.cu_tokens[s + 1] - first, h = blockIdx.y;
+    const int first = oc_first(A, s), rest = A.cu_tokens[s + 1] - first, n_new = A.span > 0 ? min(rest, A.span * OC) : rest, h = blockIdx.y;
     if (n_new <= 0) return;
     const int chunks = (n_new + OC - 1) / OC;
     const int r = lane >> 2, kc = 2 * (lane & 3);
     const int N = A.N, P = A.P, g = h / (A.heads / A.groups), units = MODE == 1 ? A.heads : A.groups, unit = MODE == 1 ? h : g;
     const int p0 = blockIdx.x * OC_COLS + pw * 16;
     const bool on = p0 < P;                                // P is a multiple of 16
-    const size_t entry0 = oc_entry(first, s);
+    const size_t entry0 = oc_entry0(A, s);
     float* S_slot = A.state + (size_t)A.seq_slots[s] * A.ld_state + (size_t)h * N * P;
     const float skip = A.skip != nullptr ? A.skip[h] : 0.f;
     if (threadIdx.x == 0) {
@@ -737,14 +741,14 @@ oc_walk_kernel(const OuterChunkArgs A) {
 }
 
 template <int NP, int MODE>
-static int launch_outer_chunked(const OuterChunkArgs& A, int n_seqs, cudaStream_t stream) {
+static int launch_outer_chunked(const OuterChunkArgs& A, int chunks, int n_seqs, cudaStream_t stream) {
     const int pre = MODE == 0 ? 2 * 3 * OC * NP * 2 : (3 * OC * (NP + 4) + 4 * NP + OC * OC_MS) * 4;
     if constexpr (MODE == 0) {
         KL_CUDA(cudaFuncSetAttribute(oc_group_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, pre));
-        launch_kernel(oc_group_kernel<NP>, dim3(A.max_chunks, A.groups + (A.heads + 3) / 4, n_seqs), OC_THREADS, pre, stream, A);
+        launch_kernel(oc_group_kernel<NP>, dim3(chunks, A.groups + (A.heads + 3) / 4, n_seqs), OC_THREADS, pre, stream, A);
     } else {
         KL_CUDA(cudaFuncSetAttribute(oc_row_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, pre));
-        launch_kernel(oc_row_kernel<NP>, dim3(A.max_chunks, A.heads, n_seqs), OC_THREADS, pre, stream, A);
+        launch_kernel(oc_row_kernel<NP>, dim3(chunks, A.heads, n_seqs), OC_THREADS, pre, stream, A);
     }
     KL_LAUNCH_CHECK();
     constexpr int smem = OcWalk<NP, MODE>::BYTES;
@@ -760,41 +764,74 @@ static long long oc_q(int N, int a_per_row) {
 static long long oc_k(int N) { return N <= 64 ? oc_k_bytes<64>() : oc_k_bytes<128>(); }
 static long long oc_round(long long bytes) { return (bytes + 255) / 256 * 256; }
 
+// What a step's scratch holds: all chunks where they take up to `limit` bytes, else as many chunks of every sequence as that (one at least), and the step
+// is worked in portions of so many.
+struct OcPlan {
+    long long units, entries, bytes;
+    int chunks, span;                      // chunks of the longest sequence; of every sequence in a portion (0: all of them at once)
+    OcPlan(int rows, int n_seqs, int max_new, int heads, int groups, int N, int a_per_row, long long limit) {
+        units = a_per_row ? heads : groups;
+        chunks = (max_new + OC - 1) / OC;
+        const long long one = units * (oc_q(N, a_per_row) + oc_k(N)) + (a_per_row ? 0 : (long long)groups * OC_PROD * 4 + (long long)heads * OC_FACS * 4);
+        entries = rows / OC + n_seqs + 1;
+        span = 0;
+        if (entries * one > limit) {
+            const long long most = limit / one / n_seqs;
+            span = most < 1 ? 1 : most < chunks ? (int)most : chunks;
+            if ((long long)span * n_seqs < entries) entries = (long long)span * n_seqs;
+            else span = 0;
+        }
+        bytes = oc_round(entries * units * oc_q(N, a_per_row)) + oc_round(entries * units * oc_k(N)) +
+                (a_per_row ? 0 : oc_round(entries * groups * OC_PROD * 4) + oc_round(entries * heads * OC_FACS * 4));
+    }
+    int portions() const { return span > 0 ? (chunks + span - 1) / span : 1; }
+};
+
 }  // namespace kl
 
 using namespace kl;
 
-// Bytes of scratch that kl_outer_chunked needs for these sizes, or -1 where it does not run them: float32 k, q and v with one decay per head,
-// or bfloat16 ones with a decay per row of S; N a multiple of 8 up to 128, P one of 16.
-KL_API long long kl_outer_chunked_scratch(int rows, int n_seqs, int max_new, int heads, int groups, int N, int P, int a_per_row, int in_dtype) {
-    if (rows <= 0 || n_seqs <= 0 || max_new <= 0 || heads <= 0 || groups <= 0 || heads % groups || heads + groups > 65535 || n_seqs > 65535) return -1;
-    if (N <= 0 || N > 128 || N % 8 || P <= 0 || P % 16) return -1;
-    if (!(in_dtype == KL_F32 && !a_per_row) && !(in_dtype == KL_BF16 && a_per_row)) return -1;
-    const long long units = a_per_row ? heads : groups, entries = rows / OC + n_seqs + 1;
-    return oc_round(entries * units * oc_q(N, a_per_row)) + oc_round(entries * units * oc_k(N)) +
-           (a_per_row ? 0 : oc_round(entries * groups * OC_PROD * 4) + oc_round(entries * heads * OC_FACS * 4));
+// 1 where the chunked form runs these sizes: float32 k, q and v with one decay per head, or bfloat16 ones with a decay per row of S; N a multiple of 8
+// up to 128, P one of 16.
+KL_API int kl_outer_chunked_fits(int n_seqs, int heads, int groups, int N, int P, int a_per_row, int in_dtype) {
+    if (n_seqs <= 0 || heads <= 0 || groups <= 0 || heads % groups || heads + groups > 65535 || n_seqs > 65535) return 0;
+    if (N <= 0 || N > 128 || N % 8 || P <= 0 || P % 16) return 0;
+    return (in_dtype == KL_F32 && !a_per_row) || (in_dtype == KL_BF16 && a_per_row);
+}
+// Bytes of scratch that kl_outer_chunked needs, and in how many portions it works a step whose scratch keeps to `limit` bytes (two launches each).
+KL_API long long kl_outer_chunked_scratch(int rows, int n_seqs, int max_new, int heads, int groups, int N, int a_per_row, long long limit) {
+    return OcPlan(rows, n_seqs, max_new, heads, groups, N, a_per_row, limit).bytes;
+}
+KL_API int kl_outer_chunked_portions(int rows, int n_seqs, int max_new, int heads, int groups, int N, int a_per_row, long long limit) {
+    return OcPlan(rows, n_seqs, max_new, heads, groups, N, a_per_row, limit).portions();
 }
 
 // q, k, v, a, c, skip, state and y as kl_outer_recurrence takes them (no normaliser); rows of k and q (and of a, with a decay per row) on
 // 16-byte boundaries.  scratch: kl_outer_chunked_scratch bytes on a 16-byte boundary.
 KL_API int kl_outer_chunked(const void* q, long long ld_q, const void* k, long long ld_k, const void* v, long long ld_v, const float* a, long long ld_a,
                             int a_per_row, const float* c, long long ld_c, const float* skip, float* state, long long ld_state, float* y,
-                            long long ld_y, void* scratch, const int* cu_tokens, const int* seq_slots, int rows, int n_seqs, int max_new, int heads,
-                            int groups, int N, int P, float q_scale, int in_dtype, cudaStream_t stream) {
+                            long long ld_y, void* scratch, long long limit, const int* cu_tokens, const int* seq_slots, int rows, int n_seqs, int max_new,
+                            int heads, int groups, int N, int P, float q_scale, int in_dtype, cudaStream_t stream) {
     if (rows <= 0 || n_seqs <= 0 || max_new <= 0) return KL_OK;
-    if (kl_outer_chunked_scratch(rows, n_seqs, max_new, heads, groups, N, P, a_per_row, in_dtype) < 0) return KL_ERR_BAD_SIZE;
+    if (!kl_outer_chunked_fits(n_seqs, heads, groups, N, P, a_per_row, in_dtype)) return KL_ERR_BAD_SIZE;
     const int w = in_dtype == KL_F32 ? 4 : 8;
     if ((((uintptr_t)q | (uintptr_t)k | (uintptr_t)scratch) & 15) || ld_q % w || ld_k % w || (a_per_row && (((uintptr_t)a & 15) || ld_a % 4))) return KL_ERR_BAD_ALIGN;
-    const long long units = a_per_row ? heads : groups, entries = rows / OC + n_seqs + 1;
+    const OcPlan plan(rows, n_seqs, max_new, heads, groups, N, a_per_row, limit);
     OuterChunkArgs A;
     A.q = q; A.ld_q = ld_q; A.k = k; A.ld_k = ld_k; A.v = v; A.ld_v = ld_v; A.a = a; A.ld_a = ld_a; A.c = c; A.ld_c = ld_c; A.skip = skip;
     A.state = state; A.ld_state = ld_state; A.y = y; A.ld_y = ld_y; A.cu_tokens = cu_tokens; A.seq_slots = seq_slots;
-    A.heads = heads; A.groups = groups; A.N = N; A.P = P; A.max_chunks = (max_new + OC - 1) / OC; A.q_scale = q_scale;
+    A.heads = heads; A.groups = groups; A.N = N; A.P = P; A.q_scale = q_scale; A.span = plan.span;
     unsigned char* at = (unsigned char*)scratch;
-    A.qp = at; at += oc_round(entries * units * oc_q(N, a_per_row));
-    A.kp = at; at += oc_round(entries * units * oc_k(N));
-    A.prod = a_per_row ? nullptr : (float*)at; at += a_per_row ? 0 : oc_round(entries * groups * OC_PROD * 4);
+    A.qp = at; at += oc_round(plan.entries * plan.units * oc_q(N, a_per_row));
+    A.kp = at; at += oc_round(plan.entries * plan.units * oc_k(N));
+    A.prod = a_per_row ? nullptr : (float*)at; at += a_per_row ? 0 : oc_round(plan.entries * groups * OC_PROD * 4);
     A.fac = a_per_row ? nullptr : (float*)at;
-    if (a_per_row) return N <= 64 ? launch_outer_chunked<64, 1>(A, n_seqs, stream) : launch_outer_chunked<128, 1>(A, n_seqs, stream);
-    return N <= 64 ? launch_outer_chunked<64, 0>(A, n_seqs, stream) : launch_outer_chunked<128, 0>(A, n_seqs, stream);
+    for (int i = 0; i < plan.portions(); ++i) {            // (S goes from one portion to the next through the slot, as the 32-bit numbers that it is)
+        A.chunk0 = i * plan.span;
+        const int chunks = plan.span > 0 ? (plan.span < plan.chunks - A.chunk0 ? plan.span : plan.chunks - A.chunk0) : plan.chunks;
+        const int rc = a_per_row ? (N <= 64 ? launch_outer_chunked<64, 1>(A, chunks, n_seqs, stream) : launch_outer_chunked<128, 1>(A, chunks, n_seqs, stream))
+                                 : (N <= 64 ? launch_outer_chunked<64, 0>(A, chunks, n_seqs, stream) : launch_outer_chunked<128, 0>(A, chunks, n_seqs, stream));
+        if (rc != KL_OK) return rc;
+    }
+    return KL_OK;
 }

@@ -932,6 +932,51 @@ def test_delta_rule_of_steps_that_the_chunks_do_not_take():
         assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize("news", [[700], [200, 1, 333, 64, 40], [97, 96]])
+@pytest.mark.parametrize("chunks", [0, 1, 7, 12])
+def test_chunks_in_portions_have_the_same_bits(monkeypatch, news, chunks):
+    """What a step's chunks take is bounded: beyond it a step is worked in portions, one chunk a sequence at the least, with the same results."""
+    from kuiperllama_b200.csrc import ops
+    step, H, G, d, dv = _step([0] * len(news), news), 4, 2, 64, 32
+    x = _delta_inputs(H, G, d, dv, step.n_tokens, len(news), 9)
+    g = torch.Generator(device=DEV).manual_seed(7)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    n, p, rows = 64, 48, step.n_tokens
+    q, k, v = (rand(rows, 2 * n), 0.3 * rand(rows, 2 * n), rand(rows, 4 * p))
+    decay = {False: torch.rand(rows, 4, device=DEV, generator=g) ** 0.1, True: torch.rand(rows, 4 * n, device=DEV, generator=g) ** 0.1}
+    qb, kb, state0 = rand(rows, 4 * n).bfloat16(), rand(rows, 4 * n).bfloat16(), 0.1 * rand(len(news), 4 * n * p)
+
+    def outer(per_row):
+        state, y = state0.clone(), torch.full((rows, 4 * p), 7.0, device=DEV)
+        ops.outer_recurrence(qb if per_row else q, kb if per_row else k, v.bfloat16() if per_row else v, decay[per_row], state, y, step, 4, 4 if per_row else 2, n, p,
+                             q_scale=0.7, chunked=True)
+        return y, state
+
+    whole = [_delta(x, step, H, G, d, dv, True), outer(False), outer(True)]
+    # bytes of a chunk of every sequence: the pieces of q and k for every unit, and what the products and factors take
+    sizes = [2 * 24576 + 4 * (12288 + 6144 + 512 + 4096), 2 * 24576 + 2 * (32 * 36 + 4) * 4 + 4 * (32 * 20 + 4) * 4, 4 * (24576 + 6144 + 512)]
+    for want, one, run in zip(whole, sizes, (lambda: _delta(x, step, H, G, d, dv, True), lambda: outer(False), lambda: outer(True))):
+        monkeypatch.setattr(ops, "CHUNK_SCRATCH", one * chunks * len(news))
+        before = ops.launch_count
+        got = run()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+        portions = -(-(-(-max(news) // 32)) // max(1, chunks))
+        if chunks <= 1 or len(news) == 1:
+            assert ops.launch_count - before in (2 * portions, 2 * portions + 1)
+        monkeypatch.undo()
+
+
+def test_scratch_of_a_long_step_is_bounded():
+    from kuiperllama_b200.csrc import ops
+    import ctypes
+    limit = ctypes.c_longlong(ops.CHUNK_SCRATCH)
+    for n, seqs in ((32768, 1), (131072, 1), (131072, 8)):
+        outer = ops.lib("outer_chunked").kl_outer_chunked_scratch(n, seqs, n, 64, 1, 128, 0, limit)
+        rows = n * (2 * 4 * 128 + 16 * 128 + 32) * 4                           # what is prepared of every row, as token by token
+        delta = ops.lib("delta_chunked").kl_delta_chunked_scratch(n, seqs, n, 16, 4, 128, 128, limit) - rows
+        assert outer <= ops.CHUNK_SCRATCH + 4096 and delta <= ops.CHUNK_SCRATCH + 4096, (outer, delta)
+
+
 def test_delta_rule_with_taps_between_16_byte_boundaries():
     """A contiguous view of the taps at another offset is served as before, token by token."""
     from kuiperllama_b200.csrc import ops
