@@ -60,6 +60,8 @@ SOURCES: Dict[str, str] = {
     "streams": "streams.cu",
     "host_tokens": "host_tokens.cpp",
 }
+# modules that what uses them does without (the interpreter's headers may be missing): the engine then goes through numpy
+OPTIONAL = ("host_tokens",)
 HEADERS: List[str] = ["common.cuh", "attention_mma.cuh", "tcgen05.cuh", "pieces.cuh", "tma_host.cuh", "attention_decode_noalloc.h"]
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -179,11 +181,21 @@ def ensure_built(name: str, quiet: bool = False) -> str:
 
 
 def build_all(quiet: bool = False, jobs: Optional[int] = None) -> Dict[str, str]:
-    """Compile every module (in parallel) and return name -> library path."""
+    """Compile every module (in parallel) and return name -> library path; an optional one that cannot be built is reported and left out."""
     jobs = jobs or min(len(SOURCES), os.cpu_count() or 2)
+
+    def one(name: str) -> Optional[str]:
+        try:
+            return ensure_built(name, quiet)
+        except ExtensionError as e:
+            if name not in OPTIONAL:
+                raise
+            _say(f"{name} is left out: {e}")
+            return None
+
     with ThreadPoolExecutor(max_workers=jobs) as pool:
-        paths = list(pool.map(lambda n: ensure_built(n, quiet), SOURCES))
-    return dict(zip(SOURCES, paths))
+        paths = list(pool.map(one, SOURCES))
+    return {name: path for name, path in zip(SOURCES, paths) if path is not None}
 
 
 if __name__ == "__main__":

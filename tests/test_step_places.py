@@ -1,6 +1,9 @@
 """The wanted places of a step: checked as one array, with the answers that one by one gave."""
 from __future__ import annotations
 
+import os
+import sysconfig
+
 import numpy as np
 import pytest
 
@@ -51,4 +54,27 @@ def test_token_ids_of_a_long_prompt():
     from kuiperllama_b200.engine import step
     tokens = [(i * 7919) % 128256 for i in range(5000)]
     ids, lo, hi = step._token_ids(tokens, len(tokens))
-    assert ids.tolist() == tokens and (lo, hi) == (min(tokens), max(tokens)) and step._host_tokens
+    assert ids.tolist() == tokens and (lo, hi) == (min(tokens), max(tokens))
+    assert step._host_tokens or not os.path.exists(os.path.join(sysconfig.get_paths()["include"], "Python.h"))
+
+
+def test_a_build_without_the_interpreters_headers_leaves_out_what_needs_them(monkeypatch):
+    """Everything else is built, a failure of anything else is one, and ids go through numpy."""
+    from kuiperllama_b200.csrc import build
+    from kuiperllama_b200.engine import step
+
+    def fails(*names):
+        def ensure_built(name, quiet=False):
+            if name in names:
+                raise build.ExtensionError(f"nvcc failed on {name}")
+            return f"{name}.so"
+        return ensure_built
+
+    monkeypatch.setattr(build, "ensure_built", fails("host_tokens"))
+    assert build.build_all(quiet=True) == {n: f"{n}.so" for n in build.SOURCES if n != "host_tokens"}
+    monkeypatch.setattr(step, "_host_tokens", None)
+    ids, lo, hi = step._token_ids([5, 2, 9], 3)
+    assert ids.tolist() == [5, 2, 9] and (lo, hi) == (2, 9) and step._host_tokens is False
+    monkeypatch.setattr(build, "ensure_built", fails("norms"))
+    with pytest.raises(build.ExtensionError):
+        build.build_all(quiet=True)
