@@ -531,6 +531,12 @@ KL_API int kl_attention_mixed_token_fits(int heads, int kv_heads, int dim, int v
     return mixed_token_plan(heads, kv_heads, dim, has_talk != 0, 1 << 20, MK_RANKS).slots > 0;
 }
 
+// The chunks of 32 keys whose scores one of `ranks` CTAs keeps at once; of more it computes the scores twice, in rounds (0: sizes that do not run).
+KL_API int kl_attention_mixed_token_room(int heads, int kv_heads, int dim, int has_talk, int ranks) {
+    if (heads <= 0 || kv_heads <= 0 || heads % kv_heads || dim <= 0 || ranks < 1 || ranks > MK_RANKS) return 0;
+    return mixed_token_plan(heads, kv_heads, dim, has_talk != 0, 1 << 20, ranks).room;
+}
+
 // `ranks` (1, 2, 4 or 8) CTAs a sequence; `chunks`: the visible chunks of 32 keys that a CTA is planned for (more of them are right too, in rounds).
 KL_API int kl_attention_mixed_token(const void* q, long long q_stride, const void* gate, long long gate_stride, void* out, long long out_stride,
                                     const void* k_cache, const void* v_cache, long long pages, const int* block_table, int blocks_per_seq,

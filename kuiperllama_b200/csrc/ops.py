@@ -1367,20 +1367,39 @@ def mixed_attention_splits(n_seqs: int, context_class: int, window: int, keep_fi
     return max(1, min(chunks, want, 32))
 
 
-def mixed_token_ranks(n_seqs: int, context_class: int, window: int, keep_first: int):
-    """(CTAs a sequence, chunks of 32 keys that each of them is planned for) of attention_mixed_token.cu: 8, 4 or 2 CTAs as long as every sequence's
-    cluster is resident at once with one CTA an SM (of 148 SMs 15 clusters of eight, 33 of four, 74 of two: a cluster stays within its part of the
-    chip), and more where a CTA would otherwise have more than 40 chunks, whose scores it computes twice.  us with 1 / 2 / 4 / 8 CTAs a sequence, 32
-    heads of 64 on 8: 15 sequences of 200 keys 22.5 / 16.8 / 12.7 / 11.2, 16 22.6 / 16.6 / 12.6 / 20.8, 33 22.8 / 16.6 / 12.9 / 31.3, 34 22.7 / 16.6 /
-    22.2 / 31.7, 74 22.7 / 17.0 / 34.5 / 53.4; 160 of 4,000 506 / 413 / 332 / 400."""
-    chunks = (16 << max(0, int(context_class))) * (PAGE // 32)
+def mixed_token_ranks(n_seqs: int, context_class: int, window: int, keep_first: int, room):
+    """(CTAs a sequence, chunks of 32 keys that each of them is planned for) of attention_mixed_token.cu: the number of CTAs whose rounds take
+    least.  A round of CTAs costs the start of one, about three chunks (and half of one for a cluster), and its chunks, 1.45 times as much where
+    a CTA has more of them than its shared memory holds the scores of (``room``, for 1, 2, 4 and 8 CTAs: it makes the scores twice then); of 148 SMs
+    15 clusters of eight run at once, 33 of four, 74 of two (a cluster stays within its part of the chip).  The longest sequence of a class is
+    somewhere between half of the class's chunks and all of them, in the lowest class between none and all: the mean over two points.
+    us with 1 / 2 / 4 / 8 CTAs a sequence: 32 heads of 64 on 8 (room 35), 15 of 200 keys 22.5 / 16.8 / 12.7 / 11.2, 16 22.6 / 16.6 / 12.6 / 20.8, 40 23.0 / 17.0 /
+    24.2 / 32.3, 76 23.1 / 32.5 / 36.5 / 63.2; 40 of 3,000 338 / 178 / 128 / 109, 76 342 / 349 / 192 / 214, 148 345 / 354 / 320 / 360; 64 of 64 (room 13), 76 of
+    3,000, window 1,024 213 / 231 / 145 / 188, 148 213 / 233 / 241 / 317; 32 of 128 (room 16), 76 of 1,000 161 / 122 / 105 / 133; 16 of 64 (room 92), 148
+    of 3,000 266 / 176 / 239 / 280."""
+    bound = (16 << max(0, int(context_class))) * (PAGE // 32)
+    points = [bound / 4, bound * 3 / 4] if context_class <= 0 else [bound * 5 / 8, bound * 7 / 8]
     if window:
-        chunks = min(chunks, (int(window) + 31) // 32 + 1 + (int(keep_first or 0) + 31) // 32)
-    sms, n = sm_count(), int(n_seqs)
-    ranks = 8 if 8 * n <= sms - 28 else 4 if 4 * n <= sms - 16 else 2 if 2 * n <= sms else 1
-    while ranks < 8 and chunks > 40 * ranks:
-        ranks *= 2
-    return ranks, -(-chunks // ranks)
+        most = (int(window) + 31) // 32 + 1 + (int(keep_first or 0) + 31) // 32
+        bound, points = min(bound, most), [min(c, most) for c in points]
+    sms, best = sm_count(), None
+    for ranks, resident, holds in zip((1, 2, 4, 8), (sms, sms, sms - 16, sms - 28), room):
+        rounds = -(-int(n_seqs) * ranks // max(1, resident // ranks * ranks))
+        cost = rounds * sum(3.2 + (0.5 if ranks > 1 else 0.0) + c / ranks * (1.45 if c / ranks > holds else 1.0) for c in points)
+        if best is None or cost < best[0]:
+            best = (cost, ranks)
+    return best[1], -(-bound // best[1])
+
+
+_mixed_rooms: Dict[tuple, tuple] = {}
+
+
+def _mixed_room(heads: int, kv_heads: int, dim: int, mix: bool) -> tuple:
+    """Chunks whose scores a CTA of attention_mixed_token.cu holds, for 1, 2, 4 and 8 CTAs a sequence."""
+    key = (heads, kv_heads, dim, mix)
+    if key not in _mixed_rooms:
+        _mixed_rooms[key] = tuple(lib("attention_mixed_token").kl_attention_mixed_token_room(heads, kv_heads, dim, int(mix), r) for r in (1, 2, 4, 8))
+    return _mixed_rooms[key]
 
 
 MIXED_SPLITS = None             # (phase 0, phase 1): fixed numbers of pieces, for comparisons
@@ -1447,7 +1466,8 @@ def attention_mixed(q: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Te
         M = lib("attention_mixed_token")
         if (M.kl_attention_mixed_token_fits(heads, kv_heads, dim, vdim, int(talk is not None)) and q.stride(0) % 2 == 0 and out.stride(0) % 2 == 0
                 and (q.data_ptr() | out.data_ptr()) % 4 == 0 and (k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0 and step.n_seqs <= 65535):
-            ranks, chunks = mixed_token_ranks(step.n_seqs, getattr(step, "context_class", 0), window, keep_first)
+            ranks, chunks = mixed_token_ranks(step.n_seqs, getattr(step, "context_class", 0), window, keep_first,
+                                              _mixed_room(heads, kv_heads, dim, talk is not None))
             _check(M.kl_attention_mixed_token(
                 _ptr(q), ctypes.c_longlong(q.stride(0)), _ptr(gate), ctypes.c_longlong(gate.stride(0) if gate is not None else 0), _ptr(out),
                 ctypes.c_longlong(out.stride(0)), _ptr(k_cache), _ptr(v_cache), ctypes.c_longlong(k_cache.shape[0]), _ptr(block_table),

@@ -67,3 +67,25 @@ def test_products_of_few_tokens_have_a_cta_for_every_sm(monkeypatch, N, K, M):
     pieces = ops.skinny_splits(N, K, M)
     assert 148 < pieces * -(-N // 128) <= 296 or pieces == 8 or pieces == -(-K // 64) // 4
     assert pieces <= 8
+
+
+# us with 1, 2, 4 and 8 CTAs a sequence, measured; rooms of 32 heads of 64 on 8, 32 of 128, 64 of 64, 16 of 64, 24 of 128
+ROOMS = {"32x64": (35, 35, 34, 34), "32x128": (16, 16, 15, 15), "64x64": (13, 13, 13, 12), "16x64": (92, 92, 92, 91), "24x128": (49, 49, 49, 49)}
+
+
+@pytest.mark.parametrize("heads,n,context_class,window,times", [
+    ("32x64", 15, 0, 0, [(22.5, 16.8, 12.7, 11.2)]), ("32x64", 16, 0, 0, [(22.6, 16.6, 12.6, 20.8)]), ("32x64", 33, 0, 0, [(22.8, 16.6, 12.9, 31.3)]),
+    ("32x64", 34, 0, 0, [(22.7, 16.6, 22.2, 31.7)]), ("32x64", 74, 0, 0, [(22.7, 17.0, 34.5, 53.4)]),
+    ("32x64", 40, 2, 0, [(338, 177.6, 127.9, 108.7)]), ("32x64", 76, 2, 0, [(342.3, 349.1, 192.2, 214.3)]), ("32x64", 148, 2, 0, [(345.1, 354.4, 320.2, 360)]),
+    ("32x64", 148, 2, 1024, [(91.9, 101.5, 147.8, 208.2)]), ("32x64", 76, 0, 0, [(23.1, 32.5, 36.5, 63.2), (51.6, 60.5, 59, 87.9), (82.7, 89, 81.1, 105.9)]),
+    ("32x128", 76, 0, 0, [(31.3, 43.4, 46.3, 74.3), (102, 84.2, 78.6, 113.7), (160.7, 122.1, 105.1, 132.8)]),
+    ("32x128", 148, 0, 0, [(36.9, 50.6, 82.2, 136.4), (109.8, 91.1, 129.5, 194.6), (172.4, 132.8, 175.7, 227.4)]),
+    ("32x128", 40, 2, 1024, [(175.1, 99.3, 78.8, 80.0)]), ("32x128", 76, 2, 0, [(456.4, 466.4, 374.2, 287.7)]),
+    ("64x64", 40, 2, 1024, [(209.6, 117.4, 95.8, 94.2)]), ("64x64", 76, 2, 1024, [(212.7, 230.7, 144.9, 188.3)]), ("64x64", 148, 2, 1024, [(212.5, 232.6, 240.9, 317)]),
+    ("16x64", 40, 2, 0, [(263.2, 88.2, 95.9, 84.5)]), ("16x64", 148, 2, 0, [(266.2, 175.5, 238.7, 279.8)]), ("24x128", 148, 2, 0, [(362.2, 264.6, 356.4, 404.9)])])
+def test_ctas_a_sequence_of_single_tokens(monkeypatch, heads, n, context_class, window, times):
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
+    ranks, chunks = ops.mixed_token_ranks(n, context_class, window, 64, ROOMS[heads])
+    total = [sum(t[i] for t in times) for i in range(4)]
+    assert total[(1, 2, 4, 8).index(ranks)] <= 1.05 * min(total), (ranks, total)
+    assert ranks * chunks >= (35 if window else 32 << context_class)
