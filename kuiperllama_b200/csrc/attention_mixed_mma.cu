@@ -17,11 +17,13 @@
 // What bounds it is the instructions of a score outside the products: 76 of phase 0's with a tanh for every size of x, an exact quotient and a mask
 // for every score, 56 now (0.72 of them a cycle and scheduler; phase 1 98, 0.50), and the tiles' uneven numbers of chunks, which several CTAs share
 // (`splits0` and `splits1`; phase 1's sums then meet in a third launch).  One prompt (32 heads of 64 on 8, window 1,024, 64 kept keys), us: 2,048 tokens 571
-// before, 414 now; 1,024 349 and 163; 64 tokens after 1,500 301 in one piece each and 67 in 16.  With 32-bit multiply-adds throughout
+// before, 408 now; 1,024 349 and 177; 64 tokens after 1,500 301 in one piece each and 54 in 16.  With 32-bit multiply-adds throughout
 // (attention_mixed_tiled.cu) 2,242 for 2,048.
 //
 // ExiledOfCode/KuiperLLama's attention is mha_kernel.cu:61,74-106 (one sequence, one query, no window, no bias).
 #include "common.cuh"
+#include "pieces.cuh"
+#include "soft_cap.cuh"
 
 namespace kl {
 
@@ -46,53 +48,6 @@ struct MixedMmaArgs {
     float scale, softcap, out_scale;
     float scale_cap, scale_cap_rest;              // scale / softcap as the sum of two numbers: a score times it is rounded once
 };
-
-// tanh(x) for |x| <= MX_SMALL: x + x^3 R(x^2) with R of degree four, the best one for the relative error of tanh (2.8e-9 of it; in 32 bits 0.76
-// units in the last place).  Scores under a soft cap lie there as a rule, and this takes seven instructions and no branch.
-constexpr float MX_SMALL = 0.6f;
-__device__ __forceinline__ float mx_tanh(float x) {
-    const float u = x * x;
-    float r = fmaf(-5.895158275961876e-3f, u, 2.0795971155166626e-2f);
-    r = fmaf(r, u, -5.3783830255270004e-2f);
-    r = fmaf(r, u, 0.13331924378871918f);
-    r = fmaf(r, u, -0.33333298563957214f);
-    return fmaf(x * u, r, x);
-}
-// v * scale / softcap, rounded once; of an infinite or huge one the leading product (tanh is 1 far before that)
-__device__ __forceinline__ float mx_capped(float v, float c, float rest) {
-    const float x = v * c;
-    return fabsf(x) < 64.f ? fmaf(v, c, v * rest) : x;
-}
-
-__device__ __forceinline__ uint32_t mx_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mx_ldm4(uint32_t a, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
-}
-__device__ __forceinline__ void mx_ldm4t(uint32_t a, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
-}
-__device__ __forceinline__ void mx_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// two numbers as three packed pairs of bfloat16 that add up to them
-__device__ __forceinline__ void mx_split(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    float2 f = __bfloat1622float2(h);
-    x -= f.x; y -= f.y;
-    const __nv_bfloat162 m = __floats2bfloat162_rn(x, y);
-    f = __bfloat1622float2(m);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(x - f.x, y - f.y);
-    a = *reinterpret_cast<const uint32_t*>(&h);
-    b = *reinterpret_cast<const uint32_t*>(&m);
-    c = *reinterpret_cast<const uint32_t*>(&l);
-}
-// the place of 16-byte piece c of row r in a tile of rows of D elements: neighbouring rows' pieces fall on different banks
-template <int D> __device__ __forceinline__ int mx_at(int r, int c) {
-    constexpr int P = D / 8;
-    if constexpr (P >= 8) return r * D + ((c ^ (r & 7)) << 3);
-    else return r * D + ((c ^ ((r / (8 / P)) & (P - 1))) << 3);
-}
 
 inline size_t mx_smem_bytes(int H, int D, int G, int phase) {
     return (size_t)(phase == 1 ? 3 : 2) * G * MX_CH * D * 2 + (size_t)(H / 2) * 2 * MX_BIAS * 4 +
@@ -148,7 +103,7 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
         for (int idx = threadIdx.x; idx < G * MX_CH * (D / 8); idx += THREADS) {
             const int row = idx / (D / 8), p = idx % (D / 8), kv = row / MX_CH, j = row % MX_CH;
             const bool in = j < valid;                                     // rows past the last key become zero
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(mx_smem(dst + (size_t)kv * MX_CH * D + mx_at<D>(j, p))),
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + (size_t)kv * MX_CH * D + pc_at<D>(j, p))),
                          "l"(in ? src + ((size_t)kv * PAGE + j) * D + p * 8 : src), "r"(in ? 16 : 0) : "memory");
         }
     };
@@ -163,7 +118,7 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
             const int h = idx / (H / 2), e = idx % (H / 2) * 2;
             const float2 t = *reinterpret_cast<const float2*>(A.talk + (size_t)h * H + e);
             uint32_t a, b, l;
-            mx_split(t.x, t.y, a, b, l);
+            pc_split(t.x, t.y, a, b, l);
             *reinterpret_cast<uint32_t*>(Ts + (size_t)h * (H + 8) + e) = a;
             *reinterpret_cast<uint32_t*>(Ts + (size_t)(H + h) * (H + 8) + e) = b;
             *reinterpret_cast<uint32_t*>(Ts + (size_t)(2 * H + h) * (H + 8) + e) = l;
@@ -218,9 +173,9 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
 #pragma unroll
             for (int n = 0; n < NT; n += 2) {
                 uint32_t b[4];
-                mx_ldm4(mx_smem(K + mx_at<D>(n * 8 + (lane & 7) + ((lane >> 4) << 3), ks * 2 + ((lane >> 3) & 1))), b);
-                mx_mma(S[n], qf[ks], b[0], b[1]);
-                mx_mma(S[n + 1], qf[ks], b[2], b[3]);
+                pc_ldm4(smem_u32(K + pc_at<D>(n * 8 + (lane & 7) + ((lane >> 4) << 3), ks * 2 + ((lane >> 3) & 1))), b);
+                pc_mma(S[n], qf[ks], b[0], b[1]);
+                pc_mma(S[n + 1], qf[ks], b[2], b[3]);
             }
         if (A.r1 != nullptr) {                                             // the bias depends on i - j alone: 39 values for the chunk
             __syncwarp();
@@ -249,16 +204,16 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) most = visible(n, e) ? fmaxf(most, fabsf(S[n][e])) : most;
             }
-            if (most * fabsf(A.scale_cap) > MX_SMALL) {
+            if (most * fabsf(A.scale_cap) > CAP_SMALL) {
 #pragma unroll
                 for (int n = 0; n < NT; ++n)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) S[n][e] = tanhf(mx_capped(S[n][e], A.scale_cap, A.scale_cap_rest));
+                    for (int e = 0; e < 4; ++e) S[n][e] = tanhf(cap_quotient(S[n][e], A.scale_cap, A.scale_cap_rest));
             } else {
 #pragma unroll
                 for (int n = 0; n < NT; ++n)
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) S[n][e] = mx_tanh(fmaf(S[n][e], A.scale_cap, S[n][e] * A.scale_cap_rest));
+                    for (int e = 0; e < 4; ++e) S[n][e] = cap_tanh(cap_small_quotient(S[n][e], A.scale_cap, A.scale_cap_rest));
             }
         }
         const float factor = A.softcap > 0.f ? A.softcap : A.scale;
@@ -318,7 +273,7 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
                             const float* p = P + (ks * 16 + kc + 8 * e) * MX_PH + r;
-                            mx_split(p[0], p[MX_PH], b[0][ks][e], b[1][ks][e], b[2][ks][e]);
+                            pc_split(p[0], p[MX_PH], b[0][ks][e], b[1][ks][e], b[2][ks][e]);
                         }
                     __syncwarp();                                          // all heads' p of these columns are read: w takes their place
 #pragma unroll
@@ -329,20 +284,20 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
                         for (int x = 0; x < 3; ++x)
 #pragma unroll
                             for (int ks = 0; ks < H / 16; ++ks)
-                                mx_ldm4(mx_smem(Ts + (size_t)(x * H + mt * 16 + (lane & 15)) * (H + 8) + ks * 16 + (lane >> 4) * 8), a[x][ks]);
+                                pc_ldm4(smem_u32(Ts + (size_t)(x * H + mt * 16 + (lane & 15)) * (H + 8) + ks * 16 + (lane >> 4) * 8), a[x][ks]);
 #pragma unroll
                         for (int ks = 0; ks < H / 16; ++ks) {
-                            mx_mma(w, a[2][ks], b[0][ks][0], b[0][ks][1]);
-                            mx_mma(w, a[1][ks], b[1][ks][0], b[1][ks][1]);
-                            mx_mma(w, a[0][ks], b[2][ks][0], b[2][ks][1]);
+                            pc_mma(w, a[2][ks], b[0][ks][0], b[0][ks][1]);
+                            pc_mma(w, a[1][ks], b[1][ks][0], b[1][ks][1]);
+                            pc_mma(w, a[0][ks], b[2][ks][0], b[2][ks][1]);
                         }
 #pragma unroll
                         for (int ks = 0; ks < H / 16; ++ks) {
-                            mx_mma(w, a[1][ks], b[0][ks][0], b[0][ks][1]);
-                            mx_mma(w, a[0][ks], b[1][ks][0], b[1][ks][1]);
+                            pc_mma(w, a[1][ks], b[0][ks][0], b[0][ks][1]);
+                            pc_mma(w, a[0][ks], b[1][ks][0], b[1][ks][1]);
                         }
 #pragma unroll
-                        for (int ks = 0; ks < H / 16; ++ks) mx_mma(w, a[0][ks], b[0][ks][0], b[0][ks][1]);
+                        for (int ks = 0; ks < H / 16; ++ks) pc_mma(w, a[0][ks], b[0][ks][0], b[0][ks][1]);
                         *reinterpret_cast<float2*>(P + (mt * 16 + r) * MX_PH + kc) = make_float2(w[0], w[1]);
                         *reinterpret_cast<float2*>(P + (mt * 16 + 8 + r) * MX_PH + kc) = make_float2(w[2], w[3]);
                     }
@@ -359,16 +314,16 @@ attention_mixed_mma_kernel(const MixedMmaArgs A) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float2 w = *reinterpret_cast<const float2*>(Ps + (h0 + (e & 1)) * MX_PH + r * MX_PQ + ks * 16 + (e >> 1) * 8 + kc);
-                    mx_split(w.x, w.y, a[0][e], a[1][e], a[2][e]);
+                    pc_split(w.x, w.y, a[0][e], a[1][e], a[2][e]);
                 }
 #pragma unroll
                 for (int n = 0; n < D / 8; n += 2) {
                     uint32_t b[4];
-                    mx_ldm4t(mx_smem(V + mx_at<D>(ks * 16 + (lane & 15), n + (lane >> 4))), b);
+                    pc_ldm4t(smem_u32(V + pc_at<D>(ks * 16 + (lane & 15), n + (lane >> 4))), b);
 #pragma unroll
                     for (int x = 2; x >= 0; --x) {
-                        mx_mma(O[n], a[x], b[0], b[1]);
-                        mx_mma(O[n + 1], a[x], b[2], b[3]);
+                        pc_mma(O[n], a[x], b[0], b[1]);
+                        pc_mma(O[n + 1], a[x], b[2], b[3]);
                     }
                 }
             }
@@ -468,8 +423,7 @@ KL_API int kl_attention_mixed_mma(const void* q, long long q_stride, const void*
     A.k_cache = (const bf16*)k_cache; A.v_cache = (const bf16*)v_cache; A.block_table = block_table; A.blocks_per_seq = blocks_per_seq;
     A.cu_tokens = cu_tokens; A.seq_slots = seq_slots; A.seq_starts = seq_starts; A.r1 = r1; A.r2 = r2; A.talk = talk; A.ml = ml;
     A.kv_heads = kv_heads; A.window = window; A.keep_first = keep_first; A.scale = scale; A.softcap = softcap; A.out_scale = out_scale;
-    A.scale_cap = softcap > 0.f ? (float)((double)scale / (double)softcap) : 0.f;
-    A.scale_cap_rest = softcap > 0.f ? (float)((double)scale / (double)softcap - (double)A.scale_cap) : 0.f;
+    cap_parts(scale, softcap, A.scale_cap, A.scale_cap_rest);
     A.rows = rows; A.n_seqs = n_seqs; A.splits0 = splits0; A.splits1 = splits1; A.part = part; A.counts = counts;
     const dim3 grid((max_new + MX_TQ - 1) / MX_TQ, n_seqs);
     int err = KL_OK;

@@ -25,6 +25,7 @@
 // ExiledOfCode/KuiperLLama's attention is mha_kernel.cu:61,74-106 (one sequence, one query, no window, no bias).
 #include "common.cuh"
 #include "pieces.cuh"
+#include "soft_cap.cuh"
 #include "tma_host.cuh"
 
 namespace kl {
@@ -74,20 +75,6 @@ template <int D> __device__ __forceinline__ int mk_at(int r, int c, int box) {
     else return (c >> 3) * box + r * 64 + (((c & 7) ^ (r & 7)) << 3);
 }
 
-// tanh(x) for |x| <= 0.6: see attention_mixed_mma.cu
-__device__ __forceinline__ float mk_tanh(float x) {
-    const float u = x * x;
-    float r = fmaf(-5.895158275961876e-3f, u, 2.0795971155166626e-2f);
-    r = fmaf(r, u, -5.3783830255270004e-2f);
-    r = fmaf(r, u, 0.13331924378871918f);
-    r = fmaf(r, u, -0.33333298563957214f);
-    return fmaf(x * u, r, x);
-}
-// v * scale / softcap, rounded once; of an infinite or huge one the leading product (tanh is 1 far before that)
-__device__ __forceinline__ float mx_capped(float v, float c, float rest) {
-    const float x = v * c;
-    return fabsf(x) < 64.f ? fmaf(v, c, v * rest) : x;
-}
 __device__ __forceinline__ void mk_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void mk_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void mk_push(uint32_t addr, float a, float b) {       // to a shared::cluster address
@@ -99,7 +86,6 @@ template <int D, int UPW>
 __global__ void __launch_bounds__(MK_THREADS + 32, 1)
 attention_mixed_token_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const MixedTokenArgs A) {
     constexpr int W = D + 8, SL = D / 32;                                  // elements of a query's row; column slices
-    constexpr float SMALL = 0.6f;
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(1024) unsigned char mk_raw[];
@@ -257,12 +243,12 @@ attention_mixed_token_kernel(const __grid_constant__ CUtensorMap map_k, const __
             if (A.softcap > 0.f) {
                 // (asked for every lane's own two scores: past the last key the page holds whatever was there before, and no visible score takes another
                 // form for it)
-                if (vis && fmaxf(fabsf(v), fabsf(v2)) * fabsf(A.scale_cap) > SMALL) {
-                    v = tanhf(mx_capped(v, A.scale_cap, A.scale_cap_rest));
-                    v2 = tanhf(mx_capped(v2, A.scale_cap, A.scale_cap_rest));
+                if (vis && fmaxf(fabsf(v), fabsf(v2)) * fabsf(A.scale_cap) > CAP_SMALL) {
+                    v = tanhf(cap_quotient(v, A.scale_cap, A.scale_cap_rest));
+                    v2 = tanhf(cap_quotient(v2, A.scale_cap, A.scale_cap_rest));
                 } else {
-                    v = mk_tanh(fmaf(v, A.scale_cap, v * A.scale_cap_rest));
-                    v2 = mk_tanh(fmaf(v2, A.scale_cap, v2 * A.scale_cap_rest));
+                    v = cap_tanh(cap_small_quotient(v, A.scale_cap, A.scale_cap_rest));
+                    v2 = cap_tanh(cap_small_quotient(v2, A.scale_cap, A.scale_cap_rest));
                 }
             }
             const float factor = A.softcap > 0.f ? A.softcap : A.scale;
@@ -558,8 +544,8 @@ KL_API int kl_attention_mixed_token(const void* q, long long q_stride, const voi
     A.block_table = block_table; A.blocks_per_seq = blocks_per_seq;
     A.cu_tokens = cu_tokens; A.seq_slots = seq_slots; A.seq_starts = seq_starts; A.r1 = r1; A.r2 = r2; A.talk = talk; A.status = status;
     A.heads = heads; A.kv_heads = kv_heads; A.window = window; A.keep_first = keep_first; A.slots = P.slots; A.room = P.room;
-    A.scale = scale; A.softcap = softcap; A.out_scale = out_scale; A.scale_cap = softcap > 0.f ? (float)((double)scale / (double)softcap) : 0.f;
-    A.scale_cap_rest = softcap > 0.f ? (float)((double)scale / (double)softcap - (double)A.scale_cap) : 0.f;
+    A.scale = scale; A.softcap = softcap; A.out_scale = out_scale;
+    cap_parts(scale, softcap, A.scale_cap, A.scale_cap_rest);
 #define KL_MK(DD, U)                                                                                                                          \
     do {                                                                                                                                      \
         KL_CUDA(cudaFuncSetAttribute(attention_mixed_token_kernel<DD, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem));         \

@@ -62,7 +62,7 @@ SOURCES: Dict[str, str] = {
 }
 # modules that what uses them does without (the interpreter's headers may be missing): the engine then goes through numpy
 OPTIONAL = ("host_tokens",)
-HEADERS: List[str] = ["common.cuh", "attention_mma.cuh", "tcgen05.cuh", "pieces.cuh", "tma_host.cuh", "attention_decode_noalloc.h"]
+HEADERS: List[str] = ["common.cuh", "attention_mma.cuh", "tcgen05.cuh", "pieces.cuh", "soft_cap.cuh", "tma_host.cuh", "attention_decode_noalloc.h"]
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared", "--expt-relaxed-constexpr", "--extended-lambda"]
