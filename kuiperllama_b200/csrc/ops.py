@@ -422,11 +422,19 @@ def mingru_scan(proj: torch.Tensor, z_col: int, x_col: int, g_col: int, bias_z: 
 # A bfloat16 step takes the chunked form from this many tokens of its longest sequence on, with at least so many rows for every sequence.  us
 # walked / in chunks, 16 heads of 128 x 128 on 4: one sequence of 64 tokens 25.1 / 28.5, 96 31.0 / 29.9, 128 37.5 / 32.0, 512 120 / 56, 2,048 444 / 169,
 # eight of 64 80 / 67, one of 64 beside 31 single tokens 42 / 150; 32 heads of 64 x 64 on 8, 64 21.6 / 25.6, 128 32.9 / 30.2, 32 of 64 134 / 162;
-# 4 heads of 128 x 128, eight of 64 29.6 / 34.1.
-DELTA_CHUNKED_FROM, DELTA_CHUNKED_ROWS = 96, 64
+# 4 heads of 128 x 128, eight of 64 29.6 / 34.1.  A captured step knows its rows, a multiple of 64 of which a replay may leave 63 empty, and not its longest
+# sequence: 128 rows with 68 tokens 25.8 / 31.1, with 128 36.8 / 33.1, with two of 64 29.6 / 36.2; 192 rows with 132 38 / 36, 192 49 / 38, two of 96 38 / 40.
+DELTA_CHUNKED_FROM, DELTA_CHUNKED_ROWS, DELTA_CHUNKED_CAPTURED = 96, 64, 192
 # Bytes that the operands of a step's chunks take at most, here and in ``outer_recurrence`` (30 KB a token with 16 heads of 128 x 128, 7 KB with 64 of 128 x
 # 64): longer steps are worked in portions, 8,900 tokens of the former in one, so what a step holds beside its rows does not grow with a prompt.
 CHUNK_SCRATCH = 256 << 20
+
+
+def delta_in_chunks(step) -> bool:
+    """Whether the sizes of a bfloat16 step ask for the chunked form of the delta rule."""
+    if step.n_tokens < DELTA_CHUNKED_ROWS * step.n_seqs:
+        return False
+    return step.max_new >= (DELTA_CHUNKED_CAPTURED if getattr(step, "captured", False) else DELTA_CHUNKED_FROM)
 
 
 def gated_delta_rule(proj: torch.Tensor, conv_col: int, b_col: int, a_col: int, conv_weight: torch.Tensor, A_log: torch.Tensor,
@@ -449,7 +457,7 @@ def gated_delta_rule(proj: torch.Tensor, conv_col: int, b_col: int, a_col: int, 
           and state.shape[1] >= conv_off + (taps - 1) * C and conv_off >= heads * vdim * dim, "gated_delta_rule: state")
     _need(out.dtype == torch.float32 and out.is_contiguous() and out.shape[0] >= n and out.shape[1] == heads * vdim, "gated_delta_rule: out")
     _need(dim <= 256, f"gated_delta_rule: key size {dim} is above 256")
-    if chunked or (chunked is None and step.max_new >= DELTA_CHUNKED_FROM and n >= DELTA_CHUNKED_ROWS * step.n_seqs):
+    if chunked or (chunked is None and delta_in_chunks(step)):
         L = lib("delta_chunked")
         # what the chunked form takes: see kl_delta_chunked_fits and kl_delta_chunked
         if (proj.dtype == torch.bfloat16 and proj.data_ptr() % 8 == 0 and proj.stride(0) % 4 == 0 and conv_col % 4 == 0 and conv_weight.data_ptr() % 16 == 0
@@ -1215,8 +1223,19 @@ def decay_lowrank(r1: torch.Tensor, W2: torch.Tensor, b: Optional[torch.Tensor],
 # A step takes the chunked form from this many tokens of its longest sequence on, with at least so many rows for every sequence: a chunk costs
 # the same for one token as for 32.  us walked / in chunks: 64 heads of 128 x 64, one sequence of 33 tokens 13.7 / 11.6, 64 18.8 / 11.7, 2,048
 # 416 / 151, eight of 40 43 / 57, eight of 64 62 / 57, one of 64 beside 31 single tokens 59 / 160; 16 heads of 64 x 128 with a decay per row, one
-# of 33 9.4 / 11.9, 64 13.8 / 12.0, 2,048 374 / 114, eight of 40 18 / 23, eight of 64 26 / 23; 32 heads of 128 x 64, 48 tokens 10.4 / 11.6.
-OUTER_CHUNKED_FROM, OUTER_CHUNKED_ROWS = 64, 48
+# of 33 9.4 / 11.9, 64 13.8 / 12.0, 2,048 374 / 114, eight of 40 18 / 23, eight of 64 26 / 23; 32 heads of 128 x 64, 48 tokens 10.4 / 11.6.  A captured step
+# knows its rows, a multiple of 64 of which a replay may leave 63 empty, and not its longest sequence: 64 rows with 4 / 20 / 48 / 64 tokens of 16 heads of
+# 64 x 128 3.6, 6.5, 10.8, 13.7 / 9.6, 10.8, 12.1, 12.2, of 32 heads of 128 x 64 5.0, 7.0, 10.2, 12.4 / 8.9, 9.1, 11.5, 11.7, of 64 heads 7.5, 10.4, 15.3,
+# 19.5 / 9.0, 9.2, 11.6, 11.7; 128 rows with 68 tokens 15.2 / 13.3, 13.4 / 13.8 and 20.0 / 14.0.
+OUTER_CHUNKED_FROM, OUTER_CHUNKED_ROWS, OUTER_CHUNKED_CAPTURED, OUTER_CHUNKED_HEADS = 64, 48, 128, 64
+
+
+def outer_in_chunks(step, heads: int, per_row: bool) -> bool:
+    """Whether the sizes of a step ask for the chunked form of ``outer_recurrence``."""
+    if step.n_tokens < OUTER_CHUNKED_ROWS * step.n_seqs:
+        return False
+    few = getattr(step, "captured", False) and (per_row or heads < OUTER_CHUNKED_HEADS)
+    return step.max_new >= (OUTER_CHUNKED_CAPTURED if few else OUTER_CHUNKED_FROM)
 
 
 def outer_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tensor, state: torch.Tensor, y: torch.Tensor, step,
@@ -1253,7 +1272,7 @@ def outer_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch
     _need(state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1 and state.shape[1] >= heads * N * P, "outer_recurrence: state")
     _need(y.dtype == torch.float32 and y.dim() == 2 and y.stride(1) == 1 and y.shape[0] >= n and y.shape[1] == heads * P, "outer_recurrence: y")
     _need(heads % groups == 0 and N <= 1024, "outer_recurrence: heads in equal groups, at most 1,024 rows of state")
-    if chunked or (chunked is None and step.max_new >= OUTER_CHUNKED_FROM and n >= OUTER_CHUNKED_ROWS * step.n_seqs):
+    if chunked or (chunked is None and outer_in_chunks(step, heads, per_row)):
         # what the chunked form takes: see kl_outer_chunked_fits; rows of q and k (and of a, with a decay per row) on 16-byte boundaries
         aligned = lambda t: t.data_ptr() % 16 == 0 and t.stride(0) * t.element_size() % 16 == 0
         L = lib("outer_chunked")

@@ -89,3 +89,14 @@ def test_ctas_a_sequence_of_single_tokens(monkeypatch, heads, n, context_class, 
     total = [sum(t[i] for t in times) for i in range(4)]
     assert total[(1, 2, 4, 8).index(ranks)] <= 1.05 * min(total), (ranks, total)
     assert ranks * chunks >= (35 if window else 32 << context_class)
+
+
+def test_recurrences_of_captured_steps_whose_rows_may_be_empty():
+    """A prompt of a few tokens is 64 rows in a captured step: it is walked, as it is alone."""
+    assert ops.delta_in_chunks(_step(96)) and not ops.delta_in_chunks(_step(95))
+    assert not ops.delta_in_chunks(_step(128, captured=True)) and ops.delta_in_chunks(_step(192, captured=True))
+    assert not ops.delta_in_chunks(_step(500, 8)) and ops.delta_in_chunks(_step(512, 8))
+    for heads, per_row in ((16, True), (64, True), (32, False)):
+        assert ops.outer_in_chunks(_step(64), heads, per_row) and not ops.outer_in_chunks(_step(63), heads, per_row)
+        assert not ops.outer_in_chunks(_step(64, captured=True), heads, per_row) and ops.outer_in_chunks(_step(128, captured=True), heads, per_row)
+    assert ops.outer_in_chunks(_step(64, captured=True), 64, False) and not ops.outer_in_chunks(_step(300, 8), 64, False)
