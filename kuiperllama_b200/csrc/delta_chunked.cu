@@ -451,7 +451,8 @@ __device__ __noinline__ void dc_tokens(const DeltaChunkArgs& A, float* S, float*
     __syncthreads();
 }
 
-template <int NP>
+// PART: of a portion of the step's chunks (A.span)
+template <int NP, bool PART>
 __global__ void __launch_bounds__(NP / 16 * 32, 1)
 dc_walk_kernel(const DeltaChunkArgs A) {
     pdl_wait();
@@ -460,13 +461,13 @@ dc_walk_kernel(const DeltaChunkArgs A) {
     extern __shared__ __align__(256) unsigned char dc_raw[];
     uint64_t* bars = reinterpret_cast<uint64_t*>(dc_raw + L::BARS);
     const int s = blockIdx.z, h = blockIdx.y, d = A.d, dv = A.dv, g = h / (A.H / A.G), C = 2 * A.G * d + A.H * dv;
-    const int first = dc_first(A, s), rest = A.cu_tokens[s + 1] - first, n_new = A.span > 0 ? min(rest, A.span * DC) : rest;
+    const int first = PART ? dc_first(A, s) : A.cu_tokens[s], rest = A.cu_tokens[s + 1] - first, n_new = PART ? min(rest, A.span * DC) : rest;
     if (n_new <= 0) return;
     const int chunks = (n_new + DC - 1) / DC;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2, kc = 2 * (lane & 3);
-    const size_t entry0 = dc_entry0(A, s);
+    const size_t entry0 = PART ? (size_t)s * A.span : dc_entry(first, s);
     float* slot = A.state + (size_t)A.seq_slots[s] * A.ld_state;
-    if (A.chunk0 == 0) {                                   // the convolution's state moves on, a share of the channels a CTA (nothing reads it any more)
+    if (!PART || A.chunk0 == 0) {                          // the convolution's state moves on, a share of the channels a CTA (nothing reads it any more)
         float* cs = slot + A.conv_off;
         const int n_ctas = gridDim.x * gridDim.y, mine = blockIdx.y * gridDim.x + blockIdx.x;
         for (int c = mine * THREADS + threadIdx.x; c < C; c += n_ctas * THREADS)
@@ -674,8 +675,9 @@ static int launch_delta_chunked(const DeltaChunkArgs& A, int chunks, int n_seqs,
     KL_CUDA(cudaFuncSetAttribute(dc_head_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, DcHead<NP>::BYTES));
     launch_kernel(dc_head_kernel<NP>, dim3(chunks, A.H, n_seqs), DC_THREADS, DcHead<NP>::BYTES, stream, A);
     KL_LAUNCH_CHECK();
-    KL_CUDA(cudaFuncSetAttribute(dc_walk_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, DcWalk<NP>::BYTES));
-    launch_kernel_after(dc_walk_kernel<NP>, dim3(A.dv / DC_COLS, A.H, n_seqs), NP / 16 * 32, DcWalk<NP>::BYTES, stream, A);
+    const auto walk = A.span > 0 ? dc_walk_kernel<NP, true> : dc_walk_kernel<NP, false>;
+    KL_CUDA(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, DcWalk<NP>::BYTES));
+    launch_kernel_after(walk, dim3(A.dv / DC_COLS, A.H, n_seqs), NP / 16 * 32, DcWalk<NP>::BYTES, stream, A);
     KL_LAUNCH_CHECK();
     return KL_OK;
 }

@@ -417,7 +417,8 @@ __device__ __noinline__ void oc_tokens(const OuterChunkArgs& A, float* S, float*
 // of 8 tokens from the four quarters' shares.  Between two barriers lie the products of a chunk, the preparation of the next one and the end of the
 // one before, none of which waits for another; everything in shared memory is there twice, and one thread copies the operands of the next
 // chunk as they lie (bulk copies).
-template <int NP, int MODE>
+// PART: of a portion of the step's chunks (A.span); without it the walk is 1.5 % faster than with a test.
+template <int NP, int MODE, bool PART>
 __global__ void __launch_bounds__(OC_WARPS * 32, NP == 64 && MODE == 1 ? 2 : 1)
 oc_walk_kernel(const OuterChunkArgs A) {
     pdl_wait();
@@ -437,14 +438,14 @@ oc_walk_kernel(const OuterChunkArgs A) {
         }
         s = __ffs(__ballot_sync(0xffffffffu, lane < gridDim.z && longer == (int)blockIdx.z)) - 1;
     }
-    const int first = oc_first(A, s), rest = A.cu_tokens[s + 1] - first, n_new = A.span > 0 ? min(rest, A.span * OC) : rest, h = blockIdx.y;
+    const int first = PART ? oc_first(A, s) : A.cu_tokens[s], rest = A.cu_tokens[s + 1] - first, n_new = PART ? min(rest, A.span * OC) : rest, h = blockIdx.y;
     if (n_new <= 0) return;
     const int chunks = (n_new + OC - 1) / OC;
     const int r = lane >> 2, kc = 2 * (lane & 3);
     const int N = A.N, P = A.P, g = h / (A.heads / A.groups), units = MODE == 1 ? A.heads : A.groups, unit = MODE == 1 ? h : g;
     const int p0 = blockIdx.x * OC_COLS + pw * 16;
     const bool on = p0 < P;                                // P is a multiple of 16
-    const size_t entry0 = oc_entry0(A, s);
+    const size_t entry0 = PART ? (size_t)s * A.span : oc_entry(first, s);
     float* S_slot = A.state + (size_t)A.seq_slots[s] * A.ld_state + (size_t)h * N * P;
     const float skip = A.skip != nullptr ? A.skip[h] : 0.f;
     if (threadIdx.x == 0) {
@@ -752,8 +753,9 @@ static int launch_outer_chunked(const OuterChunkArgs& A, int chunks, int n_seqs,
     }
     KL_LAUNCH_CHECK();
     constexpr int smem = OcWalk<NP, MODE>::BYTES;
-    KL_CUDA(cudaFuncSetAttribute(oc_walk_kernel<NP, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    launch_kernel_after(oc_walk_kernel<NP, MODE>, dim3((A.P + OC_COLS - 1) / OC_COLS, A.heads, n_seqs), OC_WARPS * 32, smem, stream, A);
+    const auto walk = A.span > 0 ? oc_walk_kernel<NP, MODE, true> : oc_walk_kernel<NP, MODE, false>;
+    KL_CUDA(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    launch_kernel_after(walk, dim3((A.P + OC_COLS - 1) / OC_COLS, A.heads, n_seqs), OC_WARPS * 32, smem, stream, A);
     KL_LAUNCH_CHECK();
     return KL_OK;
 }
