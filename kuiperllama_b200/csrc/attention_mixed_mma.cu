@@ -15,7 +15,7 @@
 // talk, p and w are 32-bit numbers.  They enter the products as the sum of three bfloat16 numbers (24 bits of mantissa); of two such
 // operands the six products down to 2^-16 of the leading one are added, smallest first, so nothing is rounded to 16 bits.
 // What bounds it is the instructions of a score outside the products: 76 of phase 0's with a tanh for every size of x, an exact quotient and a mask
-// for every score, 56 now (0.72 of them a cycle and scheduler; phase 1 98, 0.50), and the tiles' uneven numbers of chunks, which several CTAs share
+// for every score, 56 without (0.72 of them a cycle and scheduler; phase 1 98, 0.50; one more in each since a score over its cap is rounded once), and the tiles' uneven numbers of chunks, which several CTAs share
 // (`splits0` and `splits1`; phase 1's sums then meet in a third launch).  One prompt (32 heads of 64 on 8, window 1,024, 64 kept keys), us: 2,048 tokens 571
 // before, 408 now; 1,024 349 and 177; 64 tokens after 1,500 301 in one piece each and 54 in 16.  With 32-bit multiply-adds throughout
 // (attention_mixed_tiled.cu) 2,242 for 2,048.

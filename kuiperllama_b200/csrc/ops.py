@@ -1428,8 +1428,8 @@ def mixed_prompt_splits(step):
     """(phase 0, phase 1): into how many pieces at most a prompt's tiles of 8 tokens cut the 32-key chunks that they see, so that few tiles, or tiles of
     few and of many chunks, still fill the device: about 300 CTAs, twice that many for the light phase 0.  A tile of fewer chunks has as many pieces as
     chunks, which the kernels count themselves: a captured step's plan holds wherever its replays stand.
-    us with one piece each / with these, 32 heads of 64 on 8, window 1,024 and 64 kept keys: 64 tokens 26 / 20, 150 53 / 26, 300 98 / 43, 600 162 / 82,
-    1,024 266 / 163, 2,048 469 / 414, 64 after 1,500 301 / 67, four prompts of 500 216 / 185; 16 heads on 4, 300 tokens 58 / 29, 2,048 247 / 222."""
+    us with one piece each / with these, 32 heads of 64 on 8, window 1,024 and 64 kept keys: 64 tokens 26 / 21, 150 53 / 25, 300 98 / 40, 1,024 266 / 177,
+    2,048 469 / 406, 64 after 1,500 301 / 54, four prompts of 500 216 / 189; 16 heads on 4, 300 tokens 58 / 27, 2,048 247 / 219."""
     if MIXED_SPLITS is not None:
         return MIXED_SPLITS
     s1 = max(1, min(16, -(-300 // (step.n_tokens // 8 + step.n_seqs))))
