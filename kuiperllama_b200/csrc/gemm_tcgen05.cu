@@ -97,11 +97,14 @@ __device__ __forceinline__ float plain_act(const GemmArgs& args, float y) {
     y = fmaxf(y, 0.f);
     return y * y;
 }
+__device__ __forceinline__ float custom_mul(float g, float u, float alpha, float shift, float cubic) {
+    return __fdividef(g, 1.0f + __expf(-alpha * g * fmaf(cubic * g, g, 1.0f))) * (u + shift);
+}
 __device__ __forceinline__ float gated_mul(const GemmArgs& args, float g, float u) {
     if (!args.act_custom) return silu_mul(g, u);
     if (args.act_custom == 2) return fmaxf(g, 0.f) * u;
     if (args.act_limit > 0.f) { g = fminf(g, args.act_limit); u = fminf(fmaxf(u, -args.act_limit), args.act_limit); }
-    return __fdividef(g, 1.0f + __expf(-args.act_alpha * g * fmaf(args.act_cubic * g, g, 1.0f))) * (u + args.act_shift);
+    return custom_mul(g, u, args.act_alpha, args.act_shift, args.act_cubic);
 }
 
 // The squared relu on 32 accumulator columns in place.
@@ -392,14 +395,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 asm volatile("bar.sync 1, 128;" ::: "memory");             // the four epilogue warps, whatever happened
                 if (ok && quarter < 2) {
                     const int feature = tile_a * 64 + f;
+                    // (which activation is asked for a chunk too: asked for every number, 16 of the tanh form of gelu took 2,048 x 1,024 from 5.1 us with silu to 6.3)
+                    auto gate = [&](int c, float (&v)[16], auto&& act) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] = act(v[j], xch[(c + j) * 64 + f]);
+                    };
+                    const float limit = args.act_limit, alpha = args.act_alpha, shift = args.act_shift, cubic = args.act_cubic;
                     walk([&](int c, float (&v)[16]) {
-                        if (!args.act_custom) {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) v[j] = silu_mul(v[j], xch[(c + j) * 64 + f]);
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) v[j] = gated_mul(args, v[j], xch[(c + j) * 64 + f]);
-                        }
+                        if (!args.act_custom) gate(c, v, [](float g, float u) { return silu_mul(g, u); });
+                        else if (args.act_custom == 2) gate(c, v, [](float g, float u) { return fmaxf(g, 0.f) * u; });
+                        else if (limit > 0.f) gate(c, v, [&](float g, float u) { return custom_mul(fminf(g, limit), fminf(fmaxf(u, -limit), limit), alpha, shift, cubic); });
+                        else gate(c, v, [&](float g, float u) { return custom_mul(g, u, alpha, shift, cubic); });
                         if (feature < args.rows_a / 2) put_bf16(c, feature, v);
                     });
                 }
