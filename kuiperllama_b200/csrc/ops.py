@@ -1806,8 +1806,13 @@ def weights_as_rows(M: int, N: int, swiglu: bool = False) -> bool:
 
 
 def tokens_first(M: int, N: int, K: int) -> bool:
-    """Whether a product whose K cuts would be added by a kernel of their own runs with tokens as tile rows all the same."""
-    return M > 32 and one_wave(M, N) and ((K <= 2048 and (M > 64 or N >= 6144)) or (M > 128 and K <= 4096) or skinny_splits(N, K, M) == 1)
+    """Whether a product whose K cuts would be added by a kernel of their own runs with tokens as tile rows all the same.  Up to 64 tokens that is so for a short
+    K (fewer than four cuts) and for many features: a tile of tokens takes what K takes, the cuts' sum what tokens and features take.  us with tokens as
+    rows / with cuts, weights from memory: 33 tokens 640 x 640 4.1 / 4.8, 2,048 x 768 4.6 / 5.2, 2,048 x 1,024 5.3 / 4.8, 2,560 x 1,024 5.3 / 5.5, 3,072 x 1,536 6.9 /
+    6.9, 4,096 x 2,048 8.8 / 7.9, 6,144 x 2,048 9.5 / 10.3; 64 tokens 1,536 x 1,024 5.5 / 5.0, 2,048 x 1,024 5.3 / 5.9, 2,048 x 1,536 6.8 / 6.6, 3,072 x 2,048 8.8 /
+    8.5, 4,096 x 2,048 8.7 / 9.3."""
+    short = K <= 2048 and (M > 64 or K < 1024 or N * (M + 64) > 200 * K)
+    return M > 32 and one_wave(M, N) and (short or (M > 128 and K <= 4096) or skinny_splits(N, K, M) == 1)
 
 
 def gemm_skinny_partials(a: torch.Tensor, w: torch.Tensor, splits: Optional[int] = None) -> Optional[torch.Tensor]:

@@ -100,3 +100,10 @@ def test_recurrences_of_captured_steps_whose_rows_may_be_empty():
         assert ops.outer_in_chunks(_step(64), heads, per_row) and not ops.outer_in_chunks(_step(63), heads, per_row)
         assert not ops.outer_in_chunks(_step(64, captured=True), heads, per_row) and ops.outer_in_chunks(_step(128, captured=True), heads, per_row)
     assert ops.outer_in_chunks(_step(64, captured=True), 64, False) and not ops.outer_in_chunks(_step(300, 8), 64, False)
+
+
+@pytest.mark.parametrize("M,N,K,first", [(33, 640, 640, True), (48, 2048, 768, True), (33, 1536, 1024, False), (64, 2560, 1024, True), (64, 1024, 1024, False),
+                                         (33, 3072, 2048, False), (64, 3072, 2048, False), (64, 6144, 2048, True), (32, 640, 640, False), (48, 2048, 4096, False)])
+def test_products_of_33_to_64_tokens_take_the_faster_way_round(monkeypatch, M, N, K, first):
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
+    assert ops.tokens_first(M, N, K) == first
