@@ -2047,16 +2047,15 @@ def attention_tcgen05(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache
         "attention_tcgen05")
 
 
-# Keys that a token sees from which a step with a window or a sink takes tcgen05 with heads of 64, in groups of two and more heads / alone; heads
-# of 128 take it from the first on.  us on mma.sync / tcgen05, 32 heads: of 64 on 8, window 1,024, prompts of 6,000 tokens 200 / 113, 32 tokens
-# after 500 16.7 / 14.9, one prompt of 128 6.0 / 8.0, of 32 4.4 / 5.1; window 128, 2,048 tokens 26 / 22, prompts of 6,000 63 / 57; window 16, 41 /
-# 46; of 128 on 8, window 1,024, prompts of 6,000 341 / 136, 128 tokens 9.4 / 9.8, 32 tokens 6.5 / 5.8; 16 heads of 64 on 16, window 1,024,
-# 2,048 tokens 49 / 36, 32 tokens after 500 16.5 / 18.7, 64 after 1,000 35.0 / 34.2, window 128, prompts of 6,000 36 / 47.
+# Where a step with a window or a sink takes tcgen05.  Heads of 128: with windows of 128 and more (the mean over 138 steps of one to sixteen prompts is 0.79 to
+# 0.90 of mma.sync's time, 0.96 to 0.98 with windows of 16 to 64, where it is 1.4 at worst).  Heads of 64: from so many keys that a token sees on, in
+# groups of two and more heads / alone, and so many (row, head) pairs (twice as many where the group is no power of two and tiles hold empty rows): tcgen05 has
+# the larger tiles, which few rows do not fill.  us on mma.sync / tcgen05, window 1,024, 32 heads on 8: prompts of 6,000 tokens 200 / 113, 64 rows after 1,500
+# 31.5 / 29.1, 256 39 / 29.5, 512 at the start 19 / 15, after 1,500 43 / 30, 128 at the start 5.6 / 7.7; window 512, two prompts of 655 tokens 24.5 / 20.1, four of 162
+# 32.5 / 34.1; 12 heads on 4, two of 211 34.5 / 42.3; 8 on 1, 13 of 159 20 / 24; 16 on 16, 2,048 tokens 49 / 36, 256 after 1,500 32 / 37, 512 39.7 / 37.4.
 TCGEN05_WINDOW_KEYS = (512, 1024)
-# A captured step is replayed wherever its sequences stand by then, so it goes by its window and its rows alone.  us on mma.sync / tcgen05, window 1,024, 32
-# heads on 8: 64 rows at the start 4.1 / 5.5, after 1,500 31.5 / 29.1, 128 at the start 5.6 / 7.7, 256 after 1,500 39 / 29.5, 512 at the start 19 / 15, after
-# 1,500 43 / 30, eight of 64 after 700 30 / 21; 16 heads on 16: 256 after 1,500 32 / 37, 512 at the start 17.6 / 15.8, after 1,500 39.7 / 37.4.
-TCGEN05_CAPTURED_ROWS = (256, 512)
+TCGEN05_WINDOW_ROWS = 8192
+TCGEN05_WINDOW_128 = 128
 
 
 def prefill_on_tcgen05(q: torch.Tensor, q_stride: int, step, num_heads: int, num_kv_heads: int, head_dim: int, scale: float, window: int = 0,
@@ -2069,10 +2068,12 @@ def prefill_on_tcgen05(q: torch.Tensor, q_stride: int, step, num_heads: int, num
         return False
     if (not window and sink is None) or head_dim == 128:
         return True
-    alone, keys = int(group == 1), int(window or 1 << 30)
-    if getattr(step, "captured", False):
-        return step.max_new >= TCGEN05_CAPTURED_ROWS[alone] and keys >= TCGEN05_WINDOW_KEYS[alone]
-    return min(keys, getattr(step, "max_context", keys)) >= TCGEN05_WINDOW_KEYS[alone]
+    keys = int(window or 1 << 30)
+    if head_dim == 128:
+        return keys >= TCGEN05_WINDOW_128
+    if not getattr(step, "captured", False):              # (a captured step is replayed wherever its sequences stand by then)
+        keys = min(keys, getattr(step, "max_context", keys))
+    return keys >= TCGEN05_WINDOW_KEYS[int(group == 1)] and step.n_tokens * num_heads >= TCGEN05_WINDOW_ROWS * (1 if group & (group - 1) == 0 else 2)
 
 
 # Which kernel prefill steps of the bfloat16 path use for head sizes 64 and 128: "tcgen05", or "mma"

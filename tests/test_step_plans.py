@@ -19,8 +19,10 @@ def _step(rows, seqs=1, **more):
 @pytest.mark.parametrize("heads,kv_heads,hd", [(32, 8, 64), (16, 16, 64), (8, 2, 128)])
 def test_prompts_without_a_context_choose_a_kernel(heads, kv_heads, hd):
     ask = lambda **k: ops.prefill_on_tcgen05(Q, 2048, _step(300), heads, kv_heads, hd, 0.125, **k)
-    assert ask() and ask(window=4096) and ask(sink=torch.zeros(heads))
-    assert ask(window=16) == (hd == 128)
+    assert ask()
+    many = lambda **k: ops.prefill_on_tcgen05(Q, 2048, _step(2048), heads, kv_heads, hd, 0.125, **k)
+    assert many(window=4096) and many(sink=torch.zeros(heads)) and not many(window=16)
+    assert ask(window=4096) == (hd == 128 or 300 * heads >= ops.TCGEN05_WINDOW_ROWS)
 
 
 @pytest.mark.parametrize("heads,kv_heads", [(32, 8), (16, 16)])
