@@ -2066,7 +2066,7 @@ def prefill_on_tcgen05(q: torch.Tensor, q_stride: int, step, num_heads: int, num
     if not (q.dtype == torch.bfloat16 and not step.is_decode and PREFILL_KERNEL == "tcgen05" and head_dim in (64, 128) and group <= 128
             and q_stride % 8 == 0 and q.data_ptr() % 16 == 0 and (out is None or out.data_ptr() % 16 == 0) and step.max_new >= 8 and scale > 0):
         return False
-    if (not window and sink is None) or head_dim == 128:
+    if not window and sink is None:
         return True
     keys = int(window or 1 << 30)
     if head_dim == 128:
@@ -2176,6 +2176,39 @@ def attention_decode_fused(qkv: torch.Tensor, inv_freq: torch.Tensor, out: torch
 DECODE_KERNEL = "mma"
 
 
+def simt_runs(step, num_heads: int, num_kv_heads: int, head_dim: int) -> int:
+    """``runs`` of ``attention_simt`` for a step: about how many of its rows follow one another, or 0 where rows go each by itself.
+
+    A CTA of the prompt kernel has 4 to 16 rows and walks the sequences that they belong to one after the other, so a few tokens each of sequences with long
+    contexts wait for one another: 8 runs of 3 tokens after 500, 32 heads of 64, take 136 us so and 42 by rows.  With several sequences both
+    are estimated (us, fitted to 187 steps of one to sixteen sequences): by rows the longest context and all (row, key, head) products, together the
+    longest walk of a CTA and a fifth of the products; together it is where that is the better one by a third, as the walk is within 24 %."""
+    n, seqs = step.n_tokens, max(1, step.n_seqs)
+    runs = n // seqs
+    captured = getattr(step, "captured", False)           # (what its sequences bring in a replay is not known, nor what they hold by then)
+    news, starts = (None, None) if captured else (getattr(step, "host_new", None), getattr(step, "host_starts", None))
+    if seqs == 1 or not news or not starts:
+        short = min(news) < 4 if news else seqs > 1
+        return 0 if short and not (runs >= 16 and (not news or step.max_context >= 384)) else runs
+    per = num_heads // num_kv_heads
+    span = 4 if per % 4 == 0 else 8 if per % 2 == 0 else 16
+    row = tile = walk = longest = work = context = 0
+    for a, b in zip(starts, news):
+        first, last = row // span, (row + b - 1) // span
+        if first != tile:
+            tile, walk = first, 0
+        walk += a + min(b, (first + 1) * span - row)
+        longest = max(longest, walk)
+        if last != first:
+            tile, walk = last, a + b
+            longest = max(longest, walk)
+        row, work, context = row + b, work + b * (a + b / 2), max(context, a + b)
+    work *= num_heads * head_dim / 1e6
+    by_rows = 4.4 + 0.023 * context * head_dim / 64 + 1.18 * work
+    together = (6.6 + 0.034 * longest * head_dim / 64 + 0.25 * work) * (1.5 if head_dim % 8 else 1.0)
+    return runs if 1.3 * together < by_rows else 0
+
+
 def attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
               block_table: torch.Tensor, step, num_heads: int, num_kv_heads: int, head_dim: int, scale: float,
               window: int = 0) -> None:
@@ -2199,14 +2232,7 @@ def attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.
         attention_decode(q, q_stride, out, k_cache, v_cache, block_table, step.positions, step.token_slot, step.n_tokens,
                          num_heads, num_kv_heads, head_dim, scale, window)
     else:
-        # rows together: not where a sequence brings fewer than four (a CTA walks the runs that its rows fall into one after the other: 8 runs of 3
-        # tokens after 500, 32 heads of 64, 136 us against 42 by rows), unless they are few among many.  What a captured step's sequences
-        # bring in a replay is not known, nor what they hold by then.
-        runs = step.n_tokens // max(1, step.n_seqs)
-        news = None if getattr(step, "captured", False) else getattr(step, "host_new", None)
-        short = min(news) < 4 if news else step.n_seqs > 1
-        if short and not (runs >= 16 and (not news or step.max_context >= 384)):
-            runs = 0
+        runs = simt_runs(step, num_heads, num_kv_heads, head_dim)
         attention_simt(q, q_stride, out, k_cache, v_cache, block_table, step.positions, step.token_slot, step.n_tokens,
                        num_heads, num_kv_heads, head_dim, scale, window, runs=runs,
                        few_keys=step.max_new > 1 and step.max_context <= 64)

@@ -104,6 +104,16 @@ def test_recurrences_of_captured_steps_whose_rows_may_be_empty():
     assert ops.outer_in_chunks(_step(64, captured=True), 64, False) and not ops.outer_in_chunks(_step(300, 8), 64, False)
 
 
+def test_float32_rows_of_many_sequences(monkeypatch):
+    """Short runs after long contexts go by rows, whatever the average; long runs beside a short one go together."""
+    step = lambda starts, news: _step(sum(news), len(news), max_context=max(a + b for a, b in zip(starts, news)), host_starts=starts, host_new=news)
+    assert ops.simt_runs(step([0, 0, 0, 629, 12, 0, 0, 0, 0, 6, 6], [21, 25, 1, 1, 45, 56, 15, 1, 17, 3, 8]), 5, 5, 64) == 0
+    assert ops.simt_runs(step([500] * 8, [3] * 8), 32, 8, 64) == 0
+    assert ops.simt_runs(step([600, 900, 500, 662], [145, 186, 4, 1]), 32, 8, 128) > 0
+    assert ops.simt_runs(step([0, 30], [500, 300]), 32, 8, 64) == 400
+    assert ops.simt_runs(step([0], [64]), 32, 8, 64) == 64 and ops.simt_runs(step([0], [3]), 32, 8, 64) == 0
+
+
 @pytest.mark.parametrize("M,N,K,first", [(33, 640, 640, True), (48, 2048, 768, True), (33, 1536, 1024, False), (64, 2560, 1024, True), (64, 1024, 1024, False),
                                          (33, 3072, 2048, False), (64, 3072, 2048, False), (64, 6144, 2048, True), (32, 640, 640, False), (48, 2048, 4096, False)])
 def test_products_of_33_to_64_tokens_take_the_faster_way_round(monkeypatch, M, N, K, first):
