@@ -1391,13 +1391,14 @@ def mixed_token_ranks(n_seqs: int, context_class: int, window: int, keep_first: 
     least.  A round of CTAs costs the start of one, about three chunks (and half of one for a cluster), and its chunks, 1.45 times as much where
     a CTA has more of them than its shared memory holds the scores of (``room``, for 1, 2, 4 and 8 CTAs: it makes the scores twice then); of 148 SMs
     15 clusters of eight run at once, 33 of four, 74 of two (a cluster stays within its part of the chip).  The longest sequence of a class is
-    somewhere between half of the class's chunks and all of them, in the lowest class between none and all: the mean over two points.
+    somewhere between half of the class's chunks and all of them: the mean over two points.  In the lowest class, none to 32, it is counted a quarter: 64 heads
+    of 64, 76 sequences, 1 / 4 CTAs 39 / 60 for 200 keys, 120 / 99 for 600, 195 / 129 for 1,000, and the short ones do not pay for the long ones.
     us with 1 / 2 / 4 / 8 CTAs a sequence: 32 heads of 64 on 8 (room 35), 15 of 200 keys 22.5 / 16.8 / 12.7 / 11.2, 16 22.6 / 16.6 / 12.6 / 20.8, 40 23.0 / 17.0 /
     24.2 / 32.3, 76 23.1 / 32.5 / 36.5 / 63.2; 40 of 3,000 338 / 178 / 128 / 109, 76 342 / 349 / 192 / 214, 148 345 / 354 / 320 / 360; 64 of 64 (room 13), 76 of
-    3,000, window 1,024 213 / 231 / 145 / 188, 148 213 / 233 / 241 / 317; 32 of 128 (room 16), 76 of 1,000 161 / 122 / 105 / 133; 16 of 64 (room 92), 148
+    3,000, window 1,024 213 / 231 / 145 / 188, 148 213 / 233 / 241 / 317; 16 of 64 (room 92), 148
     of 3,000 266 / 176 / 239 / 280."""
     bound = (16 << max(0, int(context_class))) * (PAGE // 32)
-    points = [bound / 4, bound * 3 / 4] if context_class <= 0 else [bound * 5 / 8, bound * 7 / 8]
+    points = [bound / 4] if context_class <= 0 else [bound * 5 / 8, bound * 7 / 8]
     if window:
         most = (int(window) + 31) // 32 + 1 + (int(keep_first or 0) + 31) // 32
         bound, points = min(bound, most), [min(c, most) for c in points]
@@ -2048,7 +2049,7 @@ def attention_tcgen05(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache
 
 
 # Where a step with a window or a sink takes tcgen05.  Heads of 128: with windows of 128 and more (the mean over 138 steps of one to sixteen prompts is 0.79 to
-# 0.90 of mma.sync's time, 0.96 to 0.98 with windows of 16 to 64, where it is 1.4 at worst).  Heads of 64: from so many keys that a token sees on, in
+# 0.90 of mma.sync's time, 0.96 to 0.98 with windows of 16 to 64, where it is 1.4 at worst), and with smaller ones from 4,096 (row, head) pairs on (0.91 to 1.0).  Heads of 64: from so many keys that a token sees on, in
 # groups of two and more heads / alone, and so many (row, head) pairs (twice as many where the group is no power of two and tiles hold empty rows): tcgen05 has
 # the larger tiles, which few rows do not fill.  us on mma.sync / tcgen05, window 1,024, 32 heads on 8: prompts of 6,000 tokens 200 / 113, 64 rows after 1,500
 # 31.5 / 29.1, 256 39 / 29.5, 512 at the start 19 / 15, after 1,500 43 / 30, 128 at the start 5.6 / 7.7; window 512, two prompts of 655 tokens 24.5 / 20.1, four of 162
@@ -2070,7 +2071,7 @@ def prefill_on_tcgen05(q: torch.Tensor, q_stride: int, step, num_heads: int, num
         return True
     keys = int(window or 1 << 30)
     if head_dim == 128:
-        return keys >= TCGEN05_WINDOW_128
+        return keys >= TCGEN05_WINDOW_128 or step.n_tokens * num_heads >= TCGEN05_WINDOW_ROWS // 2
     if not getattr(step, "captured", False):              # (a captured step is replayed wherever its sequences stand by then)
         keys = min(keys, getattr(step, "max_context", keys))
     return keys >= TCGEN05_WINDOW_KEYS[int(group == 1)] and step.n_tokens * num_heads >= TCGEN05_WINDOW_ROWS * (1 if group & (group - 1) == 0 else 2)
@@ -2180,18 +2181,23 @@ def simt_runs(step, num_heads: int, num_kv_heads: int, head_dim: int) -> int:
     """``runs`` of ``attention_simt`` for a step: about how many of its rows follow one another, or 0 where rows go each by itself.
 
     A CTA of the prompt kernel has 4 to 16 rows and walks the sequences that they belong to one after the other, so a few tokens each of sequences with long
-    contexts wait for one another: 8 runs of 3 tokens after 500, 32 heads of 64, take 136 us so and 42 by rows.  With several sequences both
-    are estimated (us, fitted to 187 steps of one to sixteen sequences): by rows the longest context and all (row, key, head) products, together the
-    longest walk of a CTA and a fifth of the products; together it is where that is the better one by a third, as the walk is within 24 %."""
+    contexts wait for one another: 8 runs of 3 tokens after 500, 32 heads of 64, take 136 us so and 42 by rows.  Where a
+    sequence has fewer rows than a CTA both are estimated (us, fitted to 187 steps of one to sixteen sequences): by rows the longest context and all
+    (row, key, head) products, together the longest walk of a CTA and a fifth of the products; together it is where that is the better one, by a
+    third where a sequence brings fewer than four (the walk is estimated within 24 %)."""
     n, seqs = step.n_tokens, max(1, step.n_seqs)
     runs = n // seqs
     captured = getattr(step, "captured", False)           # (what its sequences bring in a replay is not known, nor what they hold by then)
     news, starts = (None, None) if captured else (getattr(step, "host_new", None), getattr(step, "host_starts", None))
+    per = num_heads // num_kv_heads
+    span = 4 if per % 4 == 0 else 8 if per % 2 == 0 else 16
+    if runs < span:                                       # (fewer rows than a CTA's on average: each by itself in any case)
+        return 0
+    if news and min(news) >= span and head_dim % 8 == 0:
+        return runs
     if seqs == 1 or not news or not starts:
         short = min(news) < 4 if news else seqs > 1
         return 0 if short and not (runs >= 16 and (not news or step.max_context >= 384)) else runs
-    per = num_heads // num_kv_heads
-    span = 4 if per % 4 == 0 else 8 if per % 2 == 0 else 16
     row = tile = walk = longest = work = context = 0
     for a, b in zip(starts, news):
         first, last = row // span, (row + b - 1) // span
@@ -2206,7 +2212,7 @@ def simt_runs(step, num_heads: int, num_kv_heads: int, head_dim: int) -> int:
     work *= num_heads * head_dim / 1e6
     by_rows = 4.4 + 0.023 * context * head_dim / 64 + 1.18 * work
     together = (6.6 + 0.034 * longest * head_dim / 64 + 0.25 * work) * (1.5 if head_dim % 8 else 1.0)
-    return runs if 1.3 * together < by_rows else 0
+    return runs if (1.0 if min(news) >= 4 else 1.3) * together < by_rows else 0
 
 
 def attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
