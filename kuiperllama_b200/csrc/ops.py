@@ -2181,8 +2181,8 @@ def simt_runs(step, num_heads: int, num_kv_heads: int, head_dim: int) -> int:
     """``runs`` of ``attention_simt`` for a step: about how many of its rows follow one another, or 0 where rows go each by itself.
 
     A CTA of the prompt kernel has 4 to 16 rows and walks the sequences that they belong to one after the other, so a few tokens each of sequences with long
-    contexts wait for one another: 8 runs of 3 tokens after 500, 32 heads of 64, take 136 us so and 42 by rows.  Where a
-    sequence has fewer rows than a CTA both are estimated (us, fitted to 187 steps of one to sixteen sequences): by rows the longest context and all
+    contexts wait for one another: 8 runs of 3 tokens after 500, 32 heads of 64, take 136 us so and 42 by rows.  With several
+    sequences both are estimated (us, fitted to 187 steps of one to sixteen sequences): by rows the longest context and all
     (row, key, head) products, together the longest walk of a CTA and a fifth of the products; together it is where that is the better one, by a
     third where a sequence brings fewer than four (the walk is estimated within 24 %)."""
     n, seqs = step.n_tokens, max(1, step.n_seqs)
@@ -2193,8 +2193,6 @@ def simt_runs(step, num_heads: int, num_kv_heads: int, head_dim: int) -> int:
     span = 4 if per % 4 == 0 else 8 if per % 2 == 0 else 16
     if runs < span:                                       # (fewer rows than a CTA's on average: each by itself in any case)
         return 0
-    if news and min(news) >= span and head_dim % 8 == 0:
-        return runs
     if seqs == 1 or not news or not starts:
         short = min(news) < 4 if news else seqs > 1
         return 0 if short and not (runs >= 16 and (not news or step.max_context >= 384)) else runs

@@ -111,6 +111,7 @@ def test_float32_rows_of_many_sequences(monkeypatch):
     assert ops.simt_runs(step([500] * 8, [3] * 8), 32, 8, 64) == 0
     assert ops.simt_runs(step([600, 900, 500, 662], [145, 186, 4, 1]), 32, 8, 128) > 0
     assert ops.simt_runs(step([0, 30], [500, 300]), 32, 8, 64) == 400 and ops.simt_runs(step([0, 83, 0], [118, 27, 174]), 5, 5, 64) == 106
+    assert ops.simt_runs(step([0, 224], [103, 23]), 5, 5, 64) == 0              # (16.4 us, 20.1 together)
     assert ops.simt_runs(step([0], [64]), 32, 8, 64) == 64 and ops.simt_runs(step([0], [3]), 32, 8, 64) == 0
 
 
